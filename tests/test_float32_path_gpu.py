@@ -1,0 +1,62 @@
+"""The float32 products and attention at the sizes where their forms and splits change: rows around 1, 2, 4, 8, 16, 32, 64 and 128 (skinny form, 32,
+64 and 128-row tiles), reductions cut into 1 to 8 segments, lengths that are no multiple of 4 (scalar copies) or of 32 (a ragged last
+step).  The bound of a product: K rounded multiply-adds in at least two chains, so the error stays under sqrt(K) 2^-24 of the terms' root sum of
+squares (about 1 here) times a small factor: 1e-5."""
+
+import pytest
+import torch
+
+from tests.conftest import cuda_or_skip
+
+pytestmark = pytest.mark.gpu
+ROWS = [1, 2, 3, 5, 8, 9, 16, 17, 32, 33, 64, 65, 128, 129, 300]
+
+
+@pytest.mark.parametrize("N,K", [(896, 896), (1152, 900), (20000, 96), (9728, 256), (31, 4864), (130, 333), (33, 70), (40, 2)])
+def test_products_of_every_form_agree_in_every_bit(N, K):
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    g = torch.Generator(device=dev).manual_seed(N + K)
+    x = torch.randn(max(ROWS), K, device=dev, generator=g)
+    w = torch.randn(N, K, device=dev, generator=g) / K ** 0.5
+    b = torch.randn(N, device=dev, generator=g)
+    full = ops.linear(x, w, b, torch.float32)
+    want = x.double() @ w.double().t() + b.double()
+    torch.testing.assert_close(full.double(), want, rtol=1e-5, atol=1e-5)
+    for m in ROWS:
+        assert torch.equal(ops.linear(x[-m:].contiguous(), w, b, torch.float32), full[-m:]), m
+    # operands off the 16-byte boundary take the scalar copies
+    flat = torch.empty(x.numel() + 1, device=dev)
+    flat[1:] = x.reshape(-1)
+    off = flat[1:].view_as(x)
+    assert torch.equal(ops.linear(off, w, b, torch.float32), full)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("hd,ps", [(64, 16), (128, 8), (40, 4), (17, 16), (256, 16), (320, 16)])
+@pytest.mark.parametrize("window", [None, 45])
+def test_attention_around_blocks_of_32_keys(dtype, hd, ps, window):
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    g = torch.Generator(device=dev).manual_seed(hd + ps)
+    nq, nkv, ctx = 6, 2, [1, 31, 32, 33, 64, 257, 300]
+    pages = sum(-(-c // ps) for c in ctx)
+    kc, vc = (torch.randn(pages, nkv, ps, hd, device=dev, generator=g).to(dtype) for _ in range(2))
+    order, at = torch.randperm(pages, device=dev, generator=g).int(), 0
+    bt = torch.full((len(ctx), -(-max(ctx) // ps)), -1, dtype=torch.int32, device=dev)
+    for i, c in enumerate(ctx):
+        n = -(-c // ps)
+        bt[i, :n] = order[at:at + n]
+        at += n
+    pos = torch.tensor([c - 1 for c in ctx], dtype=torch.int32, device=dev)
+    seq = torch.arange(len(ctx), dtype=torch.int32, device=dev)
+    q = torch.randn(len(ctx), nq * hd, device=dev, generator=g).to(dtype)
+    got = ops.attention_simt(q, kc, vc, bt, pos, seq, nq, nkv, hd, hd ** -0.5, window).double().reshape(len(ctx), nq, hd)
+    for i, c in enumerate(ctx):
+        lo = max(0, c - window) if window else 0
+        rows = [(int(bt[i, j // ps]), j % ps) for j in range(lo, c)]
+        k, v = (torch.stack([x[p, :, o] for p, o in rows]).double().repeat_interleave(nq // nkv, 1) for x in (kc, vc))
+        s = torch.einsum("hd,jhd->hj", q[i].double().reshape(nq, hd), k) * hd ** -0.5
+        want = torch.einsum("hj,jhd->hd", torch.softmax(s, -1), v)
+        tol = 2e-5 if dtype == torch.float32 else 1e-2
+        torch.testing.assert_close(got[i], want, rtol=tol, atol=tol)
