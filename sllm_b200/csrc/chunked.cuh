@@ -1,4 +1,5 @@
-// What the kernels that run a recurrence over prompt portions a chunk of 64 tokens at a time share (retention.cu, state_space.cu): copies
+// What the kernels that run a recurrence over prompt portions a chunk of 64 tokens at a time share (retention.cu, state_space.cu, gated_chunks.cu,
+// delta_chunks.cu): copies
 // into shared memory, a float32 product of rows and a block there, small pieces.  All arithmetic is float32 on the CUDA cores.
 #pragma once
 
@@ -61,6 +62,29 @@ __device__ __forceinline__ void rows_times_block(float (&acc)[8][TN], const floa
         o[0] = fmaf(a.z, bv[2][g].x, o[0]); o[1] = fmaf(a.z, bv[2][g].y, o[1]); o[2] = fmaf(a.z, bv[2][g].z, o[2]); o[3] = fmaf(a.z, bv[2][g].w, o[3]);
         o[0] = fmaf(a.w, bv[3][g].x, o[0]); o[1] = fmaf(a.w, bv[3][g].y, o[1]); o[2] = fmaf(a.w, bv[3][g].z, o[2]); o[3] = fmaf(a.w, bv[3][g].w, o[3]);
       }
+    }
+  }
+}
+
+// The same over the 16 tokens of a run for the run's own rows: row r0 + r takes in the tokens up to its own place and no later one (nothing that a
+// later token holds, not even times zero).
+template <int LDA, int LDB, int TN>
+__device__ __forceinline__ void rows_times_run(float (&acc)[8][TN], const float* __restrict__ A, const float* __restrict__ B, int r0) {
+  const float* b = B + 4 * (threadIdx.x & 15);
+#pragma unroll 2
+  for (int k = 0; k < 16; ++k) {
+    float4 bv[TN / 4];
+#pragma unroll
+    for (int g = 0; g < TN / 4; ++g) bv[g] = *reinterpret_cast<const float4*>(b + k * LDB + 64 * g);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const float a = A[r * LDA + k];
+      if (k <= r0 + r)
+#pragma unroll
+        for (int g = 0; g < TN / 4; ++g) {
+          float* o = acc[r] + 4 * g;
+          o[0] = fmaf(a, bv[g].x, o[0]); o[1] = fmaf(a, bv[g].y, o[1]); o[2] = fmaf(a, bv[g].z, o[2]); o[3] = fmaf(a, bv[g].w, o[3]);
+        }
     }
   }
 }

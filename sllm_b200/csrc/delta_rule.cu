@@ -77,7 +77,7 @@ struct DeltaParams {
   int rot = 0, max_pos = 0;
   float k_scale = 1.f;
   const float* skip = nullptr;         // state space: [H] D; dt logits in `gates` at off_dt + h
-  int max_len = 0;                     // > 0: requests that bring more tokens are another kernel's (retention.cu)
+  int max_len = 0;                     // > 0: requests that bring more tokens are another kernel's (retention.cu, state_space.cu, gated_chunks.cu)
 };
 
 // RPT: rows of a column per lane (dk <= 8 * RPT = DKP, the padded key size).
@@ -583,9 +583,16 @@ static int launch_delta_rule(DeltaParams p, int S, cudaStream_t stream) {
 
 static int dispatch_delta_rule(DeltaParams p, int S, cudaStream_t stream);
 
+// max_len > 0: requests that bring more tokens are left alone (another kernel's)
+static int walk_up_to(DeltaParams p, int max_len, int S, cudaStream_t stream) {
+  p.max_len = max_len;
+  if (max_len > 0 && (p.max_q <= 0 || p.max_q > max_len)) p.max_q = max_len;
+  return dispatch_delta_rule(p, S, stream);
+}
+
 SLLM_EXPORT int sllm_delta_rule(const float* proj, int ld, int off_r, int off_k, int off_v, int off_a, const float* decay,
                                 const float* a_bias, float* state, const int* q_start, const int* state_slots, float* out,
-                                int S, int H, int dk, int dv, int max_q, cudaStream_t stream) {
+                                int S, int H, int dk, int dv, int max_q, int max_len, cudaStream_t stream) {
   SLLM_REQUIRE(S >= 0 && H > 0 && H <= 65535, "delta_rule: bad sizes S=%d H=%d", S, H);
   SLLM_REQUIRE(sllm_delta_rule_supports(dk, dv), "delta_rule: a head of %d key and %d value channels is outside 1..256 keys", dk, dv);
   SLLM_REQUIRE(off_r >= 0 && off_k >= 0 && off_v >= 0 && off_a >= 0 && off_r + H * dk <= ld && off_k + H * dk <= ld &&
@@ -598,7 +605,7 @@ SLLM_EXPORT int sllm_delta_rule(const float* proj, int ld, int off_r, int off_k,
   p.max_q = max_q;           // the longest portion of the batch (0: not known)
   p.mode = 0; p.hdiv = 1; p.gates = nullptr; p.ldg = p.off_b = p.off_dt = 0; p.a_log = p.dt_bias = nullptr;
   p.r_scale = 1.f; p.inv_tau = 1.f;
-  return dispatch_delta_rule(p, S, stream);
+  return walk_up_to(p, max_len, S, stream);
 }
 
 static int dispatch_delta_rule(DeltaParams p, int S, cudaStream_t stream) {
@@ -622,7 +629,7 @@ static int dispatch_delta_rule(DeltaParams p, int S, cudaStream_t stream) {
 SLLM_EXPORT int sllm_gated_delta_rule(const float* qkv, int ld, int off_q, int off_k, int off_v, const float* gates, int ldg,
                                       int off_b, int off_dt, const float* a_log, const float* dt_bias, float* state,
                                       const int* q_start, const int* state_slots, float* out, int S, int H, int Hk, int dk, int dv,
-                                      float q_scale, int max_q, cudaStream_t stream) {
+                                      float q_scale, int max_q, int max_len, cudaStream_t stream) {
   SLLM_REQUIRE(S >= 0 && H > 0 && H <= 65535 && Hk > 0 && H % Hk == 0, "gated_delta_rule: bad sizes S=%d H=%d Hk=%d", S, H, Hk);
   SLLM_REQUIRE(sllm_delta_rule_supports(dk, dv), "gated_delta_rule: a head of %d key and %d value channels is outside 1..256 keys", dk, dv);
   SLLM_REQUIRE(off_q >= 0 && off_k >= 0 && off_v >= 0 && off_q + Hk * dk <= ld && off_k + Hk * dk <= ld && off_v + H * dv <= ld,
@@ -635,13 +642,13 @@ SLLM_EXPORT int sllm_gated_delta_rule(const float* qkv, int ld, int off_q, int o
   p.chunk = 1; p.max_q = max_q;
   p.mode = 1; p.hdiv = H / Hk; p.gates = gates; p.ldg = ldg; p.off_b = off_b; p.off_dt = off_dt; p.a_log = a_log; p.dt_bias = dt_bias;
   p.r_scale = q_scale; p.inv_tau = 1.f;
-  return dispatch_delta_rule(p, S, stream);
+  return walk_up_to(p, max_len, S, stream);
 }
 
 // Gated linear attention over q | k | v columns of `proj` [T, ld] with decay logits `z` [T, H*dk]: alpha = sigmoid(z)^(inv_tau).
 SLLM_EXPORT int sllm_gated_linear_attention(const float* proj, int ld, int off_q, int off_k, int off_v, const float* z,
                                             float* state, const int* q_start, const int* state_slots, float* out, int S, int H,
-                                            int dk, int dv, float q_scale, float inv_tau, int max_q, cudaStream_t stream) {
+                                            int dk, int dv, float q_scale, float inv_tau, int max_q, int max_len, cudaStream_t stream) {
   SLLM_REQUIRE(S >= 0 && H > 0 && H <= 65535, "gated_linear_attention: bad sizes S=%d H=%d", S, H);
   SLLM_REQUIRE(sllm_delta_rule_supports(dk, dv), "gated_linear_attention: a head of %d key and %d value channels is outside 1..256 keys", dk, dv);
   SLLM_REQUIRE(off_q >= 0 && off_k >= 0 && off_v >= 0 && off_q + H * dk <= ld && off_k + H * dk <= ld && off_v + H * dv <= ld,
@@ -653,13 +660,13 @@ SLLM_EXPORT int sllm_gated_linear_attention(const float* proj, int ld, int off_q
   p.chunk = 1; p.max_q = max_q;
   p.mode = 2; p.hdiv = 1; p.gates = nullptr; p.ldg = p.off_b = p.off_dt = 0; p.a_log = p.dt_bias = nullptr;
   p.r_scale = q_scale; p.inv_tau = inv_tau;
-  return dispatch_delta_rule(p, S, stream);
+  return walk_up_to(p, max_len, S, stream);
 }
 
 // Linear attention with a fixed decay per head (`decay` [H]) over silu'd q | k | v columns of `proj` [T, ld].
 SLLM_EXPORT int sllm_decay_linear_attention(const float* proj, int ld, int off_q, int off_k, int off_v, const float* decay,
                                             float* state, const int* q_start, const int* state_slots, float* out, int S, int H,
-                                            int dk, int dv, int max_q, cudaStream_t stream) {
+                                            int dk, int dv, int max_q, int max_len, cudaStream_t stream) {
   SLLM_REQUIRE(S >= 0 && H > 0 && H <= 65535, "decay_linear_attention: bad sizes S=%d H=%d", S, H);
   SLLM_REQUIRE(sllm_delta_rule_supports(dk, dv), "decay_linear_attention: a head of %d key and %d value channels is outside 1..256 keys", dk, dv);
   SLLM_REQUIRE(off_q >= 0 && off_k >= 0 && off_v >= 0 && off_q + H * dk <= ld && off_k + H * dk <= ld && off_v + H * dv <= ld,
@@ -671,13 +678,13 @@ SLLM_EXPORT int sllm_decay_linear_attention(const float* proj, int ld, int off_q
   p.chunk = 1; p.max_q = max_q;
   p.mode = 3; p.hdiv = 1; p.gates = nullptr; p.ldg = p.off_b = p.off_dt = 0; p.a_log = decay; p.dt_bias = nullptr;
   p.r_scale = 1.f; p.inv_tau = 1.f;
-  return dispatch_delta_rule(p, S, stream);
+  return walk_up_to(p, max_len, S, stream);
 }
 
 // Linear attention whose forget gate also writes, over q | gate logit | v columns of `proj` [T, ld]: `f_bias` and `lower` [H*dk].
 SLLM_EXPORT int sllm_forget_gate_attention(const float* proj, int ld, int off_q, int off_f, int off_v, const float* f_bias,
                                            const float* lower, float* state, const int* q_start, const int* state_slots,
-                                           float* out, int S, int H, int dk, int dv, int max_q, cudaStream_t stream) {
+                                           float* out, int S, int H, int dk, int dv, int max_q, int max_len, cudaStream_t stream) {
   SLLM_REQUIRE(S >= 0 && H > 0 && H <= 65535, "forget_gate_attention: bad sizes S=%d H=%d", S, H);
   SLLM_REQUIRE(sllm_delta_rule_supports(dk, dv), "forget_gate_attention: a head of %d key and %d value channels is outside 1..256 keys", dk, dv);
   SLLM_REQUIRE(off_q >= 0 && off_f >= 0 && off_v >= 0 && off_q + H * dk <= ld && off_f + H * dk <= ld && off_v + H * dv <= ld,
@@ -689,7 +696,7 @@ SLLM_EXPORT int sllm_forget_gate_attention(const float* proj, int ld, int off_q,
   p.chunk = 1; p.max_q = max_q;
   p.mode = 4; p.hdiv = 1; p.gates = nullptr; p.ldg = p.off_b = p.off_dt = 0; p.a_log = lower; p.dt_bias = nullptr;
   p.r_scale = 1.f; p.inv_tau = 1.f;
-  return dispatch_delta_rule(p, S, stream);
+  return walk_up_to(p, max_len, S, stream);
 }
 
 // Retention (a fixed decay per head, `decay` [H]; q and k rotated by position, k times k_scale) over q | k | v columns of
@@ -712,9 +719,7 @@ SLLM_EXPORT int sllm_retention(const float* proj, int ld, int off_q, int off_k, 
   p.mode = DR_RETENTION; p.hdiv = 1; p.gates = nullptr; p.ldg = p.off_b = p.off_dt = 0; p.a_log = decay; p.dt_bias = nullptr;
   p.r_scale = 1.f; p.inv_tau = 1.f;
   p.positions = positions; p.table = table; p.rot = rot; p.max_pos = max_pos > 0 ? max_pos : 1; p.k_scale = k_scale;
-  p.max_len = max_len;
-  if (max_len > 0 && (p.max_q <= 0 || p.max_q > max_len)) p.max_q = max_len;
-  return dispatch_delta_rule(p, S, stream);
+  return walk_up_to(p, max_len, S, stream);
 }
 
 // A state-space recurrence over x | B | C columns of `xbc` [T, ldx] (x head by head, B and C group by group: head h uses group h / (H / groups)) with step
@@ -732,9 +737,7 @@ SLLM_EXPORT int sllm_state_space(const float* xbc, int ldx, const float* dtp, in
   p.chunk = 1; p.max_q = max_q;
   p.mode = DR_STATE_SPACE; p.hdiv = H / groups; p.gates = dtp; p.ldg = ldd; p.off_b = 0; p.off_dt = off_dt; p.a_log = a_log; p.dt_bias = dt_bias;
   p.r_scale = 1.f; p.inv_tau = 1.f; p.skip = skip;
-  p.max_len = max_len;
-  if (max_len > 0 && (p.max_q <= 0 || p.max_q > max_len)) p.max_q = max_len;
-  return dispatch_delta_rule(p, S, stream);
+  return walk_up_to(p, max_len, S, stream);
 }
 
 SLLM_EXPORT int sllm_delta_out(const float* o, const float* gain, const float* proj, int ld, int off_g, float eps, void* out,

@@ -238,7 +238,7 @@ def delta_rule(proj, offs, decay, a_bias, state, step, heads: int, dk: int, dv: 
     out = torch.empty((T, heads * dv), dtype=torch.float32, device=proj.device)
     off_r, off_k, off_v, off_a = (int(o) for o in offs)
     call("sllm_delta_rule", _p(proj), ld, off_r, off_k, off_v, off_a, _p(decay), _p(a_bias), _p(state), _p(step.q_start),
-         _p(step.state_slots), _p(out), step.num_seqs, heads, dk, dv, int(step.max_q_len), _stream())
+         _p(step.state_slots), _p(out), step.num_seqs, heads, dk, dv, int(step.max_q_len), 0, _stream())
     return out
 
 
@@ -276,8 +276,10 @@ def forget_gate_attention(proj, offs, f_bias, lower, state, step, heads: int, dk
         raise KernelError(f"forget_gate_attention: state {tuple(state.shape)} or the gate's vectors do not fit {heads} heads of {dk}x{dv}")
     out = torch.empty((T, heads * dv), dtype=torch.float32, device=proj.device)
     off_q, off_f, off_v = (int(o) for o in offs)
-    call("sllm_forget_gate_attention", _p(proj), ld, off_q, off_f, off_v, _p(f_bias), _p(lower), _p(state), _p(step.q_start),
-         _p(step.state_slots), _p(out), step.num_seqs, heads, dk, dv, int(step.max_q_len), _stream())
+    longest, rest = _gated_chunks(4, proj, offs, None, lower, f_bias, 1.0, 1.0, state, step, heads, dk, dv, out)
+    if rest:
+        call("sllm_forget_gate_attention", _p(proj), ld, off_q, off_f, off_v, _p(f_bias), _p(lower), _p(state), _p(step.q_start),
+             _p(step.state_slots), _p(out), step.num_seqs, heads, dk, dv, int(step.max_q_len), longest, _stream())
     return out
 
 
@@ -322,7 +324,7 @@ def gated_delta_rule(qkv, offs, gates, off_b: int, off_dt: int, a_log, dt_bias, 
     off_q, off_k, off_v = (int(o) for o in offs)
     call("sllm_gated_delta_rule", _p(qkv), ld, off_q, off_k, off_v, _p(gates), gates.shape[1], int(off_b), int(off_dt), _p(a_log),
          _p(dt_bias), _p(state), _p(step.q_start), _p(step.state_slots), _p(out), step.num_seqs, heads, key_heads, dk, dv,
-         float(q_scale), int(step.max_q_len), _stream())
+         float(q_scale), int(step.max_q_len), 0, _stream())
     return out
 
 
@@ -338,8 +340,10 @@ def gated_linear_attention(proj, offs, z, state, step, heads: int, dk: int, dv: 
         raise KernelError(f"gated_linear_attention: z {tuple(z.shape)} or state {tuple(state.shape)} does not fit {heads} heads of {dk}x{dv}")
     out = torch.empty((T, heads * dv), dtype=torch.float32, device=proj.device)
     off_q, off_k, off_v = (int(o) for o in offs)
-    call("sllm_gated_linear_attention", _p(proj), ld, off_q, off_k, off_v, _p(z), _p(state), _p(step.q_start), _p(step.state_slots),
-         _p(out), step.num_seqs, heads, dk, dv, float(q_scale), 1.0 / float(tau), int(step.max_q_len), _stream())
+    longest, rest = _gated_chunks(2, proj, offs, z, None, None, q_scale, tau, state, step, heads, dk, dv, out)
+    if rest:
+        call("sllm_gated_linear_attention", _p(proj), ld, off_q, off_k, off_v, _p(z), _p(state), _p(step.q_start), _p(step.state_slots),
+             _p(out), step.num_seqs, heads, dk, dv, float(q_scale), 1.0 / float(tau), int(step.max_q_len), longest, _stream())
     return out
 
 
@@ -602,8 +606,10 @@ def decay_linear_attention(proj, offs, decay, state, step, heads: int, dk: int, 
         raise KernelError(f"decay_linear_attention: decay {tuple(decay.shape)} or state {tuple(state.shape)} does not fit {heads} heads of {dk}x{dv}")
     out = torch.empty((T, heads * dv), dtype=torch.float32, device=proj.device)
     off_q, off_k, off_v = (int(o) for o in offs)
-    call("sllm_decay_linear_attention", _p(proj), ld, off_q, off_k, off_v, _p(decay), _p(state), _p(step.q_start),
-         _p(step.state_slots), _p(out), step.num_seqs, heads, dk, dv, int(step.max_q_len), _stream())
+    longest, rest = _gated_chunks(3, proj, offs, None, decay, None, 1.0, 1.0, state, step, heads, dk, dv, out)
+    if rest:
+        call("sllm_decay_linear_attention", _p(proj), ld, off_q, off_k, off_v, _p(decay), _p(state), _p(step.q_start),
+             _p(step.state_slots), _p(out), step.num_seqs, heads, dk, dv, int(step.max_q_len), longest, _stream())
     return out
 
 
@@ -665,6 +671,65 @@ def portion_chunks(q_lens, ctx_lens, min_len: int, device):
     return t[:C], t[C:2 * C], t[2 * C:o], C, t[o:o + R], t[o + R:o + 2 * R], t[o + 2 * R:], R
 
 
+# Portions of at least so many tokens may run in chunks in the recurrences below (0: none does), shorter ones are walked.
+GATED_CHUNKED_FROM = 96
+# What decides (us; `_chunks_pay`): the walk takes its longest portion times a rate, that of a CTA which walks 16 columns of a head (64 where the
+# batch fills the SMs with such) and slower the more of them an SM holds; the chunks take a base for their three kernels and a rate per
+# token of all long portions.  Measured in a graph (walk / chunks): 32 heads of 64 x 64, one portion of 128, 256, 2,048 tokens: gated 32 / 34, 60 / 35,
+# 479 / 121; 16 heads of 128 x 128: forget gate 51 / 60, 95 / 60, 709 / 163.  Eight portions of 200 tokens: 79 / 117, 195 / 173; three of 700: 349 / 125, 527 / 168.  (walk, a narrow CTA's and a wide one's per token; base; chunks
+# per token, and the heads x keys x values that was measured at)
+CHUNK_COSTS = {"gated64": (0.235, 0.39, 30.0, 0.045, 32 * 64 * 64), "gated128": (0.35, 0.97, 52.0, 0.055, 16 * 128 * 128)}
+
+
+def _chunks_pay(kind: str, step, from_len: int, heads: int, dk: int, dv: int) -> bool:
+    """Whether the step's portions of ``from_len`` tokens and more are faster in chunks than walked (see `CHUNK_COSTS`)."""
+    long = [q for q in step.q_lens if q >= from_len]
+    if not long:
+        return False
+    narrow, wide, base, per_token, ref = CHUNK_COSTS[kind]
+    blocks = heads * -(-dv // 64)
+    if step.num_seqs * blocks >= num_sms():
+        rate = wide * max(1.0, len(long) * blocks / 256)
+    else:
+        rate = narrow * max(1.0, len(long) * heads * -(-dv // 16) / 180)
+    return base + sum(long) * per_token * heads * dk * dv / ref < max(long) * rate
+
+
+@functools.lru_cache(maxsize=4096)
+def gated_chunked_supports(dk: int, dv: int) -> bool:
+    return bool(lib().sllm_gated_chunked_supports(int(dk), int(dv)))
+
+
+def _long_portions(step, from_len: int, device):
+    """`portion_chunks` of a step, once per step, or None."""
+    if from_len <= 0 or step.max_q_len < from_len or not step.q_lens:
+        return None
+    key = ("chunks", from_len)
+    if key not in step.attn_tiles:
+        step.attn_tiles[key] = portion_chunks(step.q_lens, step.ctx_lens, from_len, device)
+    return step.attn_tiles[key]
+
+
+def _gated_chunks(mode: int, proj, offs, z, a, bias, q_scale: float, tau: float, state, step, heads: int, dk: int, dv: int, out):
+    """The step's long portions through the chunked form of the recurrence ``mode`` (2: a decay per channel from the logits ``z``, 3: a fixed
+    decay ``a`` per head, 4: a forget gate with lower bounds ``a`` and ``bias``); their rows of ``out`` and their states are written.
+    Returns (the longest portion left for the walk, 0 for no limit; whether any is left)."""
+    chunks = None
+    if step.max_q_len >= GATED_CHUNKED_FROM > 0 and gated_chunked_supports(dk, dv) and \
+            _chunks_pay("gated64" if dk <= 64 else "gated128", step, GATED_CHUNKED_FROM, heads, dk, dv):
+        chunks = _long_portions(step, GATED_CHUNKED_FROM, proj.device)
+    if chunks is None:
+        return 0, True
+    t0, _, n, C, seq, first, count, R = chunks
+    scratch = torch.empty((C, heads, dk, dv), dtype=torch.float32, device=proj.device)
+    keeps = torch.empty((C, heads, dk), dtype=torch.float32, device=proj.device)
+    off_q, off_k, off_v = (int(o) for o in offs)
+    call("sllm_gated_chunked", mode, _p(proj), proj.shape[1], off_q, off_k, off_v, _p(z), _p(a), _p(bias), float(q_scale), 1.0 / float(tau),
+         _p(state), _p(step.state_slots), _p(t0), _p(n), C, _p(seq), _p(first), _p(count), R, _p(scratch), _p(keeps), _p(out), heads, dk, dv, _stream())
+    launches["own"] += 2           # the three kernels of the entry point
+    return GATED_CHUNKED_FROM - 1, R < step.num_seqs
+
+
 def retention_chunked(proj, offs, off_g: int, decay, table, rotary_dim: int, k_scale: float, eps: float, state, step, chunks, heads: int,
                       dk: int, dv: int, out) -> None:
     """Retention, the heads' norm and the silu gate (columns ``off_g`` of ``proj``) for the requests that ``chunks`` (see
@@ -693,11 +758,7 @@ def retention_gated(proj, offs, off_g: int, decay, table, rotary_dim: int, k_sca
     """`retention` and what follows it in a layer: each head's output over its root mean square, times silu of columns ``off_g`` of
     ``proj``, ``[T, heads*dv]`` in ``out_dtype``.  Long prompt portions run in chunks (heads of up to 128 x 128), single tokens and short
     portions token by token; a step may hold both."""
-    chunks, longest = None, 0
-    if RETENTION_CHUNKED_FROM > 0 and step.max_q_len >= RETENTION_CHUNKED_FROM and step.q_lens and retention_chunked_supports(dk, dv):
-        if "retention" not in step.attn_tiles:
-            step.attn_tiles["retention"] = portion_chunks(step.q_lens, step.ctx_lens, RETENTION_CHUNKED_FROM, proj.device)
-        chunks, longest = step.attn_tiles["retention"], RETENTION_CHUNKED_FROM - 1
+    chunks, longest = _long_portions(step, RETENTION_CHUNKED_FROM, proj.device) if retention_chunked_supports(dk, dv) else None, RETENTION_CHUNKED_FROM - 1
     if chunks is None:
         o = retention(proj, offs, decay, table, rotary_dim, k_scale, state, step, heads, dk, dv)
         return delta_out(o, None, proj, off_g, eps, heads, dv, out_dtype, "silu")
@@ -778,12 +839,7 @@ def state_space(xbc, proj, off_dt: int, dt_bias, a_log, skip, state, step, heads
     brings one token a form of its own streams the states."""
     if xbc.shape[0] == step.num_seqs and state_space_token_supports(n, dv):
         return state_space_token(xbc, proj, off_dt, dt_bias, a_log, skip, state, step, heads, groups, n, dv)
-    chunks, longest = None, 0
-    if STATE_SPACE_CHUNKED_FROM > 0 and step.max_q_len >= STATE_SPACE_CHUNKED_FROM and step.q_lens and state_space_chunked_supports(n, dv):
-        key = ("chunks", STATE_SPACE_CHUNKED_FROM)
-        if key not in step.attn_tiles:
-            step.attn_tiles[key] = portion_chunks(step.q_lens, step.ctx_lens, STATE_SPACE_CHUNKED_FROM, xbc.device)
-        chunks, longest = step.attn_tiles[key], STATE_SPACE_CHUNKED_FROM - 1
+    chunks, longest = _long_portions(step, STATE_SPACE_CHUNKED_FROM, xbc.device) if state_space_chunked_supports(n, dv) else None, STATE_SPACE_CHUNKED_FROM - 1
     args = (xbc, proj, off_dt, dt_bias, a_log, skip, state, step)
     if chunks is None:
         return state_space_walk(*args, heads, groups, n, dv)

@@ -1,0 +1,129 @@
+"""The recurrences over long prompt portions in chunks of 64 tokens (gated_chunks.cu) against the same recurrences
+walked token by token in float64: portions that end inside a chunk, on its edge and one token beyond, beside short portions and single tokens
+that the walk keeps; head sizes on and off the kernels' padding; states that are not zero at the start.
+
+The bound: every output is a sum of at most T rounded products whose factors are themselves products of at most T decays, so its error
+against float64 grows at worst with T units of 2^-24 and in practice with the root of that; 2e-5 of the result's root mean square is about 8 sqrt(T)
+units at 640 tokens."""
+
+import numpy as np
+import pytest
+import torch
+
+from tests.conftest import cuda_or_skip
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def in_chunks(monkeypatch):
+    """Every portion that may run in chunks does, whether or not it pays."""
+    import sllm_b200.ops as ops
+    monkeypatch.setattr(ops, "_chunks_pay", lambda *a: True)
+
+
+REL = 2e-5
+LENS = [640, 1, 96, 200, 63, 64 * 2 + 1, 128, 95]
+SLOTS = [5, 0, 3, 8, 1, 7, 2, 6]
+
+
+def _step(dev, lens, slots):
+    from tests.test_rososun import _step as make
+    return make(dev, lens, slots)
+
+
+def _spans():
+    starts = np.concatenate([[0], np.cumsum(LENS)])
+    return [(int(a), int(b), s) for a, b, s in zip(starts[:-1], starts[1:], SLOTS)]
+
+
+def _close(got, want, what):
+    got, want = got.double(), want.double()
+    assert torch.isfinite(got).all(), what
+    err = (got - want).abs().max() / want.pow(2).mean().sqrt()
+    assert err < 40 * REL, f"{what}: {float(err)} of the root mean square at worst"
+    err = (got - want).norm() / want.norm()
+    assert err < REL, f"{what}: {float(err)}"
+
+
+def _walk(q, k, v, keep, S, p=None, w=None):
+    """float64, [T, H, d]: S <- keep S - w (p^T S) + k v^T, o = S^T q."""
+    out = torch.empty_like(v)
+    for t in range(q.shape[0]):
+        gone = w[t][:, :, None] * torch.einsum("hi,hij->hj", p[t], S)[:, None] if p is not None else 0.0
+        S = S * keep[t][:, :, None] - gone + k[t][:, :, None] * v[t][:, None, :]
+        out[t] = torch.einsum("hij,hi->hj", S, q[t])
+    return out, S
+
+
+def _state(g, H, dk, dv, dev):
+    return torch.randn(10, H, dk, dv, device=dev, generator=g)
+
+
+def _check(run, terms, H, dk, dv, dev, g):
+    """``run(state, step) -> o``; ``terms(a, b)``: float64 (q, k, v, keep[, p, w]) of a span's tokens."""
+    state = _state(g, H, dk, dv, dev)
+    before = state.clone()
+    o = run(state, _step(dev, LENS, SLOTS)).reshape(-1, H, dv)
+    for a, b, slot in _spans():
+        want, last = _walk(*[x[:, :, :] if x.dim() == 3 else x for x in terms(a, b)[:4]], before[slot].double(), *terms(a, b)[4:])
+        _close(o[a:b], want, f"outputs of {b - a} tokens")
+        _close(state[slot], last, f"state after {b - a} tokens")
+    untouched = [s for s in range(10) if s not in SLOTS]
+    assert torch.equal(state[untouched], before[untouched])
+
+
+SIZES = [(64, 64, 3), (128, 128, 2), (128, 64, 2), (64, 128, 2), (40, 24, 3), (72, 100, 2), (17, 5, 2)]
+
+
+@pytest.mark.parametrize("dk,dv,H", SIZES)
+@pytest.mark.parametrize("hard", [False, True])
+def test_gated_linear_attention_in_chunks(dk, dv, H, hard):
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    g = torch.Generator(device=dev).manual_seed(dk + 3 * dv)
+    T, off = sum(LENS), 3
+    proj = torch.randn(T, off + H * (2 * dk + dv), device=dev, generator=g)
+    z = torch.randn(T, H * dk, device=dev, generator=g) * (40.0 if hard else 1.0) + (0.0 if hard else 2.0)      # hard: decays from one down to e^-20
+    offs = (off, off + H * dk, off + 2 * H * dk)
+
+    def terms(a, b):
+        q, k, v = (proj[a:b, o:o + H * n].double().reshape(b - a, H, n) for o, n in zip(offs, (dk, dk, dv)))
+        return q * dk ** -0.5, k, v, (torch.nn.functional.logsigmoid(z[a:b].double()) / 8.0).exp().reshape(b - a, H, dk)
+    _check(lambda state, step: ops.gated_linear_attention(proj, offs, z, state, step, H, dk, dv, dk ** -0.5, 8.0), terms, H, dk, dv, dev, g)
+
+
+@pytest.mark.parametrize("dk,dv,H", SIZES)
+def test_decay_linear_attention_in_chunks(dk, dv, H):
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    g = torch.Generator(device=dev).manual_seed(dk + 5 * dv)
+    T = sum(LENS)
+    proj = torch.randn(T, H * (2 * dk + dv), device=dev, generator=g)
+    decay = torch.tensor([1.0 - 2.0 ** (-2.0 - 4 * h) for h in range(H)], device=dev)
+    offs = (0, H * dk, 2 * H * dk)
+    silu = torch.nn.functional.silu
+
+    def terms(a, b):
+        q, k, v = (silu(proj[a:b, o:o + H * n].double()).reshape(b - a, H, n) for o, n in zip(offs, (dk, dk, dv)))
+        return q, k, v, decay.double()[None, :, None].expand(b - a, H, 1)
+    _check(lambda state, step: ops.decay_linear_attention(proj, offs, decay, state, step, H, dk, dv), terms, H, dk, dv, dev, g)
+
+
+@pytest.mark.parametrize("dk,dv,H", SIZES)
+@pytest.mark.parametrize("hard", [False, True])
+def test_forget_gate_attention_in_chunks(dk, dv, H, hard):
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    g = torch.Generator(device=dev).manual_seed(dk + 7 * dv)
+    T = sum(LENS)
+    proj = torch.randn(T, H * (2 * dk + dv), device=dev, generator=g)
+    bias = torch.randn(H * dk, device=dev, generator=g) * (30.0 if hard else 1.0)
+    lower = torch.rand(H * dk, device=dev, generator=g) * (0.0 if hard else 0.9)
+    offs = (0, H * dk, 2 * H * dk)
+
+    def terms(a, b):
+        q, z, v = (proj[a:b, o:o + H * n].double().reshape(b - a, H, n) for o, n in zip(offs, (dk, dk, dv)))
+        f = (lower + (1 - lower) * torch.sigmoid(proj[a:b, offs[1]:offs[1] + H * dk] + bias)).double().reshape(b - a, H, dk)
+        return torch.nn.functional.silu(q), 1 - f, v, f
+    _check(lambda state, step: ops.forget_gate_attention(proj, offs, bias, lower, state, step, H, dk, dv), terms, H, dk, dv, dev, g)
