@@ -237,8 +237,10 @@ def delta_rule(proj, offs, decay, a_bias, state, step, heads: int, dk: int, dv: 
         raise KernelError(f"delta_rule: decay {tuple(decay.shape)} or state {tuple(state.shape)} does not fit {heads} heads of {dk}x{dv}")
     out = torch.empty((T, heads * dv), dtype=torch.float32, device=proj.device)
     off_r, off_k, off_v, off_a = (int(o) for o in offs)
-    call("sllm_delta_rule", _p(proj), ld, off_r, off_k, off_v, off_a, _p(decay), _p(a_bias), _p(state), _p(step.q_start),
-         _p(step.state_slots), _p(out), step.num_seqs, heads, dk, dv, int(step.max_q_len), 0, _stream())
+    longest, rest = _delta_chunks(0, proj, (off_r, off_k, off_v, off_a), decay, a_bias, None, 0, 0, None, None, 1.0, state, step, heads, heads, dk, dv, out)
+    if rest:
+        call("sllm_delta_rule", _p(proj), ld, off_r, off_k, off_v, off_a, _p(decay), _p(a_bias), _p(state), _p(step.q_start),
+             _p(step.state_slots), _p(out), step.num_seqs, heads, dk, dv, int(step.max_q_len), longest, _stream())
     return out
 
 
@@ -322,9 +324,12 @@ def gated_delta_rule(qkv, offs, gates, off_b: int, off_dt: int, a_log, dt_bias, 
         raise KernelError(f"gated_delta_rule: state {tuple(state.shape)} does not fit {heads} heads of {dk}x{dv}")
     out = torch.empty((T, heads * dv), dtype=torch.float32, device=qkv.device)
     off_q, off_k, off_v = (int(o) for o in offs)
-    call("sllm_gated_delta_rule", _p(qkv), ld, off_q, off_k, off_v, _p(gates), gates.shape[1], int(off_b), int(off_dt), _p(a_log),
-         _p(dt_bias), _p(state), _p(step.q_start), _p(step.state_slots), _p(out), step.num_seqs, heads, key_heads, dk, dv,
-         float(q_scale), int(step.max_q_len), 0, _stream())
+    longest, rest = _delta_chunks(1, qkv, (off_q, off_k, off_v, 0), None, None, gates, off_b, off_dt, a_log, dt_bias, q_scale, state, step, heads,
+                                  key_heads, dk, dv, out)
+    if rest:
+        call("sllm_gated_delta_rule", _p(qkv), ld, off_q, off_k, off_v, _p(gates), gates.shape[1], int(off_b), int(off_dt), _p(a_log),
+             _p(dt_bias), _p(state), _p(step.q_start), _p(step.state_slots), _p(out), step.num_seqs, heads, key_heads, dk, dv,
+             float(q_scale), int(step.max_q_len), longest, _stream())
     return out
 
 
@@ -673,12 +678,16 @@ def portion_chunks(q_lens, ctx_lens, min_len: int, device):
 
 # Portions of at least so many tokens may run in chunks in the recurrences below (0: none does), shorter ones are walked.
 GATED_CHUNKED_FROM = 96
+DELTA_CHUNKED_FROM = 96
 # What decides (us; `_chunks_pay`): the walk takes its longest portion times a rate, that of a CTA which walks 16 columns of a head (64 where the
 # batch fills the SMs with such) and slower the more of them an SM holds; the chunks take a base for their three kernels and a rate per
 # token of all long portions.  Measured in a graph (walk / chunks): 32 heads of 64 x 64, one portion of 128, 256, 2,048 tokens: gated 32 / 34, 60 / 35,
-# 479 / 121; 16 heads of 128 x 128: forget gate 51 / 60, 95 / 60, 709 / 163.  Eight portions of 200 tokens: 79 / 117, 195 / 173; three of 700: 349 / 125, 527 / 168.  (walk, a narrow CTA's and a wide one's per token; base; chunks
+# 479 / 121; general delta 45 / 48, 84 / 51, 931 / 333; 16 heads of 128 x 128: forget gate 51 / 60, 95 / 60, 709 / 163; gated delta 53 / 51, 99 / 58,
+# 748 / 240.  Eight portions of 200 tokens: 79 / 117, 119 / 270, 195 / 173, 223 / 240; three of 700: 349 / 125,
+# 661 / 292, 527 / 168, 551 / 260.  (walk, a narrow CTA's and a wide one's per token; base; chunks
 # per token, and the heads x keys x values that was measured at)
-CHUNK_COSTS = {"gated64": (0.235, 0.39, 30.0, 0.045, 32 * 64 * 64), "gated128": (0.35, 0.97, 52.0, 0.055, 16 * 128 * 128)}
+CHUNK_COSTS = {"gated64": (0.235, 0.39, 30.0, 0.045, 32 * 64 * 64), "gated128": (0.35, 0.97, 52.0, 0.055, 16 * 128 * 128),
+               "general": (0.42, 0.59, 40.0, 0.143, 32 * 64 * 64), "delta64": (0.30, 0.45, 42.0, 0.09, 32 * 64 * 64), "delta128": (0.37, 1.10, 42.0, 0.098, 16 * 128 * 128)}
 
 
 def _chunks_pay(kind: str, step, from_len: int, heads: int, dk: int, dv: int) -> bool:
@@ -728,6 +737,30 @@ def _gated_chunks(mode: int, proj, offs, z, a, bias, q_scale: float, tau: float,
          _p(state), _p(step.state_slots), _p(t0), _p(n), C, _p(seq), _p(first), _p(count), R, _p(scratch), _p(keeps), _p(out), heads, dk, dv, _stream())
     launches["own"] += 2           # the three kernels of the entry point
     return GATED_CHUNKED_FROM - 1, R < step.num_seqs
+
+
+@functools.lru_cache(maxsize=4096)
+def delta_chunked_supports(mode: int, dk: int, dv: int) -> bool:
+    return bool(lib().sllm_delta_chunked_supports(int(mode), int(dk), int(dv)))
+
+
+def _delta_chunks(mode: int, proj, offs, decay, a_bias, gates, off_b: int, off_dt: int, a_log, dt_bias, q_scale: float, state, step, heads: int,
+                  key_heads: int, dk: int, dv: int, out):
+    """The step's long portions through the chunked form of the delta rule ``mode`` (0: the generalized one, 1: the gated one); their rows of
+    ``out`` and their states are written.  Returns (the longest portion left for the walk, 0 for no limit; whether any is left)."""
+    chunks = None
+    if step.max_q_len >= DELTA_CHUNKED_FROM > 0 and delta_chunked_supports(mode, dk, dv) and \
+            _chunks_pay("general" if mode == 0 else "delta64" if dk <= 64 else "delta128", step, DELTA_CHUNKED_FROM, heads, dk, dv):
+        chunks = _long_portions(step, DELTA_CHUNKED_FROM, proj.device)
+    if chunks is None:
+        return 0, True
+    t0, _, n, C, seq, first, count, R = chunks
+    scratch = torch.empty(C * heads * int(lib().sllm_delta_chunked_scratch(int(dk), int(dv))), dtype=torch.float32, device=proj.device)
+    call("sllm_delta_chunked", mode, _p(proj), proj.shape[1], *(int(o) for o in offs), _p(decay), _p(a_bias), _p(gates),
+         gates.shape[1] if gates is not None else 0, int(off_b), int(off_dt), _p(a_log), _p(dt_bias), float(q_scale), _p(state), _p(step.state_slots),
+         _p(t0), _p(n), C, _p(seq), _p(first), _p(count), R, _p(scratch), _p(out), heads, key_heads, dk, dv, _stream())
+    launches["own"] += 2           # the three kernels of the entry point
+    return DELTA_CHUNKED_FROM - 1, R < step.num_seqs
 
 
 def retention_chunked(proj, offs, off_g: int, decay, table, rotary_dim: int, k_scale: float, eps: float, state, step, chunks, heads: int,

@@ -162,6 +162,11 @@ def _declare(L):
         "sllm_gated_chunked": [c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_float, c_float, c_void_p, c_void_p,
                                c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int,
                                c_int, c_void_p],
+        "sllm_delta_chunked_supports": [c_int, c_int, c_int],
+        "sllm_delta_chunked_scratch": [c_int, c_int],
+        "sllm_delta_chunked": [c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p,
+                               c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int,
+                               c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
         "sllm_softcap": [c_void_p, ctypes.c_longlong, c_float, c_void_p],
         "sllm_plain_act": [c_void_p, c_int, c_int, c_size_t, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
         "sllm_latent_rope_write": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_float, c_void_p, c_void_p, c_int,

@@ -1,4 +1,4 @@
-"""The recurrences over long prompt portions in chunks of 64 tokens (gated_chunks.cu) against the same recurrences
+"""The recurrences over long prompt portions in chunks of 64 tokens (gated_chunks.cu, delta_chunks.cu) against the same recurrences
 walked token by token in float64: portions that end inside a chunk, on its edge and one token beyond, beside short portions and single tokens
 that the walk keeps; head sizes on and off the kernels' padding; states that are not zero at the start.
 
@@ -127,3 +127,48 @@ def test_forget_gate_attention_in_chunks(dk, dv, H, hard):
         f = (lower + (1 - lower) * torch.sigmoid(proj[a:b, offs[1]:offs[1] + H * dk] + bias)).double().reshape(b - a, H, dk)
         return torch.nn.functional.silu(q), 1 - f, v, f
     _check(lambda state, step: ops.forget_gate_attention(proj, offs, bias, lower, state, step, H, dk, dv), terms, H, dk, dv, dev, g)
+
+
+@pytest.mark.parametrize("dk,dv,H,G", [(64, 64, 4, 2), (128, 128, 2, 1), (128, 64, 2, 2), (64, 128, 2, 1), (40, 24, 3, 3), (100, 72, 2, 1)])
+@pytest.mark.parametrize("hard", [False, True])
+def test_gated_delta_rule_in_chunks(dk, dv, H, G, hard):
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    g = torch.Generator(device=dev).manual_seed(dk + 11 * dv)
+    T = sum(LENS)
+    qkv = torch.randn(T, 2 * G * dk + H * dv, device=dev, generator=g)
+    gates = torch.randn(T, 2 * H + 1, device=dev, generator=g)
+    a_log = torch.rand(H, device=dev, generator=g) * (6.0 if hard else 2.0)       # hard: decays down to zero
+    dt_bias = torch.randn(H, device=dev, generator=g) - (0.0 if hard else 3.0)
+    offs = (0, G * dk, 2 * G * dk)
+
+    def terms(a, b):
+        n = b - a
+        q, k = (qkv[a:b, o:o + G * dk].double().reshape(n, G, dk) for o in offs[:2])
+        q, k = (x / (x.pow(2).sum(-1, keepdim=True) + 1e-6).sqrt() for x in (q, k))
+        q, k = (x.repeat_interleave(H // G, 1) for x in (q * dk ** -0.5, k))
+        v = qkv[a:b, offs[2]:].double().reshape(n, H, dv)
+        beta = torch.sigmoid(gates[a:b, :H].double())[:, :, None]
+        keep = torch.exp(-torch.exp(a_log.double()) * torch.nn.functional.softplus(gates[a:b, H + 1:].double() + dt_bias.double()))[:, :, None]
+        return q, k, beta * v, keep, k, beta * keep * k
+    _check(lambda state, step: ops.gated_delta_rule(qkv, offs, gates, 0, H + 1, a_log, dt_bias, state, step, H, G, dk, dv, dk ** -0.5),
+           terms, H, dk, dv, dev, g)
+
+
+@pytest.mark.parametrize("d,H", [(64, 3), (40, 2), (17, 5)])
+@pytest.mark.parametrize("hard", [False, True])
+def test_delta_rule_in_chunks(d, H, hard):
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    g = torch.Generator(device=dev).manual_seed(d + 13 * H)
+    T, C = sum(LENS), H * d
+    proj = torch.randn(T, 4 * C, device=dev, generator=g)
+    decay = torch.randn(T, C, device=dev, generator=g) * 2 + (20.0 if hard else -2.0)      # hard: every channel's decay at its smallest
+    bias = torch.randn(C, device=dev, generator=g)
+
+    def terms(a, b):
+        r, k, v, z = (proj[a:b, o * C:(o + 1) * C].double().reshape(b - a, H, d) for o in range(4))
+        u = k / (k.pow(2).sum(-1, keepdim=True) + 1e-6).sqrt()
+        keep = torch.exp(-np.exp(-0.5) * torch.sigmoid(decay[a:b].double())).reshape(b - a, H, d)
+        return r, k, v, keep, u, torch.sigmoid(z + bias.double().reshape(H, d)) * u
+    _check(lambda state, step: ops.delta_rule(proj, (0, C, 2 * C, 3 * C), decay, bias, state, step, H, d, d), terms, H, d, d, dev, g)
