@@ -1,4 +1,4 @@
-// Sampling on the device over float32 logits [R, V], one block of 1024 threads per row, and the
+// Sampling on the device over float32 logits [R, V], a cluster of eight blocks of 1024 threads per row (one block for a short row), and the
 // repetition penalty that goes before it.
 //
 // greedy: the first maximum (runtime/sampler.py:8-9).
@@ -14,20 +14,21 @@
 // as the reference's sampler works in float64.
 //
 // In this file, in order:
-//   block_argmax                     the greedy row;
+//   part_argmax, row_argmax          the greedy row, a part a block;
 //   select_key / choose_bin          the general top-k / top-p: a five-level select over the row for the
 //                                    key of the cut (by count or by mass), then the kept set is
 //                                    {key > tau} and the ties at tau up to an index;
 //   collect_candidates, select_in_candidates, draw_from_list
 //                                    the one-pass forms: every thread keeps its largest logits, and if
 //                                    the cut provably lies among those candidates the rest runs on a
-//                                    short list in shared memory (sample_top_k_fast for top_k <= 256,
-//                                    sample_top_p_fast for top_p alone on a peaked row);
+//                                    short list in shared memory (sample_top_p_fast for top_p alone on a peaked row);
+//   sample_top_k_fast                top_k <= 256: a bound below the k-th largest logit from 256 maxima, the few logits from it on;
 //   sample_rows_kernel               picks the form for its row; the general inverse CDF walks the row
 //                                    in index order (32 parts, the chosen part in 32 pieces, one warp's scan);
 //   repetition_penalty_kernel        the penalty from explicit (row, id) pairs;
 //   mark_seen_kernel, penalty_seen_kernel
 //                                    the penalty from a table of seen ids kept on the device.
+#include <cooperative_groups.h>
 #include <math.h>
 #include <stdio.h>
 
@@ -36,6 +37,7 @@
 namespace sllm {
 
 constexpr int SAMPLE_THREADS = 1024;
+constexpr int SAMPLE_SPLIT_FROM = 16384;     // logits of a row from which eight blocks share it
 
 struct MaxIdx {
   float v;
@@ -46,14 +48,14 @@ __device__ __forceinline__ MaxIdx better(MaxIdx a, MaxIdx b) {
   return a;
 }
 
-__device__ MaxIdx block_argmax(const float* __restrict__ row, int V, MaxIdx* sh) {
+// the first maximum of row[from, to), known to all threads; index 0x7fffffff: nothing there is above minus infinity
+__device__ MaxIdx part_argmax(const float* __restrict__ row, int from, int to, bool vec, MaxIdx* sh) {
   MaxIdx best{-INFINITY, 0x7fffffff};
-  if ((V & 3) == 0 && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
+  if (vec) {                                         // whole 16-byte pieces
     // four values a load, four loads in flight; a thread's indices still ascend
     const float4* row4 = reinterpret_cast<const float4*>(row);
-    const int n4 = V >> 2;
 #pragma unroll 4
-    for (int i = threadIdx.x; i < n4; i += blockDim.x) {
+    for (int i = from / 4 + threadIdx.x; i < to / 4; i += blockDim.x) {
       const float4 v = row4[i];
       if (v.x > best.v) best = MaxIdx{v.x, 4 * i};
       if (v.y > best.v) best = MaxIdx{v.y, 4 * i + 1};
@@ -61,7 +63,7 @@ __device__ MaxIdx block_argmax(const float* __restrict__ row, int V, MaxIdx* sh)
       if (v.w > best.v) best = MaxIdx{v.w, 4 * i + 3};
     }
   } else {
-    for (int i = threadIdx.x; i < V; i += blockDim.x) {
+    for (int i = from + threadIdx.x; i < to; i += blockDim.x) {
       const float v = row[i];
       if (v > best.v) best = MaxIdx{v, i};           // strict >: the first maximum wins
     }
@@ -85,8 +87,29 @@ __device__ MaxIdx block_argmax(const float* __restrict__ row, int V, MaxIdx* sh)
     if (lane == 0) sh[0] = b;
   }
   __syncthreads();
-  MaxIdx r = sh[0];
+  const MaxIdx r = sh[0];
   __syncthreads();
+  return r;
+}
+
+// A row's blocks (a cluster) and this one's part of the row, whole 16-byte pieces apart.
+struct RowPart {
+  int rank, blocks, from, to;
+  bool vec;
+};
+
+// the row's first maximum (index 0 where nothing is above minus infinity), known to the first block; all blocks of the cluster call it
+__device__ MaxIdx row_argmax(const float* __restrict__ row, const RowPart& part, MaxIdx* sh, MaxIdx* parts /* [8] shared */) {
+  MaxIdx r = part_argmax(row, part.from, part.to, part.vec, sh);
+  if (part.blocks > 1) {
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    if (threadIdx.x == 0) *cl.map_shared_rank(parts + part.rank, 0) = r;
+    cl.sync();
+    if (part.rank == 0) {
+      r = parts[0];
+      for (int b = 1; b < part.blocks; ++b) r = better(r, parts[b]);
+    }
+  }
   if (r.i == 0x7fffffff) r.i = 0;
   return r;
 }
@@ -132,23 +155,25 @@ struct Select {
   int chosen;                 // the last level's bin, -1: the target lies beyond every eligible logit
 };
 
-// f(logit, index) over the row, eight loads in flight a thread
+// f(logit, index) over row[from, to), eight loads in flight a thread
 template <class F>
-__device__ __forceinline__ void for_row(const float* __restrict__ row, int V, F f) {
-  for (int i0 = threadIdx.x; i0 < V; i0 += SAMPLE_THREADS * 8) {
+__device__ __forceinline__ void for_range(const float* __restrict__ row, int from, int to, F f) {
+  for (int i0 = from + threadIdx.x; i0 < to; i0 += SAMPLE_THREADS * 8) {
     float l[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       const int i = i0 + u * SAMPLE_THREADS;
-      l[u] = i < V ? row[i] : 0.f;
+      l[u] = i < to ? row[i] : 0.f;
     }
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       const int i = i0 + u * SAMPLE_THREADS;
-      if (i < V) f(l[u], i);
+      if (i < to) f(l[u], i);
     }
   }
 }
+template <class F>
+__device__ __forceinline__ void for_row(const float* __restrict__ row, int V, F f) { for_range(row, 0, V, f); }
 // the same over [base, base + len) cut at `end`, by one warp
 template <class F>
 __device__ __forceinline__ void for_part(const float* __restrict__ row, int base, int len, int end, F f) {
@@ -340,15 +365,11 @@ __device__ __forceinline__ bool is_kept(const Kept& kp, float l, int i) {
   return key > kp.tau || (key == kp.tau && i <= kp.i_eq);
 }
 
-// ---- a small top-k in one pass over the row ------------------------------------------------------
+// ---- candidates: every thread's largest ------------------------------------------------------------
 //
 // Each thread keeps the five largest logits of its share of the row; the four largest of every
-// thread are the candidates (4096 of them), the fifth bounds what the thread let go.  If the k-th
-// largest candidate lies above every such bound, the k largest logits of the row are all among the
-// candidates and the rest of the work (top-k's cut, top-p over what it kept, the draw in index
-// order) runs on at most k values in shared memory.  Otherwise (a thread held more than four of the
-// row's k largest) the general path above takes the row.  The probabilities of top-k's set are
-// renormalised, so the sum over the whole row is never needed here.
+// thread are the candidates (4096 of them), the fifth bounds what the thread let go.  If the cut lies above every such bound, the
+// logits above it are all among the candidates.
 
 constexpr int FAST_K = 256;                 // rows with top_k up to this try the one-pass form
 constexpr int FAST_PER_THREAD = 4;
@@ -357,8 +378,8 @@ constexpr int FAST_TIES = 1024;
 static_assert(FAST_CANDIDATES * 8 + SEL_BINS * 4 <= SAMPLE_SMEM, "the candidates live in the histograms' shared memory");
 
 struct FastShared {
-  uint32_t kept_key[FAST_K], sorted_key[FAST_K];
-  int kept_idx[FAST_K], sorted_idx[FAST_K];
+  uint32_t kept_key[FAST_K];
+  int kept_idx[FAST_K];
   double q[FAST_K];
   int tie_idx[FAST_TIES];
   int n_kept, n_ties, max_let_go, answer, last;
@@ -367,9 +388,8 @@ struct FastShared {
 
 // One pass over the row: every thread's four largest logits become the candidates (keys and
 // indices in `dyn_smem`), the largest fifth one is recorded in fs->max_let_go (31 bits), *mx_out is
-// the row's maximum (first index among equals).  WITH_SUM: *sum_out is the sum over the whole row of
+// the row's maximum (first index among equals); *sum_out is the sum over the whole row of
 // expf((logit - max) / T), from a second pass.
-template <bool WITH_SUM>
 __device__ void collect_candidates(const float* __restrict__ row, int V, float inv_t, unsigned char* dyn_smem, MaxIdx* sh_mi,
                                    double* red, FastShared* fs, MaxIdx* mx_out, double* sum_out) {
   uint32_t* cand_key = reinterpret_cast<uint32_t*>(dyn_smem);
@@ -428,24 +448,22 @@ __device__ void collect_candidates(const float* __restrict__ row, int V, float i
   __syncthreads();
   const MaxIdx mx = sh_mi[0];
   *mx_out = mx;
-  if constexpr (WITH_SUM) {
-    double part = 0.0;                              // a second, plain pass: the sum needs the maximum
-    for_row(row, V, [&](float l, int) {
-      if (l == l) part += (double)prob(l, mx.v, inv_t);
-    });
+  double part = 0.0;                              // a second, plain pass: the sum needs the maximum
+  for_row(row, V, [&](float l, int) {
+    if (l == l) part += (double)prob(l, mx.v, inv_t);
+  });
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    if (lane == 0) red[warp] = part;
-    __syncthreads();
-    if (warp == 0) {
-      double t = red[lane];
+  for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+  if (lane == 0) red[warp] = part;
+  __syncthreads();
+  if (warp == 0) {
+    double t = red[lane];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      if (lane == 0) red[32] = t;
-    }
-    __syncthreads();
-    *sum_out = red[32];
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) red[32] = t;
   }
+  __syncthreads();
+  *sum_out = red[32];
 }
 
 // The select of select_key over the candidates in shared memory (a linear level, then the key's four
@@ -541,62 +559,84 @@ __device__ void draw_from_list(const uint32_t* key, const int* idx, int n, float
   if (threadIdx.x == 0) *out = fs->answer != 0x7fffffff ? fs->answer : fs->last;
 }
 
-// true: out[row] is written.  false: the general path must take the row.  `mx` is set either way.
-__device__ bool sample_top_k_fast(const float* __restrict__ row, int V, float inv_t, int k, float pfrac, double u,
-                                  unsigned char* dyn_smem, int* bin_c, double* bin_m, Select* sel, MaxIdx* sh_mi,
-                                  FastShared* fs, MaxIdx* mx_out, int* out) {
-  uint32_t* cand_key = reinterpret_cast<uint32_t*>(dyn_smem);
-  int* cand_idx = reinterpret_cast<int*>(cand_key + FAST_CANDIDATES);
-  const int warp = threadIdx.x >> 5;
-  collect_candidates<false>(row, V, inv_t, dyn_smem, sh_mi, nullptr, fs, mx_out, nullptr);
-  const MaxIdx mx = *mx_out;
-  // the k-th largest candidate
-  select_in_candidates(cand_key, cand_idx, mx.v, inv_t, false, k, 0.0, bin_c, reinterpret_cast<float*>(cand_idx + FAST_CANDIDATES),
-                       bin_m, sel);
-  if (sel->chosen < 0) return false;
-  const uint32_t tau = sel->prefix;
-  const int n_eq = k - sel->cnt_above, ties = sel->group_cnt;
-  // every logit a thread let go must lie below tau (the bound was kept to 31 bits: compare those)
-  if ((int)(tau >> 1) <= fs->max_let_go || ties > FAST_TIES) return false;
-  // top-k's set: above tau, and the first n_eq of the ties by index
-#pragma unroll
-  for (int j = 0; j < FAST_PER_THREAD; ++j) {
-    const int c = threadIdx.x * FAST_PER_THREAD + j;
-    if (cand_idx[c] < 0) continue;
-    if (cand_key[c] > tau) {
-      const int at = atomicAdd(&fs->n_kept, 1);
-      fs->kept_key[at] = cand_key[c];
-      fs->kept_idx[at] = cand_idx[c];
-    } else if (cand_key[c] == tau) {
-      fs->tie_idx[atomicAdd(&fs->n_ties, 1)] = cand_idx[c];
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < ties) {
-    const int mine = fs->tie_idx[threadIdx.x];
-    int rank = 0;
-    for (int j = 0; j < ties; ++j) rank += fs->tie_idx[j] < mine;
-    if (rank < n_eq) {
-      const int at = atomicAdd(&fs->n_kept, 1);
-      fs->kept_key[at] = tau;
-      fs->kept_idx[at] = mine;
-    }
-  }
-  __syncthreads();
-  int m = fs->n_kept;                               // == k
-  // top-p over the kept values in descending order, ties by index (runtime/sampler.py:68-79)
-  if (pfrac >= 0.f) {
-    if (threadIdx.x < m) {
-      const uint32_t key = fs->kept_key[threadIdx.x];
-      const int idx = fs->kept_idx[threadIdx.x];
-      int rank = 0;
-      for (int j = 0; j < m; ++j) rank += fs->kept_key[j] > key || (fs->kept_key[j] == key && fs->kept_idx[j] < idx);
-      fs->sorted_key[rank] = key;
-      fs->sorted_idx[rank] = idx;
-    }
+// ---- top-k of at most 256 ------------------------------------------------------------------------
+//
+// The row's blocks and warps (a short row: its block's groups of four lanes) are 256 groups.  The k-th largest of the groups' maxima is a
+// bound at or below the row's k-th largest logit, and little more than k logits reach it (about -256 ln(1 - k / 256) of a row in no
+// particular order): they are gathered in the first block, ranked against one another, and the rest (top-p over what top-k
+// kept, the draw in index order) runs on k values in shared memory.  Two passes over the row, the second from L2, by eight SMs.
+// (32 rows of 151,936 logits, top_k 20: 34 us with the gaps of a serving step; one block a row with four candidates a thread 336 where the k-th largest lay more
+// than 24 T below the largest, which that form left to the general path.)
+
+constexpr int TOPK_GROUPS = 256, TOPK_LIST = 2048;
+constexpr uint32_t MINUS_INFINITY_KEY = 0x007fffffu;
+static_assert(TOPK_LIST * 8 <= SAMPLE_SMEM, "the list lives in the histograms' shared memory");
+
+// true: out[row] is written (by the first block).  false: the general path must take the row.  All blocks of the cluster call it; in the others
+// the result means nothing.
+__device__ bool sample_top_k_fast(const float* __restrict__ row, const RowPart& part, float inv_t, int k, float pfrac, double u,
+                                  unsigned char* dyn_smem, uint32_t* group_max /* [256] shared */, uint32_t* bound_s, int* count,
+                                  FastShared* fs, int* out) {
+  cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  uint32_t* list_key = reinterpret_cast<uint32_t*>(dyn_smem);
+  int* list_idx = reinterpret_cast<int*>(list_key + TOPK_LIST);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lanes = part.blocks > 1 ? 32 : 4;        // of a group
+  if (threadIdx.x == 0) { *count = 0; *bound_s = 0u; fs->answer = 0x7fffffff; fs->last = -1; }
+  // (key 0 belongs to no logit but one that is not a number)
+  uint32_t best = 0u;
+  for_range(row, part.from, part.to, [&](float l, int) {
+    if (l == l) best = max(best, order_key(l));
+  });
+  for (int o = 1; o < lanes; o <<= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
+  if (part.blocks > 1) {
+    if (lane < part.blocks) *cl.map_shared_rank(group_max + part.rank * 32 + warp, lane) = best;
+    cl.sync();
+  } else {
+    if (lane % 4 == 0) group_max[threadIdx.x / 4] = best;
     __syncthreads();
+  }
+  if (threadIdx.x < TOPK_GROUPS) {                   // (fewer blocks than eight do not occur beside one: every place is written)
+    const uint32_t mine = group_max[threadIdx.x];
+    int rank = 0;
+    for (int j = 0; j < TOPK_GROUPS; ++j) rank += group_max[j] > mine || (group_max[j] == mine && j < (int)threadIdx.x);
+    if (rank == k - 1) *bound_s = mine;
+  }
+  __syncthreads();
+  const uint32_t bound = *bound_s;
+  if (bound > MINUS_INFINITY_KEY) {
+    int* there = part.blocks > 1 ? cl.map_shared_rank(count, 0) : count;
+    uint32_t* keys = part.blocks > 1 ? cl.map_shared_rank(list_key, 0) : list_key;
+    int* idxs = part.blocks > 1 ? cl.map_shared_rank(list_idx, 0) : list_idx;
+    for_range(row, part.from, part.to, [&](float l, int i) {
+      if (l == l && order_key(l) >= bound) {
+        const int at = atomicAdd(there, 1);
+        if (at < TOPK_LIST) { keys[at] = order_key(l); idxs[at] = i; }
+      }
+    });
+  }
+  if (part.blocks > 1) cl.sync(); else __syncthreads();
+  if (part.rank != 0) return true;
+  const int n = *count;
+  // fewer than k groups hold a logit above minus infinity; very many ties
+  if (bound <= MINUS_INFINITY_KEY || n > TOPK_LIST) return false;
+  // the k largest in descending order, ties by index (runtime/sampler.py:60-67)
+  for (int e = threadIdx.x; e < n; e += SAMPLE_THREADS) {
+    const uint32_t key = list_key[e];
+    const int idx = list_idx[e];
+    int rank = 0;
+    for (int j = 0; j < n; ++j) rank += list_key[j] > key || (list_key[j] == key && list_idx[j] < idx);
+    if (rank < k) {
+      fs->kept_key[rank] = key;
+      fs->kept_idx[rank] = idx;
+    }
+  }
+  __syncthreads();
+  const float mx = key_value(fs->kept_key[0]);
+  int m = k;
+  if (pfrac >= 0.f) {                                // top-p over them (runtime/sampler.py:68-79)
     // the cumulative probability at every place of the sorted list, one place a thread
-    if (threadIdx.x < m) fs->q[threadIdx.x] = (double)prob(key_value(fs->sorted_key[threadIdx.x]), mx.v, inv_t);
+    if (threadIdx.x < m) fs->q[threadIdx.x] = (double)prob(key_value(fs->kept_key[threadIdx.x]), mx, inv_t);
     if (threadIdx.x == 0) fs->n_kept = m;
     __syncthreads();
     double cum = 0.0;
@@ -607,13 +647,8 @@ __device__ bool sample_top_k_fast(const float* __restrict__ row, int V, float in
     if (threadIdx.x < m && cum >= (double)pfrac * fs->red[0]) atomicMin(&fs->n_kept, (int)threadIdx.x + 1);
     __syncthreads();
     m = fs->n_kept;
-    if (threadIdx.x < m) {
-      fs->kept_key[threadIdx.x] = fs->sorted_key[threadIdx.x];
-      fs->kept_idx[threadIdx.x] = fs->sorted_idx[threadIdx.x];
-    }
-    __syncthreads();
   }
-  draw_from_list(fs->kept_key, fs->kept_idx, m, mx.v, inv_t, u, fs->red, fs, out);
+  draw_from_list(fs->kept_key, fs->kept_idx, m, mx, inv_t, u, fs->red, fs, out);
   return true;
 }
 
@@ -636,9 +671,8 @@ __device__ bool sample_top_p_fast(const float* __restrict__ row, int V, float in
   uint32_t* kept_key = reinterpret_cast<uint32_t*>(hist_m + SEL_BINS);              // [FAST_P_KEPT]
   int* kept_idx = reinterpret_cast<int*>(kept_key + FAST_P_KEPT);
   static_assert(FAST_CANDIDATES * 8 + SEL_BINS * 4 + FAST_P_KEPT * 8 <= SAMPLE_SMEM, "the lists live in the histograms' shared memory");
-  const int warp = threadIdx.x >> 5;
   double row_sum;
-  collect_candidates<true>(row, V, inv_t, dyn_smem, sh_mi, fs->red, fs, mx_out, &row_sum);
+  collect_candidates(row, V, inv_t, dyn_smem, sh_mi, fs->red, fs, mx_out, &row_sum);
   const MaxIdx mx = *mx_out;
   // the key at which the descending cumulative probability first reaches top_p of the row's sum
   select_in_candidates(cand_key, cand_idx, mx.v, inv_t, true, 0, (double)pfrac * row_sum, bin_c, hist_m, bin_m, sel);
@@ -680,9 +714,11 @@ __device__ bool sample_top_p_fast(const float* __restrict__ row, int V, float in
 __global__ void __launch_bounds__(SAMPLE_THREADS)
 sample_rows_kernel(const float* __restrict__ logits, int V, const float* __restrict__ temperature,
                    const double* __restrict__ uniform, const int* __restrict__ top_k, const float* __restrict__ top_p,
-                   int* __restrict__ out) {
-  extern __shared__ unsigned char sample_smem[];
-  __shared__ MaxIdx sh_mi[32];
+                   int* __restrict__ out, int blocks) {
+  extern __shared__ __align__(16) unsigned char sample_smem[];
+  __shared__ MaxIdx sh_mi[32], parts_mi[8];
+  __shared__ uint32_t group_max[TOPK_GROUPS], bound_s;
+  __shared__ int list_n;
   __shared__ double part_sum[SEL_WARPS];
   __shared__ int part_cnt[SEL_WARPS], part_last[SEL_WARPS];
   __shared__ int bin_c[SEL_BINS];
@@ -693,30 +729,40 @@ sample_rows_kernel(const float* __restrict__ logits, int V, const float* __restr
   __shared__ int pick_part, pick_need, i_eq_s, result;
   __shared__ double pick_before;
   pdl_launch_dependents();       // a short kernel: the successor may be set up behind it
+  if (blocks > 1) cooperative_groups::this_cluster().sync();      // nobody reaches into the shared memory of a block that has not begun
   pdl_wait();
   __shared__ FastShared fast;
-  const float* row = logits + (size_t)blockIdx.x * V;
-  const float temp = temperature ? temperature[blockIdx.x] : 0.f;
-  const int k = (top_k && temp > 0.f) ? top_k[blockIdx.x] : 0;
-  const float pfrac = (top_p && temp > 0.f) ? top_p[blockIdx.x] : -1.f;
+  const int r = blockIdx.x / blocks;
+  const float* row = logits + (size_t)r * V;
+  RowPart part;
+  part.rank = blockIdx.x % blocks;
+  part.blocks = blocks;
+  const int share = ((V + blocks - 1) / blocks + 3) & ~3;
+  part.from = min(part.rank * share, V);
+  part.to = min(part.from + share, V);
+  part.vec = (V & 3) == 0 && (reinterpret_cast<uintptr_t>(row) & 15) == 0;
+  const float temp = temperature ? temperature[r] : 0.f;
+  const int k = (top_k && temp > 0.f) ? top_k[r] : 0;
+  const float pfrac = (top_p && temp > 0.f) ? top_p[r] : -1.f;
   const bool has_k = k > 0 && k < V, has_p = pfrac >= 0.f;
   const float inv_t = temp > 0.f ? 1.0f / temp : 0.f;
   MaxIdx mx;
   if (has_k && k <= FAST_K) {
-    if (sample_top_k_fast(row, V, inv_t, k, pfrac, uniform[blockIdx.x], sample_smem, bin_c, bin_m, &sel, sh_mi, &fast, &mx,
-                          out + blockIdx.x))
-      return;
+    if (sample_top_k_fast(row, part, inv_t, k, pfrac, uniform[r], sample_smem, group_max, &bound_s, &list_n, &fast, out + r)) return;
     __syncthreads();                                 // the general path reuses what the attempt wrote
+    mx = part_argmax(row, 0, V, part.vec, sh_mi);
+    if (mx.i == 0x7fffffff) mx.i = 0;
   } else if (has_p && !has_k) {
-    if (sample_top_p_fast(row, V, inv_t, pfrac, uniform[blockIdx.x], sample_smem, bin_c, bin_m, &sel, sh_mi, &fast, &mx,
-                          out + blockIdx.x))
+    if (part.rank != 0) return;
+    if (sample_top_p_fast(row, V, inv_t, pfrac, uniform[r], sample_smem, bin_c, bin_m, &sel, sh_mi, &fast, &mx, out + r))
       return;
     __syncthreads();
   } else {
-    mx = block_argmax(row, V, sh_mi);
+    mx = row_argmax(row, part, sh_mi, parts_mi);
+    if (part.rank != 0) return;
   }
   if (!(temp > 0.f)) {
-    if (threadIdx.x == 0) out[blockIdx.x] = mx.i;
+    if (threadIdx.x == 0) out[r] = mx.i;
     return;
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -821,7 +867,7 @@ sample_rows_kernel(const float* __restrict__ logits, int V, const float* __restr
   if (threadIdx.x == 0) {
     double total = 0.0;
     for (int w = 0; w < SEL_WARPS; ++w) total += part_sum[w];
-    const double target = uniform[blockIdx.x] * total;
+    const double target = uniform[r] * total;
     double before = 0.0;
     int pick = -1, last = -1;
     for (int w = 0; w < SEL_WARPS; ++w) {
@@ -837,7 +883,7 @@ sample_rows_kernel(const float* __restrict__ logits, int V, const float* __restr
   }
   __syncthreads();
   if (pick_part < 0) {
-    if (threadIdx.x == 0) out[blockIdx.x] = result;
+    if (threadIdx.x == 0) out[r] = result;
     return;
   }
   // 3: the chosen part, again in 32 pieces of whole groups; 4: the chosen piece, group by group
@@ -875,7 +921,7 @@ sample_rows_kernel(const float* __restrict__ logits, int V, const float* __restr
   }
   __syncthreads();
   if (pick_need < 0) {
-    if (threadIdx.x == 0) out[blockIdx.x] = result;
+    if (threadIdx.x == 0) out[r] = result;
     return;
   }
   if (warp == pick_need) {
@@ -899,7 +945,7 @@ sample_rows_kernel(const float* __restrict__ logits, int V, const float* __restr
       if (hit) answer = base + o + (__ffs(hit) - 1);
       left -= __shfl_sync(0xffffffffu, incl, 31);
     }
-    if (lane == 0) out[blockIdx.x] = answer >= 0 ? answer : (last >= 0 ? last : result);
+    if (lane == 0) out[r] = answer >= 0 ? answer : (last >= 0 ? last : result);
   }
 }
 
@@ -975,7 +1021,22 @@ SLLM_EXPORT int sllm_sample_rows(const float* logits, int R, int V, const float*
     configured = true;
   }
   const int smem = (top_k || top_p) ? SAMPLE_SMEM : 0;
-  launch_kernel(sample_rows_kernel, R, SAMPLE_THREADS, smem, stream, logits, V, temperature, uniform, top_k, top_p, out);
+  // a short row is one block's (and its groups of four lanes still see more than one logit)
+  const int blocks = V >= SAMPLE_SPLIT_FROM ? 8 : 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)R * blocks);
+  cfg.blockDim = dim3(SAMPLE_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = blocks;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  cudaLaunchKernelEx(&cfg, sample_rows_kernel, logits, V, temperature, uniform, top_k, top_p, out, blocks);
   return launch_status("sample_rows");
 }
 

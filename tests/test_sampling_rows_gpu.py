@@ -1,0 +1,71 @@
+"""Rows that eight blocks share and rows of one block, around the sizes where that changes: the greedy choice, top-k with and without top-p on flat
+rows and on peaked ones (the k-th largest logit far below the largest), ties at the cut, logits that are minus infinity or not a number.  The
+choice is exact: against the same steps in float64, at uniforms that lie no closer than 1e-6 to a step of the cumulative probability."""
+
+import numpy as np
+import pytest
+import torch
+
+from tests.conftest import cuda_or_skip
+
+pytestmark = pytest.mark.gpu
+
+
+def _choose(row, t, k, p, u):
+    """(the id, the distance of u to the nearest step) in float64: top-k by value then index, top-p over it, the inverse CDF in index order."""
+    order = np.lexsort((np.arange(len(row)), -row))[:k]
+    q = np.exp((row[order] - row[order[0]]) / t)
+    if p >= 0:
+        cum = np.cumsum(q / q.sum())
+        n = int(np.searchsorted(cum, p)) + 1
+        order, q = order[:n], q[:n]
+        edge = np.abs(cum - p).min()
+    else:
+        edge = 1.0
+    by_index = np.argsort(order)
+    cum = np.cumsum(q[by_index]) / q.sum()
+    at = min(int(np.searchsorted(cum, u)), len(cum) - 1)
+    return int(order[by_index][at]), min(edge, float(np.abs(cum - u).min()))
+
+
+@pytest.mark.parametrize("V", [300, 16383, 16384, 16387, 151936])
+@pytest.mark.parametrize("k", [1, 2, 20, 255, 256])
+@pytest.mark.parametrize("peak", [0.0, 60.0])
+def test_top_k_of_long_and_short_rows(V, k, peak):
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    g = torch.Generator(device=dev).manual_seed(V + k)
+    R = 6
+    logits = torch.randn(R, V, device=dev, generator=g) * 3
+    logits[:, V // 3] += peak
+    logits[1, ::7] = -float("inf")
+    logits[2, 5] = float("nan")
+    logits[3] = (logits[3] * 2).round() / 2                  # many ties
+    logits[4, 10:] = -float("inf")
+    logits[5] = -float("inf")                                # no choice at all: any id of the row
+    rng = np.random.default_rng(V + k)
+    top_p = torch.tensor([-1.0, 0.8, 0.95, -1.0, 0.5, 0.99], device=dev)
+    for _ in range(3):
+        u = rng.random(R)
+        got = ops.sample_rows(logits, torch.full((R,), 0.7, device=dev), torch.tensor(u, device=dev),
+                              torch.full((R,), k, dtype=torch.int32, device=dev), top_p).tolist()
+        assert 0 <= got[5] < V
+        for i, row in enumerate(logits[:5].double().cpu().numpy()):
+            row = np.where(np.isnan(row), -np.inf, row)
+            want, far = _choose(row, float(np.float32(0.7)), k, float(top_p[i]), u[i])
+            assert got[i] == want or far < 1e-6, (i, got[i], want, far)
+
+
+@pytest.mark.parametrize("V", [1, 5, 16383, 16384, 16390, 151936])
+def test_greedy_of_long_and_short_rows(V):
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    g = torch.Generator(device=dev).manual_seed(V)
+    logits = torch.randn(9, V, device=dev, generator=g).round()          # the first of many equal maxima
+    logits[1] = -float("inf")
+    logits[2] = float("nan")
+    logits[3, V - 1] = 50
+    logits[4, 0] = 50
+    clean = torch.nan_to_num(logits, nan=-float("inf"), neginf=-float("inf"), posinf=float("inf"))
+    want = [int((row == row.max()).nonzero()[0]) for row in clean]
+    assert ops.sample_rows(logits).tolist() == want
