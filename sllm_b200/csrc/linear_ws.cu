@@ -1,8 +1,7 @@
-// Weight-streaming linear layer for at most 16 tokens and a modest number of output rows (the
-// attention and down projections of a decode step): y[M, N] = x[M, K] W[N, K]^T.
+// Weight-streaming linear layer for at most 16 tokens (32 for small matrices): y[M, N] = x[M, K] W[N, K]^T.
 //
 // linear_stream.cu gives 128 weight rows to a CTA and, when N is small, splits K over the grid,
-// leaving partial sums for the consumer.  Here a CTA owns 16 output rows over the whole of K and
+// leaving partial sums for the consumer.  Here a CTA owns 16 output rows at a time over the whole of K and
 // its 8 warps split K among themselves: warp w takes the 32-wide k blocks w, w+8, w+16, ...
 // (so the CTA reads 512 contiguous bytes of each row at a time), four blocks in flight per warp,
 // weights and activations both loaded straight into MMA fragments (same k permutation as in
@@ -13,18 +12,20 @@
 //              optionally through an activation: max(v, 0)^2, or gelu_tanh(v) times the token's own entry of a table
 //   residual   residual[M, N] += y (+ bias): the float32 stream is updated in place, so the next
 //              norm has nothing to add
+//   gated      act(gate) * up of a gate|up matrix whose rows alternate in blocks of 8: local row r < 8 is a pair's gate row,
+//              r + 8 its up row, act SiLU or the tanh form of GELU
 //   rotary     for the fused q|k|v matrix of an attention layer: bias, rotary encoding and the write
 //              of the new keys and values into their cache pages, so that the decode step needs no
 //              kernel between this product and the attention.  A CTA then takes the 8 rows j..j+7
 //              of a head and the 8 rows hd/2 apart: the two rows of a rotation pair are the two
 //              rows (g, g+8) of one MMA accumulator, and meet in one thread of the epilogue
 //              (ref/qwen3_5.py:355-370; cache content ref/incremental.py:135-139).
-// About N/16 CTAs keep every SM busy without splitting K over the grid; their number is rounded up
-// to a multiple of the SM count and the rows dealt evenly (N = 3584: 296 CTAs of 12 or 13 rows
-// instead of 224 of 16, of which 76 SMs would get two and 72 one).
+// About N/16 CTAs keep every SM busy without splitting K over the grid, at most two an SM, the rows dealt evenly (N = 3584: 296 CTAs of
+// 12 or 13 rows instead of 224 of 16, of which 76 SMs would get two and 72 one; N = 11264: 296 CTAs of 38 rows in three groups).
 //
 // The reference calls cublasGemmEx for these products and adds the residual in its next
 // add_rms kernel (kernels/cuda/kernels.cu:752-767, 791-839; kernels/device_decode.py:312-325).
+#include <cooperative_groups.h>
 #include <stdio.h>
 
 #include "common.cuh"
@@ -34,6 +35,7 @@ namespace sllm {
 #define WS_EPI_STORE 0
 #define WS_EPI_RESID 1
 #define WS_EPI_ROPE 2
+#define WS_EPI_GATED 3
 
 // what the rotary epilogue needs beside the product: the rows of W are q heads, then k heads, then v
 // heads of `hd` rows each; table [max_pos][2][hd/2] holds cos then sin (rotary_dim == hd), or is null
@@ -68,10 +70,13 @@ __device__ __forceinline__ void ws_mma(float (&c)[4], unsigned a0, unsigned a1, 
 }
 
 constexpr int WS_WARPS = 8;
+constexpr int WS_SLICES = 4;        // slices of K a cluster shares at most
 // k blocks a warp keeps in flight per group (two groups): with two token tiles half as many, so that the
 // activation fragments fit the registers of two CTAs an SM (four: 174 registers a thread, one CTA an SM)
 __host__ __device__ constexpr int ws_depth(int nt) { return nt == 1 ? 4 : (nt == 2 ? 2 : 1); }
 constexpr int WS_SSQ_MAX = 608;     // partial sums of squares per token a consumer takes (the producer's CTAs: at most 592 for 8192 columns)
+#define WS_GATE_SILU 0
+#define WS_GATE_GELU 1
 // with four token tiles (17..32 tokens: small matrices only, where a step is bound by its number of kernels) the table
 // is kept to what fits static shared memory beside the warps' tiles: streams of up to 3,072 columns
 __host__ __device__ constexpr int ws_ssq_max(int nt) { return nt <= 2 ? WS_SSQ_MAX : 192; }
@@ -90,38 +95,61 @@ struct WsNorm {
   float eps_in = 0.f, inv_width_in = 0.f;
   const float* gain = nullptr;       // producer (residual epilogue): the next norm's gain [N]
   __nv_bfloat16* xg_out = nullptr;   // [M, N]
-  float* ssq_out = nullptr;          // [M][(gridDim.x + 3) & ~3]
+  float* ssq_out = nullptr;          // [M][(CTAs of rows + 3) & ~3]
 };
 
 // NT: 8-token tiles (M <= 8 * NT).  OUT: float or __nv_bfloat16 (store epilogue only).  SCALED: the input
 // comes with a norm still owed (WsNorm::ssq_in).
-template <int NT, int EPI, typename OUT, bool SCALED>
+// FORM: one group of rows a CTA; several, one after the other; or one that the CTAs of a cluster share, each a slice of K (store and
+// residual epilogues).
+#define WS_ONE 0
+#define WS_WALK 1
+#define WS_SLICED 2
+template <int NT, int EPI, typename OUT, bool SCALED, int FORM>
 __global__ void __launch_bounds__(WS_WARPS * 32, 2)
 linear_ws_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ W,
                  const float* __restrict__ bias, OUT* __restrict__ out, float* __restrict__ residual,
-                 int M, int N, int K, const WsRope rope, const WsNorm norm, const int act, const TokenTable token) {
+                 int M, int N, int K, const WsRope rope, const WsNorm norm, const int act, const TokenTable token, const int slices_) {
   constexpr int WS_DEPTH = ws_depth(NT);
+  constexpr bool SLICED = FORM == WS_SLICED;
   __shared__ float red[WS_WARPS][16][8 * NT + 1];
   __shared__ float row_scale[8 * NT];
+  __shared__ float slice_sum[SLICED ? WS_SLICES : 1][SLICED ? 16 * 8 * NT : 1];
   __shared__ __align__(16) float ssq_s[SCALED ? 8 * NT : 1][SCALED ? ws_ssq_max(NT) : 4];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t4 = lane & 3;
-  // the CTA's rows [n0, n1): at most 16, the N rows dealt evenly over the grid (so that a grid of a
-  // whole number of CTAs per SM gives every SM the same bytes to stream)
-  int n0 = (int)(((long long)blockIdx.x * N) / gridDim.x), n1 = (int)(((long long)(blockIdx.x + 1) * N) / gridDim.x);
-  const int k_blocks = K / 32;
-
-  int r0 = min(n0 + g, n1 - 1), r1 = min(n0 + g + 8, n1 - 1);   // rows past the CTA's: clamped loads, skipped stores
-  if constexpr (EPI == WS_EPI_ROPE) {
-    // CTA b of a head's hd/16: rows [8c, 8c+8) of the head and the 8 rows hd/2 further
-    const int per_head = rope.hd / 16;
-    n0 = ((int)blockIdx.x / per_head) * rope.hd + ((int)blockIdx.x % per_head) * 8;
-    n1 = n0 + 16;                                  // (not a range: local row r is n0 + (r & 7) + (r >> 3) * hd/2)
-    r0 = n0 + g;
-    r1 = n0 + rope.hd / 2 + g;
-  }
-  const __nv_bfloat16* w0 = W + (size_t)r0 * K + t4 * 8;
-  const __nv_bfloat16* w1 = W + (size_t)r1 * K + t4 * 8;
+  // The CTA's rows [c0, c1), the N rows dealt evenly over the grid (so that a grid of a whole number of CTAs per SM gives
+  // every SM the same bytes to stream), taken in groups of at most 16, these too as even as they get.  Gated: the same over pairs
+  // of a gate row and its up row, in groups of at most 8.
+  constexpr int PER = EPI == WS_EPI_GATED ? 8 : 16;
+  const int units = EPI == WS_EPI_GATED ? N / 2 : N;
+  const int slices = SLICED ? slices_ : 1;
+  const int cta = blockIdx.x / slices, ctas = gridDim.x / slices, slice = blockIdx.x % slices;
+  const int c0 = (int)(((long long)cta * units) / ctas), c1 = (int)(((long long)(cta + 1) * units) / ctas);
+  const int groups = FORM != WS_WALK ? 1 : (c1 - c0 + PER - 1) / PER;
+  const int k_first = SLICED ? K / 32 * slice / slices : 0, k_blocks = SLICED ? K / 32 * (slice + 1) / slices : K / 32;      // the CTA's k blocks
+  int n0, n1;                            // the group's units
+  const __nv_bfloat16 *w0, *w1;          // the lane's two rows of the group
+  auto take = [&](int i) {
+    n0 = c0 + (int)(((long long)i * (c1 - c0)) / groups);
+    n1 = c0 + (int)(((long long)(i + 1) * (c1 - c0)) / groups);
+    int r0 = min(n0 + g, n1 - 1), r1 = min(n0 + g + 8, n1 - 1);   // rows past the group's: clamped loads, skipped stores
+    if constexpr (EPI == WS_EPI_ROPE) {
+      // CTA b of a head's hd/16: rows [8c, 8c+8) of the head and the 8 rows hd/2 further
+      const int per_head = rope.hd / 16;
+      n0 = ((int)blockIdx.x / per_head) * rope.hd + ((int)blockIdx.x % per_head) * 8;
+      n1 = n0 + 16;                                  // (not a range: local row r is n0 + (r & 7) + (r >> 3) * hd/2)
+      r0 = n0 + g;
+      r1 = n0 + rope.hd / 2 + g;
+    }
+    if constexpr (EPI == WS_EPI_GATED) {
+      r0 = r0 / 8 * 16 + r0 % 8;                     // pair q: gate row 16 (q / 8) + q % 8, up row 8 further
+      r1 = r0 + 8;
+    }
+    w0 = W + (size_t)r0 * K + t4 * 8;
+    w1 = W + (size_t)r1 * K + t4 * 8;
+  };
+  take(0);
   const __nv_bfloat16* xr[NT];
 #pragma unroll
   for (int j = 0; j < NT; ++j) xr[j] = x + (size_t)min(8 * j + g, M - 1) * K + t4 * 8;   // tokens past M: clamped, skipped
@@ -170,8 +198,10 @@ linear_ws_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __res
     }
   };
   constexpr int GROUP = WS_DEPTH * WS_WARPS;        // k blocks the CTA covers per group
-  int kb = warp;
+  const int k_mine = k_first + warp;
+  int kb = k_mine;
   load_w(wa0, wb0, kb);
+  if constexpr (SLICED) cooperative_groups::this_cluster().sync();      // nobody writes to a CTA that has not begun
   pdl_wait();
   load_x(x0, kb);
   // a norm still owed on the input: the tokens' partial sums of squares are copied to shared memory under
@@ -185,131 +215,250 @@ linear_ws_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __res
     }
     asm volatile("cp.async.commit_group;\n" ::);
   }
-  for (; kb < k_blocks; kb += 2 * GROUP) {
-    load_w(wa1, wb1, kb + GROUP);
-    load_x(x1, kb + GROUP);
-    compute(wa0, wb0, x0, kb);
-    load_w(wa0, wb0, kb + 2 * GROUP);
-    load_x(x0, kb + 2 * GROUP);
-    compute(wa1, wb1, x1, kb + GROUP);
-  }
-  pdl_launch_dependents();
+  constexpr int OUTS = (16 * 8 * NT + WS_WARPS * 32 - 1) / (WS_WARPS * 32);
+  float squares[OUTS];                   // residual epilogue: of the thread's places, over the groups
+#pragma unroll
+  for (int o = 0; o < OUTS; ++o) squares[o] = 0.f;
+  for (int group = 0; group < groups; ++group) {
+    const int m0 = n0, m1 = n1;          // (the next group's rows are taken while this one's last blocks are multiplied)
+    if constexpr (FORM != WS_ONE) {     // (also the better code for the slices: 2,048 x 11,264 10.8 us against 14.5)
+      for (kb = k_mine;; kb += 2 * GROUP) {
+        load_w(wa1, wb1, kb + GROUP);
+        load_x(x1, kb + GROUP);
+        compute(wa0, wb0, x0, kb);
+        const bool more = kb + 2 * GROUP < k_blocks;
+        if (more || group + 1 < groups) {
+          if (!more) take(group + 1);
+          load_w(wa0, wb0, more ? kb + 2 * GROUP : k_mine);
+          load_x(x0, more ? kb + 2 * GROUP : k_mine);
+        }
+        compute(wa1, wb1, x1, kb + GROUP);
+        if (!more) break;
+      }
+    } else {
+      for (; kb < k_blocks; kb += 2 * GROUP) {
+        load_w(wa1, wb1, kb + GROUP);
+        load_x(x1, kb + GROUP);
+        compute(wa0, wb0, x0, kb);
+        load_w(wa0, wb0, kb + 2 * GROUP);
+        load_x(x0, kb + 2 * GROUP);
+        compute(wa1, wb1, x1, kb + GROUP);
+      }
+    }
+    if (group + 1 == groups) pdl_launch_dependents();
 
-  if constexpr (SCALED) asm volatile("cp.async.wait_group 0;\n" ::);
-  // ---- add the warps' tiles in warp order; acc[j][c]: c0,c1 = (row g, tokens 8j+2t, +1); c2,c3 = (row g+8, ...) ----
+    // ---- add the warps' tiles in warp order; acc[j][c]: c0,c1 = (row g, tokens 8j+2t, +1); c2,c3 = (row g+8, ...) ----
+    if (group > 0) __syncthreads();      // the group before has been read
 #pragma unroll
-  for (int j = 0; j < NT; ++j)
+    for (int j = 0; j < NT; ++j)
 #pragma unroll
-    for (int c = 0; c < 4; ++c) red[warp][g + ((c & 2) ? 8 : 0)][8 * j + 2 * t4 + (c & 1)] = acc[j][c];
-  __syncthreads();
-  if constexpr (SCALED) {
-    // warp w adds the partial sums of tokens w, w + 8: lane l takes l, l + 32, ..., then the lanes are added
-#pragma unroll
-    for (int j = 0; j < NT; ++j) {
-      const int tok = warp + 8 * j;
-      float sum = 0.f;
-      if (tok < M)
-        for (int p = lane; p < norm.parts_in; p += 32) sum += ssq_s[tok][p];
-      sum = warp_sum(sum);
-      if (lane == 0) row_scale[tok] = rsqrtf(sum * norm.inv_width_in + norm.eps_in);
+      for (int c = 0; c < 4; ++c) {
+        red[warp][g + ((c & 2) ? 8 : 0)][8 * j + 2 * t4 + (c & 1)] = acc[j][c];
+        acc[j][c] = 0.f;
+      }
+    if constexpr (SCALED) {
+      if (group == 0) asm volatile("cp.async.wait_group 0;\n" ::);
     }
     __syncthreads();
-  }
-  if constexpr (EPI == WS_EPI_ROPE) {
-    const int half = rope.hd / 2;
-    const int head = n0 / rope.hd, j0 = n0 % rope.hd;            // j0 = 8c: the pair's lower dimension starts here
-    for (int idx = tid; idx < 8 * 8 * NT; idx += WS_WARPS * 32) {
-      const int i = idx % 8, tok = idx / 8;                        // consecutive threads -> consecutive dimensions of one token
-      if (tok >= M) continue;
-      float lo = 0.f, hi = 0.f;
+    if constexpr (SCALED) {
+      if (group == 0) {
+        // warp w adds the partial sums of tokens w, w + 8: lane l takes l, l + 32, ..., then the lanes are added
 #pragma unroll
-      for (int w = 0; w < WS_WARPS; ++w) { lo += red[w][i][tok]; hi += red[w][i + 8][tok]; }
-      if constexpr (SCALED) {
-        lo *= row_scale[tok];
-        hi *= row_scale[tok];
+        for (int j = 0; j < NT; ++j) {
+          const int tok = warp + 8 * j;
+          float sum = 0.f;
+          if (tok < M)
+            for (int p = lane; p < norm.parts_in; p += 32) sum += ssq_s[tok][p];
+          sum = warp_sum(sum);
+          if (lane == 0) row_scale[tok] = rsqrtf(sum * norm.inv_width_in + norm.eps_in);
+        }
+        __syncthreads();
       }
-      if (bias) { lo += bias[n0 + i]; hi += bias[n0 + half + i]; }
-      __nv_bfloat16* dst;
-      if (head < rope.nq) {
-        dst = rope.q_out + ((size_t)tok * rope.nq + head) * rope.hd;
-      } else {
-        int slot = rope.slot_mapping ? rope.slot_mapping[tok] : -1;
-        if (slot < 0 || slot / rope.page_size >= rope.num_pages) continue;     // not written (padding row, borrowed cache)
-        const bool is_k = head < rope.nq + rope.nkv;
-        const int kvh = is_k ? head - rope.nq : head - rope.nq - rope.nkv;
-        dst = (is_k ? rope.k_cache : rope.v_cache) +
-              (((size_t)(slot / rope.page_size) * rope.nkv + kvh) * rope.page_size + slot % rope.page_size) * rope.hd;
-      }
-      if (rope.table != nullptr && head < rope.nq + rope.nkv) {
-        int pos = rope.positions[tok];
-        pos = pos < 0 ? 0 : (pos >= rope.max_pos ? rope.max_pos - 1 : pos);
-        const float* cs = rope.table + (size_t)pos * rope.hd;        // cos[half] then sin[half]
-        const float c = cs[j0 + i], sn = cs[half + j0 + i];
-        const float a = lo * c - hi * sn, b = hi * c + lo * sn;
-        lo = a;
-        hi = b;
-      }
-      dst[j0 + i] = __float2bfloat16_rn(lo);
-      dst[j0 + half + i] = __float2bfloat16_rn(hi);
     }
-    return;
-  }
-  for (int idx = tid; idx < 16 * 8 * NT; idx += WS_WARPS * 32) {
-    const int row = idx % 16, tok = idx / 16;           // consecutive threads -> consecutive rows of one token
-    const int n = n0 + row;
-    const bool valid = tok < M && n < n1;               // (whole warps run the loop: 16 * 8 * NT is a multiple of 32)
-    float v = 0.f;
+    if constexpr (EPI == WS_EPI_ROPE) {
+      const int half = rope.hd / 2;
+      const int head = m0 / rope.hd, j0 = m0 % rope.hd;            // j0 = 8c: the pair's lower dimension starts here
+      for (int idx = tid; idx < 8 * 8 * NT; idx += WS_WARPS * 32) {
+        const int i = idx % 8, tok = idx / 8;                        // consecutive threads -> consecutive dimensions of one token
+        if (tok >= M) continue;
+        float lo = 0.f, hi = 0.f;
 #pragma unroll
-    for (int w = 0; w < WS_WARPS; ++w) v += red[w][row][tok];
-    if constexpr (SCALED) v *= row_scale[tok];
-    if (bias && valid) v += bias[n];
-    if constexpr (EPI == WS_EPI_RESID) {
-      float sq = 0.f;
-      if (valid) {
+        for (int w = 0; w < WS_WARPS; ++w) { lo += red[w][i][tok]; hi += red[w][i + 8][tok]; }
+        if constexpr (SCALED) {
+          lo *= row_scale[tok];
+          hi *= row_scale[tok];
+        }
+        if (bias) { lo += bias[m0 + i]; hi += bias[m0 + half + i]; }
+        __nv_bfloat16* dst;
+        if (head < rope.nq) {
+          dst = rope.q_out + ((size_t)tok * rope.nq + head) * rope.hd;
+        } else {
+          int slot = rope.slot_mapping ? rope.slot_mapping[tok] : -1;
+          if (slot < 0 || slot / rope.page_size >= rope.num_pages) continue;     // not written (padding row, borrowed cache)
+          const bool is_k = head < rope.nq + rope.nkv;
+          const int kvh = is_k ? head - rope.nq : head - rope.nq - rope.nkv;
+          dst = (is_k ? rope.k_cache : rope.v_cache) +
+                (((size_t)(slot / rope.page_size) * rope.nkv + kvh) * rope.page_size + slot % rope.page_size) * rope.hd;
+        }
+        if (rope.table != nullptr && head < rope.nq + rope.nkv) {
+          int pos = rope.positions[tok];
+          pos = pos < 0 ? 0 : (pos >= rope.max_pos ? rope.max_pos - 1 : pos);
+          const float* cs = rope.table + (size_t)pos * rope.hd;        // cos[half] then sin[half]
+          const float c = cs[j0 + i], sn = cs[half + j0 + i];
+          const float a = lo * c - hi * sn, b = hi * c + lo * sn;
+          lo = a;
+          hi = b;
+        }
+        dst[j0 + i] = __float2bfloat16_rn(lo);
+        dst[j0 + half + i] = __float2bfloat16_rn(hi);
+      }
+      return;
+    }
+    if constexpr (EPI == WS_EPI_GATED) {
+      for (int idx = tid; idx < 8 * 8 * NT; idx += WS_WARPS * 32) {
+        const int i = idx % 8, tok = idx / 8, q = m0 + i;
+        if (tok >= M || q >= m1) continue;
+        float gate = 0.f, up = 0.f;
+#pragma unroll
+        for (int w = 0; w < WS_WARPS; ++w) { gate += red[w][i][tok]; up += red[w][i + 8][tok]; }
+        if constexpr (SCALED) {
+          gate *= row_scale[tok];
+          up *= row_scale[tok];
+        }
+        if (bias) {
+          gate += bias[q / 8 * 16 + q % 8];
+          up += bias[q / 8 * 16 + q % 8 + 8];
+        }
+        out[(size_t)tok * units + q] = from_f32<OUT>((act == WS_GATE_GELU ? gelu_tanh_f32(gate) : gate * sigmoid_f32(gate)) * up);
+      }
+      continue;
+    }
+    if constexpr (SLICED) {              // the slices' sums in the first CTA, added there in the slices' order
+      cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+      for (int idx = tid; idx < 16 * 8 * NT; idx += WS_WARPS * 32) {
+        const int row = idx % 16, tok = idx / 16;
+        float v = 0.f;
+#pragma unroll
+        for (int w = 0; w < WS_WARPS; ++w) v += red[w][row][tok];
+        cl.map_shared_rank(&slice_sum[0][0], 0)[slice * (16 * 8 * NT) + idx] = v;
+      }
+      cl.sync();
+      if (slice != 0) return;
+    }
+#pragma unroll
+    for (int o = 0; o < OUTS; ++o) {
+      const int idx = tid + o * WS_WARPS * 32;
+      if (idx >= 16 * 8 * NT) break;                      // (whole warps: 16 * 8 * NT is a multiple of 32)
+      const int row = idx % 16, tok = idx / 16;           // consecutive threads -> consecutive rows of one token
+      const int n = m0 + row;
+      if (tok >= M || n >= m1) continue;
+      float v = 0.f;
+      if constexpr (SLICED) {
+        for (int w = 0; w < slices; ++w) v += slice_sum[w][idx];
+      } else {
+#pragma unroll
+        for (int w = 0; w < WS_WARPS; ++w) v += red[w][row][tok];
+      }
+      if constexpr (SCALED) v *= row_scale[tok];
+      if (bias) v += bias[n];
+      if constexpr (EPI == WS_EPI_RESID) {
         const float r = residual[(size_t)tok * N + n] + v;
         residual[(size_t)tok * N + n] = r;
         if (norm.xg_out != nullptr) {
           norm.xg_out[(size_t)tok * N + n] = __float2bfloat16_rn(r * norm.gain[n]);
-          sq = r * r;
+          squares[o] = fmaf(r, r, squares[o]);
         }
+      } else {
+        if (act == SLLM_ACT_RELU2) v = relu2_f32(v);
+        else if (act == SLLM_ACT_GELU) v = gelu_f32(v);
+        else if (act == SLLM_ACT_TOKEN) v = gelu_tanh_f32(v) * __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(token.table)[token_row(token, tok) + n]);
+        out[(size_t)tok * N + n] = from_f32<OUT>(v);
       }
-      if (norm.ssq_out != nullptr) {                    // the 16 rows of a token lie in 16 consecutive lanes
+    }
+  }
+  if constexpr (EPI == WS_EPI_RESID) {
+    if (norm.ssq_out != nullptr) {
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-        if (row == 0 && tok < M) norm.ssq_out[(size_t)tok * ((gridDim.x + 3) & ~3) + blockIdx.x] = sq;
+      for (int o = 0; o < OUTS; ++o) {                    // the 16 rows of a token lie in 16 consecutive lanes
+        const int idx = tid + o * WS_WARPS * 32;
+        if (idx >= 16 * 8 * NT) break;
+        float sq = squares[o];
+#pragma unroll
+        for (int w = 8; w > 0; w >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, w);
+        if (idx % 16 == 0 && idx / 16 < M) norm.ssq_out[(size_t)(idx / 16) * ((ctas + 3) & ~3) + cta] = sq;
       }
-    } else if (valid) {
-      if (act == SLLM_ACT_RELU2) v = relu2_f32(v);
-      else if (act == SLLM_ACT_GELU) v = gelu_f32(v);
-      else if (act == SLLM_ACT_TOKEN) v = gelu_tanh_f32(v) * __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(token.table)[token_row(token, tok) + n]);
-      out[(size_t)tok * N + n] = from_f32<OUT>(v);
     }
   }
 }
 
-// CTAs of 16 rows, or more of fewer rows where those would fill the SMs unevenly (two CTAs share an SM).  Between one
-// and two CTAs an SM: the next multiple of the SM count (N = 3584: 296 CTAs of 12 or 13 rows for 224 of 16).  Beyond two
-// an SM the fixed cost of more CTAs outweighs an uneven last wave unless the rows are long (measured at 8 tokens,
-// N = 5120: K = 5120 13.5 us with 320 CTAs, 14.5 with 592; K = 27648 61.4 against 50.4).
-static int ws_ctas(int N, int K, bool rope) {
+// CTAs (of rows) of 16 units, or more of fewer where those would fill the SMs unevenly (two CTAs share an SM): between one
+// and two CTAs an SM the next multiple of the SM count (N = 3584: 296 CTAs of 12 or 13 rows for 224 of 16).  Beyond two an SM and up to 8,192
+// rows a group a CTA, in full groups (N = 5120, 8 tokens, K = 5120: 13.5 us with 320 CTAs, 14.5 with 592, 14.4 with 296 of two groups of 8 or 9 rows)
+// unless the rows are long (K = 27648: 50.4 us with 592 against 61.4).  More rows: two CTAs an SM that walk theirs in groups, the next
+// group's first blocks in flight under this one's last and its sums, where a CTA a group paid a ramp and a tail each.
+// (8 tokens, us, this / the 128-row form of linear_stream.cu; floor at 6.65 TB/s: 11,264 x 2,048 10.9 / 17.8 / 6.9, 16,512 x 4,096 24.7 / 36.3 / 20.3,
+// 22,016 x 4,096 31.3 / 39.8 / 27.1, 152,064 x 3,584 168 / 188 / 164.)
+constexpr int WS_ONE_GROUP_ROWS = 8192;
+static int ws_ctas(int units, int per, int K, bool rope) {
   const int num_sms = sllm::num_sms();
-  int ctas = (N + 15) / 16;
+  const int ctas = (units + per - 1) / per;
   if (rope || ctas <= num_sms) return ctas;
-  int even = ctas;
-  if (ctas < 2 * num_sms) even = (ctas + num_sms - 1) / num_sms * num_sms;
-  else if (K > 8192) even = (ctas + 2 * num_sms - 1) / (2 * num_sms) * (2 * num_sms);
-  return even <= N ? even : ctas;
+  if (ctas < 2 * num_sms) return 2 * num_sms <= units ? 2 * num_sms : ctas;
+  if (ctas * 16 > WS_ONE_GROUP_ROWS) return 2 * num_sms;
+  const int even = K > 8192 ? (ctas + 2 * num_sms - 1) / (2 * num_sms) * (2 * num_sms) : ctas;
+  return even <= units ? even : ctas;
+}
+// Slices of K by the CTAs of a cluster: where the rows give less than one CTA an SM, as many (1, 2, 4) as two an SM hold, none shorter than 16 k blocks
+// (8 tokens, residual epilogue, us: 896 x 4,864 4.2 in 4 slices, 5.8 in one; 2,048 x 5,632 7.0 in 2, 8.3 in one; 2,048 x 11,264 10.8 and 12.7).
+static int ws_slices(int ctas, int K) {
+  int s = 1;
+  while (s < WS_SLICES && ctas * s * 2 <= 2 * sllm::num_sms() && K / 32 / (s * 2) >= 16) s *= 2;
+  return s;
 }
 
 template <int NT, int EPI, typename OUT>
 static int launch_ws(const __nv_bfloat16* x, const __nv_bfloat16* W, const float* bias, void* out, float* residual,
                      int M, int N, int K, cudaStream_t stream, const WsRope& rope = WsRope{}, const WsNorm& norm = WsNorm{},
                      int act = SLLM_ACT_NONE, const TokenTable& token = TokenTable{}) {
-  const int ctas = ws_ctas(N, K, EPI == WS_EPI_ROPE);
-  if (norm.ssq_in != nullptr)
-    launch_kernel(linear_ws_kernel<NT, EPI, OUT, true>, ctas, WS_WARPS * 32, 0, stream, x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token);
-  else
-    launch_kernel(linear_ws_kernel<NT, EPI, OUT, false>, ctas, WS_WARPS * 32, 0, stream, x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token);
+  const int ctas = EPI == WS_EPI_GATED ? ws_ctas(N / 2, 8, K, false) : ws_ctas(N, 16, K, EPI == WS_EPI_ROPE);
+  // (rows beyond a group a CTA: only the forms that are asked for them)
+  const bool walk = EPI != WS_EPI_ROPE && (long long)ctas * (EPI == WS_EPI_GATED ? 8 : 16) < (EPI == WS_EPI_GATED ? N / 2 : N);
+  if (norm.ssq_in != nullptr) {
+    if constexpr (EPI != WS_EPI_ROPE) {
+      if (walk) {
+        launch_kernel(linear_ws_kernel<NT, EPI, OUT, true, WS_WALK>, ctas, WS_WARPS * 32, 0, stream, x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token, 1);
+        return launch_status("linear_ws");
+      }
+    }
+    launch_kernel(linear_ws_kernel<NT, EPI, OUT, true, WS_ONE>, ctas, WS_WARPS * 32, 0, stream, x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token, 1);
+    return launch_status("linear_ws");
+  }
+  if constexpr (EPI != WS_EPI_ROPE) {
+    if (walk) {
+      launch_kernel(linear_ws_kernel<NT, EPI, OUT, false, WS_WALK>, ctas, WS_WARPS * 32, 0, stream, x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token, 1);
+      return launch_status("linear_ws");
+    }
+  }
+  if constexpr (EPI <= WS_EPI_RESID) {
+    const int slices = ws_slices(ctas, K);
+    if (slices > 1) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(ctas * slices);
+      cfg.blockDim = dim3(WS_WARPS * 32);
+      cfg.stream = stream;
+      cudaLaunchAttribute attr[2];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = slices;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[1].val.programmaticStreamSerializationAllowed = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = pdl_enabled() ? 2 : 1;
+      cudaLaunchKernelEx(&cfg, linear_ws_kernel<NT, EPI, OUT, false, WS_SLICED>, x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token, slices);
+      return launch_status("linear_ws");
+    }
+  }
+  launch_kernel(linear_ws_kernel<NT, EPI, OUT, false, WS_ONE>, ctas, WS_WARPS * 32, 0, stream, x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token, 1);
   return launch_status("linear_ws");
 }
 
@@ -323,7 +472,7 @@ SLLM_EXPORT int sllm_linear_ws_supports(int M, int N, int K) {
 
 // CTAs a launch for N output columns over a reduction of K uses: the rows of the table of partial sums of squares
 // that the residual epilogue writes when it is asked for the next norm's input (see WsNorm).
-SLLM_EXPORT int sllm_linear_ws_parts(int N, int K) { return ws_ctas(N, K, false); }
+SLLM_EXPORT int sllm_linear_ws_parts(int N, int K) { return ws_ctas(N, 16, K, false); }
 
 static bool ws_norm_in(WsNorm& n, const float* ssq_in, int parts_in, float eps_in, int width_in, int M) {
   if (ssq_in == nullptr) return true;
@@ -369,6 +518,21 @@ SLLM_EXPORT int sllm_linear_ws(const void* x, const void* W, const float* bias, 
   if (M <= 16) { GO(2) }
   GO(4)
 #undef GO
+}
+
+// out[M, N/2] = act(gate) * up (bfloat16) of the gate|up matrix W [N, K] whose rows (and biases) alternate in blocks of 8; gelu: the tanh form of GELU
+// in place of SiLU.  ssq_in: as for sllm_linear_ws.
+SLLM_EXPORT int sllm_linear_ws_gated(const void* x, const void* W, const float* bias, void* out, int gelu, int M, int N, int K,
+                                     const float* ssq_in, int parts_in, float eps_in, int width_in, cudaStream_t stream) {
+  SLLM_REQUIRE(sllm_linear_ws_supports(M, N, K) && M <= 16 && N % 16 == 0, "linear_ws_gated: sizes M=%d N=%d K=%d (needs M<=16, N%%16==0, K%%32==0)", M, N, K);
+  SLLM_REQUIRE(((uintptr_t)x & 15) == 0 && ((uintptr_t)W & 15) == 0 && out != nullptr, "linear_ws_gated: operands must be 16-byte aligned");
+  WsNorm nm;
+  SLLM_REQUIRE(ws_norm_in(nm, ssq_in, parts_in, eps_in, width_in, M), "linear_ws_gated: a table of %d partial sums (at most %d) over width %d",
+               parts_in, ws_ssq_max(M <= 16 ? 2 : 4), width_in);
+  const __nv_bfloat16 *xb = (const __nv_bfloat16*)x, *wb = (const __nv_bfloat16*)W;
+  const int act = gelu ? WS_GATE_GELU : WS_GATE_SILU;
+  if (M <= 8) return launch_ws<1, WS_EPI_GATED, __nv_bfloat16>(xb, wb, bias, out, nullptr, M, N, K, stream, WsRope{}, nm, act);
+  return launch_ws<2, WS_EPI_GATED, __nv_bfloat16>(xb, wb, bias, out, nullptr, M, N, K, stream, WsRope{}, nm, act);
 }
 
 SLLM_EXPORT int sllm_linear_ws_rope_supports(int M, int N, int K, int nq, int nkv, int hd, int rot) {

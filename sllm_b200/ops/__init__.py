@@ -197,6 +197,8 @@ def linear_act_mul(x, w_gate_up, bias, interleave: int, out_dtype, act: str) -> 
             and w_gate_up.shape[0] % 16 == 0 and _GATED_FUSED):
         M, K = x.shape
         N = w_gate_up.shape[0]
+        if ws_gated_supports(M, N, K):
+            return linear_ws_gated(x, w_gate_up, bias, act)
         if stream_supports(M, N, K):
             return linear_stream(x, w_gate_up, bias, out_dtype, act=act)
         if M > TCGEN05_MIN_ROWS and _PAIR_GEMM != "off" and pair_supports(M, N, K):
@@ -1364,7 +1366,23 @@ def linear_tc(x, w, bias, out_dtype, *, splits: int = 1, silu: bool = False, act
     return out
 
 
-WS_MAX_COLS = 8192        # wider products have CTAs enough for the 128-row streaming kernel
+WS_MAX_COLS = 8192        # wider products: see `_ws_wide`
+WS_WIDE_MIN_K = 2048
+WS_WIDE_MAX_FILL = 0.95   # up to 8 tokens
+WS_WIDE_MAX_FILL_ROWS16 = 0.7
+
+
+def _ws_wide(M: int, N: int, K: int) -> bool:
+    """Whether the warp-split kernel, two CTAs an SM that walk their rows, beats the 128-row streaming kernel on a product of more than
+    `WS_MAX_COLS` columns: unless the latter's CTAs fill its places (two an SM) in whole waves, and where a group of rows is long enough to be
+    worth its sums.  (Fill of the last wave and all, 8 tokens, us, this / the other: 0.30 10.9 / 17.8, 0.58 31.3 / 39.8, 0.73 93.8 / 104.5, 0.80 168 / 188,
+    0.84 43.9 / 46.6 and 24.7 / 24.2, 1.0 46.1 / 45.1; K = 896: 8.0 / 8.0 at a fill of 0.26 and 73 / 48 at 0.80.  16 tokens: 0.30 12.6 / 18.3, 0.58 35.2 / 45.4,
+    0.84 50.6 / 48.8 and 29.3 / 25.5, 1.0 53.1 / 46.4.)"""
+    places, ctas = 2 * num_sms(), -(-N // 128)
+    fill = ctas / (-(-ctas // places) * places)
+    return K >= WS_WIDE_MIN_K and M <= 16 and fill < (WS_WIDE_MAX_FILL if M <= 8 else WS_WIDE_MAX_FILL_ROWS16)
+
+
 WS_MAX_ROWS = 32          # one, two or four 8-token tiles (with fewer k blocks in flight the more tiles, so that two CTAs still share an SM)
 # Four tiles (17..32 tokens, one k block in flight per group) stream slowly, so only where little streams and the
 # fused epilogues save kernels: a short reduction, a matrix of at most 2^24 elements, and rows enough for one and a
@@ -1380,7 +1398,9 @@ def ws_supports(M: int, N: int, K: int) -> bool:
     """Whether the warp-split kernel is the one for this product.  With two token tiles (9..16 tokens) only where
     its 16-row CTAs fit the GPU at once: at N = 5120 (320 to 592 CTAs for 296 places) it falls behind the k-split
     kernel by more than the fused epilogues save (16 tokens, K = 27648: 64.3 against 49.2 us)."""
-    return N <= WS_MAX_COLS and ws_takes(M, N, K) and _ws_tokens_ok(M, N, K)
+    if N > WS_MAX_COLS:
+        return ws_takes(M, N, K) and _ws_wide(M, N, K)
+    return ws_takes(M, N, K) and _ws_tokens_ok(M, N, K)
 
 
 @functools.lru_cache(maxsize=4096)
@@ -1395,6 +1415,12 @@ def _ws_tokens_ok(M: int, N: int, K: int) -> bool:
     if -(-N // 16) > 2 * num_sms():
         return False
     return M <= 16 or (N * K <= WS_ROWS32_MAX_ELEMENTS and K <= WS_ROWS32_MAX_K and 2 * -(-N // 16) >= 3 * num_sms())
+
+
+@functools.lru_cache(maxsize=4096)
+def ws_gated_supports(M: int, N: int, K: int) -> bool:
+    """Whether the warp-split kernel is the one for a gate|up product with its activation."""
+    return M <= 16 and N % 16 == 0 and N > WS_MAX_COLS and ws_takes(M, N, K) and _ws_wide(M, N, K)
 
 
 class RowScale:
@@ -1416,6 +1442,19 @@ class RowScale:
 
 _NO_SCALE = (None, 0, 0.0, 0)
 MAX_SCALE_PARTS = 608          # partial sums a consumer keeps in shared memory per row
+
+
+def linear_ws_gated(x, w, bias, act: str, scale: RowScale | None = None):
+    """The warp-split streaming kernel (at most 16 tokens) with the gated epilogue: bfloat16 ``act(gate) * up`` of the gate|up matrix ``w`` whose
+    rows (and ``bias``) alternate in blocks of 8; ``act`` is ``silu`` or ``gelu_tanh``.  ``scale``: a norm still owed on ``x`` (`RowScale`)."""
+    _chk(x, w, bias, scale.ssq if scale is not None else None)
+    M, K = x.shape
+    N = w.shape[0]
+    if w.shape[1] != K:
+        raise KernelError(f"linear: x {tuple(x.shape)} does not fit w {tuple(w.shape)}")
+    out = torch.empty((M, N // 2), dtype=torch.bfloat16, device=x.device)
+    call("sllm_linear_ws_gated", _p(x), _p(w), _p(bias), _p(out), ACTIVATIONS[act], M, N, K, *(scale.args() if scale is not None else _NO_SCALE), _stream())
+    return out
 
 
 def linear_ws(x, w, bias, out_dtype, residual=None, scale: RowScale | None = None, next_gain=None, act: "str | None" = None,
@@ -1632,12 +1671,16 @@ def linear_silu_mul(x: torch.Tensor, w_gate_up: torch.Tensor, interleave: int, o
         N = w_gate_up.shape[0]
         if M > 32:
             return gemm_pair(x, w_gate_up, None, out_dtype, silu=True, scale=scale)
+        if ws_gated_supports(M, N, K):
+            return linear_ws_gated(x, w_gate_up, None, "silu", scale=scale)
         out = torch.empty((M, N // 2), dtype=torch.bfloat16, device=x.device)
         call("sllm_linear_stream_silu_scaled", _p(x), _p(w_gate_up), _p(out), M, N, K, *scale.args(), _stream())
         return out
     if x.dtype == torch.bfloat16 and out_dtype == torch.bfloat16 and interleave == 8 and x.is_cuda:
         M, K = x.shape
         N = w_gate_up.shape[0]
+        if ws_gated_supports(M, N, K):
+            return linear_ws_gated(x, w_gate_up, None, "silu")
         if stream_supports(M, N, K):
             return linear_stream(x, w_gate_up, None, out_dtype, silu=True)
         if PAIR_SILU_FROM_ROWS <= M <= TCGEN05_MIN_ROWS and N % 16 == 0 and _PAIR_GEMM != "off" and pair_supports(M, N, K):

@@ -1,0 +1,54 @@
+"""The weight-streaming product's other forms: CTAs that walk more than one group of rows (matrices of many rows), clusters that share the columns
+(matrices of few), and the gate|up product with its activation, at row counts and reductions that leave remainders of both.  The bounds: K float32
+additions of exact products, 2^-24 of the sum of their magnitudes each; for the activation also 2^-8 of the result, its bfloat16 rounding."""
+
+import pytest
+import torch
+
+from tests.conftest import cuda_or_skip
+
+pytestmark = pytest.mark.gpu
+
+
+def _product(dev, M, N, K):
+    g = torch.Generator(device=dev).manual_seed(M + N + K)
+    x = torch.randn(M, K, device=dev, generator=g).bfloat16()
+    w = (torch.randn(N, K, device=dev, generator=g) / K ** 0.5).bfloat16()
+    b = torch.randn(N, device=dev, generator=g)
+    y = x.double() @ w.double().T + b
+    bound = (K + 1) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T + b.abs())
+    return g, x, w, b, y, bound
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("N,K", [(24, 2080), (200, 4128), (1000, 4160), (2048, 1056), (5000, 64), (9480, 96), (10001, 320), (33000, 32)])
+def test_rows_and_columns_in_parts(M, N, K):
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    g, x, w, b, y, bound = _product(dev, M, N, K)
+    got = ops.linear_ws(x, w, b, torch.float32)
+    assert bool(((got - y).abs() <= bound).all())
+    stream = torch.randn(M, N, device=dev, generator=g)
+    added = stream.clone()
+    ops.linear_ws(x, w, b, torch.float32, residual=added)
+    assert bool(((added - (stream + y)).abs() <= bound + 2.0 ** -23 * (stream.abs() + y.abs())).all())
+    assert torch.equal(ops.linear_ws(x[M - 1:].contiguous(), w, b, torch.float32)[0], got[M - 1])
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("N,K", [(16, 32), (4736, 96), (4752, 320), (8208, 1056), (11264, 2048), (22016, 64)])
+@pytest.mark.parametrize("act", ["silu", "gelu_tanh"])
+def test_gate_and_up_with_their_activation(M, N, K, act):
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    _, x, w, b, y, bound = _product(dev, M, N, K)
+    gate, up = y.reshape(M, N // 16, 2, 8).unbind(2)
+    gate_off, up_off = bound.reshape(M, N // 16, 2, 8).unbind(2)
+    fn = torch.nn.functional.silu if act == "silu" else lambda v: torch.nn.functional.gelu(v, approximate="tanh")
+    want = fn(gate) * up
+    # both activations rise by at most 1.13 a unit; the float32 activation itself is good to 1e-5 of its argument
+    off = 2.0 ** -8 * want.abs() + 1.2 * (gate_off * up.abs() + up_off * gate.abs()) + 1e-5 * gate.abs() * up.abs() + 1e-30
+    got = ops.linear_ws_gated(x, w, b, act).reshape(M, N // 16, 8)
+    assert bool(((got - want).abs() <= off).all())
+    one = ops.linear_ws_gated(x[M - 1:].contiguous(), w, b, act).reshape(N // 16, 8)
+    assert torch.equal(one, got[M - 1])
