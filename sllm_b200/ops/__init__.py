@@ -267,6 +267,43 @@ def delta_out(o, gain, proj, off_g: int, eps: float, heads: int, dv: int, out_dt
     return out
 
 
+@functools.lru_cache(maxsize=4096)
+def _token_heads_fit(dk: int, dv: int) -> bool:
+    return bool(lib().sllm_recurrence_token_supports(int(dk), int(dv)))
+
+
+def recurrence_token_supports(proj, step, dk: int, dv: int) -> bool:
+    """Whether `recurrence_token` takes this step: every request brings one token, and the heads fit the kernel's registers."""
+    return proj.is_cuda and proj.shape[0] == step.num_seqs and _token_heads_fit(dk, dv)
+
+
+TOKEN_MODES = {"general_delta": 0, "gated_delta": 1, "gated": 2, "fixed": 3, "forget_gate": 4}
+
+
+def recurrence_token(kind: str, proj, offs, state, step, heads: int, dk: int, dv: int, out_dtype, *, decay=None, a=None, bias=None, gates=None,
+                     off_b: int = 0, off_dt: int = 0, key_heads: "int | None" = None, q_scale: float = 1.0, tau: float = 1.0, norm=None, out=None,
+                     out_off: int = 0) -> torch.Tensor:
+    """One token of every request through a recurrence (``general_delta``: `delta_rule`, with ``decay`` and ``a`` its bias; ``gated_delta``:
+    `gated_delta_rule`, ``a`` its a_log, ``bias`` its dt_bias; ``gated``: `gated_linear_attention`, ``decay`` its z; ``fixed``:
+    `decay_linear_attention`, ``a`` its decays; ``forget_gate``: `forget_gate_attention`, ``a`` its lower bounds, ``bias`` its bias) and, with
+    ``norm`` = (gain or None, eps, gate product or None, its column, gate activation), `delta_out` of the heads, in one kernel.  ``[S, heads*dv]`` in
+    ``out_dtype``, or columns ``out_off ..`` of ``out``."""
+    gain, eps, gate, off_g, act = norm if norm is not None else (None, 0.0, None, 0, "none")
+    _chk(proj, state, decay, a, bias, gates, gain, gate, out)
+    if any(t is not None and t.dtype != torch.float32 for t in (proj, state, decay, a, bias, gates, gain, gate)):
+        raise KernelError("recurrence_token: everything that enters the recurrence is float32")
+    S, ld = proj.shape
+    if tuple(state.shape[1:]) != (heads, dk, dv) or (decay is not None and tuple(decay.shape) != (S, heads * dk)):
+        raise KernelError(f"recurrence_token: state {tuple(state.shape)} or decay does not fit {heads} heads of {dk}x{dv}")
+    if out is None:
+        out = torch.empty((S, heads * dv), dtype=out_dtype, device=proj.device)
+    call("sllm_recurrence_token", TOKEN_MODES[kind], _p(proj), ld, *(int(o) for o in (tuple(offs) + (0,))[:4]), _p(decay), _p(a), _p(bias), _p(gates),
+         gates.shape[1] if gates is not None else 0, int(off_b), int(off_dt), int(key_heads or heads), float(q_scale), 1.0 / float(tau), _p(state),
+         _p(step.state_slots), S, heads, dk, dv, 1 if norm is not None else 0, GATE_ACTS[act], _p(gain), _p(gate),
+         gate.shape[1] if gate is not None else 0, int(off_g), float(eps), _p(out), _dtc(out.dtype), out.shape[1], int(out_off), _stream())
+    return out
+
+
 def forget_gate_attention(proj, offs, f_bias, lower, state, step, heads: int, dk: int, dv: int) -> torch.Tensor:
     """S <- diag(f) S + (1 - f) v^T; o = S^T silu(q) with f = lower + (1 - lower) sigmoid(z + f_bias) per key channel, over the
     step's tokens from and into ``state`` (float32 ``[slots, heads, dk, dv]``).  ``proj`` float32 ``[T, ld]`` holds q, the
@@ -611,6 +648,8 @@ def decay_linear_attention(proj, offs, decay, state, step, heads: int, dk: int, 
         raise KernelError("decay_linear_attention: everything that enters the recurrence is float32")
     if tuple(decay.shape) != (heads,) or tuple(state.shape[1:]) != (heads, dk, dv):
         raise KernelError(f"decay_linear_attention: decay {tuple(decay.shape)} or state {tuple(state.shape)} does not fit {heads} heads of {dk}x{dv}")
+    if recurrence_token_supports(proj, step, dk, dv):
+        return recurrence_token("fixed", proj, offs, state, step, heads, dk, dv, torch.float32, a=decay)
     out = torch.empty((T, heads * dv), dtype=torch.float32, device=proj.device)
     off_q, off_k, off_v = (int(o) for o in offs)
     longest, rest = _gated_chunks(3, proj, offs, None, decay, None, 1.0, 1.0, state, step, heads, dk, dv, out)

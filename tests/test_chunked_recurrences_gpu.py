@@ -172,3 +172,72 @@ def test_delta_rule_in_chunks(d, H, hard):
         keep = torch.exp(-np.exp(-0.5) * torch.sigmoid(decay[a:b].double())).reshape(b - a, H, d)
         return r, k, v, keep, u, torch.sigmoid(z + bias.double().reshape(H, d)) * u
     _check(lambda state, step: ops.delta_rule(proj, (0, C, 2 * C, 3 * C), decay, bias, state, step, H, d, d), terms, H, d, d, dev, g)
+
+
+# ---- single tokens ------------------------------------------------------------------------------------------------------
+
+TOKEN_SIZES = [(64, 64, 3), (128, 128, 2), (128, 64, 2), (64, 128, 2), (40, 24, 3), (72, 100, 2), (17, 4, 2)]
+
+
+@pytest.mark.parametrize("dk,dv,H", TOKEN_SIZES)
+@pytest.mark.parametrize("kind", ["general_delta", "gated_delta", "gated", "fixed", "forget_gate"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_one_token_of_every_request(kind, dk, dv, H, dtype):
+    """Against float64: a sum of at most 128 products beside the state; 2e-6 of the state's size, and the output's rounding."""
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    g = torch.Generator(device=dev).manual_seed(dk + dv + H)
+    slots = [4, 0, 7, 2, 9]
+    S, G = len(slots), H if kind != "gated_delta" or H % 2 else H // 2
+    rand = lambda *shape: torch.randn(*shape, device=dev, generator=g)  # noqa: E731
+    K, V = G * dk, H * dv
+    proj, state = rand(S, 5 + 2 * K + V + H * dk + 3), rand(10, H, dk, dv)
+    offs = (5, 5 + K, 5 + 2 * K, 5 + 2 * K + V)
+    decay, bias, a, gain, gate, gates = rand(S, H * dk), rand(H * dk), rand(H * dk), rand(V), rand(S, V + 2), rand(S, 2 * H + 1)
+    q, k, v, z = (proj[:, o:o + n].double().reshape(S, h, -1) for o, n, h in zip(offs, (K, K, V, H * dk), (G, G, H, H)))
+    kw, p, w, silu = {}, None, None, torch.nn.functional.silu
+    unit = lambda x: x / (x.pow(2).sum(-1, keepdim=True) + 1e-6).sqrt()  # noqa: E731
+    if kind == "general_delta":
+        keep = torch.exp(-np.exp(-0.5) * torch.sigmoid(decay.double())).reshape(S, H, dk)
+        p, w = unit(k), torch.sigmoid(z + a.double().reshape(H, dk)) * unit(k)
+        kw = {"decay": decay, "a": a}
+    elif kind == "gated_delta":
+        a, bias = a[:H].contiguous(), bias[:H].contiguous()
+        q, k = (unit(x).repeat_interleave(H // G, 1) for x in (q, k))
+        q, beta = q * 0.3, torch.sigmoid(gates[:, :H].double())[:, :, None]
+        keep = torch.exp(-torch.exp(a.double()) * torch.nn.functional.softplus(gates[:, H + 1:].double() + bias.double()))[:, :, None]
+        p, w, v = k, beta * keep * k, beta * v
+        kw = {"a": a, "bias": bias, "gates": gates, "off_b": 0, "off_dt": H + 1, "key_heads": G, "q_scale": 0.3}
+    elif kind == "gated":
+        q, keep = q * 0.3, (torch.nn.functional.logsigmoid(decay.double()) / 8).exp().reshape(S, H, dk)
+        kw = {"decay": decay, "q_scale": 0.3, "tau": 8.0}
+    elif kind == "fixed":
+        a = torch.rand(H, device=dev, generator=g)
+        q, k, v, keep = silu(q), silu(k), silu(v), a.double()[None, :, None]
+        kw = {"a": a}
+    else:
+        a = torch.rand(H * dk, device=dev, generator=g)
+        keep = (a.double() + (1 - a.double()) * torch.sigmoid(k.reshape(S, -1) + bias.double())).reshape(S, H, dk)
+        q, k = silu(q), 1 - keep
+        kw = {"a": a, "bias": bias}
+    before = state.clone()
+    old = state[slots].double()
+    gone = w[..., None] * torch.einsum("shi,shij->shj", p, old)[:, :, None] if p is not None else 0.0
+    new = old * keep[..., None] - gone + k[..., None] * v[:, :, None]
+    o = torch.einsum("shij,shi->shj", new, q)
+    step = _step(dev, [1] * S, slots)
+    raw = ops.recurrence_token(kind, proj, offs, state, step, H, dk, dv, torch.float32, **kw)
+    assert torch.equal(state[[1, 3, 5, 6, 8]], before[[1, 3, 5, 6, 8]])
+    size = float(new.abs().max())
+    torch.testing.assert_close(state[slots].double(), new, rtol=0, atol=2e-6 * size)
+    torch.testing.assert_close(raw.double().reshape(S, H, dv), o, rtol=2e-5, atol=2e-5 * float(o.abs().max()))
+    for act, f in (("sigmoid", torch.sigmoid), ("silu", silu), ("none", None)):
+        state.copy_(before)
+        wide = torch.zeros(S, V + 7, device=dev, dtype=dtype)
+        ops.recurrence_token(kind, proj, offs, state, step, H, dk, dv, dtype, norm=(gain, 1e-5, None if f is None else gate, 2, act), out=wide,
+                             out_off=3, **kw)
+        want = (o / (o.pow(2).mean(-1, keepdim=True) + 1e-5).sqrt()).reshape(S, V) * gain.double()
+        want = want if f is None else want * f(gate[:, 2:].double())
+        tol = 1e-4 if dtype == torch.float32 else 1e-2
+        torch.testing.assert_close(wide[:, 3:3 + V].double(), want, rtol=tol, atol=tol)
+        assert not wide[:, :3].any() and not wide[:, 3 + V:].any()
