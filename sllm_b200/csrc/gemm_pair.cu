@@ -95,11 +95,18 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
                ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
 }
 
+// A grouped product: the rows of A are sorted by group and padded so that a tile's 256 rows are one group's; row tile i belongs to group
+// tile_group[i] (device memory; -1: nobody's, no work), whose share of W starts w_rows rows and w_cols columns times the group's number into it.
+struct TpGroups {
+  const int* tile_group = nullptr;
+  int w_rows = 0, w_cols = 0;
+};
+
 template <int EPI, int BN>
 __global__ void __launch_bounds__(192, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                  const float* __restrict__ bias, void* __restrict__ out, int M, int N, int K, int* __restrict__ status,
-                 const TgExtra extra, const int ksplits, const int kb_per_split) {
+                 const TgExtra extra, const int ksplits, const int kb_per_split, const TpGroups groups) {
   extern __shared__ unsigned char tp_smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tp_smem_raw) + 1023) & ~(uintptr_t)1023);
   using C = TpCfg<BN>;
@@ -152,8 +159,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       bool gave_up = false;
       for (int unit = pair; unit < tiles && !*failed; unit += pairs) {
         const int tile = unit / ksplits, kb0 = (unit % ksplits) * kb_per_split, kb1 = min(k_blocks_all, kb0 + kb_per_split);
+        const int group = groups.tile_group != nullptr ? groups.tile_group[tile % m_tiles] : 0;
+        if (group < 0) continue;                    // (so do the MMA thread and the epilogue)
         const int m0 = (tile % m_tiles) * 2 * TP_BM + (int)rank * TP_BM;
-        const int n0 = (tile / m_tiles) * TP_BN + (int)rank * (TP_BN / 2);
+        const int n0 = (tile / m_tiles) * TP_BN + (int)rank * (TP_BN / 2) + group * groups.w_rows;
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % TP_STAGES, round = it / TP_STAGES;
           if (!mbar_wait(&empty[s], (round & 1) ^ 1) || *failed) {
@@ -165,7 +174,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           const uint32_t bar = map_to_cta(smem_u32(&full[s]), 0);
           if (rank == 0) mbar_expect_tx(&full[s], 2 * TP_STAGE_BYTES);      // both CTAs' boxes
           tma_load_2d_pair(sa, &map_a, kb * TP_BK, m0, bar);
-          tma_load_2d_pair(sa + TP_A_BYTES, &map_w, kb * TP_BK, n0, bar);
+          tma_load_2d_pair(sa + TP_A_BYTES, &map_w, kb * TP_BK + group * groups.w_cols, n0, bar);
         }
         if (gave_up) break;
       }
@@ -183,7 +192,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       const uint64_t desc0 = umma_desc(smem_u32(smem));
       int local = 0;
       uint32_t st = 0, ph = 0;                      // the stage to consume next and its barrier's parity
-      for (int unit = pair; unit < tiles && !*failed; unit += pairs, ++local) {
+      for (int unit = pair; unit < tiles && !*failed; unit += pairs) {
+        if (groups.tile_group != nullptr && groups.tile_group[unit / ksplits % m_tiles] < 0) continue;
         const int kb0 = (unit % ksplits) * kb_per_split, k_blocks = min(k_blocks_all, kb0 + kb_per_split) - kb0;
         const int b = local & 1;
         if (!mbar_wait(&acc_empty[b], ((local >> 1) & 1) ^ 1) || *failed) {     // both epilogues have drained this buffer
@@ -209,6 +219,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         }
         if (gave_up) break;
         umma_commit_pair(&acc_full[b]);             // arrives in both CTAs when every product issued so far is done
+        ++local;
       }
     }
   } else {
@@ -216,9 +227,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const int quarter = warp & 3;
     const uint32_t acc_empty_addr[2] = {map_to_cta(smem_u32(&acc_empty[0]), 0), map_to_cta(smem_u32(&acc_empty[1]), 0)};
     int local = 0;
-    for (int unit = pair; unit < tiles; unit += pairs, ++local) {
+    for (int unit = pair; unit < tiles; unit += pairs) {
       const int b = local & 1;
       const int tile = unit / ksplits, split = unit % ksplits;
+      if (groups.tile_group != nullptr && groups.tile_group[tile % m_tiles] < 0) continue;
       const int m0 = (tile % m_tiles) * 2 * TP_BM + (int)rank * TP_BM, n0 = (tile / m_tiles) * TP_BN;
       const int m = m0 + quarter * 32 + lane;
       const float row_scale = tg_row_scale(extra, m, M);        // a norm still owed on the input (1 if none): fetched while the products run
@@ -231,6 +243,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(acc_empty_addr[b]);
+        ++local;
         continue;
       }
 #pragma unroll 1
@@ -266,6 +279,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(acc_empty_addr[b]);
+      ++local;
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -566,7 +580,7 @@ static int launch_tp_wide(const CUtensorMap& ma, const CUtensorMap& mw, const fl
 
 template <int EPI, int BN>
 static int launch_tp(const CUtensorMap& ma, const CUtensorMap& mw, const float* bias, void* out, int M, int N, int K,
-                     int* status, cudaStream_t stream, const TgExtra& extra, int ksplits, int kb_per_split) {
+                     int* status, cudaStream_t stream, const TgExtra& extra, int ksplits, int kb_per_split, const TpGroups& groups = TpGroups{}) {
   auto kernel = gemm_pair_kernel<EPI, BN>;
   constexpr int TP_SMEM = TpCfg<BN>::SMEM, TP_BN = BN;
   static bool configured = false;
@@ -583,7 +597,7 @@ static int launch_tp(const CUtensorMap& ma, const CUtensorMap& mw, const float* 
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[2];
   pair_launch_config(cfg, attr, pairs, 192, TP_SMEM, stream);
-  cudaLaunchKernelEx(&cfg, kernel, ma, mw, bias, out, M, N, K, status, extra, ksplits, kb_per_split);
+  cudaLaunchKernelEx(&cfg, kernel, ma, mw, bias, out, M, N, K, status, extra, ksplits, kb_per_split, groups);
   return launch_status("gemm_pair");
 }
 
@@ -706,4 +720,32 @@ SLLM_EXPORT int sllm_gemm_pair(const void* A, const void* W, const float* bias, 
   }
 #undef GO
   SLLM_REQUIRE(false, "gemm_pair: unknown epilogue %d", epilogue);
+}
+
+// A grouped product (see TpGroups): out [M, N] (epilogue 0 float32, 1 bfloat16, 7 bfloat16 of the exact gelu) or [M, N/2] (2: silu(gate) * up, W's rows
+// interleaved in blocks of 8) of A [M, K], M a multiple of 256, row tile i times the N rows of W [w_total_rows, w_ld] from row tile_group[i] * w_rows
+// and column tile_group[i] * w_cols on; tile_group is device memory of M / 256 ints.  Tiles of group -1 are left as they are.
+SLLM_EXPORT int sllm_gemm_pair_grouped(const void* A, const void* W, void* out, int M, int N, int K, int w_total_rows, int w_ld, int w_rows,
+                                       int w_cols, const int* tile_group, int epilogue, int* status, cudaStream_t stream) {
+  SLLM_REQUIRE(sllm_gemm_pair_supports(M, N, K) && M % (2 * TP_BM) == 0 && K % TP_BK == 0 && w_cols % 8 == 0 && w_ld % 8 == 0 && w_ld >= K && w_total_rows >= N,
+               "gemm_pair_grouped: sizes M=%d N=%d K=%d of [%d, %d] (M a multiple of 256, K of 64)", M, N, K, w_total_rows, w_ld);
+  SLLM_REQUIRE(((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0 && tile_group != nullptr && out != nullptr && status != nullptr,
+               "gemm_pair_grouped: operands must be 16-byte aligned, a table of the row tiles and a status word are required");
+  SLLM_REQUIRE(epilogue != TG_EPI_SILU || N % 16 == 0, "gemm_pair_grouped: the gated epilogue needs N %% 16 == 0");
+  CUtensorMap ma, mw;
+  if (!make_map(&ma, A, M, K, TP_BM, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) || !make_map(&mw, W, w_total_rows, w_ld, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_128B)) {
+    set_error("gemm_pair_grouped: cuTensorMapEncodeTiled failed");
+    return SLLM_ERR_LAUNCH;
+  }
+  TpGroups g;
+  g.tile_group = tile_group; g.w_rows = w_rows; g.w_cols = w_cols;
+  const TgExtra extra;
+  const int kb = K / TP_BK;
+  switch (epilogue) {
+    case TG_EPI_F32: return launch_tp<TG_EPI_F32, 256>(ma, mw, nullptr, out, M, N, K, status, stream, extra, 1, kb, g);
+    case TG_EPI_BF16: return launch_tp<TG_EPI_BF16, 256>(ma, mw, nullptr, out, M, N, K, status, stream, extra, 1, kb, g);
+    case TG_EPI_SILU: return launch_tp<TG_EPI_SILU, 256>(ma, mw, nullptr, out, M, N, K, status, stream, extra, 1, kb, g);
+    case TG_EPI_GELU_ERF: return launch_tp<TG_EPI_GELU_ERF, 256>(ma, mw, nullptr, out, M, N, K, status, stream, extra, 1, kb, g);
+  }
+  SLLM_REQUIRE(false, "gemm_pair_grouped: unknown epilogue %d", epilogue);
 }

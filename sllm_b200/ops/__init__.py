@@ -1327,6 +1327,73 @@ def pair_parts(N: int, form: int = 0) -> int:
     return int(lib().sllm_gemm_pair_parts_of(int(N), int(form)))
 
 
+# ---- a mixture of experts over prompt portions, the tokens sorted by expert --------------------------------------------------
+
+MOE_TILE = 256                # rows of a tile of the grouped product: an expert's tokens are padded to whole ones
+MOE_GROUPED_OVERHEAD_US = 60  # assigning, gathering and adding up, over what the dense form pays for its activation (2,048 tokens, width 2,048)
+MOE_GROUPED_FLOPS_PER_US = 1.2e9
+
+
+def moe_grouped_pays(x, E: int, top: int, ff: int, matrices: int) -> bool:
+    """Whether a mixture of ``E`` experts of ``ff`` channels (``matrices`` of them an expert), ``top`` a token, is faster with the tokens sorted by
+    expert (an expert multiplies its own tokens, padded to tiles of 256 rows: half a tile each on average) than with every expert over every
+    token: where the multiplications saved take longer than the sorting."""
+    if not (x.is_cuda and x.dtype == torch.bfloat16 and x.shape[0] > TCGEN05_MIN_ROWS and _PAIR_GEMM == "all" and E <= 256):
+        return False
+    T, W = x.shape
+    if W % 64 or ff % 64 or not pair_supports(MOE_TILE, ff, W):
+        return False
+    rows_saved = T * E - T * top - E * MOE_TILE // 2
+    return rows_saved * 2.0 * matrices * W * ff > MOE_GROUPED_OVERHEAD_US * MOE_GROUPED_FLOPS_PER_US
+
+
+def moe_assign(idx, E: int):
+    """A row for every (token, choice) of ``idx`` (int32 ``[T, top]``) in a buffer sorted by expert: (places ``[T, top]``, the expert of every tile of 256
+    rows or -1, the token of every row or -1)."""
+    _chk(idx)
+    T, top = idx.shape
+    tiles = T * top // MOE_TILE + E
+    i32 = lambda n: torch.empty(n, dtype=torch.int32, device=idx.device)  # noqa: E731
+    place, tile_expert, row_token = i32((T, top)), i32(tiles), i32(tiles * MOE_TILE)
+    call("sllm_moe_assign", _p(idx), T, top, E, tiles, _p(place), _p(tile_expert), _p(row_token), _stream())
+    return place, tile_expert, row_token
+
+
+def moe_gather(x, row_token) -> torch.Tensor:
+    """``x[row_token]``, rows without a token left as they are."""
+    _chk(x, row_token)
+    out = torch.empty((row_token.numel(), x.shape[1]), dtype=x.dtype, device=x.device)
+    call("sllm_moe_gather", _p(x), _p(row_token), _p(out), row_token.numel(), x.shape[1] * x.element_size(), _stream())
+    return out
+
+
+def gemm_pair_grouped(x, w, tile_expert, N: int, K: int, w_rows: int, w_cols: int, out_dtype, act: "str | None" = None):
+    """`gemm_pair` with the row tiles of ``x`` (``[256 * tiles, K]``) sorted by expert: tile i times the ``N`` rows of ``w`` from row ``w_rows`` and column
+    ``w_cols`` times ``tile_expert[i]`` on.  ``act``: ``gelu`` (exact) or ``silu`` (gate and up rows alternating in blocks of 8), bfloat16."""
+    _chk(x, w, tile_expert)
+    if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or x.shape[0] != MOE_TILE * tile_expert.numel() or x.shape[1] != K:
+        raise KernelError(f"gemm_pair_grouped: x {tuple(x.shape)} does not fit {tile_expert.numel()} tiles of {MOE_TILE} rows and {K} columns, bfloat16")
+    M = x.shape[0]
+    epi = {None: 0 if out_dtype == torch.float32 else 1, "gelu": 7, "silu": 2}[act]
+    out = torch.empty((M, N // 2 if act == "silu" else N), dtype=torch.float32 if epi == 0 else torch.bfloat16, device=x.device)
+    call("sllm_gemm_pair_grouped", _p(x), _p(w), _p(out), M, N, K, w.shape[0], w.shape[1], int(w_rows), int(w_cols), _p(tile_expert), epi,
+         _p(_status_word(x.device)), _stream())
+    _tc_used["since_check"] += 1
+    return out
+
+
+def moe_combine(y, place, wts, shared=None, gate=None, residual=None):
+    """``sum_j wts[t, j] * y[place[t, j]] (+ shared[t], times gate[t, -1] if given)`` (float32 ``[T, W]``), or added into ``residual`` (returns None)."""
+    _chk(y, place, wts, shared, gate, residual)
+    T, top = place.shape
+    W = y.shape[1]
+    out = residual if residual is not None else torch.empty((T, W), dtype=torch.float32, device=y.device)
+    ld = gate.shape[1] if gate is not None else 0
+    call("sllm_moe_combine", _p(y), _p(place), _p(wts), T, top, _p(shared), _p(gate) + 4 * (ld - 1) if gate is not None else None, ld, _p(out),
+         1 if residual is not None else 0, W, _stream())
+    return None if residual is not None else out
+
+
 LINEAR_TC_MAX_ROWS = 128  # the tokens are the tensor core's N side: one tile of at most 128
 # Plain products go to it only where it beats the library: a reduction of at least this length with at
 # most this many tokens (at 7B sizes, 64 tokens: down 29.3 against 30.7 us; qkv 11.6 against 9.2 us).

@@ -9,9 +9,10 @@ two-matrix experts, and optionally one expert every token uses.
 All experts' up projections are ONE matrix (expert e's rows at e * ff, the shared expert's after them) and their down
 projections one matrix side by side: a token's activation row carries its routing weights (zero for an expert not
 chosen), so the second product adds up the weighted experts by itself, in float32, in one order whatever else the batch
-holds.  Every expert's product is computed for every token: with E experts of which ``top`` are used that is E/top times
-the arithmetic of a sorted, grouped product, and none of its bookkeeping; a decode step reads every expert's matrix
-either way once the batch holds a few tokens.
+holds.  In a decode step and a short portion every expert's product is computed for every token: E/top times the arithmetic
+of a sorted, grouped product and none of its bookkeeping, and a decode step reads every expert's matrix either way once the
+batch holds a few tokens.  Long portions sort their tokens by expert (`sorted_experts`), the weights then enter as the experts' rows are added
+up, in float32, in the order of the router's choices.
 """
 
 from __future__ import annotations
@@ -23,6 +24,16 @@ import torch
 from .. import ops
 from .base import FEED_FORWARDS, FeedForward, TensorSpec
 from .standard import Linear
+
+
+def sorted_experts(x, idx, wts, E, first, w_rows, act, down, ff, residual, shared=None, gate=None):
+    """The routed experts' term of the normed rows ``x`` with the tokens sorted by expert.  ``first`` and ``down``: the matrices of all experts (a
+    `Linear`'s weight each), ``w_rows`` rows of the first an expert; ``act(rows, w, tile_expert)``: the first product with its activation; ``shared`` (float32
+    ``[T, W]``), times the last column of ``gate`` if given, joins the sum.  Added into ``residual`` (returns None) or returned, float32."""
+    place, tile_expert, row_token = ops.moe_assign(idx, E)
+    rows = ops.moe_gather(x, row_token)
+    y = ops.gemm_pair_grouped(act(rows, first, tile_expert), down, tile_expert, down.shape[0], ff, 0, ff, torch.float32)
+    return ops.moe_combine(y, place, wts, shared, gate, residual)
 
 
 @FEED_FORWARDS.register("routed_experts")
@@ -57,6 +68,8 @@ class RoutedExperts(FeedForward):
         names = [f"e{e}" for e in range(self.E)] + (["shared"] if self.shared_ff else [])
         self.up = Linear(self._matrix(torch.cat([fetch(f"{n}.up") for n in names], dim=0)))          # [E ff + shared, W]
         self.down = Linear(self._matrix(torch.cat([fetch(f"{n}.down") for n in names], dim=1)))      # [W, E ff + shared]
+        # (the shared expert's columns once more, for portions whose tokens are sorted by expert)
+        self.shared_down = Linear(self._matrix(fetch("shared.down"))) if self.shared_ff else None
         self.router = Linear(self._matrix(fetch("router")))
         self.correction = self._f32(fetch("correction"))
 
@@ -67,7 +80,13 @@ class RoutedExperts(FeedForward):
         return ops.moe_route(self.router(x, torch.float32), self.correction, self.groups, self.keep, self.top, self.scale)
 
     def forward(self, x, step, residual=None):
-        dense, _, _ = self.route(x)
+        dense, idx, wts = self.route(x)
+        if ops.moe_grouped_pays(x, self.E, self.top, self.ff, 2):
+            shared = None
+            if self.shared_ff:
+                shared = ops.linear(ops.linear_plain_act(x, self.up.weight[self.E * self.ff:], self.dtype, "gelu"), self.shared_down.weight, None, torch.float32)
+            act = lambda rows, w, tiles: ops.gemm_pair_grouped(rows, w, tiles, self.ff, self.hidden, self.ff, 0, self.dtype, act="gelu")  # noqa: E731
+            return sorted_experts(x, idx, wts, self.E, self.up.weight, self.ff, act, self.down.weight, self.ff, residual, shared)
         act = ops.moe_act(self.up(x, self.dtype), dense, self.ff, self.dtype)        # [T, E ff + shared]
         return self.down.into(act, residual)
 
@@ -141,6 +160,8 @@ class GatedExperts(FeedForward):
             rows.append(torch.stack([g.reshape(-1, n, W), u.reshape(-1, n, W)], dim=1).reshape(2 * g.shape[0], W))
         self.gate_up = Linear(self._matrix(torch.cat(rows, dim=0)))                                # [2 (E ff + shared), W]
         self.down = Linear(self._matrix(torch.cat([fetch(f"{e}.down") for e in names], dim=1)))    # [W, E ff + shared]
+        # (the shared expert's columns once more, for portions whose tokens are sorted by expert)
+        self.shared_down = Linear(self._matrix(fetch("shared.down"))) if self.shared_ff else None
         router, bias = fetch("router"), None
         if self.shared_ff:
             router = torch.cat([router, fetch("shared.sg")], dim=0)
@@ -160,11 +181,25 @@ class GatedExperts(FeedForward):
         return ops.moe_route_top_softmax(self.router(x, torch.float32), self.top, self.scale, experts=self.E, gated=1 if self.shared_ff else 0)
 
     def forward(self, x, step, residual=None):
-        dense, _, _ = self.route(x)
+        dense, idx, wts = self.route(x)
+        if ops.moe_grouped_pays(x, self.E, self.top, self.ff, 3):
+            shared = None
+            if self.shared_ff:
+                shared = ops.linear(ops.linear_silu_mul(x, self.gate_up.weight[2 * self.E * self.ff:], self.interleave, self.dtype),
+                                    self.shared_down.weight, None, torch.float32)
+            return sorted_experts(x, idx, wts, self.E, self.gate_up.weight, 2 * self.ff, self._sorted_act, self.down.weight, self.ff, residual, shared,
+                                  dense if self.shared_ff else None)
         gu = self.gate_up(x, self.dtype)                                                                     # [T, 2 E ff]
         act = ops.gated_clamp_act(gu, self.interleave, self.limit, self.dtype, alpha=self.alpha, dense=dense, ff=self.ff, act=self.act,
                                   tail=self.shared_ff)
         return self.down.into(act, residual)
+
+    def _sorted_act(self, rows, w, tiles):
+        n = 2 * self.ff
+        if self.act == "silu" and self.interleave == 8:
+            return ops.gemm_pair_grouped(rows, w, tiles, n, self.hidden, n, 0, self.dtype, act="silu")
+        gu = ops.gemm_pair_grouped(rows, w, tiles, n, self.hidden, n, 0, self.dtype)
+        return ops.gated_clamp_act(gu, self.interleave, self.limit, self.dtype, alpha=self.alpha, ff=self.ff, act=self.act)
 
     def weight_bytes(self):
         return self.gate_up.nbytes() + self.down.nbytes() + self.router.nbytes()

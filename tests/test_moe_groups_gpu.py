@@ -1,0 +1,89 @@
+"""A mixture of experts with the tokens sorted by expert (moe_groups.cu, the grouped form of gemm_pair.cu): the sorting itself, the grouped product
+with each of its epilogues, and whole mixtures against float64 (the bound: two bfloat16 roundings of each input and activation, 2^-8 of the
+terms' root sum of squares at worst, so 1e-2 of the result's)."""
+
+import pytest
+import torch
+
+from tests.conftest import cuda_or_skip
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("T,top,E", [(1, 1, 1), (300, 2, 8), (257, 8, 8), (1000, 3, 40), (64, 1, 200), (2048, 2, 8)])
+@pytest.mark.parametrize("lopsided", [False, True])
+def test_every_choice_has_a_row_among_its_experts(T, top, E, lopsided):
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    g = torch.Generator(device=dev).manual_seed(T + E)
+    score = torch.rand(T, E, device=dev, generator=g)
+    if lopsided:
+        score[:, 0] += 2
+    idx = score.topk(top, -1).indices.int().contiguous()
+    place, tile_expert, row_token = ops.moe_assign(idx, E)
+    assert len(place.unique()) == T * top
+    assert torch.equal(tile_expert[(place // 256).long()], idx)
+    assert torch.equal(row_token[place.long()], torch.arange(T, device=dev, dtype=torch.int32)[:, None].expand(T, top))
+    assert int((row_token >= 0).sum()) == T * top
+    used = int(((torch.bincount(idx.flatten().long(), minlength=E) + 255) // 256).sum())
+    assert int((tile_expert >= 0).sum()) == used and bool((tile_expert[used:] == -1).all())
+
+
+@pytest.mark.parametrize("N,K,E", [(256, 64, 3), (1408, 192, 8), (72, 2048, 5), (520, 128, 2)])
+@pytest.mark.parametrize("act", [None, "float", "gelu", "silu"])
+def test_grouped_product(N, K, E, act):
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    if act == "silu" and N % 16:
+        pytest.skip("the gated epilogue takes whole blocks of 8 pairs")
+    g = torch.Generator(device=dev).manual_seed(N + K)
+    tiles = torch.tensor([e for e in range(E) for _ in range(1 + e % 2)] + [-1, -1], dtype=torch.int32, device=dev)
+    x = torch.randn(256 * len(tiles), K, device=dev, generator=g).bfloat16()
+    rows = torch.randn(E * N, K, device=dev, generator=g).bfloat16() / K ** 0.5                # experts below one another
+    got = ops.gemm_pair_grouped(x, rows, tiles, N, K, N, 0, torch.float32 if act == "float" else torch.bfloat16, act=None if act == "float" else act)
+    cols = rows.reshape(E, N, K).transpose(0, 1).reshape(N, E * K).contiguous()                # experts beside one another
+    side = ops.gemm_pair_grouped(x, cols, tiles, N, K, 0, K, torch.float32 if act == "float" else torch.bfloat16, act=None if act == "float" else act)
+    ops.check_tcgen05_status()
+    live = int((tiles >= 0).sum()) * 256
+    y = torch.cat([x[256 * i:256 * (i + 1)].double() @ rows[N * int(e):N * (int(e) + 1)].double().T for i, e in enumerate(tiles.tolist()) if e >= 0])
+    if act == "gelu":
+        y = torch.nn.functional.gelu(y)
+    if act == "silu":
+        gate, up = y.reshape(live, N // 16, 2, 8).unbind(2)
+        y = (torch.nn.functional.silu(gate) * up).reshape(live, N // 2)
+    tol = 2e-5 if act == "float" else 1e-2
+    torch.testing.assert_close(got[:live].double(), y, rtol=tol, atol=tol)
+    assert torch.equal(got[:live], side[:live])
+
+
+CASES = [("routed_experts", {"experts": 8, "top": 2, "groups": 4, "keep": 2, "scale": 2.0, "expert_ff": 192, "shared_ff": 384}),
+         ("routed_experts", {"experts": 6, "top": 3, "scale": 1.0, "expert_ff": 64}),
+         ("gated_experts", {"experts": 8, "top": 2, "expert_ff": 128, "limit": 7.0}),
+         ("gated_experts", {"experts": 5, "top": 1, "expert_ff": 192, "activation": "silu", "scale": 2.0}),
+         ("gated_experts", {"experts": 8, "top": 2, "expert_ff": 128, "activation": "silu", "router_bias": True, "shared_ff": 256})]
+
+
+@pytest.mark.parametrize("kind,params", CASES)
+@pytest.mark.parametrize("T", [129, 700])
+def test_a_mixture_sorted_by_expert(monkeypatch, kind, params, T):
+    import sllm_b200.ops as ops
+    from sllm_b200.config.plan import PartSpec
+    from sllm_b200.models import causal_lm  # noqa: F401  (registers the parts)
+    from sllm_b200.parts.base import FEED_FORWARDS
+    dev = cuda_or_skip()
+    W = 256
+    part = FEED_FORWARDS.build(PartSpec(kind, dict(params, hidden_size=W)), dtype=torch.bfloat16, device=dev)
+    g = torch.Generator(device=dev).manual_seed(T)
+    part.bind({s.name: torch.randn(*s.shape, device=dev, generator=g) / max(1, s.shape[-1]) ** 0.5 for s in part.tensor_specs()}.__getitem__)
+    x = torch.randn(T, W, device=dev, generator=g).bfloat16()
+    monkeypatch.setattr(ops, "moe_grouped_pays", lambda *a: False)
+    want = part.forward(x, None)
+    want = want.sum(0) if want.dim() == 3 else want
+    monkeypatch.setattr(ops, "moe_grouped_pays", lambda *a: True)
+    got = part.forward(x, None)
+    stream = torch.randn(T, W, device=dev, generator=g)
+    added = stream.clone()
+    assert part.forward(x, None, residual=added) is None
+    ops.check_tcgen05_status()
+    assert float((got - want).norm() / want.norm()) < 1e-2
+    torch.testing.assert_close(added, stream + got, rtol=1e-6, atol=1e-5)
