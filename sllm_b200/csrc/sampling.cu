@@ -155,25 +155,25 @@ struct Select {
   int chosen;                 // the last level's bin, -1: the target lies beyond every eligible logit
 };
 
-// f(logit, index) over row[from, to), eight loads in flight a thread
+// f(logit, index) over every `stride`th logit of the row from `first` on, eight loads in flight a thread
 template <class F>
-__device__ __forceinline__ void for_range(const float* __restrict__ row, int from, int to, F f) {
-  for (int i0 = from + threadIdx.x; i0 < to; i0 += SAMPLE_THREADS * 8) {
+__device__ __forceinline__ void for_strided(const float* __restrict__ row, int first, int stride, int V, F f) {
+  for (int i0 = first; i0 < V; i0 += stride * 8) {
     float l[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
-      const int i = i0 + u * SAMPLE_THREADS;
-      l[u] = i < to ? row[i] : 0.f;
+      const int i = i0 + u * stride;
+      l[u] = i < V ? row[i] : 0.f;
     }
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
-      const int i = i0 + u * SAMPLE_THREADS;
-      if (i < to) f(l[u], i);
+      const int i = i0 + u * stride;
+      if (i < V) f(l[u], i);
     }
   }
 }
 template <class F>
-__device__ __forceinline__ void for_row(const float* __restrict__ row, int V, F f) { for_range(row, 0, V, f); }
+__device__ __forceinline__ void for_row(const float* __restrict__ row, int V, F f) { for_strided(row, threadIdx.x, SAMPLE_THREADS, V, f); }
 // the same over [base, base + len) cut at `end`, by one warp
 template <class F>
 __device__ __forceinline__ void for_part(const float* __restrict__ row, int base, int len, int end, F f) {
@@ -561,7 +561,7 @@ __device__ void draw_from_list(const uint32_t* key, const int* idx, int n, float
 
 // ---- top-k of at most 256 ------------------------------------------------------------------------
 //
-// The row's blocks and warps (a short row: its block's groups of four lanes) are 256 groups.  The k-th largest of the groups' maxima is a
+// The row's blocks and warps (a short row: its block's groups of four lanes), 32 (4) logits in turn each, are 256 groups.  The k-th largest of the groups' maxima is a
 // bound at or below the row's k-th largest logit, and little more than k logits reach it (about -256 ln(1 - k / 256) of a row in no
 // particular order): they are gathered in the first block, ranked against one another, and the rest (top-p over what top-k
 // kept, the draw in index order) runs on k values in shared memory.  Two passes over the row, the second from L2, by eight SMs.
@@ -574,7 +574,7 @@ static_assert(TOPK_LIST * 8 <= SAMPLE_SMEM, "the list lives in the histograms' s
 
 // true: out[row] is written (by the first block).  false: the general path must take the row.  All blocks of the cluster call it; in the others
 // the result means nothing.
-__device__ bool sample_top_k_fast(const float* __restrict__ row, const RowPart& part, float inv_t, int k, float pfrac, double u,
+__device__ bool sample_top_k_fast(const float* __restrict__ row, int V, const RowPart& part, float inv_t, int k, float pfrac, double u,
                                   unsigned char* dyn_smem, uint32_t* group_max /* [256] shared */, uint32_t* bound_s, int* count,
                                   FastShared* fs, int* out) {
   cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
@@ -585,7 +585,8 @@ __device__ bool sample_top_k_fast(const float* __restrict__ row, const RowPart& 
   if (threadIdx.x == 0) { *count = 0; *bound_s = 0u; fs->answer = 0x7fffffff; fs->last = -1; }
   // (key 0 belongs to no logit but one that is not a number)
   uint32_t best = 0u;
-  for_range(row, part.from, part.to, [&](float l, int) {
+  const int first = part.rank * SAMPLE_THREADS + threadIdx.x, stride = part.blocks * SAMPLE_THREADS;
+  for_strided(row, first, stride, V, [&](float l, int) {
     if (l == l) best = max(best, order_key(l));
   });
   for (int o = 1; o < lanes; o <<= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
@@ -603,12 +604,13 @@ __device__ bool sample_top_k_fast(const float* __restrict__ row, const RowPart& 
     if (rank == k - 1) *bound_s = mine;
   }
   __syncthreads();
-  const uint32_t bound = *bound_s;
-  if (bound > MINUS_INFINITY_KEY) {
+  // (fewer than k groups with a logit above minus infinity: all such logits, if the list holds them)
+  const uint32_t bound = max(*bound_s, MINUS_INFINITY_KEY + 1);
+  {
     int* there = part.blocks > 1 ? cl.map_shared_rank(count, 0) : count;
     uint32_t* keys = part.blocks > 1 ? cl.map_shared_rank(list_key, 0) : list_key;
     int* idxs = part.blocks > 1 ? cl.map_shared_rank(list_idx, 0) : list_idx;
-    for_range(row, part.from, part.to, [&](float l, int i) {
+    for_strided(row, first, stride, V, [&](float l, int i) {
       if (l == l && order_key(l) >= bound) {
         const int at = atomicAdd(there, 1);
         if (at < TOPK_LIST) { keys[at] = order_key(l); idxs[at] = i; }
@@ -618,8 +620,7 @@ __device__ bool sample_top_k_fast(const float* __restrict__ row, const RowPart& 
   if (part.blocks > 1) cl.sync(); else __syncthreads();
   if (part.rank != 0) return true;
   const int n = *count;
-  // fewer than k groups hold a logit above minus infinity; very many ties
-  if (bound <= MINUS_INFINITY_KEY || n > TOPK_LIST) return false;
+  if (n < k || n > TOPK_LIST) return false;          // fewer than k logits above minus infinity; very many ties
   // the k largest in descending order, ties by index (runtime/sampler.py:60-67)
   for (int e = threadIdx.x; e < n; e += SAMPLE_THREADS) {
     const uint32_t key = list_key[e];
@@ -748,7 +749,7 @@ sample_rows_kernel(const float* __restrict__ logits, int V, const float* __restr
   const float inv_t = temp > 0.f ? 1.0f / temp : 0.f;
   MaxIdx mx;
   if (has_k && k <= FAST_K) {
-    if (sample_top_k_fast(row, part, inv_t, k, pfrac, uniform[r], sample_smem, group_max, &bound_s, &list_n, &fast, out + r)) return;
+    if (sample_top_k_fast(row, V, part, inv_t, k, pfrac, uniform[r], sample_smem, group_max, &bound_s, &list_n, &fast, out + r)) return;
     __syncthreads();                                 // the general path reuses what the attempt wrote
     mx = part_argmax(row, 0, V, part.vec, sh_mi);
     if (mx.i == 0x7fffffff) mx.i = 0;
