@@ -71,6 +71,7 @@ __device__ __forceinline__ void ws_mma(float (&c)[4], unsigned a0, unsigned a1, 
 
 constexpr int WS_WARPS = 8;
 constexpr int WS_SLICES = 4;        // slices of K a cluster shares at most
+constexpr int WS_SIDE = 4;          // groups of rows side by side in a CTA of that form
 // k blocks a warp keeps in flight per group (two groups): with two token tiles half as many, so that the
 // activation fragments fit the registers of two CTAs an SM (four: 174 registers a thread, one CTA an SM)
 __host__ __device__ constexpr int ws_depth(int nt) { return nt == 1 ? 4 : (nt == 2 ? 2 : 1); }
@@ -100,18 +101,20 @@ struct WsNorm {
 
 // NT: 8-token tiles (M <= 8 * NT).  OUT: float or __nv_bfloat16 (store epilogue only).  SCALED: the input
 // comes with a norm still owed (WsNorm::ssq_in).
-// FORM: one group of rows a CTA; several, one after the other; or one that the CTAs of a cluster share, each a slice of K (store and
-// residual epilogues).
+// FORM: one group of rows a CTA; several, one after the other; one that the CTAs of a cluster share, each a slice of K (store and
+// residual epilogues); or four side by side, two warps each (store and gated).
 #define WS_ONE 0
 #define WS_WALK 1
 #define WS_SLICED 2
+#define WS_ROWS 3
 template <int NT, int EPI, typename OUT, bool SCALED, int FORM>
 __global__ void __launch_bounds__(WS_WARPS * 32, 2)
 linear_ws_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ W,
                  const float* __restrict__ bias, OUT* __restrict__ out, float* __restrict__ residual,
                  int M, int N, int K, const WsRope rope, const WsNorm norm, const int act, const TokenTable token, const int slices_) {
   constexpr int WS_DEPTH = ws_depth(NT);
-  constexpr bool SLICED = FORM == WS_SLICED;
+  constexpr bool SLICED = FORM == WS_SLICED, ROWS = FORM == WS_ROWS;
+  constexpr int KW = ROWS ? WS_WARPS / WS_SIDE : WS_WARPS, RW = WS_WARPS / KW;      // warps of a group of rows, groups side by side
   __shared__ float red[WS_WARPS][16][8 * NT + 1];
   __shared__ float row_scale[8 * NT];
   __shared__ float slice_sum[SLICED ? WS_SLICES : 1][SLICED ? 16 * 8 * NT : 1];
@@ -131,8 +134,8 @@ linear_ws_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __res
   int n0, n1;                            // the group's units
   const __nv_bfloat16 *w0, *w1;          // the lane's two rows of the group
   auto take = [&](int i) {
-    n0 = c0 + (int)(((long long)i * (c1 - c0)) / groups);
-    n1 = c0 + (int)(((long long)(i + 1) * (c1 - c0)) / groups);
+    n0 = c0 + (int)(((long long)i * (c1 - c0)) / (ROWS ? RW : groups));
+    n1 = c0 + (int)(((long long)(i + 1) * (c1 - c0)) / (ROWS ? RW : groups));
     int r0 = min(n0 + g, n1 - 1), r1 = min(n0 + g + 8, n1 - 1);   // rows past the group's: clamped loads, skipped stores
     if constexpr (EPI == WS_EPI_ROPE) {
       // CTA b of a head's hd/16: rows [8c, 8c+8) of the head and the 8 rows hd/2 further
@@ -149,7 +152,7 @@ linear_ws_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __res
     w0 = W + (size_t)r0 * K + t4 * 8;
     w1 = W + (size_t)r1 * K + t4 * 8;
   };
-  take(0);
+  take(ROWS ? warp / KW : 0);
   const __nv_bfloat16* xr[NT];
 #pragma unroll
   for (int j = 0; j < NT; ++j) xr[j] = x + (size_t)min(8 * j + g, M - 1) * K + t4 * 8;   // tokens past M: clamped, skipped
@@ -168,7 +171,7 @@ linear_ws_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __res
   auto load_w = [&](uint4 (&wa)[WS_DEPTH], uint4 (&wb)[WS_DEPTH], int kb) {
 #pragma unroll
     for (int d = 0; d < WS_DEPTH; ++d) {
-      const int b = kb + d * WS_WARPS;
+      const int b = kb + d * KW;
       if (b < k_blocks) {
         wa[d] = ws_ldg_stream(w0 + (size_t)b * 32);
         wb[d] = ws_ldg_stream(w1 + (size_t)b * 32);
@@ -178,7 +181,7 @@ linear_ws_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __res
   auto load_x = [&](uint4 (&xv)[WS_DEPTH][NT], int kb) {
 #pragma unroll
     for (int d = 0; d < WS_DEPTH; ++d) {
-      const int b = kb + d * WS_WARPS;
+      const int b = kb + d * KW;
       if (b < k_blocks) {
 #pragma unroll
         for (int j = 0; j < NT; ++j) xv[d][j] = ws_ldg(xr[j] + (size_t)b * 32);
@@ -188,7 +191,7 @@ linear_ws_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __res
   auto compute = [&](const uint4 (&wa)[WS_DEPTH], const uint4 (&wb)[WS_DEPTH], const uint4 (&xv)[WS_DEPTH][NT], int kb) {
 #pragma unroll
     for (int d = 0; d < WS_DEPTH; ++d) {
-      if (kb + d * WS_WARPS < k_blocks) {
+      if (kb + d * KW < k_blocks) {
 #pragma unroll
         for (int j = 0; j < NT; ++j) {
           ws_mma(acc[j], wa[d].x, wb[d].x, wa[d].y, wb[d].y, xv[d][j].x, xv[d][j].y);
@@ -197,8 +200,8 @@ linear_ws_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __res
       }
     }
   };
-  constexpr int GROUP = WS_DEPTH * WS_WARPS;        // k blocks the CTA covers per group
-  const int k_mine = k_first + warp;
+  constexpr int GROUP = WS_DEPTH * KW;        // k blocks the CTA covers per group
+  const int k_mine = k_first + warp % KW;
   int kb = k_mine;
   load_w(wa0, wb0, kb);
   if constexpr (SLICED) cooperative_groups::this_cluster().sync();      // nobody writes to a CTA that has not begun
@@ -215,7 +218,7 @@ linear_ws_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __res
     }
     asm volatile("cp.async.commit_group;\n" ::);
   }
-  constexpr int OUTS = (16 * 8 * NT + WS_WARPS * 32 - 1) / (WS_WARPS * 32);
+  constexpr int OUTS = (16 * 8 * NT * RW + WS_WARPS * 32 - 1) / (WS_WARPS * 32);
   float squares[OUTS];                   // residual epilogue: of the thread's places, over the groups
 #pragma unroll
   for (int o = 0; o < OUTS; ++o) squares[o] = 0.f;
@@ -315,12 +318,13 @@ linear_ws_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __res
       return;
     }
     if constexpr (EPI == WS_EPI_GATED) {
-      for (int idx = tid; idx < 8 * 8 * NT; idx += WS_WARPS * 32) {
-        const int i = idx % 8, tok = idx / 8, q = m0 + i;
-        if (tok >= M || q >= m1) continue;
+      for (int idx = tid; idx < 8 * 8 * NT * RW; idx += WS_WARPS * 32) {
+        const int i = idx % 8, tok = idx / 8 % (8 * NT), rg = idx / (64 * NT);
+        const int q = (ROWS ? c0 + rg * (c1 - c0) / RW : m0) + i;
+        if (tok >= M || q >= (ROWS ? c0 + (rg + 1) * (c1 - c0) / RW : m1)) continue;
         float gate = 0.f, up = 0.f;
 #pragma unroll
-        for (int w = 0; w < WS_WARPS; ++w) { gate += red[w][i][tok]; up += red[w][i + 8][tok]; }
+        for (int w = 0; w < KW; ++w) { gate += red[rg * KW + w][i][tok]; up += red[rg * KW + w][i + 8][tok]; }
         if constexpr (SCALED) {
           gate *= row_scale[tok];
           up *= row_scale[tok];
@@ -348,16 +352,16 @@ linear_ws_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __res
 #pragma unroll
     for (int o = 0; o < OUTS; ++o) {
       const int idx = tid + o * WS_WARPS * 32;
-      if (idx >= 16 * 8 * NT) break;                      // (whole warps: 16 * 8 * NT is a multiple of 32)
-      const int row = idx % 16, tok = idx / 16;           // consecutive threads -> consecutive rows of one token
-      const int n = m0 + row;
-      if (tok >= M || n >= m1) continue;
+      if (idx >= 16 * 8 * NT * RW) break;                 // (whole warps: 16 * 8 * NT is a multiple of 32)
+      const int row = idx % 16, tok = idx / 16 % (8 * NT), rg = idx / (128 * NT);       // consecutive threads -> consecutive rows of one token
+      const int n = (ROWS ? c0 + rg * (c1 - c0) / RW : m0) + row;
+      if (tok >= M || n >= (ROWS ? c0 + (rg + 1) * (c1 - c0) / RW : m1)) continue;
       float v = 0.f;
       if constexpr (SLICED) {
         for (int w = 0; w < slices; ++w) v += slice_sum[w][idx];
       } else {
 #pragma unroll
-        for (int w = 0; w < WS_WARPS; ++w) v += red[w][row][tok];
+        for (int w = 0; w < KW; ++w) v += red[rg * KW + w][row][tok];
       }
       if constexpr (SCALED) v *= row_scale[tok];
       if (bias) v += bias[n];
@@ -416,6 +420,17 @@ static int ws_slices(int ctas, int K) {
   return s;
 }
 
+// Whether a CTA takes four groups of rows side by side where it would walk them: with two warps a group a short K leaves each warp a stream of
+// its own in place of one round of loads between two sums.  Where its CTAs fit the SMs at once or end in a wave that is nearly full; 9..16 tokens, whose
+// activations leave a warp half the weights in flight, only a short K at once.  (Store, us, side by side / walk / linear_stream.cu, 8 tokens: 9,728 x 896 6.1 / 7.7
+// / 8.0, 17,920 x 1,536 10.3 / 12.9 / 14.8, 11,264 x 2,048 10.4 / 10.7 / 17.8, 37,888 x 3,584 44.0 / 46.2 / 44.8, 151,936 x 1,536 74 / 87 / 81; beyond the line
+// 22,528 x 2,048 20.4 / 18.3, 22,016 x 4,096 38.5 / 31.5.  16 tokens: 9,728 x 896 7.2 / 7.6 / 8.2, 17,920 x 1,536 12.1 / 15.5 / 15.6; 11,264 x 2,048 13.6 / 12.6.)
+static bool ws_side_by_side(int M, int N, int K) {
+  const int places = 2 * sllm::num_sms(), ctas = (N + 16 * WS_SIDE - 1) / (16 * WS_SIDE);
+  if (M > 8) return K < 2048 && ctas <= places;
+  return ctas <= places || ctas * 100 >= (ctas + places - 1) / places * places * 84;
+}
+
 template <int NT, int EPI, typename OUT>
 static int launch_ws(const __nv_bfloat16* x, const __nv_bfloat16* W, const float* bias, void* out, float* residual,
                      int M, int N, int K, cudaStream_t stream, const WsRope& rope = WsRope{}, const WsNorm& norm = WsNorm{},
@@ -423,6 +438,16 @@ static int launch_ws(const __nv_bfloat16* x, const __nv_bfloat16* W, const float
   const int ctas = EPI == WS_EPI_GATED ? ws_ctas(N / 2, 8, K, false) : ws_ctas(N, 16, K, EPI == WS_EPI_ROPE);
   // (rows beyond a group a CTA: only the forms that are asked for them)
   const bool walk = EPI != WS_EPI_ROPE && (long long)ctas * (EPI == WS_EPI_GATED ? 8 : 16) < (EPI == WS_EPI_GATED ? N / 2 : N);
+  if constexpr (EPI == WS_EPI_GATED || EPI == WS_EPI_STORE) {
+    if (walk && ws_side_by_side(M, N, K)) {
+      const int n = (N + 16 * WS_SIDE - 1) / (16 * WS_SIDE);
+      if (norm.ssq_in != nullptr)
+        launch_kernel(linear_ws_kernel<NT, EPI, OUT, true, WS_ROWS>, n, WS_WARPS * 32, 0, stream, x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token, 1);
+      else
+        launch_kernel(linear_ws_kernel<NT, EPI, OUT, false, WS_ROWS>, n, WS_WARPS * 32, 0, stream, x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token, 1);
+      return launch_status("linear_ws");
+    }
+  }
   if (norm.ssq_in != nullptr) {
     if constexpr (EPI != WS_EPI_ROPE) {
       if (walk) {
@@ -469,6 +494,9 @@ using namespace sllm;
 SLLM_EXPORT int sllm_linear_ws_supports(int M, int N, int K) {
   return M >= 1 && M <= 32 && N >= 16 && K >= 32 && K % 32 == 0;
 }
+
+// whether a product of many rows takes the form with groups side by side
+SLLM_EXPORT int sllm_linear_ws_side_by_side(int M, int N, int K) { return ws_side_by_side(M, N, K); }
 
 // CTAs a launch for N output columns over a reduction of K uses: the rows of the table of partial sums of squares
 // that the residual epilogue writes when it is asked for the next norm's input (see WsNorm).

@@ -1479,14 +1479,19 @@ WS_WIDE_MAX_FILL_ROWS16 = 0.7
 
 
 def _ws_wide(M: int, N: int, K: int) -> bool:
-    """Whether the warp-split kernel, two CTAs an SM that walk their rows, beats the 128-row streaming kernel on a product of more than
-    `WS_MAX_COLS` columns: unless the latter's CTAs fill its places (two an SM) in whole waves, and where a group of rows is long enough to be
-    worth its sums.  (Fill of the last wave and all, 8 tokens, us, this / the other: 0.30 10.9 / 17.8, 0.58 31.3 / 39.8, 0.73 93.8 / 104.5, 0.80 168 / 188,
-    0.84 43.9 / 46.6 and 24.7 / 24.2, 1.0 46.1 / 45.1; K = 896: 8.0 / 8.0 at a fill of 0.26 and 73 / 48 at 0.80.  16 tokens: 0.30 12.6 / 18.3, 0.58 35.2 / 45.4,
-    0.84 50.6 / 48.8 and 29.3 / 25.5, 1.0 53.1 / 46.4.)"""
+    """Whether the warp-split kernel beats the 128-row streaming kernel on a product of more than `WS_MAX_COLS` columns.  Two CTAs an SM that walk their
+    rows: unless the latter's CTAs fill its places (two an SM) in whole waves, and where a group of rows is long enough to be
+    worth its sums.  (Fill of the last wave and all, 8 tokens, us, this / the other: 0.30 10.9 / 17.8, 0.58 31.3 / 39.8, 0.73 93.8 / 104.5,
+    0.84 43.9 / 46.6 and 24.7 / 24.2, 1.0 46.1 / 45.1.  16 tokens: 0.30 12.6 / 18.3, 0.58 35.2 / 45.4,
+    0.84 50.6 / 48.8 and 29.3 / 25.5, 1.0 53.1 / 46.4.)  CTAs of four groups side by side (the kernel's own choice): always, but for many rows of
+    a short K (151,936 x 896, 8 tokens: 49.5 / 48.9; the other figures stand in linear_ws.cu)."""
+    if M > 16 or not ws_takes(M, N, K):
+        return False
     places, ctas = 2 * num_sms(), -(-N // 128)
+    if lib().sllm_linear_ws_side_by_side(int(M), int(N), int(K)):
+        return K >= 1024 or ctas <= places
     fill = ctas / (-(-ctas // places) * places)
-    return K >= WS_WIDE_MIN_K and M <= 16 and fill < (WS_WIDE_MAX_FILL if M <= 8 else WS_WIDE_MAX_FILL_ROWS16)
+    return K >= WS_WIDE_MIN_K and fill < (WS_WIDE_MAX_FILL if M <= 8 else WS_WIDE_MAX_FILL_ROWS16)
 
 
 WS_MAX_ROWS = 32          # one, two or four 8-token tiles (with fewer k blocks in flight the more tiles, so that two CTAs still share an SM)
@@ -1505,7 +1510,7 @@ def ws_supports(M: int, N: int, K: int) -> bool:
     its 16-row CTAs fit the GPU at once: at N = 5120 (320 to 592 CTAs for 296 places) it falls behind the k-split
     kernel by more than the fused epilogues save (16 tokens, K = 27648: 64.3 against 49.2 us)."""
     if N > WS_MAX_COLS:
-        return ws_takes(M, N, K) and _ws_wide(M, N, K)
+        return _ws_wide(M, N, K)
     return ws_takes(M, N, K) and _ws_tokens_ok(M, N, K)
 
 
@@ -1526,7 +1531,7 @@ def _ws_tokens_ok(M: int, N: int, K: int) -> bool:
 @functools.lru_cache(maxsize=4096)
 def ws_gated_supports(M: int, N: int, K: int) -> bool:
     """Whether the warp-split kernel is the one for a gate|up product with its activation."""
-    return M <= 16 and N % 16 == 0 and N > WS_MAX_COLS and ws_takes(M, N, K) and _ws_wide(M, N, K)
+    return N % 16 == 0 and N > WS_MAX_COLS and _ws_wide(M, N, K)
 
 
 class RowScale:
