@@ -1976,6 +1976,7 @@ def attention_tiles(q_lens, group_size: int, device, ctx_lens=None, large_rows: 
 
 SPLIT_OVERHEAD_TILES = 3      # what a CTA of the decode form costs before and after its keys, in 64-key tiles
 MAX_SPLITS = 128              # the merge kernel keeps one weight a range in shared memory
+MERGE_TILES = 2               # the merge kernel behind a cut context (2.7 us; a short answer at 0.5B sizes, contexts below 256: 12.6 ms with it, 11.9 without)
 SPLIT_MIN_KEYS = 128          # a range has at least two key tiles (one request at 1,024 keys: 11.0 us in 4 ranges, 8.6 in 8)
 MMA_MAX_SPLITS = 32           # the mma.sync form's merge walks the ranges one after the other
 
@@ -1995,7 +1996,7 @@ def choose_splits(num_small: int, nkv: int, max_ctx: int, ctas_per_sm: int = 2, 
         if -(-max_ctx // (tiles * 64)) != s:              # so some counts leave their last ranges empty
             continue
         # (the last term: every range of every tile leaves a partial result that the merge reads again)
-        cost = -(-ctas * s // slots) * (tiles + SPLIT_OVERHEAD_TILES) + 0.5 * ctas * s / slots
+        cost = -(-ctas * s // slots) * (tiles + SPLIT_OVERHEAD_TILES) + 0.5 * ctas * s / slots + (MERGE_TILES if s > 1 else 0)
         if best_cost is None or cost < best_cost:
             best, best_cost = s, cost
     return best
