@@ -495,6 +495,8 @@ SLLM_EXPORT int sllm_linear_ws_supports(int M, int N, int K) {
   return M >= 1 && M <= 32 && N >= 16 && K >= 32 && K % 32 == 0;
 }
 
+// slices of K that the CTAs of a cluster share (no norm owed on the input)
+SLLM_EXPORT int sllm_linear_ws_slices(int N, int K) { return ws_slices(ws_ctas(N, 16, K, false), K); }
 // whether a product of many rows takes the form with groups side by side
 SLLM_EXPORT int sllm_linear_ws_side_by_side(int M, int N, int K) { return ws_side_by_side(M, N, K); }
 

@@ -1497,10 +1497,14 @@ def _ws_wide(M: int, N: int, K: int) -> bool:
 WS_MAX_ROWS = 32          # one, two or four 8-token tiles (with fewer k blocks in flight the more tiles, so that two CTAs still share an SM)
 # Four tiles (17..32 tokens, one k block in flight per group) stream slowly, so only where little streams and the
 # fused epilogues save kernels: a short reduction, a matrix of at most 2^24 elements, and rows enough for one and a
-# half CTAs an SM (q|k|v and o_proj at a hidden size of 3,584: decode at batch 24 and 32 +2.5 %; at hidden sizes of
-# 1,536 and 2,048 the k-split kernel with its norm and rotary kernels stayed the faster, 2.05 against 2.21 ms a step).
+# half CTAs an SM (q|k|v and o_proj at a hidden size of 3,584: decode at batch 24 and 32 +2.5 %; smaller ones: below).
 WS_ROWS32_MAX_ELEMENTS = int(os.environ.get("SLLM_WS_ROWS32_MAX_ELEMENTS", str(1 << 24)))
 WS_ROWS32_MAX_K = 4096
+# Smaller matrices since clusters share their columns (`_ws_rows32_ok`; not the product with the rotary epilogue, which they cannot share): where rows
+# times slices come to 0.7 of the places or the rows alone to one CTA an SM, or where K is so short that latency is all of it.  (33 steps, ms, before / since:
+# 17 requests at a width of 896 38.9 / 37.8, 24 at 1,536 63.4 / 62.2; the other designs at 2,048, 20 to 32 requests, 35.4 / 31.9, 34.1 / 32.6, 50.9 / 48.7, 34.0 / 29.9,
+# 41.0 / 38.9, 47.7 / 44.0; at 4,096 no change.  With 1,536 x 8,960 as well, 192 of 296 places, 16 requests lost what they had won.)
+WS_ROWS32_MIN_K, WS_ROWS32_SHARED_MAX_K, WS_ROWS32_SHORT_K = 512, 8192, 1024
 MAX_SCALE_PARTS_ROWS32 = 192   # the table of partial sums a four-tile consumer keeps (streams of up to 3,072 columns)
 
 
@@ -1511,7 +1515,7 @@ def ws_supports(M: int, N: int, K: int) -> bool:
     kernel by more than the fused epilogues save (16 tokens, K = 27648: 64.3 against 49.2 us)."""
     if N > WS_MAX_COLS:
         return _ws_wide(M, N, K)
-    return ws_takes(M, N, K) and _ws_tokens_ok(M, N, K)
+    return ws_takes(M, N, K) and (_ws_tokens_ok(M, N, K) or _ws_rows32_ok(M, N, K))
 
 
 @functools.lru_cache(maxsize=4096)
@@ -1526,6 +1530,14 @@ def _ws_tokens_ok(M: int, N: int, K: int) -> bool:
     if -(-N // 16) > 2 * num_sms():
         return False
     return M <= 16 or (N * K <= WS_ROWS32_MAX_ELEMENTS and K <= WS_ROWS32_MAX_K and 2 * -(-N // 16) >= 3 * num_sms())
+
+
+def _ws_rows32_ok(M: int, N: int, K: int) -> bool:
+    ctas = -(-N // 16)
+    if M > 32 or N * K > WS_ROWS32_MAX_ELEMENTS or not WS_ROWS32_MIN_K <= K <= WS_ROWS32_SHARED_MAX_K or ctas > 2 * num_sms():
+        return False
+    places = ctas * int(lib().sllm_linear_ws_slices(N, K))
+    return ctas >= num_sms() or places >= 1.4 * num_sms() or K <= WS_ROWS32_SHORT_K
 
 
 @functools.lru_cache(maxsize=4096)

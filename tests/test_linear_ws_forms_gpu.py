@@ -53,3 +53,17 @@ def test_gate_and_up_with_their_activation(M, N, K, act):
     assert bool(((got - want).abs() <= off).all())
     alone = M - 1 if M <= 8 else M - 9
     assert torch.equal(ops.linear_ws_gated(x[alone:].contiguous(), w, b, act)[-1], got[-1].reshape(-1))
+
+
+@pytest.mark.parametrize("M", [17, 24, 25, 32])
+@pytest.mark.parametrize("N,K,takes", [(896, 896, True), (896, 4864, True), (2048, 5632, True), (2048, 544, True), (1536, 8192, False), (1000, 480, False)])
+def test_more_tokens_on_small_matrices(M, N, K, takes):
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    assert ops.ws_supports(M, N, K) == takes
+    g, x, w, b, y, bound = _product(dev, M, N, K)
+    assert bool(((ops.linear_ws(x, w, b, torch.float32) - y).abs() <= bound).all())
+    stream = torch.randn(M, N, device=dev, generator=g)
+    added = stream.clone()
+    ops.linear_ws(x, w, b, torch.float32, residual=added)
+    assert bool(((added - (stream + y)).abs() <= bound + 2.0 ** -23 * (stream.abs() + y.abs())).all())
