@@ -32,6 +32,11 @@ def test_rows_and_columns_in_parts(M, N, K):
     added = stream.clone()
     ops.linear_ws(x, w, b, torch.float32, residual=added)
     assert bool(((added - (stream + y)).abs() <= bound + 2.0 ** -23 * (stream.abs() + y.abs())).all())
+    gain = torch.randn(N, device=dev, generator=g)
+    again = stream.clone()
+    xg, owed = ops.linear_ws(x, w, b, torch.float32, residual=again, next_gain=gain)
+    assert torch.equal(again, added) and torch.equal(xg, (added * gain).bfloat16())
+    torch.testing.assert_close(owed.ssq[:, :owed.parts].double().sum(1), added.double().pow(2).sum(1), rtol=N * 2.0 ** -24, atol=0)
     alone = M - 1 if M <= 8 else M - 9                       # (from 9 tokens on the rows may be dealt in another form)
     assert torch.equal(ops.linear_ws(x[alone:].contiguous(), w, b, torch.float32)[-1], got[-1])
 
