@@ -645,13 +645,15 @@ SLLM_EXPORT int sllm_gemm_pair_splits(int K, int want) {
   return (k_blocks + per - 1) / per;
 }
 
-SLLM_EXPORT int sllm_gemm_pair(const void* A, const void* W, const float* bias, void* out, int M, int N, int K,
+// w_ld: elements from one row of W to the next (0: K), a multiple of 8: columns of a wider matrix.
+SLLM_EXPORT int sllm_gemm_pair(const void* A, const void* W, const float* bias, void* out, int M, int N, int K, int w_ld,
                                int epilogue, int wide, int want_splits, const float* ssq_in, int parts_in, int stride_in, float eps_in,
                                int width_in, float* residual, const float* gain, void* xg_out, float* ssq_out, int stride_out,
                                const void* token_table, const int* token_ids, int token_off, int token_ld, int token_rows,
                                int* status, cudaStream_t stream) {
   SLLM_REQUIRE(sllm_gemm_pair_supports(M, N, K), "gemm_pair: sizes M=%d N=%d K=%d (K must be a multiple of 8)", M, N, K);
   SLLM_REQUIRE(((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0, "gemm_pair: operands must be 16-byte aligned");
+  SLLM_REQUIRE(w_ld == 0 || (w_ld >= K && w_ld % 8 == 0), "gemm_pair: rows of W %d elements apart (at least K=%d, a multiple of 8)", w_ld, K);
   SLLM_REQUIRE(status != nullptr, "gemm_pair: a status word is required");
   SLLM_REQUIRE(!tg_gated(epilogue) || N % 16 == 0, "gemm_pair: the gated epilogues need N %% 16 == 0");
   TgExtra extra;
@@ -691,7 +693,7 @@ SLLM_EXPORT int sllm_gemm_pair(const void* A, const void* W, const float* bias, 
   const int kb_per_split = (((K + TP_BK - 1) / TP_BK) + ksplits - 1) / ksplits;
   SLLM_REQUIRE(ksplits == 1 || (epilogue == TG_EPI_F32 && !wide_form && ssq_in == nullptr),
                "gemm_pair: slices of K leave a stack of float32 partial sums (plain epilogue, not the 512-wide tiles, no owed norm)");
-  if (!make_map(&ma, A, M, K, TP_BM, promo) || !make_map(&mw, W, N, K, wide_form ? wide_cols / 2 : wide == 2 ? 64 : 128, promo)) {
+  if (!make_map(&ma, A, M, K, TP_BM, promo) || !make_map(&mw, W, N, K, wide_form ? wide_cols / 2 : wide == 2 ? 64 : 128, promo, w_ld)) {
     set_error("gemm_pair: cuTensorMapEncodeTiled failed");
     return SLLM_ERR_LAUNCH;
   }

@@ -91,13 +91,13 @@ inline EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// rows x K bfloat16, row-major; boxes of box_rows x 64 elements, 128-byte swizzle, zeros outside
+// rows x K bfloat16, row-major, `ld` elements from row to row (0: K; a multiple of 8); boxes of box_rows x 64 elements, 128-byte swizzle, zeros outside
 inline bool make_map(CUtensorMap* map, const void* base, int rows, int K, int box_rows,
-                     CUtensorMapL2promotion promotion = CU_TENSOR_MAP_L2_PROMOTION_L2_128B) {
+                     CUtensorMapL2promotion promotion = CU_TENSOR_MAP_L2_PROMOTION_L2_128B, int ld = 0) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
   cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)K * 2};
+  cuuint64_t strides[1] = {(cuuint64_t)(ld > 0 ? ld : K) * 2};
   cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
   cuuint32_t elem[2] = {1, 1};
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,

@@ -1255,7 +1255,8 @@ def pair_splits(M: int, N: int, K: int) -> int:
 
 
 def gemm_pair(x, w, bias, out_dtype, *, silu: bool = False, wide: "bool | str | None" = None, scale: "RowScale | None" = None,
-              residual=None, next_gain=None, splits: int = 1, act: "str | None" = None, token: "TokenColumns | None" = None):
+              residual=None, next_gain=None, splits: int = 1, act: "str | None" = None, token: "TokenColumns | None" = None,
+              w_col: "int | None" = None):
     """The same product and epilogues as `gemm_tcgen05`, by pairs of CTAs on 256 x 256 tiles, on
     256 x 512 tiles (``wide=True``; by default where those fill the GPU at least as well; ``wide=448``, ``384`` or
     ``320``: tiles of that many columns, float32 result or residual epilogue, chosen by `pair_wide_cols` where
@@ -1267,7 +1268,8 @@ def gemm_pair(x, w, bias, out_dtype, *, silu: bool = False, wide: "bool | str | 
     ``splits`` > 1 (float32 result, no other epilogue): K in that many slices, the result a stack ``[splits', M, N]``
     of partial sums (bias in the first) for the consumer to add.  ``act="gelu_tanh"``: the gated epilogue
     ``gelu_tanh(gate + bias) * (up + bias)`` in place of ``silu``'s (rows and bias interleaved in blocks of 8); ``"relu2"``:
-    bfloat16 ``max(v, 0)^2`` of the plain result; ``"gelu"``: its exact gelu; ``"token"``: bfloat16 ``gelu_tanh(v)`` times ``token``'s columns."""
+    bfloat16 ``max(v, 0)^2`` of the plain result; ``"gelu"``: its exact gelu; ``"token"``: bfloat16 ``gelu_tanh(v)`` times ``token``'s columns.
+    ``w_col`` (a multiple of 8, as is w's width): the product with as many of w's columns as x has, from that one on."""
     _chk(x, w, bias, residual, next_gain)
     if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
         raise KernelError("gemm_pair: bfloat16 operands only")
@@ -1279,8 +1281,8 @@ def gemm_pair(x, w, bias, out_dtype, *, silu: bool = False, wide: "bool | str | 
         raise KernelError(f"gemm_pair: the {act} epilogue takes neither bias nor residual and gives bfloat16")
     M, K = x.shape
     N = w.shape[0]
-    if w.shape[1] != K:
-        raise KernelError(f"linear: x {tuple(x.shape)} does not fit w {tuple(w.shape)}")
+    if w.shape[1] != K if w_col is None else (w_col < 0 or w_col % 8 or w.shape[1] % 8 or w_col + K > w.shape[1]):
+        raise KernelError(f"linear: x {tuple(x.shape)} does not fit w {tuple(w.shape)}" + ("" if w_col is None else f" from column {w_col} on"))
     out = xg = ssq = None
     stride = 0
     plain_or_residual = not silu and (residual is not None or out_dtype == torch.float32)
@@ -1310,7 +1312,7 @@ def gemm_pair(x, w, bias, out_dtype, *, silu: bool = False, wide: "bool | str | 
         epi, out = {None: 1, "relu2": 5, "token": 6, "gelu": 7}[plain_act], torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
     if splits > 1 and (epi != 0 or scale is not None):
         raise KernelError("gemm_pair: slices of K leave float32 partial sums: no other epilogue, no owed norm")
-    call("sllm_gemm_pair", _p(x), _p(w), _p(bias), _p(out), M, N, K, epi, code, int(splits),
+    call("sllm_gemm_pair", _p(x), _p(w) + 2 * (w_col or 0), _p(bias), _p(out), M, N, K, w.shape[1], epi, code, int(splits),
          *(scale.args_with_stride() if scale is not None else (None, 0, 0, 0.0, 0)),
          _p(residual), _p(next_gain), _p(xg), _p(ssq), stride, *(token.args() if token is not None else _NO_TOKEN),
          _p(_status_word(x.device)), _stream())

@@ -68,8 +68,6 @@ class RoutedExperts(FeedForward):
         names = [f"e{e}" for e in range(self.E)] + (["shared"] if self.shared_ff else [])
         self.up = Linear(self._matrix(torch.cat([fetch(f"{n}.up") for n in names], dim=0)))          # [E ff + shared, W]
         self.down = Linear(self._matrix(torch.cat([fetch(f"{n}.down") for n in names], dim=1)))      # [W, E ff + shared]
-        # (the shared expert's columns once more, for portions whose tokens are sorted by expert)
-        self.shared_down = Linear(self._matrix(fetch("shared.down"))) if self.shared_ff else None
         self.router = Linear(self._matrix(fetch("router")))
         self.correction = self._f32(fetch("correction"))
 
@@ -84,7 +82,8 @@ class RoutedExperts(FeedForward):
         if ops.moe_grouped_pays(x, self.E, self.top, self.ff, 2):
             shared = None
             if self.shared_ff:
-                shared = ops.linear(ops.linear_plain_act(x, self.up.weight[self.E * self.ff:], self.dtype, "gelu"), self.shared_down.weight, None, torch.float32)
+                shared = ops.gemm_pair(ops.linear_plain_act(x, self.up.weight[self.E * self.ff:], self.dtype, "gelu"), self.down.weight, None, torch.float32,
+                                       w_col=self.E * self.ff)
             act = lambda rows, w, tiles: ops.gemm_pair_grouped(rows, w, tiles, self.ff, self.hidden, self.ff, 0, self.dtype, act="gelu")  # noqa: E731
             return sorted_experts(x, idx, wts, self.E, self.up.weight, self.ff, act, self.down.weight, self.ff, residual, shared)
         act = ops.moe_act(self.up(x, self.dtype), dense, self.ff, self.dtype)        # [T, E ff + shared]
@@ -160,8 +159,6 @@ class GatedExperts(FeedForward):
             rows.append(torch.stack([g.reshape(-1, n, W), u.reshape(-1, n, W)], dim=1).reshape(2 * g.shape[0], W))
         self.gate_up = Linear(self._matrix(torch.cat(rows, dim=0)))                                # [2 (E ff + shared), W]
         self.down = Linear(self._matrix(torch.cat([fetch(f"{e}.down") for e in names], dim=1)))    # [W, E ff + shared]
-        # (the shared expert's columns once more, for portions whose tokens are sorted by expert)
-        self.shared_down = Linear(self._matrix(fetch("shared.down"))) if self.shared_ff else None
         router, bias = fetch("router"), None
         if self.shared_ff:
             router = torch.cat([router, fetch("shared.sg")], dim=0)
@@ -185,8 +182,8 @@ class GatedExperts(FeedForward):
         if ops.moe_grouped_pays(x, self.E, self.top, self.ff, 3):
             shared = None
             if self.shared_ff:
-                shared = ops.linear(ops.linear_silu_mul(x, self.gate_up.weight[2 * self.E * self.ff:], self.interleave, self.dtype),
-                                    self.shared_down.weight, None, torch.float32)
+                shared = ops.gemm_pair(ops.linear_silu_mul(x, self.gate_up.weight[2 * self.E * self.ff:], self.interleave, self.dtype),
+                                       self.down.weight, None, torch.float32, w_col=self.E * self.ff)
             return sorted_experts(x, idx, wts, self.E, self.gate_up.weight, 2 * self.ff, self._sorted_act, self.down.weight, self.ff, residual, shared,
                                   dense if self.shared_ff else None)
         gu = self.gate_up(x, self.dtype)                                                                     # [T, 2 E ff]

@@ -56,6 +56,25 @@ def test_grouped_product(N, K, E, act):
     assert torch.equal(got[:live], side[:live])
 
 
+@pytest.mark.parametrize("M,N,K,cols,at", [(129, 72, 64, 128, 8), (300, 256, 200, 264, 64), (2048, 3584, 328, 1024, 512), (700, 2048, 64, 72, 0), (513, 520, 1000, 1000, 0)])
+def test_a_product_with_some_of_a_matrixs_columns(M, N, K, cols, at):
+    """The same bits as with these columns as a matrix of their own, whatever stands in the columns beside them."""
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    g = torch.Generator(device=dev).manual_seed(M + N)
+    x = torch.randn(M, K, device=dev, generator=g).bfloat16()
+    own = (torch.randn(N, K, device=dev, generator=g) / K ** 0.5).bfloat16()
+    w = torch.full((N, cols), float("nan"), device=dev).bfloat16()
+    w[:, at:at + K] = own
+    for dtype in (torch.float32, torch.bfloat16):
+        got, want = ops.gemm_pair(x, w, None, dtype, w_col=at), ops.gemm_pair(x, own, None, dtype)
+        ops.check_tcgen05_status()
+        assert torch.equal(got, want)
+    for bad in (-8, at + 4, cols - K + 8):
+        with pytest.raises(ops.KernelError):
+            ops.gemm_pair(x, w, None, torch.float32, w_col=bad)
+
+
 CASES = [("routed_experts", {"experts": 8, "top": 2, "groups": 4, "keep": 2, "scale": 2.0, "expert_ff": 192, "shared_ff": 384}),
          ("routed_experts", {"experts": 6, "top": 3, "scale": 1.0, "expert_ff": 64}),
          ("gated_experts", {"experts": 8, "top": 2, "expert_ff": 128, "limit": 7.0}),

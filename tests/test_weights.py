@@ -165,3 +165,29 @@ def test_upload_is_refused_when_the_device_has_no_room(monkeypatch):
     assert "GiB" in str(e.value) and "free" in str(e.value)
     monkeypatch.setattr(torch.cuda, "mem_get_info", lambda dev=None: (need + loading.SLACK_BYTES, 10 * need))
     loading.check_device_memory(model)
+
+
+@pytest.mark.parametrize("kind,params", [("routed_experts", {"scale": 1.0}), ("gated_experts", {"activation": "silu"})])
+def test_a_mixture_keeps_every_tensor_once(kind, params):
+    """What a mixture with a shared expert holds once bound is what the guard above counts from its specs (and the rows of zeros that pad a router): each
+    tensor is fetched once (a source that draws it gives other numbers the second time) and kept once."""
+    import torch
+    from sllm_b200.config.plan import PartSpec
+    from sllm_b200.models import causal_lm  # noqa: F401  (registers the parts)
+    from sllm_b200.parts.base import FEED_FORWARDS
+    part = FEED_FORWARDS.build(PartSpec(kind, dict(params, hidden_size=64, experts=4, top=2, expert_ff=32, shared_ff=48)),
+                               dtype=torch.bfloat16, device=torch.device("cpu"))
+    specs, fetched = {s.name: s for s in part.tensor_specs()}, []
+
+    def fetch(name):
+        fetched.append(name)
+        return torch.randn(*specs[name].shape)
+    part.bind(fetch)
+    assert sorted(fetched) == sorted(specs)
+    held = {}
+    for v in part.__dict__.values():
+        for t in (v, getattr(v, "weight", None), getattr(v, "bias", None)):
+            if isinstance(t, torch.Tensor):
+                held[t.data_ptr()] = t.numel() * t.element_size()
+    counted = sum(int(torch.tensor(s.shape).prod()) * (4 if s.role == "bias" else 2) for s in specs.values())
+    assert counted <= sum(held.values()) <= counted + 16 * 64 * 2
