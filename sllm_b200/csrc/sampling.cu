@@ -1,4 +1,4 @@
-// Sampling on the device over float32 logits [R, V], a cluster of eight blocks of 1024 threads per row (one block for a short row), and the
+// Sampling on the device over float32 logits [R, V], a cluster of up to eight blocks of 1024 threads per row (one block for a short row or where the rows are many), and the
 // repetition penalty that goes before it.
 //
 // greedy: the first maximum (runtime/sampler.py:8-9).
@@ -37,7 +37,10 @@
 namespace sllm {
 
 constexpr int SAMPLE_THREADS = 1024;
-constexpr int SAMPLE_SPLIT_FROM = 16384;     // logits of a row from which eight blocks share it
+// Logits of a row from which several blocks share it.  (One block / four, 8 rows, us: 32,000 logits: greedy 4.1 / 4.4, temperature 13.6 / 14.2, top_k 20 13.0 / 9.8;
+// 65,536: 4.8 / 4.7, 19.5 / 19.1, 18.4 / 11.3.)
+constexpr int SAMPLE_SPLIT_FROM = 49152;
+constexpr int SAMPLE_BLOCKS_LOG2 = 3;        // at most eight
 
 struct MaxIdx {
   float v;
@@ -526,16 +529,20 @@ __device__ void select_in_candidates(const uint32_t* cand_key, const int* cand_i
 }
 
 // The draw from a short list of kept tokens (keys, indices; n at most one a thread): the cumulative
-// probability in index order reaches u times the total at the answer (runtime/sampler.py:81-88).
-__device__ void draw_from_list(const uint32_t* key, const int* idx, int n, float mx, float inv_t, double u, double* red,
+// probability in index order reaches u times the total at the answer (runtime/sampler.py:81-88).  `q`: n doubles of shared memory, the
+// probabilities, made once (200 tokens: 12 us less than every thread making those before its own).
+__device__ void draw_from_list(const uint32_t* key, const int* idx, int n, float mx, float inv_t, double u, double* red, double* q,
                                FastShared* fs, int* out) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double cum = 0.0;
   int mine = -1;
+  __syncthreads();
+  if (threadIdx.x < n) q[threadIdx.x] = (double)prob(key_value(key[threadIdx.x]), mx, inv_t);
+  __syncthreads();
   if (threadIdx.x < n) {
     mine = idx[threadIdx.x];
-    for (int j = 0; j < n; ++j)
-      if (idx[j] <= mine) cum += (double)prob(key_value(key[j]), mx, inv_t);
+#pragma unroll 4
+    for (int j = 0; j < n; ++j) cum += idx[j] <= mine ? q[j] : 0.0;
   }
   double total = cum;                               // the token with the largest index holds the total
 #pragma unroll
@@ -561,11 +568,11 @@ __device__ void draw_from_list(const uint32_t* key, const int* idx, int n, float
 
 // ---- top-k of at most 256 ------------------------------------------------------------------------
 //
-// The row's blocks and warps (a short row: its block's groups of four lanes), 32 (4) logits in turn each, are 256 groups.  The k-th largest of the groups' maxima is a
+// Four lanes a block of the row, that many logits in turn, are a group, of 256.  The k-th largest of the groups' maxima is a
 // bound at or below the row's k-th largest logit, and little more than k logits reach it (about -256 ln(1 - k / 256) of a row in no
 // particular order): they are gathered in the first block, ranked against one another, and the rest (top-p over what top-k
-// kept, the draw in index order) runs on k values in shared memory.  Two passes over the row, the second from L2, by eight SMs.
-// (32 rows of 151,936 logits, top_k 20: 34 us with the gaps of a serving step; one block a row with four candidates a thread 336 where the k-th largest lay more
+// kept, the draw in index order) runs on k values in shared memory.  Two passes over the row, the second from L2, by the row's SMs.
+// (32 rows of 151,936 logits, top_k 20: 15.5 us; one block a row with four candidates a thread 51, or 306 where the k-th largest lay more
 // than 24 T below the largest, which that form left to the general path.)
 
 constexpr int TOPK_GROUPS = 256, TOPK_LIST = 2048;
@@ -578,10 +585,9 @@ __device__ bool sample_top_k_fast(const float* __restrict__ row, int V, const Ro
                                   unsigned char* dyn_smem, uint32_t* group_max /* [256] shared */, uint32_t* bound_s, int* count,
                                   FastShared* fs, int* out) {
   cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
-  uint32_t* list_key = reinterpret_cast<uint32_t*>(dyn_smem);
-  int* list_idx = reinterpret_cast<int*>(list_key + TOPK_LIST);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int lanes = part.blocks > 1 ? 32 : 4;        // of a group
+  // key above, index below it turned around: the larger the earlier in top-k's order
+  unsigned long long* list = reinterpret_cast<unsigned long long*>(dyn_smem);
+  const int lanes = 4 * part.blocks, at_group = threadIdx.x & (lanes - 1);      // of a group
   if (threadIdx.x == 0) { *count = 0; *bound_s = 0u; fs->answer = 0x7fffffff; fs->last = -1; }
   // (key 0 belongs to no logit but one that is not a number)
   uint32_t best = 0u;
@@ -590,16 +596,18 @@ __device__ bool sample_top_k_fast(const float* __restrict__ row, int V, const Ro
     if (l == l) best = max(best, order_key(l));
   });
   for (int o = 1; o < lanes; o <<= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
+  uint32_t* place = group_max + (part.rank * SAMPLE_THREADS + threadIdx.x) / lanes;
   if (part.blocks > 1) {
-    if (lane < part.blocks) *cl.map_shared_rank(group_max + part.rank * 32 + warp, lane) = best;
+    if (at_group < part.blocks) *cl.map_shared_rank(place, at_group) = best;
     cl.sync();
   } else {
-    if (lane % 4 == 0) group_max[threadIdx.x / 4] = best;
+    if (at_group == 0) *place = best;
     __syncthreads();
   }
-  if (threadIdx.x < TOPK_GROUPS) {                   // (fewer blocks than eight do not occur beside one: every place is written)
+  if (threadIdx.x < TOPK_GROUPS) {
     const uint32_t mine = group_max[threadIdx.x];
     int rank = 0;
+#pragma unroll 8
     for (int j = 0; j < TOPK_GROUPS; ++j) rank += group_max[j] > mine || (group_max[j] == mine && j < (int)threadIdx.x);
     if (rank == k - 1) *bound_s = mine;
   }
@@ -608,12 +616,11 @@ __device__ bool sample_top_k_fast(const float* __restrict__ row, int V, const Ro
   const uint32_t bound = max(*bound_s, MINUS_INFINITY_KEY + 1);
   {
     int* there = part.blocks > 1 ? cl.map_shared_rank(count, 0) : count;
-    uint32_t* keys = part.blocks > 1 ? cl.map_shared_rank(list_key, 0) : list_key;
-    int* idxs = part.blocks > 1 ? cl.map_shared_rank(list_idx, 0) : list_idx;
+    unsigned long long* all = part.blocks > 1 ? cl.map_shared_rank(list, 0) : list;
     for_strided(row, first, stride, V, [&](float l, int i) {
       if (l == l && order_key(l) >= bound) {
         const int at = atomicAdd(there, 1);
-        if (at < TOPK_LIST) { keys[at] = order_key(l); idxs[at] = i; }
+        if (at < TOPK_LIST) all[at] = (unsigned long long)order_key(l) << 32 | ~(uint32_t)i;
       }
     });
   }
@@ -623,13 +630,13 @@ __device__ bool sample_top_k_fast(const float* __restrict__ row, int V, const Ro
   if (n < k || n > TOPK_LIST) return false;          // fewer than k logits above minus infinity; very many ties
   // the k largest in descending order, ties by index (runtime/sampler.py:60-67)
   for (int e = threadIdx.x; e < n; e += SAMPLE_THREADS) {
-    const uint32_t key = list_key[e];
-    const int idx = list_idx[e];
+    const unsigned long long mine = list[e];
     int rank = 0;
-    for (int j = 0; j < n; ++j) rank += list_key[j] > key || (list_key[j] == key && list_idx[j] < idx);
+#pragma unroll 8
+    for (int j = 0; j < n; ++j) rank += list[j] > mine;
     if (rank < k) {
-      fs->kept_key[rank] = key;
-      fs->kept_idx[rank] = idx;
+      fs->kept_key[rank] = (uint32_t)(mine >> 32);
+      fs->kept_idx[rank] = (int)~(uint32_t)mine;
     }
   }
   __syncthreads();
@@ -649,7 +656,7 @@ __device__ bool sample_top_k_fast(const float* __restrict__ row, int V, const Ro
     __syncthreads();
     m = fs->n_kept;
   }
-  draw_from_list(fs->kept_key, fs->kept_idx, m, mx, inv_t, u, fs->red, fs, out);
+  draw_from_list(fs->kept_key, fs->kept_idx, m, mx, inv_t, u, fs->red, fs->q, fs, out);
   return true;
 }
 
@@ -671,7 +678,8 @@ __device__ bool sample_top_p_fast(const float* __restrict__ row, int V, float in
   float* hist_m = reinterpret_cast<float*>(cand_idx + FAST_CANDIDATES);             // [256]
   uint32_t* kept_key = reinterpret_cast<uint32_t*>(hist_m + SEL_BINS);              // [FAST_P_KEPT]
   int* kept_idx = reinterpret_cast<int*>(kept_key + FAST_P_KEPT);
-  static_assert(FAST_CANDIDATES * 8 + SEL_BINS * 4 + FAST_P_KEPT * 8 <= SAMPLE_SMEM, "the lists live in the histograms' shared memory");
+  double* kept_q = reinterpret_cast<double*>(kept_idx + FAST_P_KEPT);               // [FAST_P_KEPT]
+  static_assert(FAST_CANDIDATES * 8 + SEL_BINS * 4 + FAST_P_KEPT * 16 <= SAMPLE_SMEM, "the lists live in the histograms' shared memory");
   double row_sum;
   collect_candidates(row, V, inv_t, dyn_smem, sh_mi, fs->red, fs, mx_out, &row_sum);
   const MaxIdx mx = *mx_out;
@@ -708,14 +716,14 @@ __device__ bool sample_top_p_fast(const float* __restrict__ row, int V, float in
     }
   }
   __syncthreads();
-  draw_from_list(kept_key, kept_idx, fs->n_kept, mx.v, inv_t, u, fs->red, fs, out);
+  draw_from_list(kept_key, kept_idx, fs->n_kept, mx.v, inv_t, u, fs->red, kept_q, fs, out);
   return true;
 }
 
 __global__ void __launch_bounds__(SAMPLE_THREADS)
 sample_rows_kernel(const float* __restrict__ logits, int V, const float* __restrict__ temperature,
                    const double* __restrict__ uniform, const int* __restrict__ top_k, const float* __restrict__ top_p,
-                   int* __restrict__ out, int blocks) {
+                   int* __restrict__ out, int blocks_log2) {
   extern __shared__ __align__(16) unsigned char sample_smem[];
   __shared__ MaxIdx sh_mi[32], parts_mi[8];
   __shared__ uint32_t group_max[TOPK_GROUPS], bound_s;
@@ -730,15 +738,15 @@ sample_rows_kernel(const float* __restrict__ logits, int V, const float* __restr
   __shared__ int pick_part, pick_need, i_eq_s, result;
   __shared__ double pick_before;
   pdl_launch_dependents();       // a short kernel: the successor may be set up behind it
-  if (blocks > 1) cooperative_groups::this_cluster().sync();      // nobody reaches into the shared memory of a block that has not begun
+  if (blocks_log2 > 0) cooperative_groups::this_cluster().sync();      // nobody reaches into the shared memory of a block that has not begun
   pdl_wait();
   __shared__ FastShared fast;
-  const int r = blockIdx.x / blocks;
+  const int r = blockIdx.x >> blocks_log2;
   const float* row = logits + (size_t)r * V;
   RowPart part;
-  part.rank = blockIdx.x % blocks;
-  part.blocks = blocks;
-  const int share = ((V + blocks - 1) / blocks + 3) & ~3;
+  part.blocks = 1 << blocks_log2;
+  part.rank = blockIdx.x & (part.blocks - 1);
+  const int share = (((V + part.blocks - 1) >> blocks_log2) + 3) & ~3;
   part.from = min(part.rank * share, V);
   part.to = min(part.from + share, V);
   part.vec = (V & 3) == 0 && (reinterpret_cast<uintptr_t>(row) & 15) == 0;
@@ -1001,9 +1009,52 @@ __global__ void penalty_seen_kernel(float* __restrict__ logits, int V, const uns
   }
 }
 
+// A launch with clusters of `blocks` blocks (nullptr attribute list for one: a plain launch)
+static void sample_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[2], int rows, int blocks, int smem, cudaStream_t stream) {
+  cfg = {};
+  cfg.gridDim = dim3((unsigned)rows * blocks);
+  cfg.blockDim = dim3(SAMPLE_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = blocks;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+}
+
+// Blocks a row (log2): as many as leave every row's cluster on the GPU at once.  A block fills an SM (1,024 threads of 64 registers) and a cluster lies in one
+// GPC, so that is 15 rows of eight, 33 of four; rows that wait for a whole cluster's place pay for it however little its other
+// blocks have to do (151,936 logits, us, eight blocks / as chosen: 16 greedy rows 8.8 / 5.6, 128 38 / 10; 128 rows of top_p 0.9 212 / 73; 32 rows of top_k 20 31 / 16).
+static int row_blocks_log2(int R, int V) {
+  if (V < SAMPLE_SPLIT_FROM) return 0;
+  struct Fit {
+    int rows[SAMPLE_BLOCKS_LOG2 + 1] = {0, 0, 0, 0};
+    Fit() {
+      for (int lg = 1; lg <= SAMPLE_BLOCKS_LOG2; ++lg) {
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute attr[2];
+        sample_config(cfg, attr, num_sms(), 1 << lg, SAMPLE_SMEM, nullptr);
+        cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&rows[lg], sample_rows_kernel, &cfg) != cudaSuccess) rows[lg] = 0;
+      }
+      cudaGetLastError();
+    }
+  };
+  static const Fit fit;
+  int lg = SAMPLE_BLOCKS_LOG2;
+  while (lg > 0 && R > fit.rows[lg]) --lg;
+  return lg;
+}
+
 }  // namespace sllm
 
 using namespace sllm;
+
+// blocks that share a row in a launch of R rows of V logits
+SLLM_EXPORT int sllm_sample_rows_blocks(int R, int V) { return 1 << row_blocks_log2(R, V); }
 
 // temperature may be null (all rows greedy); uniform must hold R doubles when any temperature > 0.
 // top_k (int per row, <= 0: none) and top_p (float per row, < 0: none) may be null.
@@ -1022,22 +1073,15 @@ SLLM_EXPORT int sllm_sample_rows(const float* logits, int R, int V, const float*
     configured = true;
   }
   const int smem = (top_k || top_p) ? SAMPLE_SMEM : 0;
-  // a short row is one block's (and its groups of four lanes still see more than one logit)
-  const int blocks = V >= SAMPLE_SPLIT_FROM ? 8 : 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)R * blocks);
-  cfg.blockDim = dim3(SAMPLE_THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
+  const int lg = row_blocks_log2(R, V);
+  if (lg == 0) {
+    launch_kernel(sample_rows_kernel, R, SAMPLE_THREADS, smem, stream, logits, V, temperature, uniform, top_k, top_p, out, 0);
+    return launch_status("sample_rows");
+  }
+  cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = blocks;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  cudaLaunchKernelEx(&cfg, sample_rows_kernel, logits, V, temperature, uniform, top_k, top_p, out, blocks);
+  sample_config(cfg, attr, R, 1 << lg, smem, stream);
+  cudaLaunchKernelEx(&cfg, sample_rows_kernel, logits, V, temperature, uniform, top_k, top_p, out, lg);
   return launch_status("sample_rows");
 }
 

@@ -77,6 +77,7 @@ def _declare(L):
         "sllm_attention_simt": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int,
                                 c_int, c_int, c_float, c_int, c_int, c_void_p, c_float, c_void_p, c_int, c_void_p, c_int,
                                 c_void_p, c_void_p],
+        "sllm_sample_rows_blocks": [c_int, c_int],
         "sllm_sample_rows": [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
         "sllm_repetition_penalty": [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p],
         "sllm_mark_seen": [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p],

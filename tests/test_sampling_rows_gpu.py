@@ -69,3 +69,25 @@ def test_greedy_of_long_and_short_rows(V):
     clean = torch.nan_to_num(logits, nan=-float("inf"), neginf=-float("inf"), posinf=float("inf"))
     want = [int((row == row.max()).nonzero()[0]) for row in clean]
     assert ops.sample_rows(logits).tolist() == want
+
+
+@pytest.mark.parametrize("V", [49151, 49152, 65537, 151936])
+@pytest.mark.parametrize("R", [1, 14, 15, 16, 33, 34, 74, 75, 149])
+def test_few_rows_are_shared_by_blocks_and_many_are_not(V, R):
+    """All of a launch's blocks fit the GPU at once wherever a row has several (a block fills an SM), and a row's choice is the same however many blocks it
+    has: greedy, temperature alone, top-k with and without top-p, a top-k beyond the short form, top-p alone."""
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    blocks = ops.lib().sllm_sample_rows_blocks(R, V)
+    assert blocks in (1, 2, 4, 8) and (blocks == 1 or (R * blocks <= ops.num_sms() and V >= 49152))
+    g = torch.Generator(device=dev).manual_seed(V + R)
+    logits = torch.randn(R, V, device=dev, generator=g) * 3
+    i = torch.arange(R, device=dev) % 6
+    t = torch.where(i == 0, 0.0, 0.7)
+    k = torch.tensor([0, 0, 20, 200, 700, 0], dtype=torch.int32, device=dev)[i]
+    p = torch.tensor([-1.0, -1.0, 0.8, -1.0, 0.9, 0.95], device=dev)[i]
+    u = torch.rand(R, device=dev, generator=g, dtype=torch.float64)
+    got = ops.sample_rows(logits, t, u, k, p)
+    few = range(0, R, max(1, R // 12))
+    alone = [int(ops.sample_rows(logits[r:r + 1], t[r:r + 1], u[r:r + 1], k[r:r + 1], p[r:r + 1])) for r in few]
+    assert [int(got[r]) for r in few] == alone
