@@ -14,12 +14,16 @@
 //   and query head) the head's output is multiplied by the gate's sigmoid.  With `rel` [nkv, rel_n, nq / nkv] the score then takes in
 //   a bias by the distance from key to query (distances beyond the table: its last row) and the query head.
 //
-// Keys go by aligned blocks of 32 positions, block b to warp (b - first block) mod the block's warps.  In the scores a lane
-// is a key: it walks its own key's row (16 bytes a load where rows allow it) against the query in shared memory, so the 32
-// dot products of a block run side by side and none needs a sum over lanes; one online-softmax update a block; in the
-// weighted sum a lane is a channel and the block's 32 value rows are independent loads.  What bounds it is the latency of those loads: with
-// a key a step and a warp (every key's page, row and sum over lanes in one chain) a decode step of 3 requests at 190 keys took
-// 51 us, now 11; one token at 4,000 keys 1,020, now 70; a portion of 537 tokens 504, now 189 (14 heads of 64, 2 kv heads, float32).
+// Two ways through the keys.
+//   A key a lane (heads of up to 128 channels, from `simt_short` keys on): keys go by aligned blocks of 32 positions, block b to warp (b - first block) mod
+//   the block's warps.  In the scores a lane walks its own key's row (16 bytes a load where rows allow it) against the query in shared memory, so the 32
+//   dot products of a block run side by side and none needs a sum over lanes; one online-softmax update a block; in the
+//   weighted sum a lane is a channel and the block's 32 value rows are independent loads.  What bounds it is the latency of those loads: with
+//   a key a step and a warp (every key's page, row and sum over lanes in one chain) a decode step of 3 requests at 190 keys took
+//   51 us, now 11; one token at 4,000 keys 1,020, now 70; a portion of 537 tokens 504, now 189 (14 heads of 64, 2 kv heads, float32).
+//   Four keys a warp (wider heads, and few keys): aligned groups of four positions, a lane four channels at a time, four sums over lanes side by side, one
+//   online-softmax update.  A lane's own row is no longer a few lines of cache where heads are wide, and few keys leave most
+//   warps without a block of 32.
 // The warps' partial results are merged in warp order.  The order of every sum depends on the position alone.
 #include <math.h>
 #include <stdio.h>
@@ -30,6 +34,8 @@ namespace sllm {
 
 constexpr int ATT_WARPS = 8;
 constexpr int ATT_MAX_HD = 256;        // (instances of 64 and 128 channels too: the accumulators are registers)
+// keys below which four a warp are taken at once (128 keys of a window, 1,500 tokens, us, four a warp / a key a lane: 64 bfloat16 channels 206 / 153, 128 205 / 209, 128 float32 200 / 275)
+__host__ __device__ constexpr int simt_short(int max_hd) { return max_hd <= 64 ? 96 : 160; }
 constexpr int ATT_WIDE_HD = 640;       // a second instance for wider heads (a cached latent beside a rotated key part)
 
 // d consecutive channels of a row against the query in shared memory; VEC: 16 bytes a load (rows of whole 16-byte pieces)
@@ -54,6 +60,97 @@ __device__ __forceinline__ float simt_dot(const T* __restrict__ row, const float
   return (dot[0] + dot[1]) + (dot[2] + dot[3]);
 }
 
+// four consecutive channels from d on, zeros beyond hd
+template <typename T, bool VEC>
+__device__ __forceinline__ float4 simt_load4(const T* __restrict__ row, int d, int hd) {
+  if (VEC) {                               // (hd is a multiple of 4 then)
+    if (d >= hd) return make_float4(0.f, 0.f, 0.f, 0.f);
+    if constexpr (sizeof(T) == 4) {
+      return *reinterpret_cast<const float4*>(row + d);
+    } else {
+      const uint2 raw = *reinterpret_cast<const uint2*>(row + d);
+      const T* v = reinterpret_cast<const T*>(&raw);
+      return make_float4(to_f32(v[0]), to_f32(v[1]), to_f32(v[2]), to_f32(v[3]));
+    }
+  }
+  return make_float4(d < hd ? to_f32(row[d]) : 0.f, d + 1 < hd ? to_f32(row[d + 1]) : 0.f, d + 2 < hd ? to_f32(row[d + 2]) : 0.f,
+                     d + 3 < hd ? to_f32(row[d + 3]) : 0.f);
+}
+
+// The keys lo .. pos of one query head, four a warp: the warp's maximum m, its sum l (known to all lanes) and its weighted sum of values in acc_s.
+template <typename TC, int MAX_HD, bool VEC>
+__device__ __forceinline__ void simt_groups(const TC* __restrict__ k_cache, const TC* __restrict__ v_cache, const int* __restrict__ bt, const float* qs,
+                                            float* acc_s, int lo, int pos, int kvh, int nkv, int G, int g, int hd, int page_size, float scale,
+                                            float softcap, const float* __restrict__ rel, int rel_n, float& m, float& l) {
+  constexpr int NC = (MAX_HD + 127) / 128;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float4 acc[NC];
+#pragma unroll
+  for (int i = 0; i < NC; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int j0 = lo / 4 * 4 + warp * 4; j0 <= pos; j0 += ATT_WARPS * 4) {
+    const int j = j0 + (lane & 3);
+    const int page = j >= lo && j <= pos ? bt[j / page_size] : -1;         // a page that was given back is never dereferenced
+    const unsigned counts = __ballot_sync(0xffffffffu, page >= 0) & 15u;   // one answer for all lanes
+    if (counts == 0) continue;
+    const long long mine = page < 0 ? 0 : (((long long)page * nkv + kvh) * page_size + (j % page_size)) * hd;
+    size_t row[4];
+    float dot[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int u = 0; u < 4; ++u) row[u] = (size_t)__shfl_sync(0xffffffffu, mine, u);
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+      const int d = 4 * (lane + 32 * i);
+      if (d >= hd) break;
+      const float4 q4 = *reinterpret_cast<const float4*>(qs + d);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (counts >> u & 1) {
+          const float4 k4 = simt_load4<TC, VEC>(k_cache + row[u], d, hd);
+          dot[u] = fmaf(q4.w, k4.w, fmaf(q4.z, k4.z, fmaf(q4.y, k4.y, fmaf(q4.x, k4.x, dot[u]))));
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) dot[u] += __shfl_xor_sync(0xffffffffu, dot[u], o);
+    float s[4], m_new = m;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      s[u] = softcap > 0.f ? softcap * tanhf(dot[u] * scale / softcap) : dot[u] * scale;
+      if (rel != nullptr && counts >> u & 1) s[u] += rel[((size_t)kvh * rel_n + min(pos - j0 - u, rel_n - 1)) * G + g];
+      if (counts >> u & 1) m_new = fmaxf(m_new, s[u]);
+    }
+    const float corr = expf(m - m_new);              // exp(-inf) = 0 on the first group
+    m = m_new;
+    l *= corr;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      s[u] = counts >> u & 1 ? expf(s[u] - m_new) : 0.f;
+      l += s[u];
+    }
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+      const int d = 4 * (lane + 32 * i);
+      if (d >= hd) break;
+      acc[i].x *= corr; acc[i].y *= corr; acc[i].z *= corr; acc[i].w *= corr;
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (counts >> u & 1) {
+          const float4 v4 = simt_load4<TC, VEC>(v_cache + row[u], d, hd);
+          acc[i].x = fmaf(s[u], v4.x, acc[i].x);
+          acc[i].y = fmaf(s[u], v4.y, acc[i].y);
+          acc[i].z = fmaf(s[u], v4.z, acc[i].z);
+          acc[i].w = fmaf(s[u], v4.w, acc[i].w);
+        }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NC; ++i) {
+    const int d = 4 * (lane + 32 * i);
+    if (d < hd) *reinterpret_cast<float4*>(acc_s + d) = acc[i];            // (MAX_HD is a multiple of 4)
+  }
+}
+
 template <typename TQ, typename TC, int ATT_MAX_HD, bool VEC>
 __global__ void __launch_bounds__(ATT_WARPS * 32)
 attention_simt_kernel(const TQ* __restrict__ q, const TC* __restrict__ k_cache, const TC* __restrict__ v_cache,
@@ -61,11 +158,12 @@ attention_simt_kernel(const TQ* __restrict__ q, const TC* __restrict__ k_cache, 
                       const int* __restrict__ seq_of_token, int nq, int nkv, int hd, int page_size, float scale,
                       int window, int chunk, const float* __restrict__ sink, float softcap, const float* __restrict__ gate, int gate_ld,
                       const float* __restrict__ rel, int rel_n, TQ* __restrict__ out) {
-  __shared__ float qs[ATT_MAX_HD];
-  __shared__ float acc_s[ATT_WARPS][ATT_MAX_HD];
+  __shared__ __align__(16) float qs[ATT_MAX_HD];
+  __shared__ __align__(16) float acc_s[ATT_WARPS][ATT_MAX_HD];
   __shared__ float m_s[ATT_WARPS], l_s[ATT_WARPS];
-  __shared__ float p_s[ATT_WARPS][32];
-  __shared__ size_t row_s[ATT_WARPS][32];
+  constexpr bool NARROW = ATT_MAX_HD <= 128;
+  __shared__ float p_s[NARROW ? ATT_WARPS : 1][32];
+  __shared__ size_t row_s[NARROW ? ATT_WARPS : 1][32];
   pdl_wait();
   const int t = blockIdx.x, h = blockIdx.y;
   const int G = nq / nkv, kvh = h / G;
@@ -75,64 +173,68 @@ attention_simt_kernel(const TQ* __restrict__ q, const TC* __restrict__ k_cache, 
   int lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
   if (chunk > 0) lo = max(lo, pos / chunk * chunk);
 
-  for (int d = threadIdx.x; d < hd; d += blockDim.x) qs[d] = to_f32(q[((size_t)t * nq + h) * hd + d]);
+  for (int d = threadIdx.x; d < ATT_MAX_HD; d += blockDim.x) qs[d] = d < hd ? to_f32(q[((size_t)t * nq + h) * hd + d]) : 0.f;
   __syncthreads();
 
-  float acc[ATT_MAX_HD / 32];
+  float m = -INFINITY, l = 0.f;
+  if (!NARROW || pos - lo < simt_short(ATT_MAX_HD)) {
+    simt_groups<TC, ATT_MAX_HD, VEC>(k_cache, v_cache, bt, qs, acc_s[warp], lo, pos, kvh, nkv, G, h % G, hd, page_size, scale, softcap, rel, rel_n, m, l);
+  } else if constexpr (NARROW) {
+    float acc[ATT_MAX_HD / 32];
 #pragma unroll
-  for (int i = 0; i < ATT_MAX_HD / 32; ++i) acc[i] = 0.f;
-  float m = -INFINITY, l = 0.f;                      // l: this lane's keys alone; added up over the lanes at the end
-
-  for (int j0 = lo / 32 * 32 + warp * 32; j0 <= pos; j0 += ATT_WARPS * 32) {
-    const int j = j0 + lane;
-    const int page = j >= lo && j <= pos ? bt[j / page_size] : -1;         // a page that was given back is never dereferenced
-    const size_t row = page < 0 ? 0 : (((size_t)page * nkv + kvh) * page_size + (j % page_size)) * hd;
-    float s = -INFINITY;
-    if (page >= 0) {
-      const float dot = simt_dot<TC, VEC>(k_cache + row, qs, hd);
-      s = softcap > 0.f ? softcap * tanhf(dot * scale / softcap) : dot * scale;
-      if (rel != nullptr) s += rel[((size_t)kvh * rel_n + min(pos - j, rel_n - 1)) * G + h % G];
-    }
-    const unsigned counts = __ballot_sync(0xffffffffu, page >= 0);
-    if (counts == 0) continue;
-    const float m_new = fmaxf(m, warp_max(s));
-    const float corr = expf(m - m_new);              // exp(-inf) = 0 on the first block
-    const float p = page < 0 ? 0.f : expf(s - m_new);
-    l = l * corr + p;
-    m = m_new;
-    p_s[warp][lane] = p;
-    row_s[warp][lane] = row;                         // (a key that does not count: row 0 of the pages, times zero is not taken)
-    __syncwarp();
+    for (int i = 0; i < ATT_MAX_HD / 32; ++i) acc[i] = 0.f;
+    // l: this lane's keys alone; added up over the lanes at the end
+    for (int j0 = lo / 32 * 32 + warp * 32; j0 <= pos; j0 += ATT_WARPS * 32) {
+      const int j = j0 + lane;
+      const int page = j >= lo && j <= pos ? bt[j / page_size] : -1;         // a page that was given back is never dereferenced
+      const size_t row = page < 0 ? 0 : (((size_t)page * nkv + kvh) * page_size + (j % page_size)) * hd;
+      float s = -INFINITY;
+      if (page >= 0) {
+        const float dot = simt_dot<TC, VEC>(k_cache + row, qs, hd);
+        s = softcap > 0.f ? softcap * tanhf(dot * scale / softcap) : dot * scale;
+        if (rel != nullptr) s += rel[((size_t)kvh * rel_n + min(pos - j, rel_n - 1)) * G + h % G];
+      }
+      const unsigned counts = __ballot_sync(0xffffffffu, page >= 0);
+      if (counts == 0) continue;
+      const float m_new = fmaxf(m, warp_max(s));
+      const float corr = expf(m - m_new);              // exp(-inf) = 0 on the first block
+      const float p = page < 0 ? 0.f : expf(s - m_new);
+      l = l * corr + p;
+      m = m_new;
+      p_s[warp][lane] = p;
+      row_s[warp][lane] = row;                         // (a key that does not count: row 0 of the pages, times zero is not taken)
+      __syncwarp();
 #pragma unroll
-    for (int i = 0; i < ATT_MAX_HD / 32; ++i) acc[i] *= corr;
-    if (counts == 0xffffffffu) {
+      for (int i = 0; i < ATT_MAX_HD / 32; ++i) acc[i] *= corr;
+      if (counts == 0xffffffffu) {
 #pragma unroll 8
-      for (int u = 0; u < 32; ++u) {
-        const float pu = p_s[warp][u];
-        const TC* vr = v_cache + row_s[warp][u];
+        for (int u = 0; u < 32; ++u) {
+          const float pu = p_s[warp][u];
+          const TC* vr = v_cache + row_s[warp][u];
 #pragma unroll
-        for (int i = 0; i < ATT_MAX_HD / 32; ++i)
-          if (lane + 32 * i < hd) acc[i] = fmaf(pu, to_f32(vr[lane + 32 * i]), acc[i]);
-      }
-    } else {
-      for (unsigned left = counts; left != 0; left &= left - 1) {
-        const int u = __ffs(left) - 1;
-        const float pu = p_s[warp][u];
-        const TC* vr = v_cache + row_s[warp][u];
+          for (int i = 0; i < ATT_MAX_HD / 32; ++i)
+            if (lane + 32 * i < hd) acc[i] = fmaf(pu, to_f32(vr[lane + 32 * i]), acc[i]);
+        }
+      } else {
+        for (unsigned left = counts; left != 0; left &= left - 1) {
+          const int u = __ffs(left) - 1;
+          const float pu = p_s[warp][u];
+          const TC* vr = v_cache + row_s[warp][u];
 #pragma unroll
-        for (int i = 0; i < ATT_MAX_HD / 32; ++i)
-          if (lane + 32 * i < hd) acc[i] = fmaf(pu, to_f32(vr[lane + 32 * i]), acc[i]);
+          for (int i = 0; i < ATT_MAX_HD / 32; ++i)
+            if (lane + 32 * i < hd) acc[i] = fmaf(pu, to_f32(vr[lane + 32 * i]), acc[i]);
+        }
       }
+      __syncwarp();
     }
-    __syncwarp();
-  }
-  l = warp_sum(l);
-  if (lane == 0) { m_s[warp] = m; l_s[warp] = l; }
+    l = warp_sum(l);
 #pragma unroll
-  for (int i = 0; i < ATT_MAX_HD / 32; ++i) {
-    const int d = lane + 32 * i;
-    if (d < hd) acc_s[warp][d] = acc[i];
+    for (int i = 0; i < ATT_MAX_HD / 32; ++i) {
+      const int d = lane + 32 * i;
+      if (d < hd) acc_s[warp][d] = acc[i];
+    }
   }
+  if (lane == 0) { m_s[warp] = m; l_s[warp] = l; }
   __syncthreads();
   float mm = -INFINITY;
 #pragma unroll
@@ -159,7 +261,7 @@ template <typename T>
 static int simt_launch(const T* q, const T* k_cache, const T* v_cache, const int* block_tables, int max_pages, const int* positions,
                        const int* seq_of_token, int num_tokens, int nq, int nkv, int hd, int page_size, float scale, int window, int chunk,
                        const float* sink, float softcap, const float* gate, int gate_ld, const float* rel, int rel_n, T* out, cudaStream_t stream) {
-  const bool vec = hd * (int)sizeof(T) % 16 == 0 && (reinterpret_cast<uintptr_t>(k_cache) & 15) == 0;
+  const bool vec = hd * (int)sizeof(T) % 16 == 0 && ((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) == 0;
   auto kernel = hd <= 64 ? (vec ? attention_simt_kernel<T, T, 64, true> : attention_simt_kernel<T, T, 64, false>)
               : hd <= 128 ? (vec ? attention_simt_kernel<T, T, 128, true> : attention_simt_kernel<T, T, 128, false>)
               : hd <= ATT_MAX_HD ? (vec ? attention_simt_kernel<T, T, ATT_MAX_HD, true> : attention_simt_kernel<T, T, ATT_MAX_HD, false>)

@@ -60,3 +60,32 @@ def test_attention_around_blocks_of_32_keys(dtype, hd, ps, window):
         want = torch.einsum("hj,jhd->hd", torch.softmax(s, -1), v)
         tol = 2e-5 if dtype == torch.float32 else 1e-2
         torch.testing.assert_close(got[i], want, rtol=tol, atol=tol)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("hd,nkv", [(64, 2), (100, 2), (128, 2), (132, 2), (255, 2), (300, 1), (576, 1), (640, 1)])
+@pytest.mark.parametrize("window,softcap", [(None, 0.0), (90, 5.0), (150, 0.0)])
+def test_attention_four_keys_a_warp(dtype, hd, nkv, window, softcap):
+    """Wide heads and, of narrow ones, contexts and windows on both sides of the line between the two ways through the keys, with all that a score and a
+    head pass, pages before the window given back: against the same in float32."""
+    import sllm_b200.ops as ops
+    from tests import torch_ops as ref
+    dev = cuda_or_skip()
+    g = torch.Generator(device=dev).manual_seed(hd)
+    nq, ps, ctx = 4, 8, [1, 3, 4, 5, 95, 96, 97, 98, 159, 160, 161, 162, 290]
+    per = -(-max(ctx) // ps)
+    kc, vc = (torch.randn(len(ctx) * per, nkv, ps, hd, device=dev, generator=g).to(dtype) for _ in range(2))
+    bt = torch.randperm(len(ctx) * per, device=dev, generator=g).int().reshape(len(ctx), per).contiguous()
+    for i, c in enumerate(ctx):
+        if window:
+            bt[i, :max(0, c - window) // ps] = -1
+    pos = torch.tensor([c - 1 for c in ctx], dtype=torch.int32, device=dev)
+    seq = torch.arange(len(ctx), dtype=torch.int32, device=dev)
+    q = torch.randn(len(ctx), nq * hd, device=dev, generator=g).to(dtype)
+    sink = torch.randn(nq, device=dev, generator=g)
+    gate = (torch.randn(len(ctx), nq + 3, device=dev, generator=g), 3)
+    args = (bt, pos, seq, nq, nkv, hd, hd ** -0.5, window, None, sink, softcap, gate)
+    got = ops.attention_simt(q, kc, vc, *args).float()
+    want = ref.attention_simt(q.float(), kc.float(), vc.float(), *args)
+    tol = 2e-5 if dtype == torch.float32 else 1e-2           # (bfloat16: the result's own rounding, 2^-8)
+    torch.testing.assert_close(got, want, rtol=tol, atol=tol)
