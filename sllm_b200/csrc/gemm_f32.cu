@@ -12,9 +12,9 @@
 //   of its own (cp.async, 6 stages of 32 rows x 32 k), a lane per row of W, so nothing but its own copies is waited for.  The
 //   S segments of the same 32 rows are the warps of a cluster of CTAs of two warps, so that a matrix of 896 rows still
 //   reaches 112 SMs with 40 KB in flight on each; they meet in distributed shared memory.
-// * Beyond: `gemm_f32_tile_kernel`, bound by the FMA pipes and by issue slots: 128 x 128 (64 or 32 x 128) tiles, 8 x 8 (4 x 8) results
+// * Beyond: `gemm_f32_tile_kernel`, bound by the FMA pipes and by issue slots: tiles of 128, 64 or 32 x 128 or 64, 8 x 8 (4 x 8, 4 x 4) results
 //   a thread, a three-stage cp.async ring; the S segments of a tile are the CTAs of a cluster, which add up through distributed shared
-//   memory.  The packed form matters here: it halves the issue slots of the multiply-adds, which leaves room for the loads from shared memory.
+//   memory, or where the tiles alone fill the GPU one CTA's, one after the other.  The packed form matters here: it halves the issue slots of the multiply-adds, which leaves room for the loads from shared memory.
 //
 // Measured (us; floor: W at 6.65 TB/s): 3 rows, 9,728 x 896 10.0 (floor 5.2; 82 with the one 64 x 64 tile form there was before), 896 x 4,864 10.4
 // (2.6; 342), 151,936 x 896 93 (82; 503); 537 rows 259 (36 TFLOP/s; 314) and 150 (31; 297); 2,048 rows of 9,728 x 896 844 (42 TFLOP/s of 74; 1,015).
@@ -157,42 +157,56 @@ gemm_f32_skinny_kernel(const float* __restrict__ A, const float* __restrict__ W,
 
 // ---- tiles --------------------------------------------------------------------------------------------------------------
 
-constexpr int TL_BN = 128, TL_BK = 32, TL_PITCH = TL_BK + 4, TL_STAGES = 3;
+constexpr int TL_BK = 32, TL_PITCH = TL_BK + 4, TL_STAGES = 3;
 
-__host__ __device__ constexpr int tl_stage_floats(int BM) { return (BM + TL_BN) * TL_PITCH; }
+__host__ __device__ constexpr int tl_stage_floats(int BM, int BN) { return (BM + BN) * TL_PITCH; }
 // the ring, and afterwards the tile's partial sums
-__host__ __device__ constexpr int tl_smem(int BM) { return 4 * TL_STAGES * tl_stage_floats(BM); }
-static_assert(TL_STAGES * tl_stage_floats(32) >= 32 * TL_BN && TL_STAGES * tl_stage_floats(128) >= 128 * TL_BN, "the ring holds a tile");
+__host__ __device__ constexpr int tl_smem(int BM, int BN) { return 4 * TL_STAGES * tl_stage_floats(BM, BN); }
+static_assert(TL_STAGES * tl_stage_floats(32, 128) >= 32 * 128 && TL_STAGES * tl_stage_floats(128, 128) >= 128 * 128, "the ring holds a tile");
+__host__ __device__ constexpr int tl_threads(int BM) { return BM == 32 ? 128 : 256; }
 
-template <int BM, bool VEC>
-__global__ void __launch_bounds__(BM == 32 ? 128 : 256, BM == 128 ? 1 : 2)
+// FOLD: a CTA takes all the segments of its tile, one after the other; else the segments are the CTAs of a cluster (or there is one).
+template <int BM, int BN, bool VEC, bool FOLD>
+__global__ void __launch_bounds__(tl_threads(BM), BM == 128 ? 1 : 2)
 gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
                      int M, int N, int K, int S, int seg) {
-  constexpr int THREADS = BM == 32 ? 128 : 256, TM = BM == 128 ? 8 : 4, TN = 8;
+  constexpr int THREADS = tl_threads(BM), TM = BM == 128 ? 8 : 4, TN = BN / 16;
   constexpr int WM = TM * 4, WN = TN * 8;            // a warp's share: lanes 4 x 8, the rows of a lane 4 (of W: 8) apart
-  constexpr int WARPS_N = TL_BN / WN;
+  constexpr int WARPS_N = BN / WN;
+  static_assert(BM / WM * WARPS_N == THREADS / 32, "the warps' shares are the tile");
   extern __shared__ __align__(16) float sm[];
   // eight consecutive rows are what a quarter of a warp reads, and a pitch of 36 floats puts them on different banks
   const int tid = threadIdx.x, lane = tid % 32, warp = tid / 32;
   const int mt = warp / WARPS_N * WM + lane / 8, nt = warp % WARPS_N * WN + lane % 8;
-  const int n0 = blockIdx.x * TL_BN, m0 = blockIdx.y * BM;
-  const int kl = tid % 8 * 4, row = tid / 8;         // eight threads a row when staging
+  const int n0 = blockIdx.x * BN, m0 = blockIdx.y * BM;
   pdl_wait();
-  const int s = blockIdx.z, k0 = s * seg, kend = min(K, k0 + seg);
+  const int s = FOLD ? 0 : blockIdx.z, k0 = s * seg, kend = FOLD ? K : min(K, k0 + seg);
   const int steps = kend > k0 ? (kend - k0 + TL_BK - 1) / TL_BK : 0;
+  const int fold = FOLD ? seg / TL_BK : 0;           // steps of a segment (a whole number: `launch`)
   unsigned long long two[TM][TN];
+  float sum[FOLD ? TM : 1][FOLD ? TN : 1];           // the segments before
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
     for (int j = 0; j < TN; ++j) two[i][j] = 0;
   auto stage = [&](int it) {
-    float* st = sm + (it % TL_STAGES) * tl_stage_floats(BM) + row * TL_PITCH + kl;
-    const int k = k0 + it * TL_BK + kl, from = k < K ? k : 0;
+    float* st = sm + (it % TL_STAGES) * tl_stage_floats(BM, BN);
+    if constexpr (VEC) {                             // eight threads a row
+      const int kl = tid % 8 * 4, row = tid / 8, k = k0 + it * TL_BK + kl, from = k < K ? k : 0;
+      st += row * TL_PITCH + kl;
 #pragma unroll
-    for (int i = 0; i < BM; i += THREADS / 8) f32_stage4<VEC>(st + i * TL_PITCH, A + (size_t)min(m0 + row + i, M - 1) * K + from, k, kend);
+      for (int i = 0; i < BM; i += THREADS / 8) f32_stage4<true>(st + i * TL_PITCH, A + (size_t)min(m0 + row + i, M - 1) * K + from, k, kend);
 #pragma unroll
-    for (int i = 0; i < TL_BN; i += THREADS / 8)
-      f32_stage4<VEC>(st + (BM + i) * TL_PITCH, W + (size_t)min(n0 + row + i, N - 1) * K + from, k, kend);
+      for (int i = 0; i < BN; i += THREADS / 8)
+        f32_stage4<true>(st + (BM + i) * TL_PITCH, W + (size_t)min(n0 + row + i, N - 1) * K + from, k, kend);
+    } else {                                         // a warp a row: neighbouring lanes copy neighbouring numbers
+      const int k = k0 + it * TL_BK + lane, from = k < K ? k : 0, bytes = k < kend ? 4 : 0;
+      st += warp * TL_PITCH + lane;
+#pragma unroll 4
+      for (int i = 0; i < BM; i += THREADS / 32) f32_copy4(st + i * TL_PITCH, A + (size_t)min(m0 + warp + i, M - 1) * K + from, bytes);
+#pragma unroll 4
+      for (int i = 0; i < BN; i += THREADS / 32) f32_copy4(st + (BM + i) * TL_PITCH, W + (size_t)min(n0 + warp + i, N - 1) * K + from, bytes);
+    }
   };
 #pragma unroll
   for (int p = 0; p < TL_STAGES - 1; ++p) {
@@ -204,10 +218,21 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
     __syncthreads();
     if (it + TL_STAGES - 1 < steps) stage(it + TL_STAGES - 1);
     f32_commit();
-    const float* as = sm + (it % TL_STAGES) * tl_stage_floats(BM) + mt * TL_PITCH;
-    const float* ws = sm + (it % TL_STAGES) * tl_stage_floats(BM) + (BM + nt) * TL_PITCH;
+    const float* as = sm + (it % TL_STAGES) * tl_stage_floats(BM, BN) + mt * TL_PITCH;
+    const float* ws = sm + (it % TL_STAGES) * tl_stage_floats(BM, BN) + (BM + nt) * TL_PITCH;
+    if (FOLD && it % fold == 0 && it > 0) {
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+          sum[i][j] = it == fold ? f32_both(two[i][j]) : sum[i][j] + f32_both(two[i][j]);
+          two[i][j] = 0;
+        }
+    }
+    const int left = kend - k0 - it * TL_BK;         // (what lies beyond is zeros)
 #pragma unroll
     for (int k = 0; k < TL_BK; k += 4) {
+      if (!VEC && k >= left) break;
       ulonglong2 a[TM];
 #pragma unroll
       for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(as + i * 4 * TL_PITCH + k);
@@ -222,7 +247,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
     }
   }
   f32_wait<0>();
-  if (S == 1) {
+  if (FOLD || S == 1) {
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
       const int m = m0 + mt + i * 4;
@@ -230,28 +255,33 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
 #pragma unroll
       for (int j = 0; j < TN; ++j) {
         const int n = n0 + nt + j * 8;
-        if (n < N) C[(size_t)m * N + n] = f32_both(two[i][j]) + (bias ? bias[n] : 0.f);
+        if (n >= N) continue;
+        float v = f32_both(two[i][j]);
+        if constexpr (FOLD) v = sum[i][j] + v;
+        C[(size_t)m * N + n] = v + (bias ? bias[n] : 0.f);
       }
     }
     return;
   }
-  __syncthreads();                                   // everybody has read the last stage
+  if constexpr (!FOLD) {
+    __syncthreads();                                 // everybody has read the last stage
 #pragma unroll
-  for (int i = 0; i < TM; ++i)
+    for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) sm[(mt + i * 4) * TL_BN + nt + j * 8] = f32_both(two[i][j]);
-  cg::cluster_group cl = cg::this_cluster();
-  cl.sync();
-  // each CTA of the cluster adds up its share of the tile's rows, the segments in order
-  const int share = BM / S;
-  for (int i = tid; i < share * TL_BN; i += THREADS) {
-    const int r = s * share + i / TL_BN, c = i % TL_BN;
-    if (m0 + r >= M || n0 + c >= N) continue;
-    float v = *cl.map_shared_rank(sm + r * TL_BN + c, 0);
-    for (int o = 1; o < S; ++o) v += *cl.map_shared_rank(sm + r * TL_BN + c, o);
-    C[(size_t)(m0 + r) * N + n0 + c] = v + (bias ? bias[n0 + c] : 0.f);
+      for (int j = 0; j < TN; ++j) sm[(mt + i * 4) * BN + nt + j * 8] = f32_both(two[i][j]);
+    cg::cluster_group cl = cg::this_cluster();
+    cl.sync();
+    // each CTA of the cluster adds up its share of the tile's rows, the segments in order
+    const int share = BM / S;
+    for (int i = tid; i < share * BN; i += THREADS) {
+      const int r = s * share + i / BN, c = i % BN;
+      if (m0 + r >= M || n0 + c >= N) continue;
+      float v = *cl.map_shared_rank(sm + r * BN + c, 0);
+      for (int o = 1; o < S; ++o) v += *cl.map_shared_rank(sm + r * BN + c, o);
+      C[(size_t)(m0 + r) * N + n0 + c] = v + (bias ? bias[n0 + c] : 0.f);
+    }
+    cl.sync();                                       // nobody leaves while its sums are being read
   }
-  cl.sync();                                         // nobody leaves while its sums are being read
 }
 
 // Segments of K: as many (1, 2, 4, 8) as give the skinny kernel four warps of 32 rows an SM, none shorter than 64.  A warp is bound by the
@@ -294,12 +324,51 @@ static int launch_skinny(const float* A, const float* W, const float* bias, floa
                          4 * SK_WARPS * SK_STAGES * sk_stage_floats(MT), dim3(cluster, 1, 1), A, W, bias, C, M, N, K, S, seg, stream);
 }
 
-template <int BM, bool VEC>
+template <int BM, int BN, bool VEC, bool FOLD>
 static int launch_tiles(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int S, int seg, cudaStream_t stream) {
-  const int rows = (M + BM - 1) / BM;
+  const int rows = (M + BM - 1) / BM, cols = (N + BN - 1) / BN;
   SLLM_REQUIRE(rows <= 65535, "gemm_f32: M=%d is too large for one launch", M);
-  return launch_clusters(gemm_f32_tile_kernel<BM, VEC>, dim3((N + TL_BN - 1) / TL_BN, rows, S), BM == 32 ? 128 : 256, tl_smem(BM),
-                         dim3(1, 1, S), A, W, bias, C, M, N, K, S, seg, stream);
+  const int parts = FOLD ? 1 : S;
+  return launch_clusters(gemm_f32_tile_kernel<BM, BN, VEC, FOLD>, dim3(cols, rows, parts), tl_threads(BM), tl_smem(BM, BN), dim3(1, 1, parts), A, W, bias, C,
+                         M, N, K, S, seg, stream);
+}
+
+// The forms of the tiles and what they take, us: a step of 32 k of a CTA no less than `wait` (latency) nor than `work` times the CTAs that share its SM; `once` a
+// tile; `cluster` the pass over the cluster's sums, times the CTAs an SM; `launch`.  Fitted to 26 matrices of 24 x 1,024 to 32,000 x 512 with 17 to 4,096 rows; without
+// whole 16-byte pieces (`vec` false) copies of 4 bytes weigh on every step.
+struct TileForm {
+  int bm, bn, per_sm, fold;
+  float wait[2], work[2], once[2], cluster[2], launch[2], margin;      // [whole pieces]; margin: how much better it must look, the model's error
+};
+constexpr TileForm TILE_FORMS[] = {
+    {32, 64, 4, 0, {0.82f, 0.66f}, {0.46f, 0.47f}, {0.f, 0.f}, {1.68f, 0.88f}, {1.96f, 2.19f}, 1.2f},
+    {32, 128, 3, 0, {1.66f, 1.18f}, {0.91f, 0.86f}, {0.f, 0.f}, {3.92f, 2.11f}, {1.48f, 2.37f}, 1.0f},
+    {64, 128, 2, 0, {2.38f, 1.95f}, {1.52f, 1.74f}, {0.f, 0.f}, {5.42f, 3.2f}, {0.97f, 2.38f}, 1.0f},
+    {64, 64, 2, 1, {1.64f, 1.15f}, {1.32f, 1.03f}, {0.f, 0.f}, {0.f, 0.f}, {0.41f, 1.72f}, 1.2f},
+    {64, 128, 2, 1, {2.69f, 2.28f}, {2.12f, 1.85f}, {0.f, 0.f}, {0.f, 0.f}, {0.02f, 3.16f}, 1.1f},
+    {128, 128, 1, 1, {3.99f, 3.34f}, {0.04f, 2.43f}, {0.f, 3.7f}, {0.f, 0.f}, {0.f, 0.06f}, 1.1f},
+};
+// The form that finishes first: waves of CTAs an SM, and never faster than W streams in once per row of tiles (2 TB/s).  (us, one form for all rows before: 64 x
+// 64 matrix, 2,048 rows 8.4 -> 3.4; 2,304 x 768, 2,048 rows 243 -> 169 with the segments in turn; 896 x 896, 130 rows 19.3 -> 13.1.)
+static int tile_form(int M, int N, int K, int S, int seg, bool vec) {
+  const int sms = num_sms();
+  int best = 2;
+  float least = 0.f;
+  for (int f = 0; f < (int)(sizeof(TILE_FORMS) / sizeof(TileForm)); ++f) {
+    const TileForm& t = TILE_FORMS[f];
+    if (t.fold && S == 1) continue;                  // (that is the form without)
+    if (t.bm < 64 && M > 65535 * t.bm) continue;     // (a launch's rows of tiles)
+    const long long rows = (M + t.bm - 1) / t.bm, ctas = rows * ((N + t.bn - 1) / t.bn) * (t.fold ? 1 : S), per = (ctas + sms - 1) / sms;
+    const float steps = (float)((t.fold || seg > K ? K + TL_BK - 1 : seg) / TL_BK);
+    const auto wave = [&](long long n) { return n == 0 ? 0.f : t.once[vec] + steps * fmaxf(t.wait[vec], (float)n * t.work[vec]); };
+    float us = t.launch[vec] + (float)(per / t.per_sm) * wave(t.per_sm) + wave(per % t.per_sm) + (S > 1 ? t.cluster[vec] * (float)per : 0.f);
+    us = t.margin * fmaxf(us, (float)rows * (float)N * (float)K * 2e-6f);
+    if (least == 0.f || us < least) {
+      best = f;
+      least = us;
+    }
+  }
+  return best;
 }
 
 template <bool VEC>
@@ -310,12 +379,14 @@ static int launch(const float* A, const float* W, const float* bias, float* C, i
   if (M <= 4) return launch_skinny<4, VEC>(A, W, bias, C, M, N, K, S, seg, stream);
   if (M <= 8) return launch_skinny<8, VEC>(A, W, bias, C, M, N, K, S, seg, stream);
   if (M <= 16) return launch_skinny<16, VEC>(A, W, bias, C, M, N, K, S, seg, stream);
-  if (M <= 32) return launch_tiles<32, VEC>(A, W, bias, C, M, N, K, S, seg, stream);
-  // 128-row tiles (one CTA an SM) or 64-row tiles (two): whichever needs less time in waves
-  const long long cols = (long long)((N + TL_BN - 1) / TL_BN) * S, sms = num_sms();
-  const long long big = ((M + 127) / 128 * cols + sms - 1) / sms * 2, small = ((M + 63) / 64 * cols + 2 * sms - 1) / (2 * sms) * 2;
-  if (M > 64 && big < small) return launch_tiles<128, VEC>(A, W, bias, C, M, N, K, S, seg, stream);
-  return launch_tiles<64, VEC>(A, W, bias, C, M, N, K, S, seg, stream);
+  switch (tile_form(M, N, K, S, seg, VEC)) {
+    case 0: return launch_tiles<32, 64, VEC, false>(A, W, bias, C, M, N, K, S, seg, stream);
+    case 1: return launch_tiles<32, 128, VEC, false>(A, W, bias, C, M, N, K, S, seg, stream);
+    case 2: return launch_tiles<64, 128, VEC, false>(A, W, bias, C, M, N, K, S, seg, stream);
+    case 3: return launch_tiles<64, 64, VEC, true>(A, W, bias, C, M, N, K, S, seg, stream);
+    case 4: return launch_tiles<64, 128, VEC, true>(A, W, bias, C, M, N, K, S, seg, stream);
+  }
+  return launch_tiles<128, 128, VEC, true>(A, W, bias, C, M, N, K, S, seg, stream);
 }
 
 }  // namespace sllm

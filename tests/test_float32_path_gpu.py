@@ -89,3 +89,24 @@ def test_attention_four_keys_a_warp(dtype, hd, nkv, window, softcap):
     want = ref.attention_simt(q.float(), kc.float(), vc.float(), *args)
     tol = 2e-5 if dtype == torch.float32 else 1e-2           # (bfloat16: the result's own rounding, 2^-8)
     torch.testing.assert_close(got, want, rtol=tol, atol=tol)
+
+
+@pytest.mark.parametrize("N,K", [(64, 64), (512, 512), (2304, 768), (896, 1792), (257, 1001), (3000, 130), (4100, 36)])
+def test_every_number_of_rows_takes_a_form_of_the_same_bits(N, K):
+    """Rows from one tile to many waves of them: tiles of all sizes, segments over a cluster and one after the other."""
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    g = torch.Generator(device=dev).manual_seed(N + K)
+    x = torch.randn(4133, K, device=dev, generator=g)
+    w = torch.randn(N, K, device=dev, generator=g) / K ** 0.5
+    b = torch.randn(N, device=dev, generator=g)
+    few = torch.cat([ops.linear(x[i:i + 16].contiguous(), w, b, torch.float32) for i in range(0, 64, 16)])
+    torch.testing.assert_close(few.double(), x[:64].double() @ w.double().t() + b.double(), rtol=1e-5, atol=1e-5)
+    last = ops.linear(x[-9:].contiguous(), w, b, torch.float32)
+    for m in (17, 31, 64, 100, 129, 257, 543, 1025, 2050, 4133):
+        y = ops.linear(x[-m:].contiguous() if m > 64 else x[:m].contiguous(), w, b, torch.float32)
+        if m > 64:
+            assert torch.equal(y[-9:], last), m
+            torch.testing.assert_close(y[:7].double(), x[-m:][:7].double() @ w.double().t() + b.double(), rtol=1e-5, atol=1e-5)
+        else:
+            assert torch.equal(y, few[:m]), m
