@@ -1336,14 +1336,14 @@ MOE_GROUPED_OVERHEAD_US = 60  # assigning, gathering and adding up, over what th
 MOE_GROUPED_FLOPS_PER_US = 1.2e9
 
 
-def moe_grouped_pays(x, E: int, top: int, ff: int, matrices: int) -> bool:
+def moe_grouped_pays(x, E: int, top: int, ff: int, matrices: int, shared_ff: int = 0) -> bool:
     """Whether a mixture of ``E`` experts of ``ff`` channels (``matrices`` of them an expert), ``top`` a token, is faster with the tokens sorted by
     expert (an expert multiplies its own tokens, padded to tiles of 256 rows: half a tile each on average) than with every expert over every
     token: where the multiplications saved take longer than the sorting."""
     if not (x.is_cuda and x.dtype == torch.bfloat16 and x.shape[0] > TCGEN05_MIN_ROWS and _PAIR_GEMM == "all" and E <= 256):
         return False
     T, W = x.shape
-    if W % 64 or ff % 64 or not pair_supports(MOE_TILE, ff, W):
+    if W % 64 or ff % 64 or shared_ff % 8 or not pair_supports(MOE_TILE, ff, W):      # (a row of the down matrix holds the shared expert's channels too)
         return False
     rows_saved = T * E - T * top - E * MOE_TILE // 2
     return rows_saved * 2.0 * matrices * W * ff > MOE_GROUPED_OVERHEAD_US * MOE_GROUPED_FLOPS_PER_US

@@ -79,7 +79,7 @@ class RoutedExperts(FeedForward):
 
     def forward(self, x, step, residual=None):
         dense, idx, wts = self.route(x)
-        if ops.moe_grouped_pays(x, self.E, self.top, self.ff, 2):
+        if ops.moe_grouped_pays(x, self.E, self.top, self.ff, 2, self.shared_ff):
             shared = None
             if self.shared_ff:
                 shared = ops.gemm_pair(ops.linear_plain_act(x, self.up.weight[self.E * self.ff:], self.dtype, "gelu"), self.down.weight, None, torch.float32,
@@ -179,7 +179,7 @@ class GatedExperts(FeedForward):
 
     def forward(self, x, step, residual=None):
         dense, idx, wts = self.route(x)
-        if ops.moe_grouped_pays(x, self.E, self.top, self.ff, 3):
+        if ops.moe_grouped_pays(x, self.E, self.top, self.ff, 3, self.shared_ff):
             shared = None
             if self.shared_ff:
                 shared = ops.gemm_pair(ops.linear_silu_mul(x, self.gate_up.weight[2 * self.E * self.ff:], self.interleave, self.dtype),

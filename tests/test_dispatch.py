@@ -75,3 +75,30 @@ def test_slices_of_k_for_results_of_few_tiles(ops_with_sms):
     if sms == 148:
         assert ops.pair_splits(197, 3584, 18944) > 1 and ops.pair_splits(512, 3584, 18944) > 1
         assert ops.pair_splits(2048, 3584, 18944) == 1 and ops.pair_splits(2048, 37888, 3584) == 1
+
+
+class _Rows:
+    """bfloat16 rows on a device, as far as a decision looks at them."""
+    is_cuda = True
+
+    def __init__(self, *shape):
+        import torch
+        self.shape, self.dtype = shape, torch.bfloat16
+
+
+@pytest.fixture
+def any_pair_product(ops_with_sms, monkeypatch):
+    ops, sms = ops_with_sms
+    monkeypatch.setattr(ops, "pair_supports", lambda M, N, K: K % 8 == 0)
+    return ops, sms
+
+
+def test_a_mixture_is_sorted_only_where_its_matrices_rows_suit_the_product(any_pair_product):
+    """The grouped product reads the experts' columns of the down matrix, whose rows end with the shared expert's: whole 16-byte pieces."""
+    ops, _ = any_pair_product
+    sizes = dict(E=8, top=2, ff=4096, matrices=3)
+    assert ops.moe_grouped_pays(_Rows(4096, 4096), **sizes)
+    assert ops.moe_grouped_pays(_Rows(4096, 4096), **sizes, shared_ff=104)
+    for shared in (100, 4, 1):
+        assert not ops.moe_grouped_pays(_Rows(4096, 4096), **sizes, shared_ff=shared)
+    assert not ops.moe_grouped_pays(_Rows(4096, 4096), 8, 2, 4096 + 32, 3) and not ops.moe_grouped_pays(_Rows(4096, 4096 + 32), 8, 2, 4096, 3)

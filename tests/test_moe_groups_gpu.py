@@ -106,3 +106,24 @@ def test_a_mixture_sorted_by_expert(monkeypatch, kind, params, T):
     ops.check_tcgen05_status()
     assert float((got - want).norm() / want.norm()) < 1e-2
     torch.testing.assert_close(added, stream + got, rtol=1e-6, atol=1e-5)
+
+
+@pytest.mark.parametrize("shared_ff", [100, 96])
+def test_a_shared_expert_of_any_size_beside_experts_of_whole_tiles(shared_ff):
+    """Long portions by the dispatch's own choice: no size that the product over all experts takes is refused."""
+    import sllm_b200.ops as ops
+    from sllm_b200.config.plan import PartSpec
+    from sllm_b200.models import causal_lm  # noqa: F401  (registers the parts)
+    from sllm_b200.parts.base import FEED_FORWARDS
+    dev = cuda_or_skip()
+    part = FEED_FORWARDS.build(PartSpec("gated_experts", {"hidden_size": 1024, "experts": 8, "top": 2, "expert_ff": 1024, "activation": "silu",
+                                                           "shared_ff": shared_ff}), dtype=torch.bfloat16, device=dev)
+    g = torch.Generator(device=dev).manual_seed(shared_ff)
+    part.bind({s.name: torch.randn(*s.shape, device=dev, generator=g) / s.shape[-1] ** 0.5 for s in part.tensor_specs()}.__getitem__)
+    x = torch.randn(4000, 1024, device=dev, generator=g).bfloat16()
+    y = part.forward(x, None)
+    ops.check_tcgen05_status()
+    y = y.sum(0) if y.dim() == 3 else y
+    one = part.forward(x[-100:].contiguous(), None)
+    one = one.sum(0) if one.dim() == 3 else one
+    assert float((y[-100:] - one).norm() / one.norm()) < 1e-2
