@@ -1332,21 +1332,37 @@ def pair_parts(N: int, form: int = 0) -> int:
 # ---- a mixture of experts over prompt portions, the tokens sorted by expert --------------------------------------------------
 
 MOE_TILE = 256                # rows of a tile of the grouped product: an expert's tokens are padded to whole ones
-MOE_GROUPED_OVERHEAD_US = 60  # assigning, gathering and adding up, over what the dense form pays for its activation (2,048 tokens, width 2,048)
+# Assigning, gathering and adding up, over what the dense form pays for its activation: a part of its own and one with the rows the experts' tiles hold
+# times the width (us; us per 2^20 elements), and the products' rate.
+MOE_GROUPED_OVERHEAD_US, MOE_GROUPED_US_PER_MI = 45.0, 1.57
 MOE_GROUPED_FLOPS_PER_US = 1.2e9
+MOE_GROUPED_BYTES = 256 << 20
 
 
 def moe_grouped_pays(x, E: int, top: int, ff: int, matrices: int, shared_ff: int = 0) -> bool:
     """Whether a mixture of ``E`` experts of ``ff`` channels (``matrices`` of them an expert), ``top`` a token, is faster with the tokens sorted by
-    expert (an expert multiplies its own tokens, padded to tiles of 256 rows: half a tile each on average) than with every expert over every
-    token: where the multiplications saved take longer than the sorting."""
+    expert than with every expert over every token: where the multiplications saved, in rows of whole tiles of 256 on both sides, take longer than the
+    sorting; and whether its buffers are little larger than the other form's (`MOE_GROUPED_BYTES` are always allowed).
+    (us, sorted / every expert: width 2,048, 8 experts of 1,408, 2 used: 256 tokens 118 / 75, 700 124 / 128, 2,048 187 / 286; 64 experts, 6 used: 256
+    427 / 286, 300 421 / 465, 2,048 495 / 1,724; width 4,096, 8 experts of 14,336: 256 684 / 645, 300 683 / 1,076.)"""
     if not (x.is_cuda and x.dtype == torch.bfloat16 and x.shape[0] > TCGEN05_MIN_ROWS and _PAIR_GEMM == "all" and E <= 256):
         return False
     T, W = x.shape
     if W % 64 or ff % 64 or shared_ff % 8 or not pair_supports(MOE_TILE, ff, W):      # (a row of the down matrix holds the shared expert's channels too)
         return False
-    rows_saved = T * E - T * top - E * MOE_TILE // 2
-    return rows_saved * 2.0 * matrices * W * ff > MOE_GROUPED_OVERHEAD_US * MOE_GROUPED_FLOPS_PER_US
+    tokens = T * top / E                                        # an expert's, on average: half a tile is padding, or most of its only one
+    rows = min(E * max(MOE_TILE, tokens + MOE_TILE // 2), T * top * MOE_TILE)
+    saved = -(-T // MOE_TILE) * MOE_TILE * E - rows
+    if saved * 2.0 * matrices * W * ff <= (MOE_GROUPED_OVERHEAD_US + MOE_GROUPED_US_PER_MI * rows * W / 2 ** 20) * MOE_GROUPED_FLOPS_PER_US:
+        return False
+    return moe_grouped_bytes(T, W, E, top, ff, matrices, shared_ff) <= max(1.25 * 2 * matrices * T * (E * ff + shared_ff), MOE_GROUPED_BYTES)
+
+
+def moe_grouped_bytes(T: int, W: int, E: int, top: int, ff: int, matrices: int, shared_ff: int = 0) -> int:
+    """Bytes of the buffers that the sorted form holds at once: of every row either the gathered token or the float32 result beside the activation (gate and
+    up too where a kernel of its own takes them), and the shared expert's."""
+    rows = (T * top // MOE_TILE + E) * MOE_TILE
+    return rows * max(2 * W + 2 * ff * (matrices - 1), 2 * ff * matrices, 2 * ff + 4 * W) + (T * (2 * shared_ff + 4 * W) if shared_ff else 0)
 
 
 def moe_assign(idx, E: int):

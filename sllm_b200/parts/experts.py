@@ -18,6 +18,7 @@ up, in float32, in the order of the router's choices.
 from __future__ import annotations
 
 import math
+from contextlib import suppress
 
 import torch
 
@@ -31,8 +32,8 @@ def sorted_experts(x, idx, wts, E, first, w_rows, act, down, ff, residual, share
     `Linear`'s weight each), ``w_rows`` rows of the first an expert; ``act(rows, w, tile_expert)``: the first product with its activation; ``shared`` (float32
     ``[T, W]``), times the last column of ``gate`` if given, joins the sum.  Added into ``residual`` (returns None) or returned, float32."""
     place, tile_expert, row_token = ops.moe_assign(idx, E)
-    rows = ops.moe_gather(x, row_token)
-    y = ops.gemm_pair_grouped(act(rows, first, tile_expert), down, tile_expert, down.shape[0], ff, 0, ff, torch.float32)
+    hidden = act(ops.moe_gather(x, row_token), first, tile_expert)              # (the gathered rows are given back here)
+    y = ops.gemm_pair_grouped(hidden, down, tile_expert, down.shape[0], ff, 0, ff, torch.float32)
     return ops.moe_combine(y, place, wts, shared, gate, residual)
 
 
@@ -80,14 +81,18 @@ class RoutedExperts(FeedForward):
     def forward(self, x, step, residual=None):
         dense, idx, wts = self.route(x)
         if ops.moe_grouped_pays(x, self.E, self.top, self.ff, 2, self.shared_ff):
-            shared = None
-            if self.shared_ff:
-                shared = ops.gemm_pair(ops.linear_plain_act(x, self.up.weight[self.E * self.ff:], self.dtype, "gelu"), self.down.weight, None, torch.float32,
-                                       w_col=self.E * self.ff)
-            act = lambda rows, w, tiles: ops.gemm_pair_grouped(rows, w, tiles, self.ff, self.hidden, self.ff, 0, self.dtype, act="gelu")  # noqa: E731
-            return sorted_experts(x, idx, wts, self.E, self.up.weight, self.ff, act, self.down.weight, self.ff, residual, shared)
+            with suppress(torch.OutOfMemoryError):           # (nothing is written before all buffers are there: the other form needs no more than ever)
+                return self._sorted(x, idx, wts, residual)
         act = ops.moe_act(self.up(x, self.dtype), dense, self.ff, self.dtype)        # [T, E ff + shared]
         return self.down.into(act, residual)
+
+    def _sorted(self, x, idx, wts, residual):
+        shared = None
+        if self.shared_ff:
+            shared = ops.gemm_pair(ops.linear_plain_act(x, self.up.weight[self.E * self.ff:], self.dtype, "gelu"), self.down.weight, None, torch.float32,
+                                   w_col=self.E * self.ff)
+        act = lambda rows, w, tiles: ops.gemm_pair_grouped(rows, w, tiles, self.ff, self.hidden, self.ff, 0, self.dtype, act="gelu")  # noqa: E731
+        return sorted_experts(x, idx, wts, self.E, self.up.weight, self.ff, act, self.down.weight, self.ff, residual, shared)
 
     def weight_bytes(self):
         return self.up.nbytes() + self.down.nbytes() + self.router.nbytes() + 4 * self.E
@@ -180,16 +185,20 @@ class GatedExperts(FeedForward):
     def forward(self, x, step, residual=None):
         dense, idx, wts = self.route(x)
         if ops.moe_grouped_pays(x, self.E, self.top, self.ff, 3, self.shared_ff):
-            shared = None
-            if self.shared_ff:
-                shared = ops.gemm_pair(ops.linear_silu_mul(x, self.gate_up.weight[2 * self.E * self.ff:], self.interleave, self.dtype),
-                                       self.down.weight, None, torch.float32, w_col=self.E * self.ff)
-            return sorted_experts(x, idx, wts, self.E, self.gate_up.weight, 2 * self.ff, self._sorted_act, self.down.weight, self.ff, residual, shared,
-                                  dense if self.shared_ff else None)
+            with suppress(torch.OutOfMemoryError):           # (as in `RoutedExperts`)
+                return self._sorted(x, idx, wts, dense, residual)
         gu = self.gate_up(x, self.dtype)                                                                     # [T, 2 E ff]
         act = ops.gated_clamp_act(gu, self.interleave, self.limit, self.dtype, alpha=self.alpha, dense=dense, ff=self.ff, act=self.act,
                                   tail=self.shared_ff)
         return self.down.into(act, residual)
+
+    def _sorted(self, x, idx, wts, dense, residual):
+        shared = None
+        if self.shared_ff:
+            shared = ops.gemm_pair(ops.linear_silu_mul(x, self.gate_up.weight[2 * self.E * self.ff:], self.interleave, self.dtype),
+                                   self.down.weight, None, torch.float32, w_col=self.E * self.ff)
+        return sorted_experts(x, idx, wts, self.E, self.gate_up.weight, 2 * self.ff, self._sorted_act, self.down.weight, self.ff, residual, shared,
+                              dense if self.shared_ff else None)
 
     def _sorted_act(self, rows, w, tiles):
         n = 2 * self.ff

@@ -102,3 +102,21 @@ def test_a_mixture_is_sorted_only_where_its_matrices_rows_suit_the_product(any_p
     for shared in (100, 4, 1):
         assert not ops.moe_grouped_pays(_Rows(4096, 4096), **sizes, shared_ff=shared)
     assert not ops.moe_grouped_pays(_Rows(4096, 4096), 8, 2, 4096 + 32, 3) and not ops.moe_grouped_pays(_Rows(4096, 4096 + 32), 8, 2, 4096, 3)
+
+
+def test_a_mixture_is_sorted_where_that_saves_more_than_it_costs(any_pair_product):
+    """Up to 256 tokens every expert's product is one tile of rows in either form, so sorting saves nothing, however many experts there are; from some
+    hundred tokens on it pays, the later the smaller the matrices.  Never where its buffers would be much the larger ones."""
+    ops, _ = any_pair_product
+    sizes = [(4096, 64, 2, 1408, 3), (4096, 8, 2, 14336, 3), (4096, 256, 8, 2048, 3), (2048, 8, 2, 1408, 2), (2048, 128, 8, 768, 3), (1024, 4, 1, 256, 3)]
+    for W, E, top, ff, mats in sizes:
+        for T in (1, 128, 129, 150, 200, 256):
+            assert not ops.moe_grouped_pays(_Rows(T, W), E, top, ff, mats), (T, W, E)
+        for T in (129, 300, 700, 2048, 8192, 32768):
+            if ops.moe_grouped_pays(_Rows(T, W), E, top, ff, mats):
+                assert ops.moe_grouped_bytes(T, W, E, top, ff, mats) <= max(256 << 20, 1.25 * T * E * ff * 2 * mats), (T, W, E)
+    for T, W, E, top, ff, mats, shared, want in [(300, 2048, 64, 6, 1408, 3, 2816, True), (300, 4096, 8, 2, 14336, 3, 0, True), (512, 2048, 8, 2, 1408, 3, 2816, False),
+                                                 (2048, 2048, 8, 2, 1408, 2, 2816, True), (1024, 2048, 8, 2, 1408, 2, 2816, False), (4096, 1024, 16, 4, 512, 2, 512, True),
+                                                 (512, 1024, 16, 4, 512, 2, 512, False), (4096, 1024, 4, 1, 256, 3, 0, False), (2048, 4096, 8, 2, 2752, 3, 0, True),
+                                                 (2048, 4096, 256, 8, 1024, 3, 0, True), (512, 4096, 256, 8, 1024, 3, 0, False)]:
+        assert ops.moe_grouped_pays(_Rows(T, W), E, top, ff, mats, shared) == want, (T, W, E, ff)

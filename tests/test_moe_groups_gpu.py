@@ -127,3 +127,31 @@ def test_a_shared_expert_of_any_size_beside_experts_of_whole_tiles(shared_ff):
     one = part.forward(x[-100:].contiguous(), None)
     one = one.sum(0) if one.dim() == 3 else one
     assert float((y[-100:] - one).norm() / one.norm()) < 1e-2
+
+
+@pytest.mark.parametrize("kind,params", CASES)
+def test_no_room_for_the_sorted_rows(monkeypatch, kind, params):
+    """Where the sorted form's buffers cannot be had, the mixture runs as it does for short portions, and a stream that it adds to has been added to once."""
+    import sllm_b200.ops as ops
+    from sllm_b200.config.plan import PartSpec
+    from sllm_b200.models import causal_lm  # noqa: F401  (registers the parts)
+    from sllm_b200.parts.base import FEED_FORWARDS
+    dev = cuda_or_skip()
+    part = FEED_FORWARDS.build(PartSpec(kind, dict(params, hidden_size=256)), dtype=torch.bfloat16, device=dev)
+    g = torch.Generator(device=dev).manual_seed(5)
+    part.bind({s.name: torch.randn(*s.shape, device=dev, generator=g) / max(1, s.shape[-1]) ** 0.5 for s in part.tensor_specs()}.__getitem__)
+    x = torch.randn(300, 256, device=dev, generator=g).bfloat16()
+    stream = torch.randn(300, 256, device=dev, generator=g)
+    want, got = stream.clone(), stream.clone()
+    monkeypatch.setattr(ops, "moe_grouped_pays", lambda *a: False)
+    term = part.forward(x, None, residual=want)
+
+    def full(*a, **kw):
+        raise torch.OutOfMemoryError("no room (raised by the test)")
+    for at in ("moe_gather", "moe_combine"):
+        got.copy_(stream)
+        with monkeypatch.context() as m:
+            m.setattr(ops, "moe_grouped_pays", lambda *a: True)
+            m.setattr(ops, at, full)
+            same = part.forward(x, None, residual=got)
+        assert torch.equal(got, want) and (same is None) == (term is None) and (term is None or torch.equal(same, term))
