@@ -272,9 +272,9 @@ def _token_heads_fit(dk: int, dv: int) -> bool:
     return bool(lib().sllm_recurrence_token_supports(int(dk), int(dv)))
 
 
-def recurrence_token_supports(proj, step, dk: int, dv: int) -> bool:
-    """Whether `recurrence_token` takes this step: every request brings one token, and the heads fit the kernel's registers."""
-    return proj.is_cuda and proj.shape[0] == step.num_seqs and _token_heads_fit(dk, dv)
+def recurrence_token_supports(proj, state, step, dk: int, dv: int) -> bool:
+    """Whether `recurrence_token` takes this step: every request brings one token, the heads fit the kernel's registers, and the states lie on 16 bytes."""
+    return proj.is_cuda and proj.shape[0] == step.num_seqs and state.data_ptr() % 16 == 0 and _token_heads_fit(dk, dv)
 
 
 TOKEN_MODES = {"general_delta": 0, "gated_delta": 1, "gated": 2, "fixed": 3, "forget_gate": 4}
@@ -648,7 +648,7 @@ def decay_linear_attention(proj, offs, decay, state, step, heads: int, dk: int, 
         raise KernelError("decay_linear_attention: everything that enters the recurrence is float32")
     if tuple(decay.shape) != (heads,) or tuple(state.shape[1:]) != (heads, dk, dv):
         raise KernelError(f"decay_linear_attention: decay {tuple(decay.shape)} or state {tuple(state.shape)} does not fit {heads} heads of {dk}x{dv}")
-    if recurrence_token_supports(proj, step, dk, dv):
+    if recurrence_token_supports(proj, state, step, dk, dv):
         return recurrence_token("fixed", proj, offs, state, step, heads, dk, dv, torch.float32, a=decay)
     out = torch.empty((T, heads * dv), dtype=torch.float32, device=proj.device)
     off_q, off_k, off_v = (int(o) for o in offs)

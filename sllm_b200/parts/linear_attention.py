@@ -71,7 +71,7 @@ class GatedLinearAttention(Mixer):
     def mix(self, x, step: StepContext, cache: LayerCache, position=None, write_cache=True):
         proj = self.inp(x, torch.float32)                                            # [T, 2K + 2V] float32
         z = self.a2(self.a1(x, self.dtype), torch.float32)                           # [T, K] decay logits, float32
-        if ops.recurrence_token_supports(proj, step, self.dim, self.vdim):
+        if ops.recurrence_token_supports(proj, cache.states["gla"], step, self.dim, self.vdim):
             return ops.recurrence_token("gated", proj, self.offs, cache.states["gla"], step, self.heads, self.dim, self.vdim, self.dtype, decay=z,
                                         q_scale=self.dim ** -0.5, tau=self.tau, norm=(self.gain, self.eps, proj, self.off_g, "silu"))
         o = ops.gated_linear_attention(proj, self.offs, z, cache.states["gla"], step, self.heads, self.dim, self.vdim,
@@ -267,7 +267,7 @@ class ForgetGateAttention(Mixer):
         if proj is None:
             proj = self.inp(x, torch.float32)                                        # [T, 2K + V] float32
         offs = tuple(o + proj_off for o in self.offs)
-        if ops.recurrence_token_supports(proj, step, self.dim, self.vdim):
+        if ops.recurrence_token_supports(proj, cache.states["forget_gate"], step, self.dim, self.vdim):
             return ops.recurrence_token("forget_gate", proj, offs, cache.states["forget_gate"], step, self.heads, self.dim, self.vdim, self.dtype,
                                         a=self.lower, bias=self.f_bias, norm=(self.gain, self.eps, None, 0, "none"), out=out, out_off=out_off)
         o = ops.forget_gate_attention(proj, offs, self.f_bias, self.lower, cache.states["forget_gate"], step, self.heads,

@@ -241,3 +241,23 @@ def test_one_token_of_every_request(kind, dk, dv, H, dtype):
         tol = 1e-4 if dtype == torch.float32 else 1e-2
         torch.testing.assert_close(wide[:, 3:3 + V].double(), want, rtol=tol, atol=tol)
         assert not wide[:, :3].any() and not wide[:, 3 + V:].any()
+
+
+@pytest.mark.parametrize("lens", [[1, 1, 1], [130, 1, 97]])
+def test_states_off_the_16_byte_boundary(lens):
+    """A state that is a view at an odd float is taken by every form, as it is where it starts on 16 bytes."""
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    g = torch.Generator(device=dev).manual_seed(8)
+    H, d = 3, 64
+    proj = torch.randn(sum(lens), 3 * H * d, device=dev, generator=g)
+    decay = torch.tensor([0.5, 0.9, 0.99], device=dev)
+    step = _step(dev, lens, [2, 0, 3])
+    state = torch.randn(4, H, d, d, device=dev, generator=g)
+    off = torch.zeros(state.numel() + 1, device=dev)[1:].view_as(state).copy_(state)
+    assert off.is_contiguous() and off.data_ptr() % 16 != 0
+    offs = (0, H * d, 2 * H * d)
+    want = ops.decay_linear_attention(proj, offs, decay, state, step, H, d, d)
+    got = ops.decay_linear_attention(proj, offs, decay, off, step, H, d, d)
+    torch.testing.assert_close(got, want, rtol=2e-5, atol=2e-5 * float(want.abs().max()))
+    torch.testing.assert_close(off, state, rtol=2e-5, atol=2e-5 * float(state.abs().max()))
