@@ -295,6 +295,10 @@ def recurrence_token(kind: str, proj, offs, state, step, heads: int, dk: int, dv
     S, ld = proj.shape
     if tuple(state.shape[1:]) != (heads, dk, dv) or (decay is not None and tuple(decay.shape) != (S, heads * dk)):
         raise KernelError(f"recurrence_token: state {tuple(state.shape)} or decay does not fit {heads} heads of {dk}x{dv}")
+    per_head = kind in ("gated_delta", "fixed")
+    if any(t is not None and t.numel() != (heads if per_head else heads * dk) for t in (a, bias)) or (gain is not None and gain.numel() != heads * dv) or \
+            any(t is not None and t.shape[0] != S for t in (gates, gate)):
+        raise KernelError(f"recurrence_token: the rule's vectors, the norm's gain or the gates' rows do not fit {S} tokens and {heads} heads of {dk}x{dv}")
     if out is None:
         out = torch.empty((S, heads * dv), dtype=out_dtype, device=proj.device)
     call("sllm_recurrence_token", TOKEN_MODES[kind], _p(proj), ld, *(int(o) for o in (tuple(offs) + (0,))[:4]), _p(decay), _p(a), _p(bias), _p(gates),

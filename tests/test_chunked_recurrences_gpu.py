@@ -261,3 +261,19 @@ def test_states_off_the_16_byte_boundary(lens):
     got = ops.decay_linear_attention(proj, offs, decay, off, step, H, d, d)
     torch.testing.assert_close(got, want, rtol=2e-5, atol=2e-5 * float(want.abs().max()))
     torch.testing.assert_close(off, state, rtol=2e-5, atol=2e-5 * float(state.abs().max()))
+
+
+@pytest.mark.parametrize("short", ["a", "bias", "gain", "gate"])
+def test_vectors_that_do_not_fit_are_refused(short):
+    """As `forget_gate_attention` refuses them: the kernel would read past their ends."""
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    H, d, S = 3, 64, 2
+    x = {"a": torch.zeros(H * d, device=dev), "bias": torch.zeros(H * d, device=dev), "gain": torch.zeros(H * d, device=dev), "gate": torch.zeros(S, H * d, device=dev)}
+    proj, state = torch.zeros(S, 3 * H * d, device=dev), torch.zeros(3, H, d, d, device=dev)
+    run = lambda: ops.recurrence_token("forget_gate", proj, (0, H * d, 2 * H * d), state, _step(dev, [1] * S, [0, 1]), H, d, d, torch.float32,  # noqa: E731
+                                       a=x["a"], bias=x["bias"], norm=(x["gain"], 1e-5, x["gate"], 0, "silu"))
+    run()
+    x[short] = x[short][:-1].contiguous()
+    with pytest.raises(ops.KernelError):
+        run()
