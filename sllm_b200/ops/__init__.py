@@ -272,8 +272,16 @@ def _token_heads_fit(dk: int, dv: int) -> bool:
     return bool(lib().sllm_recurrence_token_supports(int(dk), int(dv)))
 
 
-def recurrence_token_supports(proj, state, step, dk: int, dv: int) -> bool:
-    """Whether `recurrence_token` takes this step: every request brings one token, the heads fit the kernel's registers, and the states lie on 16 bytes."""
+# A rule that removes before it writes sums over the state twice, which a CTA of 256 threads a head of at most 16 x 16 does slower than the walk's warps once the
+# heads are many.  (32 such heads, us, this / the walk and the norm behind it: 16 requests 6.8 / 8.1, 33 11.9 / 11.1, 128 39 / 30; a rule without a removal 14 / 28.)
+TOKEN_SMALL_HEAD, TOKEN_SMALL_HEADS = 256, 1024
+
+
+def recurrence_token_supports(proj, state, step, dk: int, dv: int, removes: bool = False) -> bool:
+    """Whether `recurrence_token` takes this step: every request brings one token, the heads fit the kernel's registers (and, with a rule that ``removes``, are
+    not very many small ones), and the states lie on 16 bytes."""
+    if removes and dk * dv <= TOKEN_SMALL_HEAD and step.num_seqs * state.shape[1] > TOKEN_SMALL_HEADS:
+        return False
     return proj.is_cuda and proj.shape[0] == step.num_seqs and state.data_ptr() % 16 == 0 and _token_heads_fit(dk, dv)
 
 

@@ -74,7 +74,7 @@ class GeneralDelta(Mixer):
         proj = self.inp(x, torch.float32)                                            # [T, 5C + R] float32
         lora = ops.tanh_cols(proj, o["w1"], self.rank, self.dtype)                   # [T, R]
         decay = self.w2(lora, torch.float32)                                         # [T, C] decay logits, float32
-        if ops.recurrence_token_supports(proj, cache.states["delta"], step, self.dim, self.dim):
+        if ops.recurrence_token_supports(proj, cache.states["delta"], step, self.dim, self.dim, removes=True):
             y = ops.recurrence_token("general_delta", proj, (o["r"], o["k"], o["v"], o["a"]), cache.states["delta"], step, self.heads, self.dim,
                                      self.dim, self.dtype, decay=decay, a=self.a_bias, norm=(self.gain, self.eps, proj, o["g"], "sigmoid"))
             return self.out.into(y, residual)
@@ -149,7 +149,7 @@ class GatedDelta(Mixer):
     def mix(self, x, step: StepContext, cache: LayerCache, position=None, write_cache=True):
         proj = self.inp(x, torch.float32)                                            # [T, C + 2H + V] float32
         cv = ops.short_conv_silu(proj, 0, self.conv_w, cache.states.get("conv"), step)      # [T, C] float32
-        if ops.recurrence_token_supports(cv, cache.states["delta"], step, self.dim, self.vdim):
+        if ops.recurrence_token_supports(cv, cache.states["delta"], step, self.dim, self.vdim, removes=True):
             return ops.recurrence_token("gated_delta", cv, self.offs, cache.states["delta"], step, self.heads, self.dim, self.vdim, self.dtype,
                                         a=self.a_log, bias=self.dt_bias, gates=proj, off_b=self.off_b, off_dt=self.off_a, key_heads=self.kv_heads,
                                         q_scale=self.dim ** -0.5, norm=(self.gain, self.eps, proj, self.off_g, "silu"))

@@ -120,3 +120,16 @@ def test_a_mixture_is_sorted_where_that_saves_more_than_it_costs(any_pair_produc
                                                  (512, 1024, 16, 4, 512, 2, 512, False), (4096, 1024, 4, 1, 256, 3, 0, False), (2048, 4096, 8, 2, 2752, 3, 0, True),
                                                  (2048, 4096, 256, 8, 1024, 3, 0, True), (512, 4096, 256, 8, 1024, 3, 0, False)]:
         assert ops.moe_grouped_pays(_Rows(T, W), E, top, ff, mats, shared) == want, (T, W, E, ff)
+
+
+def test_single_tokens_of_very_many_small_heads(ops_with_sms, monkeypatch):
+    import torch
+    ops, _ = ops_with_sms
+    monkeypatch.setattr(ops, "_token_heads_fit", lambda dk, dv: True)
+
+    class Step:
+        num_seqs = 64
+    for d, heads, removes, want in [(16, 16, True, True), (16, 17, True, False), (16, 64, False, True), (20, 64, True, True), (8, 64, True, False), (64, 64, True, True)]:
+        state = torch.empty(1, heads, d, d)
+        assert state.data_ptr() % 16 == 0
+        assert ops.recurrence_token_supports(_Rows(64, 4096), state, Step, d, d, removes) == want, (d, heads, removes)
