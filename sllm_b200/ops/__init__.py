@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import functools
 import os
+from contextlib import suppress
 
 import torch
 
@@ -772,6 +773,54 @@ def _long_portions(step, from_len: int, device):
     return step.attn_tiles[key]
 
 
+CHUNK_SCRATCH_BYTES = 256 << 20      # what the chunks of a recurrence may hold at once beside the step's own tensors (8,192 tokens of 16 heads of 128 x 128 in four groups: 940 us, in one 882)
+
+
+def chunk_groups(counts, most: int):
+    """Requests of ``counts`` chunks each, dealt in order to groups of at most ``most`` chunks: per group its first chunk, its chunks, and (request, its first
+    chunk counted in the group, how many) of every request with chunks there."""
+    starts = [sum(counts[:r]) for r in range(len(counts))]
+    total, groups = sum(counts), []
+    for a in range(0, total, most):
+        b = min(a + most, total)
+        runs = [(r, max(f, a) - a, min(f + c, b) - max(f, a)) for r, (f, c) in enumerate(zip(starts, counts)) if f < b and f + c > a]
+        groups.append((a, b - a, runs))
+    return groups
+
+
+def _portion_groups(step, from_len: int, chunk_bytes: int, device):
+    """The step's long portions as (requests, chunks at once, groups of them: (first tokens, lengths, chunks, requests' rows, first chunks, counts, runs) on the
+    device) such that a group's scratch of ``chunk_bytes`` a chunk stays within `CHUNK_SCRATCH_BYTES`, or None.  A request whose chunks fall to several groups
+    goes on from its state's slot, where the group before left it."""
+    chunks = _long_portions(step, from_len, device)
+    if chunks is None:
+        return None
+    t0, _, n, C, seq, first, count, R = chunks
+    most = max(1, CHUNK_SCRATCH_BYTES // chunk_bytes)
+    if C <= most:
+        return R, C, [(t0, n, C, seq, first, count, R)]
+    most = -(-C // -(-C // most))            # (groups of one size)
+    key = ("chunk groups", from_len, most)
+    if key not in step.attn_tiles:
+        long = [(s, -(-q // RETENTION_CHUNK)) for s, q in enumerate(step.q_lens) if q >= from_len]
+        groups = chunk_groups([c for _, c in long], most)
+        flat = [v for _, _, runs in groups for v in [long[r][0] for r, _, _ in runs] + [f for _, f, _ in runs] + [c for _, _, c in runs]]
+        table, at, out = torch.tensor(flat, dtype=torch.int32).to(device, non_blocking=True), 0, []
+        for a, c, runs in groups:
+            k = len(runs)
+            out.append((t0[a:a + c], n[a:a + c], c, table[at:at + k], table[at + k:at + 2 * k], table[at + 2 * k:at + 3 * k], k))
+            at += 3 * k
+        step.attn_tiles[key] = out
+    return R, most, step.attn_tiles[key]
+
+
+def _scratch(floats: int, device):
+    """float32 scratch, or None where there is no room for it: the walk needs none."""
+    with suppress(torch.OutOfMemoryError):
+        return torch.empty(floats, dtype=torch.float32, device=device)
+    return None
+
+
 def _gated_chunks(mode: int, proj, offs, z, a, bias, q_scale: float, tau: float, state, step, heads: int, dk: int, dv: int, out):
     """The step's long portions through the chunked form of the recurrence ``mode`` (2: a decay per channel from the logits ``z``, 3: a fixed
     decay ``a`` per head, 4: a forget gate with lower bounds ``a`` and ``bias``); their rows of ``out`` and their states are written.
@@ -779,16 +828,19 @@ def _gated_chunks(mode: int, proj, offs, z, a, bias, q_scale: float, tau: float,
     chunks = None
     if step.max_q_len >= GATED_CHUNKED_FROM > 0 and gated_chunked_supports(dk, dv) and \
             _chunks_pay("gated64" if dk <= 64 else "gated128", step, GATED_CHUNKED_FROM, heads, dk, dv):
-        chunks = _long_portions(step, GATED_CHUNKED_FROM, proj.device)
+        chunks = _portion_groups(step, GATED_CHUNKED_FROM, 4 * heads * dk * (dv + 1), proj.device)
     if chunks is None:
         return 0, True
-    t0, _, n, C, seq, first, count, R = chunks
-    scratch = torch.empty((C, heads, dk, dv), dtype=torch.float32, device=proj.device)
-    keeps = torch.empty((C, heads, dk), dtype=torch.float32, device=proj.device)
+    R, most, groups = chunks
+    scratch = _scratch(most * heads * dk * (dv + 1), proj.device)
+    if scratch is None:
+        return 0, True
     off_q, off_k, off_v = (int(o) for o in offs)
-    call("sllm_gated_chunked", mode, _p(proj), proj.shape[1], off_q, off_k, off_v, _p(z), _p(a), _p(bias), float(q_scale), 1.0 / float(tau),
-         _p(state), _p(step.state_slots), _p(t0), _p(n), C, _p(seq), _p(first), _p(count), R, _p(scratch), _p(keeps), _p(out), heads, dk, dv, _stream())
-    launches["own"] += 2           # the three kernels of the entry point
+    for t0, n, C, seq, first, count, runs in groups:
+        call("sllm_gated_chunked", mode, _p(proj), proj.shape[1], off_q, off_k, off_v, _p(z), _p(a), _p(bias), float(q_scale), 1.0 / float(tau),
+             _p(state), _p(step.state_slots), _p(t0), _p(n), C, _p(seq), _p(first), _p(count), runs, _p(scratch), _p(scratch) + 4 * most * heads * dk * dv, _p(out),
+             heads, dk, dv, _stream())
+        launches["own"] += 2           # the three kernels of the entry point
     return GATED_CHUNKED_FROM - 1, R < step.num_seqs
 
 
@@ -804,15 +856,19 @@ def _delta_chunks(mode: int, proj, offs, decay, a_bias, gates, off_b: int, off_d
     chunks = None
     if step.max_q_len >= DELTA_CHUNKED_FROM > 0 and delta_chunked_supports(mode, dk, dv) and \
             _chunks_pay("general" if mode == 0 else "delta64" if dk <= 64 else "delta128", step, DELTA_CHUNKED_FROM, heads, dk, dv):
-        chunks = _long_portions(step, DELTA_CHUNKED_FROM, proj.device)
+        floats = heads * int(lib().sllm_delta_chunked_scratch(int(dk), int(dv)))
+        chunks = _portion_groups(step, DELTA_CHUNKED_FROM, 4 * floats, proj.device)
     if chunks is None:
         return 0, True
-    t0, _, n, C, seq, first, count, R = chunks
-    scratch = torch.empty(C * heads * int(lib().sllm_delta_chunked_scratch(int(dk), int(dv))), dtype=torch.float32, device=proj.device)
-    call("sllm_delta_chunked", mode, _p(proj), proj.shape[1], *(int(o) for o in offs), _p(decay), _p(a_bias), _p(gates),
-         gates.shape[1] if gates is not None else 0, int(off_b), int(off_dt), _p(a_log), _p(dt_bias), float(q_scale), _p(state), _p(step.state_slots),
-         _p(t0), _p(n), C, _p(seq), _p(first), _p(count), R, _p(scratch), _p(out), heads, key_heads, dk, dv, _stream())
-    launches["own"] += 2           # the three kernels of the entry point
+    R, most, groups = chunks
+    scratch = _scratch(most * floats, proj.device)
+    if scratch is None:
+        return 0, True
+    for t0, n, C, seq, first, count, runs in groups:
+        call("sllm_delta_chunked", mode, _p(proj), proj.shape[1], *(int(o) for o in offs), _p(decay), _p(a_bias), _p(gates),
+             gates.shape[1] if gates is not None else 0, int(off_b), int(off_dt), _p(a_log), _p(dt_bias), float(q_scale), _p(state), _p(step.state_slots),
+             _p(t0), _p(n), C, _p(seq), _p(first), _p(count), runs, _p(scratch), _p(out), heads, key_heads, dk, dv, _stream())
+        launches["own"] += 2           # the three kernels of the entry point
     return DELTA_CHUNKED_FROM - 1, R < step.num_seqs
 
 

@@ -277,3 +277,40 @@ def test_vectors_that_do_not_fit_are_refused(short):
     x[short] = x[short][:-1].contiguous()
     with pytest.raises(ops.KernelError):
         run()
+
+
+@pytest.mark.parametrize("kind", ["gated", "fixed", "forget_gate", "gated_delta", "general_delta"])
+def test_chunks_within_a_bound_on_their_scratch(monkeypatch, kind):
+    """A step whose chunks would hold more than the bound runs them in groups, with the same bits and scratch for one group; where there is no room even for that
+    the portions are walked, as they were before there were chunks."""
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    g = torch.Generator(device=dev).manual_seed(3)
+    H, d, T = 2, 64, sum(LENS)
+    C = H * d
+    proj, z, v1, v2 = (torch.randn(*s, device=dev, generator=g) for s in ((T, 4 * C), (T, C), (C,), (C,)))
+    lower, head, heads = torch.rand(C, device=dev, generator=g) * 0.9, torch.tensor([0.9, 0.99], device=dev), torch.zeros(H, device=dev) - 2
+    offs = (0, C, 2 * C)
+    run = {"gated": lambda s, t: ops.gated_linear_attention(proj, offs, z, s, t, H, d, d, 0.1, 8.0),
+           "fixed": lambda s, t: ops.decay_linear_attention(proj, offs, head, s, t, H, d, d),
+           "forget_gate": lambda s, t: ops.forget_gate_attention(proj, offs, v1, lower, s, t, H, d, d),
+           "gated_delta": lambda s, t: ops.gated_delta_rule(proj, offs, z, 0, H, heads, heads, s, t, H, H, d, d, 0.1),
+           "general_delta": lambda s, t: ops.delta_rule(proj, offs + (3 * C,), z, v2, s, t, H, d, d)}[kind]
+    before = _state(g, H, d, d, dev)
+    want_state = before.clone()
+    want = run(want_state, _step(dev, LENS, SLOTS))
+    per = 4 * H * (d * (d + 1) if kind in ("gated", "fixed", "forget_gate") else int(ops.lib().sllm_delta_chunked_scratch(d, d)))
+    sizes, empty = [], ops._scratch
+    for chunks in (1, 3, 4, 11):
+        with monkeypatch.context() as m:
+            m.setattr(ops, "CHUNK_SCRATCH_BYTES", chunks * per + per - 4)
+            m.setattr(ops, "_scratch", lambda floats, device: sizes.append(4 * floats) or empty(floats, device))
+            state = before.clone()
+            assert torch.equal(run(state, _step(dev, LENS, SLOTS)), want) and torch.equal(state, want_state)
+        assert per <= sizes.pop() <= chunks * per and not sizes
+    with monkeypatch.context() as m:
+        m.setattr(ops, "_scratch", lambda floats, device: None)
+        state = before.clone()
+        got = run(state, _step(dev, LENS, SLOTS))
+    _close(got, want, "walked")
+    _close(state, want_state, "states walked")

@@ -133,3 +133,19 @@ def test_single_tokens_of_very_many_small_heads(ops_with_sms, monkeypatch):
         state = torch.empty(1, heads, d, d)
         assert state.data_ptr() % 16 == 0
         assert ops.recurrence_token_supports(_Rows(64, 4096), state, Step, d, d, removes) == want, (d, heads, removes)
+
+
+@pytest.mark.parametrize("most", [1, 2, 3, 5, 7, 100])
+def test_chunks_of_long_portions_in_groups(most):
+    """Every chunk is in one group, in order; a request's chunks go on where the group before stopped."""
+    import sllm_b200.ops as ops
+    counts = [10, 2, 1, 4, 1]
+    seen = []
+    for a, n, runs in ops.chunk_groups(counts, most):
+        assert 1 <= n <= most and a == len(seen) and sum(c for _, _, c in runs) == n
+        at = 0
+        for r, first, c in runs:
+            assert first == at and c >= 1
+            seen += [r] * c
+            at += c
+    assert seen == [r for r, c in enumerate(counts) for _ in range(c)]
