@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import functools
 import os
+from collections import namedtuple
 from contextlib import suppress
 
 import torch
@@ -733,15 +734,23 @@ def portion_chunks(q_lens, ctx_lens, min_len: int, device):
 # Portions of at least so many tokens may run in chunks in the recurrences below (0: none does), shorter ones are walked.
 GATED_CHUNKED_FROM = 96
 DELTA_CHUNKED_FROM = 96
-# What decides (us; `_chunks_pay`): the walk takes its longest portion times a rate, that of a CTA which walks 16 columns of a head (64 where the
-# batch fills the SMs with such) and slower the more of them an SM holds; the chunks take a base for their three kernels and a rate per
-# token of all long portions.  Measured in a graph (walk / chunks): 32 heads of 64 x 64, one portion of 128, 256, 2,048 tokens: gated 32 / 34, 60 / 35,
-# 479 / 121; general delta 45 / 48, 84 / 51, 931 / 333; 16 heads of 128 x 128: forget gate 51 / 60, 95 / 60, 709 / 163; gated delta 53 / 51, 99 / 58,
-# 748 / 240.  Eight portions of 200 tokens: 79 / 117, 119 / 270, 195 / 173, 223 / 240; three of 700: 349 / 125,
-# 661 / 292, 527 / 168, 551 / 260.  (walk, a narrow CTA's and a wide one's per token; base; chunks
-# per token, and the heads x keys x values that was measured at)
-CHUNK_COSTS = {"gated64": (0.235, 0.39, 30.0, 0.045, 32 * 64 * 64), "gated128": (0.35, 0.97, 52.0, 0.055, 16 * 128 * 128),
-               "general": (0.42, 0.59, 40.0, 0.143, 32 * 64 * 64), "delta64": (0.30, 0.45, 42.0, 0.09, 32 * 64 * 64), "delta128": (0.37, 1.10, 42.0, 0.098, 16 * 128 * 128)}
+# What decides (us; `_chunks_pay`), fitted to 12 to 24 sizes of heads each and 36 shapes of a step (1 to 100 requests, portions of 96 to 4,096 tokens, alone and beside short ones).
+# The walk: `start`, and a rate a token of its longest portion, that of a CTA which walks 16 columns of a head (64 where the batch fills the SMs with such; `wide`), no less than
+# `busy` for every CTA an SM, of which `fixed` does not shrink with the keys.  The chunks: `base`, `part` for two (chunk, head) an SM or every two, then a
+# chunk's `serial` piece of the longest portion or (the delta rules) `scan` times the (portion, head, 16 columns) an SM, for the others `scan` times the states'
+# elements an SM; `rest` where short portions are walked beside them.  Heads are padded to 64 or 128 in the chunks, not in the walk.
+# Measured (walk / chunks): 32 heads of 64 x 64, one portion of 128, 256, 2,048 tokens: gated 32 / 34, 60 / 35, 479 / 121; general delta 45 / 48, 84 / 51, 931 / 333;
+# 16 heads of 128 x 128, gated delta: 53 / 51, 99 / 58, 748 / 240, eight portions of 200 tokens 223 / 240; 4 heads of 16 x 16, general delta, 100 portions of 96: 44 / 205.
+ChunkCosts = namedtuple("ChunkCosts", "start narrow wide busy busy_wide fixed base part serial scan rest")
+CHUNK_COSTS = {"gated64": ChunkCosts(7.3, 0.226, 0.342, 0.142, 0.206, 0.68, 9.3, 24.2, 0.1, 6.2, 9.4),
+               "gated128": ChunkCosts(10.3, 0.312, 0.507, 0.216, 0.468, 0.92, 0.0, 58.5, 0.0, 9.2, 32.4),
+               "fixed64": ChunkCosts(7.4, 0.262, 0.365, 0.142, 0.221, 0.66, 13.6, 22.6, 0.1, 4.9, 10.1),
+               "fixed128": ChunkCosts(11.2, 0.350, 0.558, 0.228, 0.518, 1.0, 12.2, 47.6, 0.0, 7.3, 32.9),
+               "forget64": ChunkCosts(7.7, 0.251, 0.351, 0.138, 0.211, 0.63, 11.0, 20.6, 0.1, 4.6, 9.9),
+               "forget128": ChunkCosts(11.6, 0.347, 0.561, 0.231, 0.513, 1.0, 11.7, 42.0, 0.0, 7.1, 34.6),
+               "delta64": ChunkCosts(7.8, 0.331, 0.430, 0.177, 0.279, 0.84, 0.0, 29.7, 3.2, 2.25, 8.4),
+               "delta128": ChunkCosts(11.4, 0.348, 0.625, 0.237, 0.582, 0.97, 0.0, 48.7, 3.47, 4.61, 27.1),
+               "general": ChunkCosts(5.8, 0.335, 0.507, 0.219, 0.332, 0.46, 0.0, 51.4, 3.1, 2.46, 4.1)}
 
 
 def _chunks_pay(kind: str, step, from_len: int, heads: int, dk: int, dv: int) -> bool:
@@ -749,13 +758,20 @@ def _chunks_pay(kind: str, step, from_len: int, heads: int, dk: int, dv: int) ->
     long = [q for q in step.q_lens if q >= from_len]
     if not long:
         return False
-    narrow, wide, base, per_token, ref = CHUNK_COSTS[kind]
-    blocks = heads * -(-dv // 64)
-    if step.num_seqs * blocks >= num_sms():
-        rate = wide * max(1.0, len(long) * blocks / 256)
+    c, sms, blocks = CHUNK_COSTS[kind], num_sms(), heads * -(-dv // 64)
+    pad_k, pad_v = 64 if dk <= 64 else 128, 64 if dv <= 64 else 128
+    if step.num_seqs * blocks >= sms:
+        rate = max(c.wide, c.busy_wide * len(long) * blocks / sms)
     else:
-        rate = narrow * max(1.0, len(long) * heads * -(-dv // 16) / 180)
-    return base + sum(long) * per_token * heads * dk * dv / ref < max(long) * rate
+        rate = max(c.narrow, c.busy * len(long) * heads * -(-dv // 16) / sms)
+    walk = c.start + max(long) * rate * (c.fixed + (1 - c.fixed) * dk / pad_k)
+    counts = [-(-q // RETENTION_CHUNK) for q in long]
+    chunks = c.base + c.part * max(1.0, sum(counts) * heads / (2 * sms)) * (pad_k + pad_v) / (2 * pad_k) + (c.rest if len(long) < step.num_seqs else 0.0)
+    if not kind.startswith(("delta", "general")):
+        chunks += c.serial * max(counts) + c.scan * sum(counts) * heads * dk * dv / (4096 * sms)
+    else:
+        chunks += max(counts) * max(c.serial, c.scan * len(long) * heads * pad_v / (16 * sms))
+    return chunks < walk
 
 
 @functools.lru_cache(maxsize=4096)
@@ -821,13 +837,16 @@ def _scratch(floats: int, device):
     return None
 
 
+GATED_KINDS = {2: "gated", 3: "fixed", 4: "forget"}
+
+
 def _gated_chunks(mode: int, proj, offs, z, a, bias, q_scale: float, tau: float, state, step, heads: int, dk: int, dv: int, out):
     """The step's long portions through the chunked form of the recurrence ``mode`` (2: a decay per channel from the logits ``z``, 3: a fixed
     decay ``a`` per head, 4: a forget gate with lower bounds ``a`` and ``bias``); their rows of ``out`` and their states are written.
     Returns (the longest portion left for the walk, 0 for no limit; whether any is left)."""
     chunks = None
     if step.max_q_len >= GATED_CHUNKED_FROM > 0 and gated_chunked_supports(dk, dv) and \
-            _chunks_pay("gated64" if dk <= 64 else "gated128", step, GATED_CHUNKED_FROM, heads, dk, dv):
+            _chunks_pay(GATED_KINDS[mode] + ("64" if dk <= 64 else "128"), step, GATED_CHUNKED_FROM, heads, dk, dv):
         chunks = _portion_groups(step, GATED_CHUNKED_FROM, 4 * heads * dk * (dv + 1), proj.device)
     if chunks is None:
         return 0, True

@@ -149,3 +149,23 @@ def test_chunks_of_long_portions_in_groups(most):
             seen += [r] * c
             at += c
     assert seen == [r for r, c in enumerate(counts) for _ in range(c)]
+
+
+def test_portions_run_in_chunks_where_that_is_faster(monkeypatch):
+    """Shapes measured in both forms, on both sides of the line (148 SMs): heads whose padding or very many short portions make the chunks the slower
+    form, and long portions of which the walk is one chain."""
+    import sllm_b200.ops as ops
+    monkeypatch.setattr(ops, "num_sms", lambda: 148)
+
+    class Step:
+        def __init__(self, lens):
+            self.q_lens, self.num_seqs = lens, len(lens)
+    for kind, heads, dk, dv, lens, want in [
+            ("gated64", 32, 64, 64, [2048], True), ("gated64", 32, 64, 64, [96], False), ("gated64", 64, 64, 64, [100] * 40, False), ("gated64", 32, 64, 64, [100] * 100, False),
+            ("gated64", 8, 16, 16, [150] * 16, False), ("gated64", 32, 64, 64, [2048] + [1] * 7, True), ("gated64", 4, 32, 32, [1, 2, 3], False),
+            ("gated128", 16, 128, 128, [2048], True), ("gated128", 16, 128, 128, [128], False), ("gated128", 16, 128, 128, [1000, 100, 100, 100], True),
+            ("forget128", 16, 128, 128, [400] * 5, True), ("forget128", 16, 128, 128, [128], False), ("fixed64", 64, 64, 64, [1001, 700, 600], True), ("fixed64", 8, 16, 16, [96] * 100, False),
+            ("delta64", 16, 64, 64, [512], True), ("delta64", 4, 32, 32, [96] * 100, False), ("delta128", 16, 128, 128, [2048], True),
+            ("delta128", 32, 128, 128, [1000] * 8, True), ("delta128", 8, 128, 64, [96] * 100, False),
+            ("general", 32, 64, 64, [2048], True), ("general", 32, 64, 64, [200] * 8, False), ("general", 4, 16, 16, [96] * 100, False), ("general", 8, 32, 32, [150] * 16, False)]:
+        assert ops._chunks_pay(kind, Step(lens), 96, heads, dk, dv) == want, (kind, heads, dk, len(lens), lens[0])
