@@ -1456,6 +1456,8 @@ def moe_assign(idx, E: int):
     """A row for every (token, choice) of ``idx`` (int32 ``[T, top]``) in a buffer sorted by expert: (places ``[T, top]``, the expert of every tile of 256
     rows or -1, the token of every row or -1)."""
     _chk(idx)
+    if idx.dtype != torch.int32 or idx.dim() != 2:
+        raise KernelError(f"moe_assign: the router's choices are int32 [tokens, choices], got {idx.dtype} {tuple(idx.shape)}")
     T, top = idx.shape
     tiles = T * top // MOE_TILE + E
     i32 = lambda n: torch.empty(n, dtype=torch.int32, device=idx.device)  # noqa: E731
@@ -1467,6 +1469,8 @@ def moe_assign(idx, E: int):
 def moe_gather(x, row_token) -> torch.Tensor:
     """``x[row_token]``, rows without a token left as they are."""
     _chk(x, row_token)
+    if row_token.dtype != torch.int32:
+        raise KernelError(f"moe_gather: the rows' tokens are int32, got {row_token.dtype}")
     out = torch.empty((row_token.numel(), x.shape[1]), dtype=x.dtype, device=x.device)
     call("sllm_moe_gather", _p(x), _p(row_token), _p(out), row_token.numel(), x.shape[1] * x.element_size(), _stream())
     return out
@@ -1476,8 +1480,8 @@ def gemm_pair_grouped(x, w, tile_expert, N: int, K: int, w_rows: int, w_cols: in
     """`gemm_pair` with the row tiles of ``x`` (``[256 * tiles, K]``) sorted by expert: tile i times the ``N`` rows of ``w`` from row ``w_rows`` and column
     ``w_cols`` times ``tile_expert[i]`` on.  ``act``: ``gelu`` (exact) or ``silu`` (gate and up rows alternating in blocks of 8), bfloat16."""
     _chk(x, w, tile_expert)
-    if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or x.shape[0] != MOE_TILE * tile_expert.numel() or x.shape[1] != K:
-        raise KernelError(f"gemm_pair_grouped: x {tuple(x.shape)} does not fit {tile_expert.numel()} tiles of {MOE_TILE} rows and {K} columns, bfloat16")
+    if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or tile_expert.dtype != torch.int32 or x.shape[0] != MOE_TILE * tile_expert.numel() or x.shape[1] != K:
+        raise KernelError(f"gemm_pair_grouped: x {tuple(x.shape)} does not fit {tile_expert.numel()} tiles (int32) of {MOE_TILE} rows and {K} columns, bfloat16")
     M = x.shape[0]
     epi = {None: 0 if out_dtype == torch.float32 else 1, "gelu": 7, "silu": 2}[act]
     out = torch.empty((M, N // 2 if act == "silu" else N), dtype=torch.float32 if epi == 0 else torch.bfloat16, device=x.device)
@@ -1492,6 +1496,9 @@ def moe_combine(y, place, wts, shared=None, gate=None, residual=None):
     _chk(y, place, wts, shared, gate, residual)
     T, top = place.shape
     W = y.shape[1]
+    if place.dtype != torch.int32 or tuple(wts.shape) != (T, top) or any(t is not None and t.dtype != torch.float32 for t in (y, wts, shared, gate, residual)) or \
+            any(t is not None and tuple(t.shape) != (T, W) for t in (shared, residual)) or (gate is not None and gate.shape[0] != T):
+        raise KernelError(f"moe_combine: places int32 and weights float32 [{T}, {top}], float32 rows of {W}, the shared expert's and the stream's [{T}, {W}]")
     out = residual if residual is not None else torch.empty((T, W), dtype=torch.float32, device=y.device)
     ld = gate.shape[1] if gate is not None else 0
     call("sllm_moe_combine", _p(y), _p(place), _p(wts), T, top, _p(shared), _p(gate) + 4 * (ld - 1) if gate is not None else None, ld, _p(out),

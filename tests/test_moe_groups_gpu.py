@@ -155,3 +155,22 @@ def test_no_room_for_the_sorted_rows(monkeypatch, kind, params):
             m.setattr(ops, at, full)
             same = part.forward(x, None, residual=got)
         assert torch.equal(got, want) and (same is None) == (term is None) and (term is None or torch.equal(same, term))
+
+
+def test_tables_of_another_type_are_refused():
+    """The kernels read them as 32-bit numbers: wider ones would be other experts, and other rows."""
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    idx = torch.zeros(300, 2, dtype=torch.int32, device=dev)
+    place, tile_expert, row_token = ops.moe_assign(idx, 4)
+    x, w = torch.zeros(300, 64, device=dev).bfloat16(), torch.zeros(64, 256, device=dev).bfloat16()
+    rows = ops.moe_gather(x, row_token)
+    y = ops.gemm_pair_grouped(rows, w, tile_expert, 64, 64, 0, 64, torch.float32)
+    wts, stream = torch.zeros(300, 2, device=dev), torch.zeros(300, 64, device=dev)
+    assert ops.moe_combine(y, place, wts, residual=stream) is None
+    for bad in (lambda: ops.moe_assign(idx.long(), 4), lambda: ops.moe_assign(idx.float(), 4), lambda: ops.moe_assign(idx.reshape(-1), 4),
+                lambda: ops.moe_gather(x, row_token.long()), lambda: ops.gemm_pair_grouped(rows, w, tile_expert.long(), 64, 64, 0, 64, torch.float32),
+                lambda: ops.moe_combine(y, place.long(), wts), lambda: ops.moe_combine(y, place, wts.double()), lambda: ops.moe_combine(y, place, wts[:, :1].contiguous()),
+                lambda: ops.moe_combine(y, place, wts, shared=stream[:, :32].contiguous()), lambda: ops.moe_combine(y, place, wts, residual=stream.bfloat16())):
+        with pytest.raises(ops.KernelError):
+            bad()
