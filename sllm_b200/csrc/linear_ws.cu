@@ -401,20 +401,23 @@ linear_ws_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __res
 // unless the rows are long (K = 27648: 50.4 us with 592 against 61.4).  More rows: two CTAs an SM that walk theirs in groups, the next
 // group's first blocks in flight under this one's last and its sums, where a CTA a group paid a ramp and a tail each.
 // (8 tokens, us, this / the 128-row form of linear_stream.cu; floor at 6.65 TB/s: 11,264 x 2,048 10.9 / 17.8 / 6.9, 16,512 x 4,096 24.7 / 36.3 / 20.3,
-// 22,016 x 4,096 31.3 / 39.8 / 27.1, 152,064 x 3,584 168 / 188 / 164.)
-constexpr int WS_ONE_GROUP_ROWS = 8192;
+// 22,016 x 4,096 31.3 / 39.8 / 27.1, 152,064 x 3,584 168 / 188 / 164.)  A short K leaves a group too little to stream under its sums (20,000 x 1,024: 12.9 walked, 11.9 a CTA a group).
+constexpr int WS_ONE_GROUP_ROWS = 8192, WS_WALK_MIN_K = 1280;
 static int ws_ctas(int units, int per, int K, bool rope) {
   const int num_sms = sllm::num_sms();
   const int ctas = (units + per - 1) / per;
   if (rope || ctas <= num_sms) return ctas;
   if (ctas < 2 * num_sms) return 2 * num_sms <= units ? 2 * num_sms : ctas;
-  if (ctas * 16 > WS_ONE_GROUP_ROWS) return 2 * num_sms;
+  if (ctas * 16 > WS_ONE_GROUP_ROWS) return K >= WS_WALK_MIN_K ? 2 * num_sms : ctas;
   const int even = K > 8192 ? (ctas + 2 * num_sms - 1) / (2 * num_sms) * (2 * num_sms) : ctas;
   return even <= units ? even : ctas;
 }
-// Slices of K by the CTAs of a cluster: where the rows give less than one CTA an SM, as many (1, 2, 4) as two an SM hold, none shorter than 16 k blocks
-// (8 tokens, residual epilogue, us: 896 x 4,864 4.2 in 4 slices, 5.8 in one; 2,048 x 5,632 7.0 in 2, 8.3 in one; 2,048 x 11,264 10.8 and 12.7).
-static int ws_slices(int ctas, int K) {
+// Slices of K by the CTAs of a cluster: where the rows give less than one CTA an SM, as many (1, 2, 4) as two an SM hold, none shorter than 16 k blocks, and
+// only of a K that is worth the pass over the cluster's sums.
+// (us, in slices / in one. 8 tokens, residual epilogue: 896 x 4,864 4.5 / 6.1; 2,048 x 2,048 4.2 / 4.6; 2,048 x 1,536 3.8 / 4.2; 1,024 x 1,024 2.9 / 2.8. 8 tokens, store: 512 x
+// 2,560 3.1 / 3.9; 256 x 2,048 2.7 / 2.5; 1,024 x 1,024 2.8 / 2.2. 16 tokens: 512 x 2,048 2.9 / 3.3; 2,048 x 1,536 4.3 / 3.6.)
+static int ws_slices(int ctas, int K, int M, bool residual) {
+  if (K < (M > 8 ? 2048 : residual ? 1536 : 2080)) return 1;
   int s = 1;
   while (s < WS_SLICES && ctas * s * 2 <= 2 * sllm::num_sms() && K / 32 / (s * 2) >= 16) s *= 2;
   return s;
@@ -439,7 +442,7 @@ static int launch_ws(const __nv_bfloat16* x, const __nv_bfloat16* W, const float
   // (rows beyond a group a CTA: only the forms that are asked for them)
   const bool walk = EPI != WS_EPI_ROPE && (long long)ctas * (EPI == WS_EPI_GATED ? 8 : 16) < (EPI == WS_EPI_GATED ? N / 2 : N);
   if constexpr (EPI == WS_EPI_GATED || EPI == WS_EPI_STORE) {
-    if (walk && ws_side_by_side(M, N, K)) {
+    if (N > WS_ONE_GROUP_ROWS && ws_side_by_side(M, N, K)) {
       const int n = (N + 16 * WS_SIDE - 1) / (16 * WS_SIDE);
       if (norm.ssq_in != nullptr)
         launch_kernel(linear_ws_kernel<NT, EPI, OUT, true, WS_ROWS>, n, WS_WARPS * 32, 0, stream, x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token, 1);
@@ -465,7 +468,7 @@ static int launch_ws(const __nv_bfloat16* x, const __nv_bfloat16* W, const float
     }
   }
   if constexpr (EPI <= WS_EPI_RESID) {
-    const int slices = ws_slices(ctas, K);
+    const int slices = ws_slices(ctas, K, M, EPI == WS_EPI_RESID);
     if (slices > 1) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(ctas * slices);
@@ -495,8 +498,8 @@ SLLM_EXPORT int sllm_linear_ws_supports(int M, int N, int K) {
   return M >= 1 && M <= 32 && N >= 16 && K >= 32 && K % 32 == 0;
 }
 
-// slices of K that the CTAs of a cluster share (no norm owed on the input)
-SLLM_EXPORT int sllm_linear_ws_slices(int N, int K) { return ws_slices(ws_ctas(N, 16, K, false), K); }
+// slices of K that the CTAs of a cluster share at more than 8 tokens (no norm owed on the input)
+SLLM_EXPORT int sllm_linear_ws_slices(int N, int K) { return ws_slices(ws_ctas(N, 16, K, false), K, 32, false); }
 // whether a product of many rows takes the form with groups side by side
 SLLM_EXPORT int sllm_linear_ws_side_by_side(int M, int N, int K) { return ws_side_by_side(M, N, K); }
 

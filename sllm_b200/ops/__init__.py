@@ -1616,7 +1616,7 @@ WS_ROWS32_MAX_K = 4096
 # times slices come to 0.7 of the places or the rows alone to one CTA an SM, or where K is so short that latency is all of it.  (33 steps, ms, before / since:
 # 17 requests at a width of 896 38.9 / 37.8, 24 at 1,536 63.4 / 62.2; the other designs at 2,048, 20 to 32 requests, 35.4 / 31.9, 34.1 / 32.6, 50.9 / 48.7, 34.0 / 29.9,
 # 41.0 / 38.9, 47.7 / 44.0; at 4,096 no change.  With 1,536 x 8,960 as well, 192 of 296 places, 16 requests lost what they had won.)
-WS_ROWS32_MIN_K, WS_ROWS32_SHARED_MAX_K, WS_ROWS32_SHORT_K = 512, 8192, 1024
+WS_ROWS32_MIN_K, WS_ROWS32_SHARED_MAX_K, WS_ROWS32_SHORT_K, WS_ROWS32_SLICED_K = 512, 8192, 1024, 2048
 MAX_SCALE_PARTS_ROWS32 = 192   # the table of partial sums a four-tile consumer keeps (streams of up to 3,072 columns)
 
 
@@ -1648,8 +1648,15 @@ def _ws_rows32_ok(M: int, N: int, K: int) -> bool:
     ctas = -(-N // 16)
     if M > 32 or N * K > WS_ROWS32_MAX_ELEMENTS or not WS_ROWS32_MIN_K <= K <= WS_ROWS32_SHARED_MAX_K or ctas > 2 * num_sms():
         return False
-    places = ctas * int(lib().sllm_linear_ws_slices(N, K))
+    places = ctas * (int(lib().sllm_linear_ws_slices(N, K)) if K >= WS_ROWS32_SLICED_K else 2)
     return ctas >= num_sms() or places >= 1.4 * num_sms() or K <= WS_ROWS32_SHORT_K
+
+
+def _ws_stack_pays(M: int, N: int, K: int) -> bool:
+    """Whether a consumer that adds partial sums is better served by the k-split kernel although the warp-split one takes the product: 17 to 32 tokens and rows for one
+    to one and a half CTAs an SM, beyond what clusters share.  (24 tokens, the product and the norm behind it, us: 2,560 x 2,560 10.0 accumulated, 8.0 from slices; 3,072 x 3,072 10.8 / 9.9;
+    2,560 x 4,096 12.2 / 9.8; the product alone, which cannot leave slices: 7.3 against 24.7 from the k-split kernel unsliced.)"""
+    return M > 16 and not _ws_tokens_ok(M, N, K) and -(-N // 16) >= num_sms() and stream_supports(M, N, K)
 
 
 @functools.lru_cache(maxsize=4096)
@@ -1738,7 +1745,7 @@ def can_accumulate(x: torch.Tensor, w: torch.Tensor) -> bool:
     M, K = x.shape
     N = w.shape[0]
     if ws_supports(M, N, K):
-        return True
+        return not _ws_stack_pays(M, N, K)
     # (a result of so few tiles that it is better cut along K leaves partial sums, which a norm kernel adds)
     return _pair_rows(M) and N % 4 == 0 and pair_supports(M, N, K) and pair_splits(M, N, K) == 1
 
@@ -1809,7 +1816,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias, out_dtype: torch.dtype, allow
         raise KernelError("linear: CUDA only")
     M, K = x.shape
     N = w.shape[0]
-    if ws_supports(M, N, K):
+    if ws_supports(M, N, K) and not (allow_partials and out_dtype == torch.float32 and _ws_stack_pays(M, N, K)):
         return linear_ws(x, w, bias, out_dtype)
     if stream_supports(M, N, K):
         splits = _stream_splits(N, K) if (allow_partials and out_dtype == torch.float32) else 1
@@ -1865,7 +1872,7 @@ def linear_plain_act(x, w, out_dtype, act: str, token: "TokenColumns | None" = N
         M, K = x.shape
         N = w.shape[0]
         large = N * K >= LINEAR_TC_LARGE
-        if ws_supports(M, N, K) or (M <= 16 and not large and ws_takes(M, N, K)):
+        if ws_supports(M, N, K) and not _ws_stack_pays(M, N, K) or (M <= 16 and not large and ws_takes(M, N, K)):
             return linear_ws(x, w, None, out_dtype, act=act, token=token)
         if act in ("relu2", "gelu") and large and M >= LINEAR_TC_WIDE_FROM_ROWS and linear_tc_takes(M, N, K):
             return linear_tc(x, w, None, out_dtype, act=act)

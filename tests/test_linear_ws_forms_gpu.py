@@ -72,3 +72,33 @@ def test_more_tokens_on_small_matrices(M, N, K, takes):
     added = stream.clone()
     ops.linear_ws(x, w, b, torch.float32, residual=added)
     assert bool(((added - (stream + y)).abs() <= bound + 2.0 ** -23 * (stream.abs() + y.abs())).all())
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16, 24])
+@pytest.mark.parametrize("N,K", [(256, 1024), (1000, 1536), (2048, 1536), (512, 2048), (130, 2080), (2048, 2048), (20000, 1024), (19000, 1280)])
+def test_around_the_reductions_that_are_cut(M, N, K):
+    """Reductions on both sides of the lines from which clusters share them and from which rows are walked."""
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    g, x, w, b, y, bound = _product(dev, M, N, K)
+    assert bool(((ops.linear_ws(x, w, b, torch.float32) - y).abs() <= bound).all())
+    stream = torch.randn(M, N, device=dev, generator=g)
+    added = stream.clone()
+    ops.linear_ws(x, w, b, torch.float32, residual=added)
+    assert bool(((added - (stream + y)).abs() <= bound + 2.0 ** -23 * (stream.abs() + y.abs())).all())
+
+
+@pytest.mark.parametrize("N,K,slices", [(2560, 2560, True), (3072, 3072, True), (2048, 2048, False), (4096, 2048, False), (3584, 3584, False)])
+def test_partial_sums_for_those_who_add_them(N, K, slices):
+    """17 to 32 tokens and rows for one to one and a half CTAs an SM: a consumer that adds partial sums gets slices of K, one that cannot the whole product, and both
+    are the product."""
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    if ops.num_sms() != 148:
+        pytest.skip("the sizes are those of 148 SMs")
+    _, x, w, _, y, bound = _product(dev, 24, N, K)
+    y, bound = x.double() @ w.double().T, bound + 1
+    parts = ops.linear(x, w, None, torch.float32, True)
+    assert (parts.dim() == 3) == slices and ops.can_accumulate(x, w) == (not slices)
+    for got in (parts.double().sum(0) if slices else parts, ops.linear(x, w, None, torch.float32)):
+        assert got.dim() == 2 and float((got - y).norm() / y.norm()) < 1e-5
