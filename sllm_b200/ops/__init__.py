@@ -2107,7 +2107,10 @@ def attention_tiles(q_lens, group_size: int, device, ctx_lens=None, large_rows: 
 
 SPLIT_OVERHEAD_TILES = 3      # what a CTA of the decode form costs before and after its keys, in 64-key tiles
 MAX_SPLITS = 128              # the merge kernel keeps one weight a range in shared memory
-MERGE_TILES = 2               # the merge kernel behind a cut context (2.7 us; a short answer at 0.5B sizes, contexts below 256: 12.6 ms with it, 11.9 without)
+# The merge kernel behind a cut context, in key tiles of a CTA (2.7 us; a short answer at 0.5B sizes, contexts below 256: 12.6 ms with it, 11.9 without).  It also decides in
+# bands of longer contexts whose CTAs come to one or two waves (28 query heads of 128, us, in one range / as without this term): 160 (tile, KV head) pairs at 768 keys 21.4 / 23.5 in
+# three, 1,024 keys 27.4 / 28.2; 200 pairs at 2,048 49.8 / 53.3 in four; 224 pairs at 4,096 93.5 / 97.5 in five; 300 pairs at 512 27.6 / 32.7 in two.
+MERGE_TILES = 2
 SPLIT_MIN_KEYS = 128          # a range has at least two key tiles (one request at 1,024 keys: 11.0 us in 4 ranges, 8.6 in 8)
 MMA_MAX_SPLITS = 32           # the mma.sync form's merge walks the ranges one after the other
 

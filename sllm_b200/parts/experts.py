@@ -8,11 +8,11 @@ two-matrix experts, and optionally one expert every token uses.
 
 All experts' up projections are ONE matrix (expert e's rows at e * ff, the shared expert's after them) and their down
 projections one matrix side by side: a token's activation row carries its routing weights (zero for an expert not
-chosen), so the second product adds up the weighted experts by itself, in float32, in one order whatever else the batch
-holds.  In a decode step and a short portion every expert's product is computed for every token: E/top times the arithmetic
-of a sorted, grouped product and none of its bookkeeping, and a decode step reads every expert's matrix either way once the
-batch holds a few tokens.  Long portions sort their tokens by expert (`sorted_experts`), the weights then enter as the experts' rows are added
-up, in float32, in the order of the router's choices.
+chosen), so the second product adds up the weighted experts by itself, in float32, in one order.  In a decode step and a
+short portion every expert's product is computed for every token: E/top times the arithmetic of a sorted, grouped product
+and none of its bookkeeping, and a decode step reads every expert's matrix either way once the batch holds a few tokens.
+Long portions sort their tokens by expert (`sorted_experts`); the weights then enter as the experts' rows are added up, in
+float32, in the order of the router's choices.
 """
 
 from __future__ import annotations
@@ -118,7 +118,8 @@ class GatedExperts(FeedForward):
     alternating in blocks of 8, or all of the expert's gate rows before its up rows where ff is no multiple of 8) and their
     down projections one matrix side by side, the shared expert behind the others; w_sg is a row of the router's matrix (which is
     padded with rows of zeros to a size the products' kernels take).  A token's activation row carries its routing weights, so the second product
-    adds up the weighted experts in float32 in one order whatever the batch holds."""
+    adds up the weighted experts in float32 in one order; where a step's tokens are sorted by expert (`ops.moe_grouped_pays`, which looks at
+    the whole step) the weights enter behind it, so a portion's last bits depend on the portions beside it."""
 
     def __init__(self, params, **kw):
         super().__init__(params, **kw)

@@ -39,6 +39,9 @@ def test_the_cut_of_a_context_fills_whole_waves(ops_with_sms):
         assert ops.choose_splits(64, 4, 4096, 2) == 1
         assert ops.choose_splits(1, 4, 32768, 2) == 74             # 296 CTAs of seven key tiles
         assert ops.choose_splits(1, 4, 1024, 2) == 8               # ranges of two key tiles, not fewer
+        for pairs, ctx in ((32, 256), (148, 256), (160, 768), (160, 1024), (196, 1024), (200, 2048), (220, 2048), (224, 4096), (232, 4096), (300, 512)):
+            assert ops.choose_splits(pairs, 1, ctx, 2) == 1, (pairs, ctx)      # a wave or two of whole contexts: a cut and its merge do not pay
+        assert ops.choose_splits(120, 1, 512, 2) == 2 and ops.choose_splits(32, 1, 512, 2) == 4
 
 
 def test_tile_shapes_of_a_prompt_portions_products(ops_with_sms):
