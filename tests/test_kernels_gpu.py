@@ -935,8 +935,8 @@ def test_an_rmsnorm_owed_by_one_product_and_paid_by_the_next(M, H, K):
     def produce(into):
         if M <= 16:
             return ops.linear_accumulate_norm(x, w, b, into, gain, eps)      # as the engine calls it
-        # 17..32 tokens: the dispatch has no use for the warp-split kernel with a norm here (the matrices it sends
-        # there at so many tokens have more CTAs than the four-tile table holds); the kernel is called directly
+        # 17..32 tokens: the dispatch sends only some of these sizes to the warp-split kernel with a norm (small matrices, whose
+        # CTAs fit the four-tile table); the kernel is called directly for all that do
         xg_, scale_ = ops.linear_ws(x, w, b, torch.float32, residual=into, next_gain=gain)
         scale_.eps = eps
         return xg_, scale_

@@ -102,3 +102,44 @@ def test_partial_sums_for_those_who_add_them(N, K, slices):
     assert (parts.dim() == 3) == slices and ops.can_accumulate(x, w) == (not slices)
     for got in (parts.double().sum(0) if slices else parts, ops.linear(x, w, None, torch.float32)):
         assert got.dim() == 2 and float((got - y).norm() / y.norm()) < 1e-5
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("N,K", [(8208, 128), (9728, 896), (17920, 1536), (22016, 4096)])
+@pytest.mark.parametrize("parts", [1, 56, 296, 592])
+def test_gate_and_up_with_a_norm_owed_on_their_input(M, N, K, parts):
+    """Groups of rows side by side and one after the other, with the tokens' partial sums of squares of every size of table a producer leaves.  The bound: that of the
+    product, times the row's scale, 2^-20 more for the scale's own sum and root."""
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    g, x, w, b, _, _ = _product(dev, M, N, K)
+    ssq = torch.full((M, (parts + 3) & ~3), float("nan"), device=dev)          # (what lies beyond the parts is never read)
+    ssq[:, :parts] = torch.rand(M, parts, device=dev, generator=g) * 4 * K / parts
+    eps = 1e-5
+    scale = (ssq[:, :parts].double().sum(1, keepdim=True) / K + eps).rsqrt()
+    plain = x.double() @ w.double().T
+    y = plain * scale + b
+    bound = (K + 1) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T * scale + b.abs()) + 2.0 ** -20 * plain.abs() * scale
+    for act, fn in (("silu", torch.nn.functional.silu), ("gelu_tanh", lambda v: torch.nn.functional.gelu(v, approximate="tanh"))):
+        gate, up = y.reshape(M, N // 16, 2, 8).unbind(2)
+        gate_off, up_off = bound.reshape(M, N // 16, 2, 8).unbind(2)
+        want = fn(gate) * up
+        off = 2.0 ** -8 * want.abs() + 1.2 * (gate_off * up.abs() + up_off * gate.abs()) + 1e-5 * gate.abs() * up.abs() + 1e-30
+        got = ops.linear_ws_gated(x, w, b, act, scale=ops.RowScale(ssq, parts, eps, K)).reshape(M, N // 16, 8)
+        assert bool(((got - want).abs() <= off).all())
+
+
+@pytest.mark.parametrize("M", [17, 24, 32])
+@pytest.mark.parametrize("N,K", [(896, 896), (896, 4864), (2048, 5632), (2048, 2048)])
+def test_the_next_norms_input_from_more_tokens(M, N, K):
+    """17 to 32 tokens on small matrices, the columns shared by clusters: the stream, the next norm's input and its partial sums, as the dispatch has them made."""
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    g, x, w, b, y, bound = _product(dev, M, N, K)
+    assert ops.can_accumulate_norm(x, w)
+    stream, gain = torch.randn(M, N, device=dev, generator=g), torch.randn(N, device=dev, generator=g)
+    added = stream.clone()
+    xg, owed = ops.linear_accumulate_norm(x, w, b, added, gain, 1e-6)
+    assert bool(((added - (stream + y)).abs() <= bound + 2.0 ** -23 * (stream.abs() + y.abs())).all())
+    assert torch.equal(xg, (added * gain).bfloat16()) and owed.width == N and owed.eps == 1e-6 and owed.parts <= ops.MAX_SCALE_PARTS_ROWS32
+    torch.testing.assert_close(owed.ssq[:, :owed.parts].double().sum(1), added.double().pow(2).sum(1), rtol=N * 2.0 ** -24, atol=0)

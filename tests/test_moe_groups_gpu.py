@@ -1,6 +1,6 @@
 """A mixture of experts with the tokens sorted by expert (moe_groups.cu, the grouped form of gemm_pair.cu): the sorting itself, the grouped product
-with each of its epilogues, and whole mixtures against float64 (the bound: two bfloat16 roundings of each input and activation, 2^-8 of the
-terms' root sum of squares at worst, so 1e-2 of the result's)."""
+with each of its epilogues, and whole mixtures in both forms, against one another and against float64 (the bound: two bfloat16 roundings of each input and
+activation, 2^-8 of the terms' root sum of squares at worst, so 1e-2 of the result's)."""
 
 import pytest
 import torch
@@ -106,6 +106,49 @@ def test_a_mixture_sorted_by_expert(monkeypatch, kind, params, T):
     ops.check_tcgen05_status()
     assert float((got - want).norm() / want.norm()) < 1e-2
     torch.testing.assert_close(added, stream + got, rtol=1e-6, atol=1e-5)
+
+
+def _in_float64(part, kind, params, tensors, x):
+    """The mixture from the router's own choices and weights, expert by expert."""
+    dense, idx, wts = part.route(x)
+    t = {n: v.bfloat16().double() for n, v in tensors.items()}
+    x, silu = x.double(), torch.nn.functional.silu
+
+    def expert(n):
+        if kind == "routed_experts":
+            return torch.nn.functional.gelu(x @ t[f"{n}.up"].T) @ t[f"{n}.down"].T
+        gate, up = x @ t[f"{n}.gate"].T, x @ t[f"{n}.up"].T
+        if params.get("activation") == "silu":
+            return (silu(gate) * up) @ t[f"{n}.down"].T
+        gate, up = gate.clamp(max=params["limit"]), up.clamp(-params["limit"], params["limit"])
+        return (gate * torch.sigmoid(1.702 * gate) * (up + 1)) @ t[f"{n}.down"].T
+    out = sum(((idx == e) * wts).double().sum(-1, keepdim=True) * expert(f"e{e}") for e in range(params["experts"]))
+    if params.get("shared_ff"):
+        out = out + expert("shared") * (torch.sigmoid(x @ t["shared.sg"].T) if kind == "gated_experts" else 1.0)
+    return out
+
+
+@pytest.mark.parametrize("kind,params", CASES)
+@pytest.mark.parametrize("sort", [False, True])
+def test_a_mixture_in_float64(monkeypatch, kind, params, sort):
+    import sllm_b200.ops as ops
+    from sllm_b200.config.plan import PartSpec
+    from sllm_b200.models import causal_lm  # noqa: F401  (registers the parts)
+    from sllm_b200.parts.base import FEED_FORWARDS
+    dev = cuda_or_skip()
+    part = FEED_FORWARDS.build(PartSpec(kind, dict(params, hidden_size=256)), dtype=torch.bfloat16, device=dev)
+    g = torch.Generator(device=dev).manual_seed(7)
+    tensors = {s.name: torch.randn(*s.shape, device=dev, generator=g) / max(1, s.shape[-1]) ** 0.5 for s in part.tensor_specs()}
+    part.bind(tensors.__getitem__)
+    x = torch.randn(530, 256, device=dev, generator=g).bfloat16()
+    monkeypatch.setattr(ops, "moe_grouped_pays", lambda *a: sort)
+    y = part.forward(x, None)
+    ops.check_tcgen05_status()
+    y = (y.sum(0) if y.dim() == 3 else y).double()
+    want = _in_float64(part, kind, params, tensors, x)
+    assert float((y - want).norm() / want.norm()) < 1e-2
+    worst = (y - want).norm(dim=1) / want.norm(dim=1).clamp(min=0.1 * float(want.norm(dim=1).mean()))
+    assert float(worst.max()) < 3e-2                         # no token with another expert's rows or weights
 
 
 @pytest.mark.parametrize("shared_ff", [100, 96])
