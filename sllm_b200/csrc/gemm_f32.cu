@@ -17,7 +17,7 @@
 //   memory, or where the tiles alone fill the GPU one CTA's, one after the other.  The packed form matters here: it halves the issue slots of the multiply-adds, which leaves room for the loads from shared memory.
 //
 // Measured (us; floor: W at 6.65 TB/s): 3 rows, 9,728 x 896 10.0 (floor 5.2; 82 with the one 64 x 64 tile form there was before), 896 x 4,864 10.4
-// (2.6; 342), 151,936 x 896 93 (82; 503); 537 rows 259 (36 TFLOP/s; 314) and 150 (31; 297); 2,048 rows of 9,728 x 896 844 (42 TFLOP/s of 74; 1,015).
+// (2.6; 342), 151,936 x 896 93 (82; 503); 543 rows 260 (36 TFLOP/s; 314) and 149 (32; 299); 2,048 rows of 9,728 x 896 844 (42 TFLOP/s of 74; 1,015).
 // The tiles are bound by the multiply-add pipes (59 % active) and the reads of shared memory beside them (75 %).
 #include <cooperative_groups.h>
 #include <stdio.h>
