@@ -1025,6 +1025,13 @@ static void sample_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[2
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
 }
 
+// Raises the kernel's limit of shared memory; what fits the GPU is asked with it raised, whichever call of a process comes first.
+static bool sample_smem_raised() {
+  static bool raised = false;
+  if (!raised) raised = cudaFuncSetAttribute(sample_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_SMEM) == cudaSuccess;
+  return raised;
+}
+
 // Blocks a row (log2): as many as leave every row's cluster on the GPU at once.  A block fills an SM (1,024 threads of 64 registers) and a cluster lies in one
 // GPC, so that is 15 rows of eight, 33 of four; rows that wait for a whole cluster's place pay for it however little its other
 // blocks have to do (151,936 logits, us, eight blocks / as chosen: 16 greedy rows 8.8 / 5.6, 128 38 / 10; 128 rows of top_p 0.9 212 / 73; 32 rows of top_k 20 31 / 16).
@@ -1043,6 +1050,7 @@ static int row_blocks_log2(int R, int V) {
       cudaGetLastError();
     }
   };
+  if (!sample_smem_raised()) return 0;
   static const Fit fit;
   int lg = SAMPLE_BLOCKS_LOG2;
   while (lg > 0 && R > fit.rows[lg]) --lg;
@@ -1064,13 +1072,9 @@ SLLM_EXPORT int sllm_sample_rows(const float* logits, int R, int V, const float*
   SLLM_REQUIRE(temperature == nullptr || uniform != nullptr, "sample_rows: temperatures without uniforms");
   SLLM_REQUIRE(temperature != nullptr || (top_k == nullptr && top_p == nullptr), "sample_rows: filters without temperatures");
   if (R == 0) return SLLM_OK;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(sample_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_SMEM) != cudaSuccess) {
-      set_error("sample_rows: cannot raise the shared memory limit");
-      return SLLM_ERR_LAUNCH;
-    }
-    configured = true;
+  if (!sample_smem_raised()) {
+    set_error("sample_rows: cannot raise the shared memory limit");
+    return SLLM_ERR_LAUNCH;
   }
   const int smem = (top_k || top_p) ? SAMPLE_SMEM : 0;
   const int lg = row_blocks_log2(R, V);

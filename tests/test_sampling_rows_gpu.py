@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 import torch
 
-from tests.conftest import cuda_or_skip
+from tests.conftest import ROOT, cuda_or_skip
 
 pytestmark = pytest.mark.gpu
 
@@ -91,3 +91,14 @@ def test_few_rows_are_shared_by_blocks_and_many_are_not(V, R):
     few = range(0, R, max(1, R // 12))
     alone = [int(ops.sample_rows(logits[r:r + 1], t[r:r + 1], u[r:r + 1], k[r:r + 1], p[r:r + 1])) for r in few]
     assert [int(got[r]) for r in few] == alone
+
+
+def test_blocks_a_row_asked_before_the_first_launch():
+    """The answer is kept for the process, so it must not depend on whether a row has been sampled yet."""
+    import subprocess
+    import sys
+    cuda_or_skip()
+    code = "import torch, sllm_b200.ops as ops; torch.zeros(1, device='cuda'); print(ops.lib().sllm_sample_rows_blocks(1, 151936))"
+    done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, cwd=ROOT)
+    assert done.returncode == 0, done.stderr
+    assert int(done.stdout.split()[-1]) == 8
