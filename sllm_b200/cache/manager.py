@@ -104,6 +104,7 @@ class CacheManager:
         self.kv_storage = []       # per group: tensor [runs, 2, pages, nkv, page_size, hd] (1 for 2 where keys are the values)
         self.state_storage = {}    # (run, name) -> tensor [slots, *shape]
         self.slot_tables = {}      # name -> tensor [slots, ...] of per-request state that others own (`register_slot_table`)
+        self._slot_rows = None     # all of these, as one kernel zeroes their rows (`zero_rows`)
         self.reuse_count = 0       # pages handed out that had been held before
         self._ever_used = [set() for _ in self.groups]
 
@@ -157,15 +158,32 @@ class CacheManager:
         return True
 
     # ---- life of a request -----------------------------------------------------------
-    def add_request(self, req_id) -> RequestCache:
+    def add_request(self, req_id, zero: bool = True) -> RequestCache:
+        """``zero`` false: the caller zeroes the request's rows itself, together with those of the others it admits (`zero_rows`)."""
         if req_id in self.requests:
             raise ValueError(f"request {req_id!r} is already live")
         slot = self.slots.allocate(req_id)
         req = RequestCache(req_id, slot, 0, [[] for _ in self.groups])
         self.requests[req_id] = req
-        for t in (*self.state_storage.values(), *self.slot_tables.values()):
-            t[slot].zero_()
+        if zero:
+            self.zero_rows([req])
         return req
+
+    def zero_rows(self, reqs) -> None:
+        """The rows of these requests in every per-request table become zero: one kernel for all of them where the tables lie on a GPU (a fill a row and
+        table otherwise)."""
+        tables = (*self.state_storage.values(), *self.slot_tables.values())
+        if not reqs or not tables:
+            return
+        if all(t.is_cuda and t.is_contiguous() and t.device == tables[0].device for t in tables):
+            if self._slot_rows is None:
+                from .. import ops
+                self._slot_rows = ops.SlotRows(tables)
+            self._slot_rows.zero([r.slot for r in reqs])
+            return
+        for r in reqs:
+            for t in tables:
+                t[r.slot].zero_()
 
     def register_slot_table(self, name: str, table) -> None:
         """Per-request state of fixed size that lives outside the model (the sampler's table of
@@ -174,6 +192,7 @@ class CacheManager:
         if table.shape[0] != self.max_requests + 1:
             raise ValueError(f"slot table {name!r} has {table.shape[0]} rows, the cache has {self.max_requests} + 1 slots")
         self.slot_tables[name] = table
+        self._slot_rows = None
 
     def reserve(self, req_id, total_tokens: int) -> None:
         """Grow the request's tables to hold ``total_tokens``.  Takes all pages
@@ -311,6 +330,7 @@ class CacheManager:
         self.state_storage = {
             (run, s.name): torch.zeros((self.max_requests + 1,) + tuple(s.shape), dtype=torch.float32, device=device)
             for run, states in self.state_runs.items() for s in states}
+        self._slot_rows = None
         caches: list[LayerCache] = []
         for run, entry in enumerate(self.needs):
             how, what = entry[0], entry[1]

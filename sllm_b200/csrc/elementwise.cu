@@ -53,6 +53,29 @@ __global__ void embed_gather_kernel(const TW* __restrict__ table, const int* __r
 }
 
 // ---------------------------------------------------------------------------
+// The rows of newly admitted requests in every per-request table, zeroed together: table t starts at rows[2t] and has rows of
+// rows[2t + 1] bytes; a grid column a (table, slot).  Bound by launches: a fill per (request, layer's state) left the device idle between 1.4 us fills
+// (16 requests of 8 layers: 128 of them, 1.5 ms before a step's first kernel; one launch: 4 us for their 16 MB).
+// ---------------------------------------------------------------------------
+constexpr int ZERO_SLOTS = 64;                    // slots of a launch
+constexpr int ZERO_CHUNK = 64 * 1024;             // bytes of a CTA
+struct ZeroSlots { int slot[ZERO_SLOTS]; };
+
+__global__ void __launch_bounds__(256) zero_rows_kernel(const long long* __restrict__ rows, const ZeroSlots slots) {
+  pdl_launch_dependents();       // a short kernel: the successor may be set up behind it
+  pdl_wait();
+  const long long bytes = rows[2 * blockIdx.x + 1];
+  const long long b0 = (long long)blockIdx.z * ZERO_CHUNK, b1 = b0 + ZERO_CHUNK < bytes ? b0 + ZERO_CHUNK : bytes;
+  if (b0 >= bytes) return;
+  unsigned char* p = reinterpret_cast<unsigned char*>(rows[2 * blockIdx.x]) + (long long)slots.slot[blockIdx.y] * bytes;
+  const long long h = b0 + ((16 - ((unsigned long long)(p + b0) & 15)) & 15);          // a row may start on any byte (a table of bytes with an odd vocabulary)
+  const long long head = h < b1 ? h : b1, tail = head + (b1 - head) / 16 * 16;
+  for (long long i = b0 + threadIdx.x; i < head; i += 256) p[i] = 0;
+  for (long long i = head + threadIdx.x * 16; i < tail; i += 256 * 16) *reinterpret_cast<uint4*>(p + i) = make_uint4(0, 0, 0, 0);
+  for (long long i = tail + threadIdx.x; i < b1; i += 256) p[i] = 0;
+}
+
+// ---------------------------------------------------------------------------
 // residual += sum of `parts` delta slices (if any); out = residual * rsqrt(mean(residual^2)+eps) * w
 // Formula ref/standard.py:25-31; fusion with the add as kernels/cuda/kernels.cu:791-839;
 // 1/sqrtf, not rsqrtf (kernels.cu:818-820).  The sum over a row is taken in an order
@@ -418,6 +441,22 @@ using namespace sllm;
 SLLM_EXPORT const char* sllm_last_error() { return g_error; }
 
 // streaming multiprocessors of the current device: the dispatch sizes its splits for them
+// rows: device, [tables][2] (start, bytes of a row); most_bytes: the longest row; slots: host
+SLLM_EXPORT int sllm_zero_rows(const long long* rows, int tables, long long most_bytes, const int* slots, int n, cudaStream_t stream) {
+  SLLM_REQUIRE(tables >= 0 && tables <= (1 << 20) && n >= 0 && most_bytes >= 0 && most_bytes / ZERO_CHUNK < 65535, "zero_rows: %d tables, %d slots, rows of %lld bytes", tables, n, most_bytes);
+  if (tables == 0 || most_bytes == 0) return SLLM_OK;
+  for (int i = 0; i < n; i += ZERO_SLOTS) {
+    const int m = n - i < ZERO_SLOTS ? n - i : ZERO_SLOTS;
+    ZeroSlots z = {};
+    for (int k = 0; k < m; ++k) {
+      SLLM_REQUIRE(slots[i + k] >= 0, "zero_rows: slot %d", slots[i + k]);
+      z.slot[k] = slots[i + k];
+    }
+    launch_kernel(zero_rows_kernel, dim3((unsigned)tables, (unsigned)m, (unsigned)((most_bytes + ZERO_CHUNK - 1) / ZERO_CHUNK)), 256, 0, stream, rows, z);
+  }
+  return launch_status("zero_rows");
+}
+
 SLLM_EXPORT int sllm_num_sms() { return sllm::num_sms(); }
 
 SLLM_EXPORT int sllm_embed_gather(const void* table, int table_dtype, const int* ids, float* out, int T, int H,

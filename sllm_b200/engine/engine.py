@@ -120,9 +120,8 @@ class Engine:
             pool = cache.groups[gi].pool
             if need > pool.free_count:
                 raise OutOfPages(f"step needs {need} pages in group {gi}, {pool.free_count} free of {pool.capacity}")
+        cache.zero_rows([cache.add_request(e.req_id, zero=False) for e in entries if e.req_id not in cache.requests])
         for e, tot in zip(entries, totals):
-            if e.req_id not in cache.requests:
-                cache.add_request(e.req_id)
             cache.reserve(e.req_id, tot)
 
         # ---- the description: packed into one pinned buffer, one copy --------------------

@@ -160,7 +160,7 @@ class Scheduler:
                 planned_ids.add(r.req_id)
                 budget -= n
         # admission (pump): skip what does not fit, keep its place
-        skipped = []
+        skipped, admitted = [], []
         while self.waiting and len(self.running) < self.max_num_seqs and budget > 0:
             r = self.waiting.popleft()
             n = min(r.pending, self.chunk_size, budget)
@@ -171,13 +171,14 @@ class Scheduler:
             if n <= 0 or not self.cache.can_reserve(r.req_id, total):
                 skipped.append(r)
                 continue
-            self.cache.add_request(r.req_id)
+            admitted.append(self.cache.add_request(r.req_id, zero=False))
             self.cache.reserve(r.req_id, total)
             r.status = "running"
             self.running.append(r)
             plan.append(Planned(r, r.num_computed, n, r.num_computed + n == r.num_tokens))
             planned_ids.add(r.req_id)
             budget -= n
+        self.cache.zero_rows(admitted)
         self.waiting.extendleft(reversed(skipped))
         self._trim_to_row_tiles(plan)
         return plan

@@ -9,6 +9,7 @@ float32 path, runs in this package's own kernels.
 
 from __future__ import annotations
 
+import ctypes
 import functools
 import os
 from collections import namedtuple
@@ -70,6 +71,27 @@ def embed_gather(table: torch.Tensor, ids: torch.Tensor, scale: float = 1.0) -> 
     out = torch.empty((T, H), dtype=torch.float32, device=table.device)
     call("sllm_embed_gather", _p(table), _dt(table), _p(ids), _p(out), T, H, V, float(scale), _stream())
     return out
+
+
+class SlotRows:
+    """Tables of per-request rows (``[slots, ...]`` each, contiguous, on one device), to be zeroed a request at a time in all of them at once: what a request's
+    admission does to the state it will carry."""
+
+    def __init__(self, tables):
+        _chk(*tables)
+        self.tables = list(tables)                # (their addresses stand in `rows`)
+        self.slots = min(t.shape[0] for t in self.tables)
+        sizes = [t[0].numel() * t.element_size() for t in self.tables]
+        self.most = max(sizes)
+        self.rows = torch.tensor([[t.data_ptr(), n] for t, n in zip(self.tables, sizes)], dtype=torch.int64).to(self.tables[0].device)
+
+    def zero(self, slots) -> None:
+        """Rows ``slots`` of every table become zero, in one launch (for up to 64 of them)."""
+        slots = [int(s) for s in slots]
+        if not all(0 <= s < self.slots for s in slots):
+            raise KernelError(f"SlotRows: slots {slots} of {self.slots}")
+        if slots:
+            call("sllm_zero_rows", _p(self.rows), len(self.tables), self.most, (ctypes.c_int * len(slots))(*slots), len(slots), _stream())
 
 
 # ---- a stream of several copies ------------------------------------------------------------------------

@@ -1022,3 +1022,19 @@ def test_attention_tma_decode(nq, nkv, hd, ps, window, case, consecutive):
         ops.check_tcgen05_status()
         assert not out.isnan().any(), "a row was not written, or a masked slot held garbage"
         torch.testing.assert_close(out.float(), want, rtol=2e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("admitted", [[0], [3, 1], list(range(70))])
+def test_rows_of_admitted_requests_are_zeroed_in_every_table(admitted):
+    """Rows of any size and start (bytes of an odd vocabulary, one float, more than a CTA's share), more slots than a launch takes: the named rows and no others."""
+    ops = _ops()
+    S = 75
+    shapes = [((S, 1), torch.float32), ((S, 3, 40, 150), torch.float32), ((S, 151937), torch.uint8), ((S, 15), torch.uint8), ((S, 16384), torch.float32)]
+    tables = [torch.full(shape, 7, dtype=dt, device="cuda") for shape, dt in shapes]
+    ops.SlotRows(tables).zero(admitted)
+    for t in tables:
+        want = torch.full_like(t, 7)
+        want[torch.tensor(admitted, device="cuda")] = 0
+        assert torch.equal(t, want)
+    with pytest.raises(ops.KernelError):
+        ops.SlotRows(tables).zero([S])
