@@ -65,6 +65,16 @@ __device__ __forceinline__ float block_sum(float v, float* red /* >= 33 floats *
   return red[32];
 }
 
+// The same sum (the same order, the same bits) with one barrier in place of three: every warp adds the warps' sums itself.  `red` (32 floats) is
+// this sum's own: nobody writes to it again.
+__device__ __forceinline__ float block_sum_once(float v, float* red) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+  v = warp_sum(v);
+  if (lane == 0) red[warp] = v;
+  __syncthreads();
+  return warp_sum(lane < nw ? red[lane] : 0.f);
+}
+
 // ---- activations a product's epilogue (or the kernel behind a product) applies to a plain, ungated result ----------------
 #define SLLM_ACT_NONE 0
 #define SLLM_ACT_RELU2 1       // max(v, 0)^2
@@ -106,6 +116,8 @@ void set_error(const char* msg);   // remembers the text for sllm_last_error()
 // graph): 3.24 ms so; 3.29 ms with no early release in the short kernels; 6.05 ms with the release
 // at the top of every kernel; 3.33 ms with SLLM_PDL=0 in the environment (the attribute off, plain
 // stream order).
+// A kernel that loads straight behind pdl_wait() what an earlier kernel wrote takes that pointer without __restrict__: a load from a const __restrict__ pointer is free to move, and moves, in
+// front of the wait.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

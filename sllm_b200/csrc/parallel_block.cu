@@ -288,6 +288,121 @@ norm_pair_kernel(const float* __restrict__ stream, const float* __restrict__ gai
   }
 }
 
+// The same with the row in registers, two vectors of four a thread (W a multiple of 4, at most 8,192; every pointer 16-byte aligned): the gains, which no kernel of
+// the step writes, are loaded before the wait, and nothing behind the sum waits for memory.  (In a graph of such kernels, us, before / now: 16 rows of 2,048 4.1 / 1.4, 2,292 rows of 4,096 32 / 14.)
+constexpr int NORM_PAIR_V = 2;
+template <typename TO>
+__global__ void __launch_bounds__(1024)
+norm_pair_vec_kernel(const float* stream, const float* gain_a, const float* gain_b, float eps,
+                     TO* out_a, TO* out_b, int W) {
+  __shared__ float red[32];
+  pdl_launch_dependents();
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 a[NORM_PAIR_V], b[NORM_PAIR_V], x[NORM_PAIR_V];
+#pragma unroll
+  for (int k = 0; k < NORM_PAIR_V; ++k) {
+    const int i = (threadIdx.x + k * blockDim.x) * 4;
+    a[k] = i < W ? pb_load4(gain_a + i) : zero;
+    b[k] = i < W && gain_b != nullptr ? pb_load4(gain_b + i) : zero;
+  }
+  pdl_wait();
+  const size_t base = (size_t)blockIdx.x * W;
+  float ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < NORM_PAIR_V; ++k) {
+    const int i = (threadIdx.x + k * blockDim.x) * 4;
+    x[k] = i < W ? pb_load4(stream + base + i) : zero;
+  }
+#pragma unroll
+  for (int k = 0; k < NORM_PAIR_V; ++k) {
+    ss = fmaf(x[k].x, x[k].x, ss); ss = fmaf(x[k].y, x[k].y, ss); ss = fmaf(x[k].z, x[k].z, ss); ss = fmaf(x[k].w, x[k].w, ss);
+  }
+  const float inv = 1.0f / sqrtf(block_sum_once(ss, red) / (float)W + eps);
+#pragma unroll
+  for (int k = 0; k < NORM_PAIR_V; ++k) {
+    const int i = (threadIdx.x + k * blockDim.x) * 4;
+    if (i >= W) continue;
+    const float4 v = make_float4(x[k].x * inv, x[k].y * inv, x[k].z * inv, x[k].w * inv);
+    pb_store4(out_a + base + i, make_float4(v.x * a[k].x, v.y * a[k].y, v.z * a[k].z, v.w * a[k].w));
+    if (out_b != nullptr) pb_store4(out_b + base + i, make_float4(v.x * b[k].x, v.y * b[k].y, v.z * b[k].z, v.w * b[k].w));
+  }
+}
+
+// group_norm_shift_kernel for a stream with nothing pending whose groups are multiples of 128 channels (W up to 4,096; every pointer 16-byte aligned): a warp holds V
+// pieces of 128 channels of its row, and of the other row, in registers; a piece's squares are added in the warp, a group's pieces in order, so the bits do not depend on
+// V.  Few rows are bound by latency: one piece a warp, the gain and the mix loaded before the wait, the row's place in its request beside the row itself.  Many rows (GNS_MANY_ROWS
+// an SM) by what is in flight and by blocks that come and go: two pieces with a shift, four without.  (In a graph of such kernels, 4 groups, us, before / now: with a shift 8 rows of 2,048
+// 3.3 / 2.3, 8 rows of 4,096 4.9 / 3.0, 2,048 rows of 2,048 25.7 / 12.9 (14.2 with one piece), 2,292 rows of 4,096 181 / 35 (60); plain 8 rows of 4,096 2.7 / 1.7, 2,292 rows of 4,096
+// 14.7 / 14.5 (31.8).)
+constexpr int GNS_MANY_ROWS = 2;
+template <typename TO, int V, bool MIX>
+__global__ void __launch_bounds__(1024 / V)
+group_norm_shift_regs_kernel(const float* stream, const float* gain, const float* mix, float* state, const int* seq_of_token, const int* q_start,
+                             const int* state_slots, TO* out_h, TO* out_hs, int W, int groups, float eps) {
+  __shared__ float red[2][32];
+  pdl_launch_dependents();
+  const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int gs = W / groups, pieces = gs / 128;
+  float4 w[V], m[MIX ? V : 1], x[V], ox[MIX ? V : 1], hp[MIX ? V : 1];
+  auto at = [&](int k) { return (warp * V + k) * 128 + lane * 4; };
+#pragma unroll
+  for (int k = 0; k < V; ++k) {
+    w[k] = pb_load4(gain + at(k));
+    if constexpr (MIX) m[k] = pb_load4(mix + at(k));
+  }
+  pdl_wait();
+#pragma unroll
+  for (int k = 0; k < V; ++k) x[k] = pb_load4(stream + (size_t)t * W + at(k));
+  int other_t = t;
+  bool first = false;
+  float* slot = nullptr;
+  if constexpr (MIX) {                     // the other row: the one before, or for a portion's first token the portion's last
+    const int s = seq_of_token[t];
+    first = t == q_start[s];
+    other_t = first ? q_start[s + 1] - 1 : t - 1;
+    slot = state + (size_t)state_slots[s] * W;
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      ox[k] = other_t != t ? pb_load4(stream + (size_t)other_t * W + at(k)) : x[k];
+      hp[k] = first ? pb_load4(slot + at(k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+  auto squares = [](float4 v) { return warp_sum(fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, v.x * v.x)))); };
+#pragma unroll
+  for (int k = 0; k < V; ++k) {
+    const float sx = squares(x[k]);
+    if (lane == 0) red[0][warp * V + k] = sx;
+    if constexpr (MIX) {
+      const float so = squares(ox[k]);
+      if (lane == 0) red[1][warp * V + k] = so;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < V; ++k) {
+    const int i = at(k), p0 = (warp * V + k) / pieces * pieces;
+    float ssx = 0.f, sso = 0.f;
+    for (int p = p0; p < p0 + pieces; ++p) {
+      ssx += red[0][p];
+      if (MIX) sso += red[1][p];
+    }
+    const float r = 1.0f / sqrtf(ssx / (float)gs + eps);
+    const float4 h = make_float4(x[k].x * r * w[k].x, x[k].y * r * w[k].y, x[k].z * r * w[k].z, x[k].w * r * w[k].w);
+    if (out_h != nullptr) pb_store4(out_h + (size_t)t * W + i, h);
+    if constexpr (MIX) {
+      const float orr = 1.0f / sqrtf(sso / (float)gs + eps);
+      const float4 oh = make_float4(ox[k].x * orr * w[k].x, ox[k].y * orr * w[k].y, ox[k].z * orr * w[k].z, ox[k].w * orr * w[k].w);
+      float4 prev = oh;
+      if (first) {
+        prev = hp[k];
+        pb_store4(slot + i, oh);
+      }
+      pb_store4(out_hs + (size_t)t * W + i, make_float4(h.x + (prev.x - h.x) * m[k].x, h.y + (prev.y - h.y) * m[k].y,
+                                                        h.z + (prev.z - h.z) * m[k].z, h.w + (prev.w - h.w) * m[k].w));
+    }
+  }
+}
+
 }  // namespace sllm
 
 using namespace sllm;
@@ -326,6 +441,20 @@ SLLM_EXPORT int sllm_group_norm_shift(const float* stream, const float* rinv, co
   auto aligned = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
   const bool vec = W % 4 == 0 && (W / groups) % 4 == 0 && aligned(stream) && aligned(gain) && aligned(mix) && aligned(state) &&
                    aligned(out_h) && aligned(out_hs);
+  if (vec && rinv == nullptr && W % 128 == 0 && (W / groups) % 128 == 0 && W <= 4096 && (out_dtype == SLLM_F32 || out_dtype == SLLM_BF16)) {
+    const bool many = T > GNS_MANY_ROWS * num_sms();
+#define SLLM_GNR(TO, V_, MIX_)                                                                                                                        \
+  launch_kernel(group_norm_shift_regs_kernel<TO, V_, MIX_>, T, W / 4 / V_, 0, stream_, stream, gain, mix, state, seq_of_token, q_start, state_slots, (TO*)out_h, \
+                (TO*)out_hs, W, groups, eps)
+#define SLLM_GNR_FORM(TO)                                                             \
+  if (mix != nullptr) { if (many && W % 256 == 0) SLLM_GNR(TO, 2, true); else SLLM_GNR(TO, 1, true); } \
+  else { if (many && W % 512 == 0) SLLM_GNR(TO, 4, false); else SLLM_GNR(TO, 1, false); }
+    if (out_dtype == SLLM_F32) { SLLM_GNR_FORM(float) }
+    else { SLLM_GNR_FORM(__nv_bfloat16) }
+#undef SLLM_GNR_FORM
+#undef SLLM_GNR
+    return launch_status("group_norm_shift");
+  }
 #define SLLM_GNS(TO, VEC_)                                                                                                 \
   launch_kernel(group_norm_shift_kernel<TO, VEC_>, T, threads, smem, stream_, stream, rinv, gain, mix, state, seq_of_token, \
                 q_start, state_slots, (TO*)out_h, (TO*)out_hs, W, groups, eps)
@@ -385,6 +514,15 @@ SLLM_EXPORT int sllm_norm_pair(const float* stream, const float* gain_a, const f
                                int out_dtype, int T, int W, cudaStream_t stream_) {
   SLLM_REQUIRE(T >= 0 && W > 0 && gain_a && out_a && ((gain_b == nullptr) == (out_b == nullptr)), "norm_pair: bad arguments T=%d W=%d", T, W);
   if (T == 0) return SLLM_OK;
+  auto aligned = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
+  if (W % 4 == 0 && W <= 8192 && aligned(stream) && aligned(gain_a) && aligned(gain_b) && aligned(out_a) && aligned(out_b) && (out_dtype == SLLM_F32 || out_dtype == SLLM_BF16)) {
+    const int vec_threads = (W / 4 + 32 * NORM_PAIR_V - 1) / (32 * NORM_PAIR_V) * 32;
+    if (out_dtype == SLLM_F32)
+      launch_kernel(norm_pair_vec_kernel<float>, T, vec_threads, 0, stream_, stream, gain_a, gain_b, eps, (float*)out_a, (float*)out_b, W);
+    else
+      launch_kernel(norm_pair_vec_kernel<__nv_bfloat16>, T, vec_threads, 0, stream_, stream, gain_a, gain_b, eps, (__nv_bfloat16*)out_a, (__nv_bfloat16*)out_b, W);
+    return launch_status("norm_pair");
+  }
   const int threads = W >= 2048 ? 256 : 128;
   if (out_dtype == SLLM_F32)
     launch_kernel(norm_pair_kernel<float>, T, threads, 0, stream_, stream, gain_a, gain_b, eps, (float*)out_a, (float*)out_b, W);
