@@ -62,6 +62,9 @@ __device__ __forceinline__ uint4 ws_ldg(const void* p) {       // activations: s
   asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
+__device__ __forceinline__ void ws_copy4(void* smem, const void* p) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(p) : "memory");
+}
 __device__ __forceinline__ void ws_mma(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3,
                                        unsigned b0, unsigned b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
@@ -119,6 +122,14 @@ linear_ws_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __res
   __shared__ float row_scale[8 * NT];
   __shared__ float slice_sum[SLICED ? WS_SLICES : 1][SLICED ? 16 * 8 * NT : 1];
   __shared__ __align__(16) float ssq_s[SCALED ? 8 * NT : 1][SCALED ? ws_ssq_max(NT) : 4];
+  // What the thread's own outputs will need beside the product, copied under the stream of weights: a load behind the last sums is a miss in HBM for what no kernel of the step
+  // writes (gain, bias, cos and sin: a step's weights push them out of L2), one in L2 for the stream.  (In a graph of such products, us, before / now: residual
+  // with the next norm's input 896 x 896, one token 2.74 / 2.36, 3,584 x 3,584, 8 tokens 7.80 / 7.11, 2,048 x 5,632, 32 tokens 10.3 / 9.3; rotary 1,152 x 896, one token 3.43 / 2.81.)
+  // (A residual form that itself has a norm owed does without, and two token tiles with a norm owed keep no bias: shared memory.)
+  constexpr bool AHEAD = (EPI == WS_EPI_RESID && !SCALED && (FORM == WS_ONE || FORM == WS_SLICED)) || EPI == WS_EPI_ROPE;
+  constexpr bool BIAS_AHEAD = !(SCALED && NT == 2);
+  constexpr int AHEAD_N = EPI == WS_EPI_ROPE ? 64 * NT : (16 * 8 * NT + WS_WARPS * 32 - 1) / (WS_WARPS * 32) * WS_WARPS * 32;
+  __shared__ float ahead[AHEAD ? (EPI == WS_EPI_ROPE ? (BIAS_AHEAD ? 4 : 2) : 3) : 1][AHEAD ? AHEAD_N : 1];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t4 = lane & 3;
   // The CTA's rows [c0, c1), the N rows dealt evenly over the grid (so that a grid of a whole number of CTAs per SM gives
@@ -203,10 +214,46 @@ linear_ws_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __res
   constexpr int GROUP = WS_DEPTH * KW;        // k blocks the CTA covers per group
   const int k_mine = k_first + warp % KW;
   int kb = k_mine;
+  int ahead_pos = 0, ahead_slot = -1;
+  if constexpr (EPI == WS_EPI_ROPE) {         // (the step's description was there before the step's first kernel)
+    const int tok = tid / 8;
+    if (tid < AHEAD_N && tok < M) {
+      if (rope.table != nullptr) ahead_pos = rope.positions[tok];
+      if (rope.slot_mapping != nullptr) ahead_slot = rope.slot_mapping[tok];
+    }
+  }
   load_w(wa0, wb0, kb);
+  if constexpr (EPI == WS_EPI_ROPE) {
+    const int tok = tid / 8, i = tid % 8, half = rope.hd / 2, j = n0 % rope.hd + i;
+    if (tid < AHEAD_N && tok < M) {
+      const float* cs = rope.table + (size_t)min(max(ahead_pos, 0), rope.max_pos - 1) * rope.hd;        // cos[half] then sin[half]
+      if (rope.table != nullptr) {
+        ws_copy4(&ahead[0][tid], cs + j);
+        ws_copy4(&ahead[1][tid], cs + half + j);
+      }
+      if (BIAS_AHEAD && bias) {
+        ws_copy4(&ahead[BIAS_AHEAD ? 2 : 0][tid], bias + n0 + i);
+        ws_copy4(&ahead[BIAS_AHEAD ? 3 : 0][tid], bias + n0 + half + i);
+      }
+    }
+  }
+  auto resid_at = [&](auto&& use) {           // the thread's outputs of the CTA's only group
+    for (int idx = tid; idx < 16 * 8 * NT; idx += WS_WARPS * 32) {
+      const int tok = idx / 16, n = n0 + idx % 16;
+      if (tok < M && n < n1 && slice == 0) use(idx, tok, n);
+    }
+  };
+  if constexpr (EPI == WS_EPI_RESID && AHEAD) {
+    resid_at([&](int idx, int, int n) {
+      if (norm.gain != nullptr) ws_copy4(&ahead[0][idx], norm.gain + n);
+      if (bias) ws_copy4(&ahead[1][idx], bias + n);
+    });
+  }
   if constexpr (SLICED) cooperative_groups::this_cluster().sync();      // nobody writes to a CTA that has not begun
   pdl_wait();
   load_x(x0, kb);
+  if constexpr (EPI == WS_EPI_RESID && AHEAD) resid_at([&](int idx, int tok, int n) { ws_copy4(&ahead[2][idx], residual + (size_t)tok * N + n); });
+  if constexpr (AHEAD) asm volatile("cp.async.commit_group;\n" ::);
   // a norm still owed on the input: the tokens' partial sums of squares are copied to shared memory under
   // the stream and added after the loop
   if constexpr (SCALED) {
@@ -259,8 +306,8 @@ linear_ws_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __res
         red[warp][g + ((c & 2) ? 8 : 0)][8 * j + 2 * t4 + (c & 1)] = acc[j][c];
         acc[j][c] = 0.f;
       }
-    if constexpr (SCALED) {
-      if (group == 0) asm volatile("cp.async.wait_group 0;\n" ::);
+    if constexpr (SCALED || AHEAD) {
+      if (group == 0) asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     }
     __syncthreads();
     if constexpr (SCALED) {
@@ -281,9 +328,8 @@ linear_ws_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __res
     if constexpr (EPI == WS_EPI_ROPE) {
       const int half = rope.hd / 2;
       const int head = m0 / rope.hd, j0 = m0 % rope.hd;            // j0 = 8c: the pair's lower dimension starts here
-      for (int idx = tid; idx < 8 * 8 * NT; idx += WS_WARPS * 32) {
-        const int i = idx % 8, tok = idx / 8;                        // consecutive threads -> consecutive dimensions of one token
-        if (tok >= M) continue;
+      const int i = tid % 8, tok = tid / 8;                          // consecutive threads -> consecutive dimensions of one token; at most one output a thread
+      if (tid < AHEAD_N && tok < M) {
         float lo = 0.f, hi = 0.f;
 #pragma unroll
         for (int w = 0; w < WS_WARPS; ++w) { lo += red[w][i][tok]; hi += red[w][i + 8][tok]; }
@@ -291,23 +337,22 @@ linear_ws_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __res
           lo *= row_scale[tok];
           hi *= row_scale[tok];
         }
-        if (bias) { lo += bias[m0 + i]; hi += bias[m0 + half + i]; }
+        if (bias) {
+          lo += BIAS_AHEAD ? ahead[BIAS_AHEAD ? 2 : 0][tid] : bias[m0 + i];
+          hi += BIAS_AHEAD ? ahead[BIAS_AHEAD ? 3 : 0][tid] : bias[m0 + half + i];
+        }
         __nv_bfloat16* dst;
         if (head < rope.nq) {
           dst = rope.q_out + ((size_t)tok * rope.nq + head) * rope.hd;
         } else {
-          int slot = rope.slot_mapping ? rope.slot_mapping[tok] : -1;
-          if (slot < 0 || slot / rope.page_size >= rope.num_pages) continue;     // not written (padding row, borrowed cache)
+          if (ahead_slot < 0 || ahead_slot / rope.page_size >= rope.num_pages) return;     // not written (padding row, borrowed cache)
           const bool is_k = head < rope.nq + rope.nkv;
           const int kvh = is_k ? head - rope.nq : head - rope.nq - rope.nkv;
           dst = (is_k ? rope.k_cache : rope.v_cache) +
-                (((size_t)(slot / rope.page_size) * rope.nkv + kvh) * rope.page_size + slot % rope.page_size) * rope.hd;
+                (((size_t)(ahead_slot / rope.page_size) * rope.nkv + kvh) * rope.page_size + ahead_slot % rope.page_size) * rope.hd;
         }
         if (rope.table != nullptr && head < rope.nq + rope.nkv) {
-          int pos = rope.positions[tok];
-          pos = pos < 0 ? 0 : (pos >= rope.max_pos ? rope.max_pos - 1 : pos);
-          const float* cs = rope.table + (size_t)pos * rope.hd;        // cos[half] then sin[half]
-          const float c = cs[j0 + i], sn = cs[half + j0 + i];
+          const float c = ahead[0][tid], sn = ahead[1][tid];
           const float a = lo * c - hi * sn, b = hi * c + lo * sn;
           lo = a;
           hi = b;
@@ -364,12 +409,12 @@ linear_ws_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __res
         for (int w = 0; w < KW; ++w) v += red[rg * KW + w][row][tok];
       }
       if constexpr (SCALED) v *= row_scale[tok];
-      if (bias) v += bias[n];
+      if (bias) v += EPI == WS_EPI_RESID && AHEAD ? ahead[AHEAD ? 1 : 0][AHEAD ? idx : 0] : bias[n];
       if constexpr (EPI == WS_EPI_RESID) {
-        const float r = residual[(size_t)tok * N + n] + v;
+        const float r = (AHEAD ? ahead[AHEAD ? 2 : 0][AHEAD ? idx : 0] : residual[(size_t)tok * N + n]) + v;
         residual[(size_t)tok * N + n] = r;
         if (norm.xg_out != nullptr) {
-          norm.xg_out[(size_t)tok * N + n] = __float2bfloat16_rn(r * norm.gain[n]);
+          norm.xg_out[(size_t)tok * N + n] = __float2bfloat16_rn(r * (AHEAD ? ahead[0][AHEAD ? idx : 0] : norm.gain[n]));
           squares[o] = fmaf(r, r, squares[o]);
         }
       } else {
