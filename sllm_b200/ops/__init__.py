@@ -1674,6 +1674,12 @@ def _ws_rows32_ok(M: int, N: int, K: int) -> bool:
     return ctas >= num_sms() or places >= 1.4 * num_sms() or K <= WS_ROWS32_SHORT_K
 
 
+def _ws_rope32_ok(N: int, K: int) -> bool:
+    """Whether the rotary epilogue is worth it for 17 to 32 tokens on a small matrix, which gives its CTAs no slices to share: where K is so short that latency is all of it.  The product then
+    takes a norm still owed and writes the caches, so that a norm kernel and the rotary kernel fall away (32 requests at 0.5B sizes, us a layer: 3.4 + 2.2 + 1.7 in three kernels, 5.4 in one)."""
+    return K <= WS_ROWS32_SHORT_K and -(-N // 16) <= 2 * num_sms()
+
+
 def _ws_stack_pays(M: int, N: int, K: int) -> bool:
     """Whether a consumer that adds partial sums is better served by the k-split kernel although the warp-split one takes the product: 17 to 32 tokens and rows for one
     to one and a half CTAs an SM, beyond what clusters share.  (24 tokens, the product and the norm behind it, us: 2,560 x 2,560 10.0 accumulated, 8.0 from slices; 3,072 x 3,072 10.8 / 9.9;
@@ -1966,14 +1972,15 @@ def linear_silu_mul(x: torch.Tensor, w_gate_up: torch.Tensor, interleave: int, o
 _QKV_ROPE = os.environ.get("SLLM_QKV_ROPE_FUSED", "1") != "0"     # 0: the product, then the rotary kernel
 
 
-def qkv_rope_supports(x, w, table, rotary_dim, nq, nkv, hd, k_cache) -> bool:
+def qkv_rope_supports(x, w, table, rotary_dim, nq, nkv, hd, k_cache, owed: bool = False) -> bool:
     """Whether `linear_rope_kv_write` takes the product: bfloat16, few tokens, the whole head rotated
-    (or no rotation at all), a head size that is a multiple of 16."""
+    (or no rotation at all), a head size that is a multiple of 16.  ``owed``: its input has a norm still owed,
+    which the product would pay and no other kernel for 17 to 32 tokens does (`_ws_rope32_ok`)."""
     if not (_QKV_ROPE and x.is_cuda and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and k_cache.dtype == torch.bfloat16):
         return False
     rot = int(rotary_dim) if table is not None else 0
     M, K = x.shape
-    return M <= WS_MAX_ROWS and _ws_tokens_ok(M, w.shape[0], K) and bool(lib().sllm_linear_ws_rope_supports(int(M), int(w.shape[0]), int(K), int(nq), int(nkv),
+    return M <= WS_MAX_ROWS and (_ws_tokens_ok(M, w.shape[0], K) or (owed and _ws_rope32_ok(w.shape[0], K))) and bool(lib().sllm_linear_ws_rope_supports(int(M), int(w.shape[0]), int(K), int(nq), int(nkv),
                                                                           int(hd), rot))
 
 

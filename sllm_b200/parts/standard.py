@@ -205,7 +205,7 @@ class Attention(Mixer):
         rot = getattr(position, "rotary_dim", 0) if table is not None else 0
         slots = g.slot_mapping if write_cache else None
         owed = x if isinstance(x, OwedNorm) else None
-        fused = owed is not None and ops.qkv_rope_supports(owed.x, self.qkv.weight, table, rot, self.nq, self.nkv, self.hd, cache.k)
+        fused = owed is not None and ops.qkv_rope_supports(owed.x, self.qkv.weight, table, rot, self.nq, self.nkv, self.hd, cache.k, owed=True)
         if owed is not None and not fused and not ops.linear_scaled_supports(owed.x, self.qkv.weight):
             x, owed = owed.plain(), None
         if owed is not None and fused:
