@@ -63,6 +63,41 @@ __device__ __forceinline__ void ls_mma(float (&c)[4], unsigned a0, unsigned a1, 
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// acc[j][c]: c0,c1 = (row g, tokens 8j+2t, +1); c2,c3 = (row g+8, same tokens) of the 16 rows from n0
+template <int NT, int EPI, typename OUT>
+__device__ __forceinline__ void ls_finish(const float (&acc)[NT][4], int n0, int g, int t4, const float* __restrict__ bias, OUT* __restrict__ out, int M, int N) {
+  const int row_a = n0 + g, row_b = n0 + g + 8;
+  if constexpr (EPI == EPI_SILU || EPI == EPI_GELU) {
+    // rows g (gate i) and g+8 (up i) of this 16-row tile; the output column is (n0/16)*8 + g
+    const int col = (n0 >> 4) * 8 + g;
+    const int I = N >> 1;
+    if (row_b < N) {
+      const float bias_g = (EPI == EPI_GELU && bias) ? bias[row_a] : 0.f, bias_u = (EPI == EPI_GELU && bias) ? bias[row_b] : 0.f;
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int tok = 8 * j + 2 * t4 + c;
+          if (tok < M) {
+            const float gate = acc[j][c] + bias_g, up = acc[j][c + 2] + bias_u;
+            if constexpr (EPI == EPI_GELU)
+              out[(size_t)tok * I + col] = from_f32<OUT>(0.5f * gate * (1.0f + tanhf(0.7978845608028654f * (gate + 0.044715f * gate * gate * gate))) * up);
+            else
+              out[(size_t)tok * I + col] = from_f32<OUT>(gate * (1.0f / (1.0f + expf(-gate))) * up);
+          }
+        }
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int tok = 8 * j + 2 * t4 + (c & 1), row = (c & 2) ? row_b : row_a;
+        if (tok < M && row < N) out[(size_t)tok * N + row] = from_f32<OUT>(acc[j][c] + (bias ? bias[row] : 0.f));
+      }
+  }
+}
+
 // NT: 8-token tiles (M <= 8*NT).  OUT: float or __nv_bfloat16.  SCALED: the rows of the result are scaled
 // (LsScale; unsplit launches only).
 template <int NT, int EPI, typename OUT, bool SCALED>
@@ -115,14 +150,15 @@ linear_stream_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       const uint4 ra = a[2 * b], rb = a[2 * b + 1];         // rows g and g+8: 8 consecutive k each
+      uint4 xv[NT];
 #pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        const uint4 xv = *reinterpret_cast<const uint4*>(xb + (size_t)(8 * j + g) * LS_XSTRIDE + b * 32 + t4 * 8);
-        // first MMA: k slots (2t,2t+1) <- elements 0,1; slots (2t+8,2t+9) <- elements 2,3
-        ls_mma(acc[j], ra.x, rb.x, ra.y, rb.y, xv.x, xv.y);
-        // second MMA: elements 4,5 and 6,7
-        ls_mma(acc[j], ra.z, rb.z, ra.w, rb.w, xv.z, xv.w);
-      }
+      for (int j = 0; j < NT; ++j) xv[j] = *reinterpret_cast<const uint4*>(xb + (size_t)(8 * j + g) * LS_XSTRIDE + b * 32 + t4 * 8);
+      // first MMA: k slots (2t,2t+1) <- elements 0,1; slots (2t+8,2t+9) <- elements 2,3; second: elements 4,5 and 6,7.  A tile's second depends on its first, so the tiles'
+      // first ones come before their second ones.
+#pragma unroll
+      for (int j = 0; j < NT; ++j) ls_mma(acc[j], ra.x, rb.x, ra.y, rb.y, xv[j].x, xv[j].y);
+#pragma unroll
+      for (int j = 0; j < NT; ++j) ls_mma(acc[j], ra.z, rb.z, ra.w, rb.w, xv[j].z, xv[j].w);
     }
   };
 
@@ -182,9 +218,9 @@ linear_stream_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
       for (int c = 0; c < 4; ++c) acc[j][c] *= row_scale[8 * j + 2 * t4 + (c & 1)];
   }
 
-  // ---- epilogue: acc[j][c]: c0,c1 = (row g, tokens 8j+2t, +1); c2,c3 = (row g+8, same tokens) ----
-  const int row_a = n0 + g, row_b = n0 + g + 8;
+  // ---- epilogue ----
   if (gridDim.y > 1) {
+    const int row_a = n0 + g, row_b = n0 + g + 8;
 #pragma unroll
     for (int j = 0; j < NT; ++j)
 #pragma unroll
@@ -195,40 +231,129 @@ linear_stream_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
       }
     return;
   }
-  if constexpr (EPI == EPI_SILU || EPI == EPI_GELU) {
-    // rows g (gate i) and g+8 (up i) of this 16-row tile; the output column is (n0/16)*8 + g
-    const int col = (n0 >> 4) * 8 + g;
-    const int I = N >> 1;
-    if (row_b < N) {
-      const float bias_g = (EPI == EPI_GELU && bias) ? bias[row_a] : 0.f, bias_u = (EPI == EPI_GELU && bias) ? bias[row_b] : 0.f;
+  ls_finish<NT, EPI, OUT>(acc, n0, g, t4, bias, out, M, N);
+}
+
+// The same product with all of the activations in shared memory (a short K): no barrier in the stream, so it is bound by the weights in flight alone.  Above, a chunk of 128
+// columns waits for its activations from L2 between two barriers, which for 32 tokens and K = 896 was seven round trips of a kernel whose weights take 2.7 us.
+// A CTA of four warps takes 64 rows, so that 9,728 rows are 152 CTAs for 148 SMs and a warp's products a quarter of a scheduler's; a warp keeps LR_DEPTH chunks (16 KB) in flight, the
+// first of them before the wait; the activations lie in the order the lanes read them, 16 bytes each.  The k order of every sum is that of the form above, so are the bits.
+// (In a graph of such products, us, this / the form above: one token, output head 151,936 x 896 42.5 / 48.0; 8 tokens, gate|up with the activation 4,864 x 896 4.5 / 7.6, 8,192 x 1,024 6.1 / 9.0,
+// with a norm owed 6.7 / 9.0; 16 tokens 5.2 / 7.9, 7.1 / 9.3, 7.7 / 9.6; 12,288 x 1,536 11.2 / 14.1; 32 tokens with a norm owed 9,728 x 896 12.0 / 13.6, 4,864 x 896 8.5 / 12.2.)
+constexpr int LR_WARPS = 4, LR_DEPTH = 4, LR_X_MAX = 100 * 1024;
+
+template <int NT, int EPI, typename OUT, bool SCALED>
+__global__ void __launch_bounds__(LR_WARPS * 32)
+linear_resident_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ W, const float* __restrict__ bias, OUT* __restrict__ out,
+                       int M, int N, int K, const LsScale scale) {
+  extern __shared__ __align__(16) unsigned char ls_smem[];               // [K / 32][NT][32 lanes] 16 bytes
+  __shared__ float row_scale[8 * NT];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t4 = lane & 3;
+  const int n0 = (blockIdx.x * LR_WARPS + warp) * 16;
+  const int chunks = K / LS_KC;
+  const int r0 = min(n0 + g, N - 1), r1 = min(n0 + g + 8, N - 1);      // rows past N are clamped for the loads and skipped at the store
+  const __nv_bfloat16* w0 = W + (size_t)r0 * K + t4 * 8;
+  const __nv_bfloat16* w1 = W + (size_t)r1 * K + t4 * 8;
+  uint4 w[LR_DEPTH][8];
+  auto load_w = [&](uint4 (&a)[8], int chunk) {
+    if (chunk >= chunks) return;
 #pragma unroll
-      for (int j = 0; j < NT; ++j)
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const int tok = 8 * j + 2 * t4 + c;
-          if (tok < M) {
-            const float gate = acc[j][c] + bias_g, up = acc[j][c + 2] + bias_u;
-            if constexpr (EPI == EPI_GELU)
-              out[(size_t)tok * I + col] = from_f32<OUT>(0.5f * gate * (1.0f + tanhf(0.7978845608028654f * (gate + 0.044715f * gate * gate * gate))) * up);
-            else
-              out[(size_t)tok * I + col] = from_f32<OUT>(gate * (1.0f / (1.0f + expf(-gate))) * up);
-          }
-        }
+    for (int b = 0; b < 4; ++b) {
+      a[2 * b] = ldg_stream(w0 + (size_t)chunk * LS_KC + b * 32);
+      a[2 * b + 1] = ldg_stream(w1 + (size_t)chunk * LS_KC + b * 32);
     }
-  } else {
+  };
+#pragma unroll
+  for (int d = 0; d < LR_DEPTH; ++d) load_w(w[d], d);
+  pdl_wait();
+  for (int e = tid; e < K / 32 * NT * 32; e += LR_WARPS * 32) {
+    const int l = e & 31, j = (e >> 5) % NT, b = (e >> 5) / NT, row = 8 * j + (l >> 2);
+    if (row < M) ls_cp_async_16(ls_smem + (size_t)e * 16, x + (size_t)row * K + b * 32 + (l & 3) * 8, true);       // (tokens past M: what lies there, in columns that nobody stores)
+  }
+  asm volatile("cp.async.commit_group;\n" ::);
+  if constexpr (SCALED) {              // eight lanes a token, four partial sums a load: every load of a thread is under way before the first is added
+    constexpr int LANES = LR_WARPS * 32 / (8 * NT) < 8 ? LR_WARPS * 32 / (8 * NT) : 8;
+    const int stride = (scale.parts + 3) & ~3, tok = tid / LANES, q = tid % LANES;
+    float sum = 0.f;
+    if (tok < M) {
+      const float* s = scale.ssq + (size_t)tok * stride;
+#pragma unroll 4
+      for (int p = q * 4; p < scale.parts; p += LANES * 4) {
+        const float4 v = __ldcg(reinterpret_cast<const float4*>(s + p));
+        sum += v.x + (p + 1 < scale.parts ? v.y : 0.f) + (p + 2 < scale.parts ? v.z : 0.f) + (p + 3 < scale.parts ? v.w : 0.f);
+      }
+    }
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (q == 0 && tok < 8 * NT) row_scale[tok] = rsqrtf(sum * scale.inv_width + scale.eps);
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+  float acc[NT][4];
+#pragma unroll
+  for (int j = 0; j < NT; ++j)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[j][c] = 0.f;
+  for (int c0 = 0; c0 < chunks; c0 += LR_DEPTH) {
+#pragma unroll
+    for (int d = 0; d < LR_DEPTH; ++d) {
+      const int c = c0 + d;
+      if (c >= chunks) break;
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const uint4 ra = w[d][2 * b], rb = w[d][2 * b + 1];
+        uint4 xv[NT];
+#pragma unroll
+        for (int j = 0; j < NT; ++j) xv[j] = *reinterpret_cast<const uint4*>(ls_smem + ((size_t)((c * 4 + b) * NT + j) * 32 + lane) * 16);
+        // (a token tile's two products depend on one another: the tiles' first ones, then their second ones)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) ls_mma(acc[j], ra.x, rb.x, ra.y, rb.y, xv[j].x, xv[j].y);
+#pragma unroll
+        for (int j = 0; j < NT; ++j) ls_mma(acc[j], ra.z, rb.z, ra.w, rb.w, xv[j].z, xv[j].w);
+      }
+      load_w(w[d], c + LR_DEPTH);
+    }
+  }
+  pdl_launch_dependents();
+  if constexpr (SCALED) {
 #pragma unroll
     for (int j = 0; j < NT; ++j)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int tok = 8 * j + 2 * t4 + (c & 1), row = (c & 2) ? row_b : row_a;
-        if (tok < M && row < N) out[(size_t)tok * N + row] = from_f32<OUT>(acc[j][c] + (bias ? bias[row] : 0.f));
-      }
+      for (int c = 0; c < 4; ++c) acc[j][c] *= row_scale[8 * j + 2 * t4 + (c & 1)];
   }
+  ls_finish<NT, EPI, OUT>(acc, n0, g, t4, bias, out, M, N);
+}
+
+// Where the activations fit; with four token tiles the products of a warp (mma.sync, some 30 cycles each) are what takes the time, so there only where the form above is
+// worse off still: a norm owed, whose partial sums it adds token after token behind the stream, or too few rows for its CTAs.  (17 tokens, us, this / the form above: 9,728 x 896
+// with the activation 10.4 / 9.6, with a norm owed 11.0 / 13.4; 4,096 x 1,024 7.2 / 10.3, 6,144 x 1,536 10.3 / 15.3, 8,192 x 1,024 9.8 / 10.6, 32 tokens 11.0 / 10.6.)
+constexpr int LR_MANY_TOKENS_ROWS = 7168;
+static bool ls_resident(int M, int N, int K, int splits, bool scaled) {
+  const int nt = M <= 8 ? 1 : (M <= 16 ? 2 : 4);
+  return splits == 1 && M <= 32 && K * 16 * nt <= LR_X_MAX && (nt < 4 || scaled || N <= LR_MANY_TOKENS_ROWS);
+}
+
+template <int NT, int EPI, typename OUT, bool SCALED>
+static int launch_resident(const __nv_bfloat16* x, const __nv_bfloat16* W, const float* bias, void* out, int M, int N, int K, cudaStream_t stream, const LsScale& scale) {
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(linear_resident_kernel<NT, EPI, OUT, SCALED>, cudaFuncAttributeMaxDynamicSharedMemorySize, LR_X_MAX) != cudaSuccess) {
+      set_error("linear_stream: cannot raise the shared memory limit");
+      return SLLM_ERR_LAUNCH;
+    }
+    configured = true;
+  }
+  launch_kernel(linear_resident_kernel<NT, EPI, OUT, SCALED>, (N + LR_WARPS * 16 - 1) / (LR_WARPS * 16), LR_WARPS * 32, (size_t)K * 16 * NT, stream, x, W, bias, (OUT*)out, M, N, K, scale);
+  return launch_status("linear_stream");
 }
 
 template <int NT, int EPI, typename OUT, bool SCALED = false>
 static int launch_ls(const __nv_bfloat16* x, const __nv_bfloat16* W, const float* bias, void* out, float* partial,
                      int M, int N, int K, int splits, cudaStream_t stream, const LsScale& scale = LsScale{}) {
+  if constexpr (NT <= 4) {
+    if (ls_resident(M, N, K, splits, SCALED)) return launch_resident<NT, EPI, OUT, SCALED>(x, W, bias, out, M, N, K, stream, scale);
+  }
   constexpr size_t smem = sizeof(__nv_bfloat16) * 2 * 8 * NT * LS_XSTRIDE + (SCALED ? sizeof(float) * 8 * NT * LS_SSQ_MAX : 0);
   static bool configured = false;
   if (!configured && smem + 1024 > 48 * 1024) {      // (the kernel has a little static shared memory too)

@@ -203,11 +203,11 @@ linear_ws_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __res
 #pragma unroll
     for (int d = 0; d < WS_DEPTH; ++d) {
       if (kb + d * KW < k_blocks) {
+        // (a token tile's two products depend on one another: the tiles' first ones, then their second ones)
 #pragma unroll
-        for (int j = 0; j < NT; ++j) {
-          ws_mma(acc[j], wa[d].x, wb[d].x, wa[d].y, wb[d].y, xv[d][j].x, xv[d][j].y);
-          ws_mma(acc[j], wa[d].z, wb[d].z, wa[d].w, wb[d].w, xv[d][j].z, xv[d][j].w);
-        }
+        for (int j = 0; j < NT; ++j) ws_mma(acc[j], wa[d].x, wb[d].x, wa[d].y, wb[d].y, xv[d][j].x, xv[d][j].y);
+#pragma unroll
+        for (int j = 0; j < NT; ++j) ws_mma(acc[j], wa[d].z, wb[d].z, wa[d].w, wb[d].w, xv[d][j].z, xv[d][j].w);
       }
     }
   };

@@ -1569,6 +1569,17 @@ def linear_tc_supports(M: int, N: int, K: int) -> bool:
     return linear_tc_takes(M, N, K) and M >= _tc_from_rows(N, K)
 
 
+LINEAR_TC_UNSPLIT = 12 << 20
+
+
+@functools.lru_cache(maxsize=4096)
+def _tc_unsplit_pays(M: int, N: int, K: int) -> bool:
+    """Whether a product of 17 to 32 tokens that cannot leave partial sums (or applies gate|up's activation) is better off here than with the streaming kernel although its matrix is
+    under `LINEAR_TC_LARGE`: there mma.sync's rate bounds four token tiles.  (32 tokens, us, streaming / this one: store 9,728 x 896 9.4 / 9.0, 12,288 x 1,536 16.3 / 12.7, 10,240 x 2,048
+    21.0 / 15.0; gate|up 17,920 x 1,536 20.2 / 16.0, with a norm owed 19.9 and here a norm kernel of 1.4 before it; 11,264 x 2,048 24.5 / 17.6 and 26.5.)"""
+    return STREAM_MAX_ROWS >= M >= LINEAR_TC_LARGE_FROM_ROWS and N * K >= LINEAR_TC_UNSPLIT and linear_tc_takes(M, N, K)
+
+
 @functools.lru_cache(maxsize=4096)
 def _tc_splits(N: int, K: int) -> int:
     """Slices of K so that (tiles of 128 rows) x slices comes to about one unit per SM, each slice
@@ -1848,6 +1859,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias, out_dtype: torch.dtype, allow
         return linear_ws(x, w, bias, out_dtype)
     if stream_supports(M, N, K):
         splits = _stream_splits(N, K) if (allow_partials and out_dtype == torch.float32) else 1
+        if splits == 1 and _tc_unsplit_pays(M, N, K):
+            return linear_tc(x, w, bias, out_dtype)
         return linear_stream(x, w, bias, out_dtype, splits=splits)
     if allow_partials and out_dtype == torch.float32 and M <= LINEAR_TC_SPLIT_MAX_ROWS and K >= LINEAR_TC_SPLIT_MIN_K \
             and linear_tc_supports(M, N, K):
@@ -1926,7 +1939,7 @@ def silu_scaled_supports(x, w_gate_up, interleave: int, out_dtype) -> bool:
     N = w_gate_up.shape[0]
     if not (x.is_cuda and x.dtype == torch.bfloat16 and out_dtype == torch.bfloat16 and interleave == 8 and N % 16 == 0):
         return False
-    return (M <= 32 and stream_supports(M, N, K)) or (M > TCGEN05_MIN_ROWS and _PAIR_GEMM != "off" and pair_supports(M, N, K))
+    return (M <= 32 and stream_supports(M, N, K) and not _tc_unsplit_pays(M, N, K)) or (M > TCGEN05_MIN_ROWS and _PAIR_GEMM != "off" and pair_supports(M, N, K))
 
 
 def linear_silu_mul(x: torch.Tensor, w_gate_up: torch.Tensor, interleave: int, out_dtype: torch.dtype,
@@ -1951,8 +1964,10 @@ def linear_silu_mul(x: torch.Tensor, w_gate_up: torch.Tensor, interleave: int, o
         N = w_gate_up.shape[0]
         if ws_gated_supports(M, N, K):
             return linear_ws_gated(x, w_gate_up, None, "silu")
-        if stream_supports(M, N, K):
+        if stream_supports(M, N, K) and not (N % 16 == 0 and _tc_unsplit_pays(M, N, K)):
             return linear_stream(x, w_gate_up, None, out_dtype, silu=True)
+        if N % 16 == 0 and _tc_unsplit_pays(M, N, K):
+            return linear_tc(x, w_gate_up, None, out_dtype, silu=True)
         if PAIR_SILU_FROM_ROWS <= M <= TCGEN05_MIN_ROWS and N % 16 == 0 and _PAIR_GEMM != "off" and pair_supports(M, N, K):
             # 64..128 tokens: still bound by reading W once, and the pair kernel's narrow tiles (two accumulators, the
             # epilogue under the next tile) stream it faster than `linear_tc`, whose accumulator is 128 columns wide there

@@ -143,3 +143,32 @@ def test_the_next_norms_input_from_more_tokens(M, N, K):
     assert bool(((added - (stream + y)).abs() <= bound + 2.0 ** -23 * (stream.abs() + y.abs())).all())
     assert torch.equal(xg, (added * gain).bfloat16()) and owed.width == N and owed.eps == 1e-6 and owed.parts <= ops.MAX_SCALE_PARTS_ROWS32
     torch.testing.assert_close(owed.ssq[:, :owed.parts].double().sum(1), added.double().pow(2).sum(1), rtol=N * 2.0 ** -24, atol=0)
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32])
+@pytest.mark.parametrize("N,K", [(16, 128), (1000, 896), (4864, 896), (7168, 1536), (7184, 1536), (9728, 896), (200, 3200), (64, 6400), (8192, 1664)])
+def test_streams_with_resident_activations(M, N, K):
+    """The streaming kernel where all activations fit its shared memory and just beyond: plain, with the activation, with a norm owed on the input (tables of one, some and
+    many partial sums, the rest of them never read), rows and tokens that leave remainders."""
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    g, x, w, b, y, bound = _product(dev, M, N, K)
+    assert bool(((ops.linear_stream(x, w, b, torch.float32) - y).abs() <= bound).all())
+    if N % 16:
+        return
+    for parts in (0, 1, 57, 592):
+        scale, plain, off = 1.0, x.double() @ w.double().T, (K + 1) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+        if parts == 0:
+            got = ops.linear_stream(x, w, None, torch.bfloat16, silu=True)
+        else:
+            ssq = torch.full((M, (parts + 3) & ~3), float("nan"), device=dev)
+            ssq[:, :parts] = torch.rand(M, parts, device=dev, generator=g) * 4 * K / parts
+            scale = (ssq[:, :parts].double().sum(1, keepdim=True) / K + 1e-5).rsqrt()
+            got = torch.empty(M, N // 2, dtype=torch.bfloat16, device=dev)
+            ops.call("sllm_linear_stream_silu_scaled", x.data_ptr(), w.data_ptr(), got.data_ptr(), M, N, K, *ops.RowScale(ssq, parts, 1e-5, K).args(), ops._stream())
+        z, zo = plain * scale, off * scale + 2.0 ** -20 * (plain * scale).abs()
+        gate, up = z.reshape(M, N // 16, 2, 8).unbind(2)
+        gate_off, up_off = zo.reshape(M, N // 16, 2, 8).unbind(2)
+        want = torch.nn.functional.silu(gate) * up
+        lim = 2.0 ** -8 * want.abs() + 1.2 * (gate_off * up.abs() + up_off * gate.abs()) + 1e-5 * gate.abs() * up.abs() + 1e-30
+        assert bool(((got.reshape(M, N // 16, 8) - want).abs() <= lim).all())
