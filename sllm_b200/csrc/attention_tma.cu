@@ -17,8 +17,13 @@
 // uninitialised value.  Every mbarrier wait is bounded; a wait that runs out records a code in the
 // status word and the CTA leaves through the common exit.
 //
+// Up to TA_CLUSTER ranges of a context are the CTAs of a cluster: each leaves its partial result in its own shared memory, and the cluster's CTAs share the rows'
+// columns and add the ranges over distributed shared memory, so that there is neither scratch nor a second kernel (that one took 3.5 to 4.2 us of a layer, of which
+// its launch and the trip of the partial results through memory were most).  More ranges go through scratch and attention_tma_combine_kernel.
+//
 // Takes head sizes 64 and 128 and page sizes that divide 64; the host falls back to
 // attention_mma.cu otherwise.
+#include <cooperative_groups.h>
 #include <math.h>
 #include <stdio.h>
 
@@ -33,6 +38,7 @@ namespace sllm {
 constexpr int TA_BN = 64;          // keys per tile
 constexpr int TA_STAGES = 3;
 constexpr int TA_THREADS = 160;    // four compute warps and the producer warp
+constexpr int TA_CLUSTER = 8;      // ranges of a context that a cluster merges
 constexpr int TA_BT_CACHE = 2048;  // block-table entries the producer keeps in shared memory
 
 struct AttnTmaParams {
@@ -47,6 +53,7 @@ struct AttnTmaParams {
   const int* tile_row0;          // [tiles]
   int* status;
   int max_pages, page_size, nq, nkv, window, num_splits, total_tokens;
+  int cluster;                   // the ranges are a cluster's CTAs
   int block;     // > 0: a query sees only keys of its own block of this many positions (counted from 0)
   int page_runs;                 // the run maps are valid: a tile of pages with consecutive ids is fetched as one box
   float scale_log2;
@@ -87,6 +94,11 @@ attention_tma_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   volatile int* failed = reinterpret_cast<volatile int*>(empty + TA_STAGES);
   int* bt_s = const_cast<int*>(reinterpret_cast<volatile int*>(failed + 2));      // [TA_BT_CACHE]
 
+  // a range's own result, for the cluster's merge: behind the warps' merge buffer, over the stages
+  float* own_o = reinterpret_cast<float*>(kv_s) + 4 * 16 * HD + 128;             // [16][HD]
+  float* own_lse = own_o + 16 * HD;                                              // [16]
+  static_assert(sizeof(float) * (5 * 16 * HD + 144) <= TA_STAGES * 2 * KV_BYTES, "a range's result");
+
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t4 = lane & 3;
   if (tid == 0) {
@@ -121,8 +133,11 @@ attention_tma_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   int key_lo = 0;
   if (p.window > 0) key_lo = max(0, pos0 + row0 / G - p.window + 1);
   if (p.block > 0) key_lo = max(key_lo, (pos0 + row0 / G) / p.block * p.block);
+  // (a context so short that one range holds it needs no merge: every CTA of the cluster finds the same)
+  const int chunk = ((ctx + p.num_splits - 1) / p.num_splits + TA_BN - 1) / TA_BN * TA_BN;
+  const bool merge = p.cluster && chunk < ctx;
+  const bool alone = p.num_splits == 1 || (p.cluster && !merge);
   if (p.num_splits > 1) {
-    const int chunk = ((ctx + p.num_splits - 1) / p.num_splits + TA_BN - 1) / TA_BN * TA_BN;
     key_lo = max(key_lo, split * chunk);
     key_hi = min(key_hi, (split + 1) * chunk);
   }
@@ -417,19 +432,24 @@ attention_tma_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __g
           const float4 v = *reinterpret_cast<const float4*>(mo + (w * 16 + r) * HD + d4);
           acc.x += v.x * f[w]; acc.y += v.y * f[w]; acc.z += v.z * f[w]; acc.w += v.w * f[w];
         }
-        if (p.sink != nullptr && p.num_splits == 1) lt += exp2f(p.sink[kvh * G + row % G] * 1.4426950408889634f - mt);
+        if (p.sink != nullptr && alone) lt += exp2f(p.sink[kvh * G + row % G] * 1.4426950408889634f - mt);
         float inv = lt > 0.f ? 1.f / lt : 0.f;
-        if (p.gate != nullptr && p.num_splits == 1) inv *= sigmoid_f32(p.gate[(size_t)(q0 + row / G) * p.gate_ld + kvh * G + row % G]);
+        if (p.gate != nullptr && alone) inv *= sigmoid_f32(p.gate[(size_t)(q0 + row / G) * p.gate_ld + kvh * G + row % G]);
         const size_t orow = (size_t)(q0 + row / G) * p.nq + kvh * G + row % G;
-        if (p.num_splits > 1) {
+        if (merge) {
+          *reinterpret_cast<float4*>(own_o + r * HD + d4) = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
+          if (d4 == 0) own_lse[r] = lt > 0.f ? mt + log2f(lt) : -INFINITY;
+        } else if (!alone) {
           float* po = p.part_o + ((size_t)split * p.total_tokens * p.nq + orow) * HD + d4;
           *reinterpret_cast<float4*>(po) = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
           if (d4 == 0) p.part_lse[(size_t)split * p.total_tokens * p.nq + orow] = lt > 0.f ? mt + log2f(lt) : -INFINITY;
-        } else {
+        } else if (!p.cluster || split == 0) {
           *reinterpret_cast<uint2*>(p.out + orow * HD + d4) =
               make_uint2(pack_bf16(acc.x * inv, acc.y * inv), pack_bf16(acc.z * inv, acc.w * inv));
         }
       }
+    } else if (merge && tid < 16) {
+      own_lse[tid] = -INFINITY;
     }
   }
   // common exit: if something gave up, let the copies that were issued land before the shared
@@ -439,6 +459,37 @@ attention_tma_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   if (*failed && tid == 0) {
     for (int s = 0; s < TA_STAGES; ++s) mbar_wait(&full[s], 0, TMA_DRAIN_NS);
   }
+  if (!merge) return;
+  // ---------------- the cluster's merge: out[row] = sum_s w_s o_s[row], w_s = 2^(lse_s - max) / sum ----------------
+  cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  cl.sync();                                              // every range's result is in its CTA's shared memory
+  for (int idx = split * TA_THREADS + tid; idx < 16 * (HD / 4); idx += p.num_splits * TA_THREADS) {
+    const int r = idx / (HD / 4), d4 = (idx % (HD / 4)) * 4, row = row0 + r;
+    if (row >= rows_total) continue;
+    float lse[TA_CLUSTER], mt = -INFINITY, tot = 0.f;
+    float4 o[TA_CLUSTER];
+#pragma unroll
+    for (int s = 0; s < TA_CLUSTER; ++s) {
+      lse[s] = s < p.num_splits ? *cl.map_shared_rank(own_lse + r, s) : -INFINITY;
+      if (s < p.num_splits) o[s] = *reinterpret_cast<const float4*>(cl.map_shared_rank(own_o + r * HD + d4, s));
+    }
+#pragma unroll
+    for (int s = 0; s < TA_CLUSTER; ++s) mt = fmaxf(mt, lse[s]);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int s = 0; s < TA_CLUSTER; ++s) {
+      if (s >= p.num_splits || lse[s] == -INFINITY) continue;      // a range without a key of this row weighs nothing
+      const float w = exp2f(lse[s] - mt);
+      tot += w;
+      acc.x = fmaf(w, o[s].x, acc.x); acc.y = fmaf(w, o[s].y, acc.y); acc.z = fmaf(w, o[s].z, acc.z); acc.w = fmaf(w, o[s].w, acc.w);
+    }
+    if (p.sink != nullptr) tot += exp2f(p.sink[kvh * G + row % G] * 1.4426950408889634f - mt);
+    float inv = tot > 0.f ? 1.f / tot : 0.f;
+    if (p.gate != nullptr) inv *= sigmoid_f32(p.gate[(size_t)(q0 + row / G) * p.gate_ld + kvh * G + row % G]);
+    *reinterpret_cast<uint2*>(p.out + ((size_t)(q0 + row / G) * p.nq + kvh * G + row % G) * HD + d4) =
+        make_uint2(pack_bf16(acc.x * inv, acc.y * inv), pack_bf16(acc.z * inv, acc.w * inv));
+  }
+  cl.sync();                                              // nobody leaves while its shared memory is read
 }
 
 constexpr int TA_MAX_SPLITS = 128;     // the merge keeps one weight a range in shared memory
@@ -573,6 +624,23 @@ static int launch_ta(const CUtensorMap& mk, const CUtensorMap& mv, const CUtenso
     configured = true;
   }
   dim3 grid((unsigned)tiles * p.nkv, 1, p.num_splits);
+  if (p.cluster) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(TA_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = p.num_splits;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, attention_tma_decode_kernel<HD, CAP, REL>, mk, mv, rk, rv, p);
+    return launch_status("attention_tma");
+  }
   launch_kernel(attention_tma_decode_kernel<HD, CAP, REL>, grid, TA_THREADS, smem, stream, mk, mv, rk, rv, p);
   int rc = launch_status("attention_tma");
   if (rc != SLLM_OK) return rc;
@@ -605,6 +673,17 @@ SLLM_EXPORT int sllm_attention_tma_ctas_per_sm(int hd) {
   return by_smem < by_threads ? (by_smem < 1 ? 1 : by_smem) : by_threads;
 }
 
+// Whether so many ranges are merged without scratch and without a second kernel: as clusters, which fit all at once only up to some 85 % of the places (more than two CTAs of a
+// cluster leave places of a GPC idle; beyond that they take a second wave).  (Pairs of (tile, KV head) x ranges of two key tiles, one KV head of 128, us, as clusters / through scratch:
+// 44 x 4 9.0 / 10.1, 62 x 4 9.3 / 10.5, 70 x 4 9.6 / 10.7, 74 x 4 16.5 / 11.0; 31 x 8 9.8 / 10.6, 35 x 8 16.9 / 10.9; 148 x 2 9.6 / 11.1; heads of 64: 66 x 4 7.7 / 9.2, 94 x 4 8.0 / 9.6,
+// 105 x 4 13.7 / 9.6.)
+static bool ta_clustered(int tiles, int nkv, int num_splits, int hd) {
+  if (num_splits < 2 || num_splits > TA_CLUSTER) return false;
+  const long long places = (long long)sllm_attention_tma_ctas_per_sm(hd) * num_sms(), ctas = (long long)tiles * nkv * num_splits;
+  return num_splits == 2 ? ctas <= places : ctas * 100 <= places * 85;
+}
+SLLM_EXPORT int sllm_attention_tma_clustered(int tiles, int nkv, int num_splits, int hd) { return ta_clustered(tiles, nkv, num_splits, hd) ? 1 : 0; }
+
 // The decode form only: every tile holds at most 16 (token, head-in-group) rows.  num_pages: pages in the
 // cache tensors [num_pages, nkv, page_size, hd].  status: one int of device memory, zero before the launch.
 SLLM_EXPORT int sllm_attention_tma_decode(const void* q, const void* k_cache, const void* v_cache, long long num_pages,
@@ -619,7 +698,8 @@ SLLM_EXPORT int sllm_attention_tma_decode(const void* q, const void* k_cache, co
   SLLM_REQUIRE(sllm_attention_tma_supports(hd, page_size), "attention_tma: head_dim=%d page_size=%d not taken", hd, page_size);
   SLLM_REQUIRE(max_pages > 0 && tiles >= 0 && total_tokens >= 0 && num_pages > 0, "attention_tma: bad sizes");
   SLLM_REQUIRE(num_splits >= 1 && num_splits <= TA_MAX_SPLITS && nkv <= 65535, "attention_tma: bad grid nkv=%d splits=%d", nkv, num_splits);
-  SLLM_REQUIRE(num_splits == 1 || (part_o && part_lse), "attention_tma: split-KV needs scratch");
+  const bool cluster = ta_clustered(tiles, nkv, num_splits, hd);
+  SLLM_REQUIRE(num_splits == 1 || cluster || (part_o && part_lse), "attention_tma: split-KV needs scratch");
   SLLM_REQUIRE(status != nullptr, "attention_tma: a status word is required");
   SLLM_REQUIRE(((uintptr_t)k_cache & 15) == 0 && ((uintptr_t)v_cache & 15) == 0, "attention_tma: the cache must be 16-byte aligned");
   if (tiles == 0) return SLLM_OK;
@@ -636,6 +716,7 @@ SLLM_EXPORT int sllm_attention_tma_decode(const void* q, const void* k_cache, co
                     cache_map(v_cache, rows, page_size, hd, &rv, nkv);
   AttnTmaParams p;
   p.page_runs = runs ? 1 : 0;
+  p.cluster = cluster ? 1 : 0;
   p.q = (const __nv_bfloat16*)q; p.out = (__nv_bfloat16*)out; p.part_o = part_o; p.part_lse = part_lse;
   p.block_tables = block_tables; p.q_start = q_start; p.ctx_len = ctx_len; p.tile_seq = tile_seq; p.tile_row0 = tile_row0;
   p.status = status; p.max_pages = max_pages; p.page_size = page_size; p.nq = nq; p.nkv = nkv; p.window = window; p.block = block;

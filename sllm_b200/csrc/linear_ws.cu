@@ -479,6 +479,26 @@ static bool ws_side_by_side(int M, int N, int K) {
   return ctas <= places || ctas * 100 >= (ctas + places - 1) / places * places * 84;
 }
 
+// The kernel, told once what shared memory it wants beside L1: what two CTAs need, at least WS_CARVEOUT per cent.  The loads in flight lie in L1, and an SM keeps the split that the kernel
+// before had as long as the next one's shared memory fits: behind the decode attention, which takes all of it, this kernel ran with 28 KB of L1 (at 7B sizes gate|up 65 us in place of 45,
+// down 67 in place of 25, as soon as no small kernel stood between them).  (8 requests at 7B sizes, 8 of 240 keys at a width of 2,048, 16 of 300, one of 700 at 4,096, ms: no preference 195, 20.0, 29.4, 17.2;
+// 0 per cent beyond what fits 131.6, 19.8, 29.4, 16.8; 30 131.6, 19.4, 28.6, 16.6; 60 138.9, 21.4, 28.9, 18.4.)
+constexpr int WS_CARVEOUT = 30, WS_SM_SHARED = 228 * 1024;
+template <int NT, int EPI, typename OUT, bool SCALED, int FORM>
+static auto ws_kernel() {
+  auto kernel = linear_ws_kernel<NT, EPI, OUT, SCALED, FORM>;
+  static bool told = false;
+  if (!told) {
+    cudaFuncAttributes at;
+    if (cudaFuncGetAttributes(&at, kernel) == cudaSuccess) {
+      const int fit = (int)(2 * (at.sharedSizeBytes + 1024) * 100 / WS_SM_SHARED) + 1;
+      cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, fit > WS_CARVEOUT ? fit : WS_CARVEOUT);      // (a preference; nothing depends on it but time)
+    }
+    told = true;
+  }
+  return kernel;
+}
+
 template <int NT, int EPI, typename OUT>
 static int launch_ws(const __nv_bfloat16* x, const __nv_bfloat16* W, const float* bias, void* out, float* residual,
                      int M, int N, int K, cudaStream_t stream, const WsRope& rope = WsRope{}, const WsNorm& norm = WsNorm{},
@@ -490,25 +510,25 @@ static int launch_ws(const __nv_bfloat16* x, const __nv_bfloat16* W, const float
     if (N > WS_ONE_GROUP_ROWS && ws_side_by_side(M, N, K)) {
       const int n = (N + 16 * WS_SIDE - 1) / (16 * WS_SIDE);
       if (norm.ssq_in != nullptr)
-        launch_kernel(linear_ws_kernel<NT, EPI, OUT, true, WS_ROWS>, n, WS_WARPS * 32, 0, stream, x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token, 1);
+        launch_kernel(ws_kernel<NT, EPI, OUT, true, WS_ROWS>(), n, WS_WARPS * 32, 0, stream, x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token, 1);
       else
-        launch_kernel(linear_ws_kernel<NT, EPI, OUT, false, WS_ROWS>, n, WS_WARPS * 32, 0, stream, x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token, 1);
+        launch_kernel(ws_kernel<NT, EPI, OUT, false, WS_ROWS>(), n, WS_WARPS * 32, 0, stream, x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token, 1);
       return launch_status("linear_ws");
     }
   }
   if (norm.ssq_in != nullptr) {
     if constexpr (EPI != WS_EPI_ROPE) {
       if (walk) {
-        launch_kernel(linear_ws_kernel<NT, EPI, OUT, true, WS_WALK>, ctas, WS_WARPS * 32, 0, stream, x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token, 1);
+        launch_kernel(ws_kernel<NT, EPI, OUT, true, WS_WALK>(), ctas, WS_WARPS * 32, 0, stream, x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token, 1);
         return launch_status("linear_ws");
       }
     }
-    launch_kernel(linear_ws_kernel<NT, EPI, OUT, true, WS_ONE>, ctas, WS_WARPS * 32, 0, stream, x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token, 1);
+    launch_kernel(ws_kernel<NT, EPI, OUT, true, WS_ONE>(), ctas, WS_WARPS * 32, 0, stream, x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token, 1);
     return launch_status("linear_ws");
   }
   if constexpr (EPI != WS_EPI_ROPE) {
     if (walk) {
-      launch_kernel(linear_ws_kernel<NT, EPI, OUT, false, WS_WALK>, ctas, WS_WARPS * 32, 0, stream, x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token, 1);
+      launch_kernel(ws_kernel<NT, EPI, OUT, false, WS_WALK>(), ctas, WS_WARPS * 32, 0, stream, x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token, 1);
       return launch_status("linear_ws");
     }
   }
@@ -527,11 +547,11 @@ static int launch_ws(const __nv_bfloat16* x, const __nv_bfloat16* W, const float
       attr[1].val.programmaticStreamSerializationAllowed = 1;
       cfg.attrs = attr;
       cfg.numAttrs = pdl_enabled() ? 2 : 1;
-      cudaLaunchKernelEx(&cfg, linear_ws_kernel<NT, EPI, OUT, false, WS_SLICED>, x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token, slices);
+      cudaLaunchKernelEx(&cfg, ws_kernel<NT, EPI, OUT, false, WS_SLICED>(), x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token, slices);
       return launch_status("linear_ws");
     }
   }
-  launch_kernel(linear_ws_kernel<NT, EPI, OUT, false, WS_ONE>, ctas, WS_WARPS * 32, 0, stream, x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token, 1);
+  launch_kernel(ws_kernel<NT, EPI, OUT, false, WS_ONE>(), ctas, WS_WARPS * 32, 0, stream, x, W, bias, (OUT*)out, residual, M, N, K, rope, norm, act, token, 1);
   return launch_status("linear_ws");
 }
 

@@ -2180,6 +2180,37 @@ def choose_splits(num_small: int, nkv: int, max_ctx: int, ctas_per_sm: int = 2, 
     return best
 
 
+# The TMA-fed form merges up to eight ranges in the kernel itself, as a cluster (`sllm_attention_tma_clustered`; the figures stand there): some 1.3 us more for the CTAs, against the
+# 2.7 us and more of the merge kernel, so a range may then be a single key tile.  (Us, as it was / so: 8 requests of 240 keys, 16 query heads and one KV head of 128, whole 8.9, four
+# clustered ranges 7.2; 4 of 200 keys, 14 / 2 heads of 64, 6.8 / 5.3; 16 of 300 keys, 16 / 2 of 128, four ranges and the merge kernel 9.7, eight clustered 8.6.)
+CLUSTER_MERGE_TILES = 1
+CLUSTER_MIN_KEYS = 64
+
+
+@functools.lru_cache(maxsize=4096)
+def tma_clustered(tiles: int, nkv: int, splits: int, hd: int) -> bool:
+    """Whether the TMA-fed decode form merges so many ranges of so many (tile, KV head) pairs in clusters, without scratch."""
+    return bool(lib().sllm_attention_tma_clustered(int(tiles), int(nkv), int(splits), int(hd)))
+
+
+@functools.lru_cache(maxsize=4096)
+def choose_tma_splits(num_small: int, nkv: int, max_ctx: int, hd: int) -> int:
+    """`choose_splits` for the TMA-fed decode form: the same cost, with the cheaper merge of ranges that are a cluster's."""
+    per_sm = _tma_ctas_per_sm(hd)
+    ctas, slots = max(num_small * nkv, 1), max(1, per_sm * num_sms())
+
+    def cost(s):
+        tiles = -(-(-(-max_ctx // s)) // 64)
+        merge = 0 if s == 1 else CLUSTER_MERGE_TILES if tma_clustered(num_small, nkv, s, hd) else MERGE_TILES
+        return -(-ctas * s // slots) * (tiles + SPLIT_OVERHEAD_TILES) + 0.5 * ctas * s / slots + merge
+    best = choose_splits(num_small, nkv, max_ctx, per_sm)
+    for s in range(1, min(max_ctx // CLUSTER_MIN_KEYS, 8) + 1):
+        tiles = -(-(-(-max_ctx // s)) // 64)
+        if -(-max_ctx // (tiles * 64)) == s and (s == 1 or tma_clustered(num_small, nkv, s, hd)) and cost(s) < cost(best):
+            best = s
+    return best
+
+
 def attention_mma(q, k_cache, v_cache, block_tables, q_start, ctx_len, tiles, decode: bool, num_splits: int,
                   nq, nkv, hd, scale, window, out=None, block=None, sink=None, softcap: float = 0.0, gate=None, rel=None):
     """The tensor-core attention kernel on one tile list (see `attention_tiles`); the merge of a split context
@@ -2223,7 +2254,8 @@ def attention_tma_decode(q, k_cache, v_cache, block_tables, q_start, ctx_len, ti
     if out is None:
         out = torch.empty_like(q)
     part_o = part_lse = None
-    if num_splits > 1:
+    scratch = num_splits > 1 and not tma_clustered(tiles[2], nkv, num_splits, hd)
+    if scratch:
         part_o = torch.empty((num_splits, T, nq, hd), dtype=torch.float32, device=q.device)
         part_lse = torch.empty((num_splits, T, nq), dtype=torch.float32, device=q.device)
     call("sllm_attention_tma_decode", _p(q), _p(k_cache), _p(v_cache), k_cache.shape[0], _p(out), _p(part_o),
@@ -2231,7 +2263,7 @@ def attention_tma_decode(q, k_cache, v_cache, block_tables, q_start, ctx_len, ti
          tiles[2], num_splits, T, nq, nkv, hd, k_cache.shape[2], float(scale), int(window or 0), int(block or 0),
          _p(sink), float(softcap or 0.0), *_gate_args(gate), *(rel.args() if rel else _NO_REL)[:2], _p(_status_word(q.device)), _stream())
     _tc_used["since_check"] += 1
-    if num_splits > 1:
+    if scratch:
         launches["own"] += 1
     return out
 
@@ -2367,7 +2399,7 @@ def paged_attention(q, k_cache, v_cache, step, group: int, nq, nkv, hd, scale, w
         if small:
             small_ctx = max((c for c, n in zip(step.ctx_lens, step.q_lens) if n * G <= 16), default=step.max_ctx_len) \
                 if step.ctx_lens else step.max_ctx_len
-            splits = choose_splits(small[2], nkv, small_ctx, per_sm, 0 if tma else MMA_MAX_SPLITS)
+            splits = choose_tma_splits(small[2], nkv, small_ctx, hd) if tma else choose_splits(small[2], nkv, small_ctx, per_sm, MMA_MAX_SPLITS)
         tc_splits = choose_tc_splits(large[2], nkv, step.max_ctx_len) if (large and use_tc and not block and not window) else (1, 0)
         parts = block_parts(step.q_lens, step.ctx_lens, G, block, k_cache.shape[2], q.device, rows) if (large and use_tc and block) else None
         step.attn_tiles[key] = (small, large, splits, rows, tc_splits, parts)

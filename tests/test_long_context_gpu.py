@@ -162,3 +162,39 @@ def test_the_decode_forms_merge_leaves_other_kernels_rows_alone(nq, nkv, hd):
             assert bool((out[1:41] == 77.0).all()), f"{name}, {splits} ranges: the portion's rows were written"
             torch.testing.assert_close(out[[0, 41]].float(), want[[0, 41]], rtol=2e-2, atol=2e-2,
                                        msg=lambda m: f"{name}, {splits} ranges: {m}")
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("lens", [[1], [64], [65, 3, 200], [1000, 512, 0, 700], [130] * 30])
+@pytest.mark.parametrize("splits", [1, 2, 3, 5, 8, 9])
+def test_ranges_merged_by_a_cluster(splits, lens, hd):
+    """The decode form with its context in ranges that a cluster merges (up to eight that fit the GPU at once) and in ranges that go through scratch: contexts that one range holds, ranges
+    without a key, a row without context, a sink and a gate; against float64.  The bound: bfloat16 probabilities and results, 2^-8 each of what is averaged."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import sllm_b200.ops as ops
+    dev, nkv, G, ps = "cuda", 2, 7, 16
+    nq, B = nkv * G, len(lens)
+    g = torch.Generator(device=dev).manual_seed(splits + B)
+    rand = lambda *s: torch.randn(*s, device=dev, generator=g)  # noqa: E731
+    per = max(1, -(-max(lens) // ps))
+    kc, vc = rand(B * per, nkv, ps, hd).bfloat16(), rand(B * per, nkv, ps, hd).bfloat16()
+    bt = torch.arange(B * per, device=dev, dtype=torch.int32).reshape(B, per)
+    q, sink, gate = rand(B, nq * hd).bfloat16(), rand(nq), rand(B, nq + 3)
+    q_start, ctx = torch.arange(B + 1, device=dev, dtype=torch.int32), torch.tensor(lens, device=dev, dtype=torch.int32)
+    small, _ = ops.attention_tiles([1] * B, G, dev)
+    assert ops.tma_clustered(B, nkv, splits, hd) == (2 <= splits <= 8 and B * nkv * splits <= (1.0 if splits == 2 else 0.85) * ops._tma_ctas_per_sm(hd) * ops.num_sms())
+    for s, gt in ((None, None), (sink, (gate, 3))):
+        got = ops.attention_tma_decode(q, kc, vc, bt, q_start, ctx, small, splits, nq, nkv, hd, hd ** -0.5, None, sink=s, gate=gt)
+        ops.check_tcgen05_status()
+        for b, n in enumerate(lens):
+            if n == 0:
+                assert not bool(got[b].any())
+                continue
+            k = kc[b * per:(b + 1) * per].permute(1, 0, 2, 3).reshape(nkv, -1, hd)[:, :n].double().repeat_interleave(G, 0)
+            v = vc[b * per:(b + 1) * per].permute(1, 0, 2, 3).reshape(nkv, -1, hd)[:, :n].double().repeat_interleave(G, 0)
+            z = torch.einsum("hd,hnd->hn", q[b].reshape(nq, hd).double(), k) * hd ** -0.5
+            w = z.exp() / (z.exp().sum(1, keepdim=True) + (s.double().exp()[:, None] if s is not None else 0))
+            f = gate[b, 3:].double().sigmoid()[:, None] if gt is not None else 1.0
+            want, size = torch.einsum("hn,hnd->hd", w, v) * f, torch.einsum("hn,hnd->hd", w, v.abs()) * f
+            assert bool(((got[b].reshape(nq, hd) - want).abs() <= 3 * 2.0 ** -8 * size + 1e-6).all()), (b, n)
