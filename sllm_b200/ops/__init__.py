@@ -1828,6 +1828,9 @@ def linear_scaled_supports(x: torch.Tensor, w: torch.Tensor) -> bool:
             and pair_supports(M, w.shape[0], K))
 
 
+LINEAR_NARROW_MAX_COLS = 15    # a router's logits: fewer columns than a tile of any other kernel (figures in linear_stream.cu)
+
+
 def _stream_splits(N: int, K: int) -> int:
     ctas = -(-N // 128)
     return max(1, min(2 * num_sms() // ctas, K // 128, 16))
@@ -1874,6 +1877,11 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias, out_dtype: torch.dtype, allow
         if allow_partials and out_dtype == torch.float32 and pair_splits(M, N, K) > 1:
             return gemm_pair(x, w, bias, out_dtype, splits=pair_splits(M, N, K))
         return gemm_pair(x, w, bias, out_dtype)
+    if 1 <= M <= TCGEN05_MIN_ROWS and 1 <= N <= LINEAR_NARROW_MAX_COLS and K >= 8 and K % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 \
+            and out_dtype in (torch.float32, torch.bfloat16) and (bias is None or bias.dtype == torch.float32):
+        out = torch.empty((M, N), dtype=out_dtype, device=x.device)
+        call("sllm_linear_narrow", _p(x), _p(w), _p(bias), _p(out), _dtc(out_dtype), M, N, K, _stream())
+        return out
     launches["library"] += 1
     if out_dtype == torch.float32:
         out = torch.mm(x, w.t(), out_dtype=torch.float32)

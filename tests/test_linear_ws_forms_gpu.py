@@ -172,3 +172,17 @@ def test_streams_with_resident_activations(M, N, K):
         want = torch.nn.functional.silu(gate) * up
         lim = 2.0 ** -8 * want.abs() + 1.2 * (gate_off * up.abs() + up_off * gate.abs()) + 1e-5 * gate.abs() * up.abs() + 1e-30
         assert bool(((got.reshape(M, N // 16, 8) - want).abs() <= lim).all())
+
+
+@pytest.mark.parametrize("M", [1, 16, 33, 128])
+@pytest.mark.parametrize("N,K", [(1, 8), (8, 2048), (9, 4096), (15, 4104), (8, 264), (7, 11008)])
+def test_few_columns(M, N, K):
+    """Products narrower than a tile: no library kernel, both result types, with and without a bias."""
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    _, x, w, b, y, bound = _product(dev, M, N, K)
+    before = ops.launches["library"]
+    assert bool(((ops.linear(x, w, b, torch.float32) - y).abs() <= bound).all())
+    plain = y - b
+    assert bool(((ops.linear(x, w, None, torch.bfloat16) - plain).abs() <= bound + 2.0 ** -8 * plain.abs()).all())
+    assert ops.launches["library"] == before
