@@ -148,7 +148,7 @@ post_add_norm_kernel(float* __restrict__ stream, const float* __restrict__ term,
 // Two vectors of four a thread, so a row of 4,096 takes 512 threads.  One row (a decode step of one request) is bound by latency: both gains, which no kernel of the
 // step writes, are loaded before the wait (they had been two misses in HBM, each behind a sum), and a sum takes one barrier.  Many rows are bound by what is in
 // flight: 16 bytes a load, the stream's and the term's together.  (In a graph of such kernels, us, before / now: one row of 4,096 5.6 / 2.2; 2,292 rows of 4,096 with a
-// bfloat16 reader 68 / 28.)  The choice does not look at the number of rows, so a row's bits do not depend on its neighbours.
+// bfloat16 reader 68 / 28, 25 with the gains kept over the rows.)  The choice does not look at the number of rows, so a row's bits do not depend on its neighbours.
 constexpr int PAN_V = 2;
 __device__ __forceinline__ float4 sw_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void sw_store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
@@ -220,21 +220,24 @@ __device__ __forceinline__ float pan_add(PanRow& r, float* x, const float* term,
 template <typename TO>
 __global__ void __launch_bounds__(1024)
 post_add_norm_vec_kernel(float* stream, const float* term, int parts, size_t part_stride, const float* post_gain,
-                         float post_eps, const float* pre_gain, float pre_eps, TO* h, int W) {
+                         float post_eps, const float* pre_gain, float pre_eps, TO* h, int T, int W) {
   __shared__ float red[2][32];
   pdl_launch_dependents();
   PanRow r;
   pan_gains(r, term != nullptr ? post_gain : nullptr, pre_gain, W);
   pdl_wait();
-  const size_t base = (size_t)blockIdx.x * W;
-  const float ss = pan_add(r, stream + base, term, base, parts, part_stride, post_eps, W, red[0]);
-  if (h == nullptr) return;
-  const float inv = pre_gain != nullptr ? 1.0f / sqrtf(block_sum_once(ss, red[1]) / (float)W + pre_eps) : 1.f;      // (no gain: the reader takes the stream as it is)
+  for (int row = blockIdx.x; row < T; row += gridDim.x) {
+    if (row != (int)blockIdx.x) __syncthreads();         // the sums of the row before have been read
+    const size_t base = (size_t)row * W;
+    const float ss = pan_add(r, stream + base, term, base, parts, part_stride, post_eps, W, red[0]);
+    if (h == nullptr) continue;
+    const float inv = pre_gain != nullptr ? 1.0f / sqrtf(block_sum_once(ss, red[1]) / (float)W + pre_eps) : 1.f;      // (no gain: the reader takes the stream as it is)
 #pragma unroll
-  for (int k = 0; k < PAN_V; ++k) {
-    const int i = pan_at(k);
-    const float4 y = r.y[k], g = r.pre[k];
-    if (i < W) sw_store4(h + base + i, pre_gain != nullptr ? make_float4(y.x * inv * g.x, y.y * inv * g.y, y.z * inv * g.z, y.w * inv * g.w) : y);
+    for (int k = 0; k < PAN_V; ++k) {
+      const int i = pan_at(k);
+      const float4 y = r.y[k], g = r.pre[k];
+      if (i < W) sw_store4(h + base + i, pre_gain != nullptr ? make_float4(y.x * inv * g.x, y.y * inv * g.y, y.z * inv * g.z, y.w * inv * g.w) : y);
+    }
   }
 }
 
@@ -298,6 +301,12 @@ static bool pan_vec(int W, int most_threads, size_t part_stride, std::initialize
   for (const void* p : pointers)
     if (((uintptr_t)p & 15) != 0) return false;
   return true;
+}
+// CTAs: as many as are on the SMs at once (64 registers a thread), each with its gains for all its rows (they are as many bytes from L2 as a row and its term:
+// 2,292 rows of 4,096, a CTA a row 27.7 us, so 25.4; bits as before)
+static unsigned pan_ctas(int T, int threads) {
+  const int most = num_sms() * (1024 / threads > 1 ? 1024 / threads : 1);
+  return (unsigned)(T < most ? T : most);
 }
 static int pan_threads(int W) { return (W / 4 + 32 * PAN_V - 1) / (32 * PAN_V) * 32; }
 
@@ -588,10 +597,11 @@ SLLM_EXPORT int sllm_post_add_norm(float* stream_, const float* term, int parts,
   if (T == 0) return SLLM_OK;
   if (pan_vec(W, 1024, part_stride, {stream_, term, post_gain, pre_gain, h}) && (h == nullptr || h_dtype == SLLM_F32 || h_dtype == SLLM_BF16)) {
     if (h == nullptr || h_dtype == SLLM_F32)
-      launch_kernel(post_add_norm_vec_kernel<float>, (unsigned)T, pan_threads(W), 0, stream, stream_, term, parts, part_stride, post_gain, post_eps, pre_gain, pre_eps, (float*)h, W);
+      launch_kernel(post_add_norm_vec_kernel<float>, pan_ctas(T, pan_threads(W)), pan_threads(W), 0, stream, stream_, term, parts, part_stride, post_gain, post_eps, pre_gain, pre_eps,
+                    (float*)h, T, W);
     else
-      launch_kernel(post_add_norm_vec_kernel<__nv_bfloat16>, (unsigned)T, pan_threads(W), 0, stream, stream_, term, parts, part_stride, post_gain, post_eps, pre_gain, pre_eps,
-                    (__nv_bfloat16*)h, W);
+      launch_kernel(post_add_norm_vec_kernel<__nv_bfloat16>, pan_ctas(T, pan_threads(W)), pan_threads(W), 0, stream, stream_, term, parts, part_stride, post_gain, post_eps, pre_gain, pre_eps,
+                    (__nv_bfloat16*)h, T, W);
     return launch_status("post_add_norm");
   }
 #define PAN(TO_, PER_)                                                                                                      \
