@@ -430,11 +430,11 @@ __global__ void __launch_bounds__(AttThreads<DECODE>::value) attention_mma_kerne
 
 // out[row] = sum_s w_s part_o[s][row], w_s = 2^(lse_s - max) / sum: the splits of one row merged.
 template <int HD>
-__global__ void attention_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_lse,
+__global__ void attention_combine_kernel(const float* part_o, const float* part_lse,
                                              __nv_bfloat16* __restrict__ out, int rows, int num_splits,
-                                             const int* __restrict__ tile_seq, const int* __restrict__ q_start, int nq,
+                                             const int* tile_seq, const int* q_start, int nq,
                                              const float* __restrict__ sink, int out_ld, int out_off, int vdim, float out_scale,
-                                             const float* __restrict__ gate, int gate_ld) {
+                                             const float* gate, int gate_ld) {
   // One CTA per (tile, query head, token of the tile's request): the rows the decode form wrote and no others, so
   // that a step's other rows (a prompt portion's, the prefill form's) are neither read nor touched.  The step's
   // description is read before the wait for the kernel before.

@@ -48,9 +48,9 @@ __device__ __forceinline__ void pw_add(float* acc, const uint4& raw, __nv_bfloat
 // channels, and the loads of eight rows are in flight together: a block of 64 tokens is two round trips to memory.
 template <typename TC, bool VEC>
 __global__ void __launch_bounds__(PW_WARPS * 32)
-pool_kv_write_kernel(const TC* __restrict__ k_cache, const TC* __restrict__ v_cache, const int* __restrict__ block_tables,
-                     int max_pages, const int* __restrict__ positions, const int* __restrict__ seq_of_token,
-                     const int* __restrict__ pool_slots, TC* __restrict__ pk_cache, TC* __restrict__ pv_cache, int pool_pages,
+pool_kv_write_kernel(const TC* k_cache, const TC* v_cache, const int* block_tables,
+                     int max_pages, const int* positions, const int* seq_of_token,
+                     const int* pool_slots, TC* __restrict__ pk_cache, TC* __restrict__ pv_cache, int pool_pages,
                      int nkv, int D, int page_size, int pool) {
   extern __shared__ float pw_sm[];               // [2][PW_WARPS][D]
   constexpr int E = VEC ? 16 / (int)sizeof(TC) : 1;
@@ -129,10 +129,10 @@ pool_kv_write_kernel(const TC* __restrict__ k_cache, const TC* __restrict__ v_ca
 
 template <typename TC>
 __global__ void __launch_bounds__(AP_WARPS * 32)
-attention_pooled_simt_kernel(const TC* __restrict__ q, const TC* __restrict__ k_cache, const TC* __restrict__ v_cache,
-                             const TC* __restrict__ pk_cache, const TC* __restrict__ pv_cache,
-                             const int* __restrict__ block_tables, int max_pages, const int* __restrict__ pool_tables,
-                             int pool_max_pages, const int* __restrict__ positions, const int* __restrict__ seq_of_token,
+attention_pooled_simt_kernel(const TC* q, const TC* k_cache, const TC* v_cache,
+                             const TC* pk_cache, const TC* pv_cache,
+                             const int* block_tables, int max_pages, const int* pool_tables,
+                             int pool_max_pages, const int* positions, const int* seq_of_token,
                              int nq, int nkv, int D, int vdim, int page_size, float scale, int window, int pool,
                              const float* __restrict__ sink, float out_scale, TC* __restrict__ out, int out_ld, int out_off) {
   __shared__ float qs[AP_MAX_D];

@@ -42,7 +42,7 @@ constexpr int ATT_WIDE_HD = 640;       // a second instance for wider heads (a c
 
 // d consecutive channels of a row against the query in shared memory; VEC: 16 bytes a load (rows of whole 16-byte pieces)
 template <typename T, bool VEC>
-__device__ __forceinline__ float simt_dot(const T* __restrict__ row, const float* qs, int d) {
+__device__ __forceinline__ float simt_dot(const T* row, const float* qs, int d) {
   float dot[4] = {0.f, 0.f, 0.f, 0.f};               // four chains
   if (VEC) {
     constexpr int P = 16 / sizeof(T);
@@ -64,7 +64,7 @@ __device__ __forceinline__ float simt_dot(const T* __restrict__ row, const float
 
 // four consecutive channels from d on, zeros beyond hd
 template <typename T, bool VEC>
-__device__ __forceinline__ float4 simt_load4(const T* __restrict__ row, int d, int hd) {
+__device__ __forceinline__ float4 simt_load4(const T* row, int d, int hd) {
   if (VEC) {                               // (hd is a multiple of 4 then)
     if (d >= hd) return make_float4(0.f, 0.f, 0.f, 0.f);
     if constexpr (sizeof(T) == 4) {
@@ -81,7 +81,7 @@ __device__ __forceinline__ float4 simt_load4(const T* __restrict__ row, int d, i
 
 // The keys lo .. pos of one query head, four a warp: the warp's maximum m, its sum l (known to all lanes) and its weighted sum of values in acc_s.
 template <typename TC, int MAX_HD, bool VEC>
-__device__ __forceinline__ void simt_groups(const TC* __restrict__ k_cache, const TC* __restrict__ v_cache, const int* __restrict__ bt, const float* qs,
+__device__ __forceinline__ void simt_groups(const TC* k_cache, const TC* v_cache, const int* bt, const float* qs,
                                             float* acc_s, int lo, int pos, int kvh, int nkv, int G, int g, int hd, int page_size, float scale,
                                             float softcap, const float* __restrict__ rel, int rel_n, float& m, float& l) {
   constexpr int NC = (MAX_HD + 127) / 128;
@@ -155,10 +155,10 @@ __device__ __forceinline__ void simt_groups(const TC* __restrict__ k_cache, cons
 
 template <typename TQ, typename TC, int ATT_MAX_HD, bool VEC>
 __global__ void __launch_bounds__(ATT_WARPS * 32)
-attention_simt_kernel(const TQ* __restrict__ q, const TC* __restrict__ k_cache, const TC* __restrict__ v_cache,
-                      const int* __restrict__ block_tables, int max_pages, const int* __restrict__ positions,
-                      const int* __restrict__ seq_of_token, int nq, int nkv, int hd, int page_size, float scale,
-                      int window, int chunk, const float* __restrict__ sink, float softcap, const float* __restrict__ gate, int gate_ld,
+attention_simt_kernel(const TQ* q, const TC* k_cache, const TC* v_cache,
+                      const int* block_tables, int max_pages, const int* positions,
+                      const int* seq_of_token, int nq, int nkv, int hd, int page_size, float scale,
+                      int window, int chunk, const float* __restrict__ sink, float softcap, const float* gate, int gate_ld,
                       const float* __restrict__ rel, int rel_n, TQ* __restrict__ out) {
   __shared__ __align__(16) float qs[ATT_MAX_HD];
   __shared__ __align__(16) float acc_s[ATT_WARPS][ATT_MAX_HD];

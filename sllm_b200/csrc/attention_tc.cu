@@ -606,9 +606,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
 
 // The ranges' results of one (token, head) row merged: weights 2^(lse - max lse), ranges without a key skipped.
 template <int HD>
-__global__ void attention_tc_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_lse,
+__global__ void attention_tc_combine_kernel(const float* part_o, const float* part_lse,
                                             __nv_bfloat16* __restrict__ out, int rows, int num_splits, int nq,
-                                            const float* __restrict__ sink, const float* __restrict__ gate, int gate_ld) {
+                                            const float* __restrict__ sink, const float* gate, int gate_ld) {
   pdl_launch_dependents();       // a short kernel: the successor may be set up behind it
   pdl_wait();
   const int row = blockIdx.x;

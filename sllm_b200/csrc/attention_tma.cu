@@ -496,10 +496,10 @@ constexpr int TA_MAX_SPLITS = 128;     // the merge keeps one weight a range in 
 constexpr int TA_MERGE_WARPS = 8;      // at most
 
 template <int HD>
-__global__ void attention_tma_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_lse,
+__global__ void attention_tma_combine_kernel(const float* part_o, const float* part_lse,
                                              __nv_bfloat16* __restrict__ out, int rows, int num_splits,
-                                             const int* __restrict__ tile_seq, const int* __restrict__ q_start, int nq,
-                                             const float* __restrict__ sink, const float* __restrict__ gate, int gate_ld) {
+                                             const int* tile_seq, const int* q_start, int nq,
+                                             const float* __restrict__ sink, const float* gate, int gate_ld) {
   // One CTA per (tile, query head, token of the tile's request): the rows the decode form wrote and no others, so
   // that a step's other rows (a prompt portion's, the prefill form's) are neither read nor touched.  The step's
   // description is read before the wait for the kernel before.  The ranges' weights are found by the threads side

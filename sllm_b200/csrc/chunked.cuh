@@ -21,7 +21,7 @@ __device__ __forceinline__ void rc_commit() { asm volatile("cp.async.commit_grou
 __device__ __forceinline__ float4 rc_load4(const float* p, bool ok) { return ok ? *reinterpret_cast<const float4*>(p) : make_float4(0.f, 0.f, 0.f, 0.f); }
 // `rows` rows of `cols` floats (ld apart) into dst[i * LD + j] (DR x DC of it), zeros beyond; by cp.async where `vec`
 template <int DR, int DC, int LD>
-__device__ __forceinline__ void load_block(float* __restrict__ dst, const float* __restrict__ src, size_t ld, int rows, int cols, bool vec) {
+__device__ __forceinline__ void load_block(float* __restrict__ dst, const float* src, size_t ld, int rows, int cols, bool vec) {
   if (vec) {
 #pragma unroll 4
     for (int e = threadIdx.x; e < DR * (DC / 4); e += blockDim.x) {

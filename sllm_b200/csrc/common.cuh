@@ -116,8 +116,10 @@ void set_error(const char* msg);   // remembers the text for sllm_last_error()
 // graph): 3.24 ms so; 3.29 ms with no early release in the short kernels; 6.05 ms with the release
 // at the top of every kernel; 3.33 ms with SLLM_PDL=0 in the environment (the attribute off, plain
 // stream order).
-// A kernel that loads straight behind pdl_wait() what an earlier kernel wrote takes that pointer without __restrict__: a load from a const __restrict__ pointer is free to move, and moves, in
-// front of the wait.
+// What a step's kernels write is never reached through a __restrict__ pointer or __ldg(): both say that nobody else writes there while the kernel runs, and with this
+// launch attribute the kernel runs while the one before it still writes, so such a load is free to move in front of the wait.  Matrices, gains, biases and tables, which no kernel of a
+// step writes, keep it: they may be read before the wait, and are, so they have to be in place before the last kernel of this library that the stream holds was launched.  Results that a
+// kernel only writes keep it too (a store does not move in front of the wait).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

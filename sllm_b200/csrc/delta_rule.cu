@@ -500,9 +500,9 @@ __global__ void __launch_bounds__(DR_THREADS) delta_rule_kernel(const DeltaParam
 // (gate_act 0) or z * sigmoid(z) (gate_act 1), or no gate at all (gate_act 2: `proj` is not read); `gain` may be null (ones);
 // a warp per (t, h).
 template <typename TO>
-__global__ void delta_out_kernel(const float* __restrict__ o, const float* __restrict__ gain, const float* __restrict__ proj,
+__global__ void delta_out_kernel(const float* o, const float* __restrict__ gain, const float* proj,
                                  int ld, int off_g, float eps, TO* __restrict__ out, int rows, int H, int dv, int gate_act,
-                                 int out_ld, int out_off, const int* __restrict__ seq_of_token, const int* __restrict__ q_start, int max_len) {
+                                 int out_ld, int out_off, const int* seq_of_token, const int* q_start, int max_len) {
   pdl_launch_dependents();
   pdl_wait();
   const int lane = threadIdx.x & 31;
@@ -528,9 +528,9 @@ __global__ void delta_out_kernel(const float* __restrict__ o, const float* __res
 // the same with a CTA per (t, h): a "head" of many hundred channels (one norm over all of a row's heads together)
 template <typename TO>
 __global__ void __launch_bounds__(256)
-delta_out_wide_kernel(const float* __restrict__ o, const float* __restrict__ gain, const float* __restrict__ proj, int ld, int off_g,
-                      float eps, TO* __restrict__ out, int H, int dv, int gate_act, int out_ld, int out_off, const int* __restrict__ seq_of_token,
-                      const int* __restrict__ q_start, int max_len) {
+delta_out_wide_kernel(const float* o, const float* __restrict__ gain, const float* proj, int ld, int off_g,
+                      float eps, TO* __restrict__ out, int H, int dv, int gate_act, int out_ld, int out_off, const int* seq_of_token,
+                      const int* q_start, int max_len) {
   __shared__ float red[33];
   pdl_launch_dependents();
   pdl_wait();

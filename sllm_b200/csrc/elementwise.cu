@@ -42,7 +42,7 @@ int num_sms() {
 // VEC: rows of whole 16-byte pieces, every pointer on such a border: a thread a piece.  The first kernel of a decode step, bound by its one miss: a channel at a time a row of
 // 4,096 was four round trips (in a graph of such kernels, one row of 4,096 / 16 of 2,048 / 2,292 of 4,096, us: 3.6 / 2.35 / 17.4 before, 1.5 / 1.3 / 11.9 so).
 template <typename TW, bool VEC>
-__global__ void embed_gather_kernel(const TW* __restrict__ table, const int* __restrict__ ids,
+__global__ void embed_gather_kernel(const TW* __restrict__ table, const int* ids,
                                     float* __restrict__ out, int H, int V, float scale) {
   pdl_launch_dependents();       // a short kernel: the successor may be set up behind it
   pdl_wait();
@@ -112,7 +112,7 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
 
 // Any width and alignment, read from memory in every pass.
 template <typename TD, typename TO>
-__global__ void add_rmsnorm_kernel(float* __restrict__ residual, const TD* __restrict__ delta, int parts,
+__global__ void add_rmsnorm_kernel(float* residual, const TD* delta, int parts,
                                    size_t part_stride, const float* __restrict__ w, float eps,
                                    TO* __restrict__ out, int H) {
   __shared__ float red[33];
@@ -179,7 +179,7 @@ add_rmsnorm_few_kernel(float* residual, const TD* delta, int parts, size_t part_
 // row in registers (one read of the stream, no second pass) and a row takes few threads, which
 // leaves many rows resident per SM and many loads in flight.  One part only.
 template <typename TD, typename TO, int VPT>
-__global__ void add_rmsnorm_rows_kernel(float* __restrict__ residual, const TD* __restrict__ delta,
+__global__ void add_rmsnorm_rows_kernel(float* residual, const TD* delta,
                                         const float* __restrict__ w, float eps, TO* __restrict__ out, int H) {
   __shared__ float red[33];
   pdl_launch_dependents();       // a short kernel: the successor may be set up behind it
@@ -222,7 +222,7 @@ __global__ void add_rmsnorm_rows_kernel(float* __restrict__ residual, const TD* 
 // silu(z) = z / (1 + exp(-z))  (ref/qwen3_5.py:28-29; kernels/cuda/kernels.cu:898-907)
 // ---------------------------------------------------------------------------
 template <typename TI, typename TO>
-__global__ void silu_mul_kernel(const TI* __restrict__ gu, TO* __restrict__ out, int I, int blk, size_t n) {
+__global__ void silu_mul_kernel(const TI* gu, TO* __restrict__ out, int I, int blk, size_t n) {
   pdl_launch_dependents();       // a short kernel: the successor may be set up behind it
   pdl_wait();
   size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -237,8 +237,8 @@ __global__ void silu_mul_kernel(const TI* __restrict__ gu, TO* __restrict__ out,
 
 // out[r, :] = sum over parts of x[part][rows[r], :]
 template <typename T>
-__global__ void gather_rows_kernel(const T* __restrict__ x, int parts, size_t part_stride,
-                                   const int* __restrict__ rows, T* __restrict__ out, int H, int n_src) {
+__global__ void gather_rows_kernel(const T* x, int parts, size_t part_stride,
+                                   const int* rows, T* __restrict__ out, int H, int n_src) {
   pdl_launch_dependents();       // a short kernel: the successor may be set up behind it
   pdl_wait();
   int r = rows[blockIdx.x];
@@ -268,11 +268,11 @@ __global__ void gather_rows_kernel(const T* __restrict__ x, int parts, size_t pa
 // they are added here in order.  A block takes `hpb` consecutive heads of one token (one head when
 // few tokens leave the GPU idle otherwise, all heads for prompt portions).
 template <typename TI, typename TC>
-__global__ void rope_kv_write_kernel(const TI* __restrict__ qkv, int parts, size_t part_stride,
+__global__ void rope_kv_write_kernel(const TI* qkv, int parts, size_t part_stride,
                                      const float* __restrict__ bias,
-                                     const int* __restrict__ positions, const float* __restrict__ table,
+                                     const int* positions, const float* __restrict__ table,
                                      int rot, int max_pos, int nq, int nkv, int hd, int hpb,
-                                     const int* __restrict__ slot_mapping, int page_size, int num_pages,
+                                     const int* slot_mapping, int page_size, int num_pages,
                                      TC* __restrict__ k_cache, TC* __restrict__ v_cache, TC* __restrict__ q_out) {
   pdl_launch_dependents();       // a short kernel: the successor may be set up behind it
   pdl_wait();
@@ -333,10 +333,10 @@ __global__ void rope_kv_write_kernel(const TI* __restrict__ qkv, int parts, size
 // hd % 8 == 0.  An item is (head, chunk of 8 dims); the chunk below rot/2 also takes its partner
 // rot/2 further, the chunks between rot/2 and rot are done by their partners.
 template <typename TI>
-__global__ void rope_kv_write_vec_kernel(const TI* __restrict__ qkv, const float* __restrict__ bias,
-                                         const int* __restrict__ positions, const float* __restrict__ table,
+__global__ void rope_kv_write_vec_kernel(const TI* qkv, const float* __restrict__ bias,
+                                         const int* positions, const float* __restrict__ table,
                                          int rot, int max_pos, int nq, int nkv, int hd, int hpb,
-                                         const int* __restrict__ slot_mapping, int page_size, int num_pages,
+                                         const int* slot_mapping, int page_size, int num_pages,
                                          __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache,
                                          __nv_bfloat16* __restrict__ q_out) {
   pdl_launch_dependents();       // a short kernel: the successor may be set up behind it
@@ -424,7 +424,7 @@ __global__ void rope_kv_write_vec_kernel(const TI* __restrict__ qkv, const float
 // ---------------------------------------------------------------------------
 // x[i] = cap * tanh(x[i] / cap), in place (a model's capped logits)
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) softcap_kernel(float* __restrict__ x, size_t n, float cap) {
+__global__ void __launch_bounds__(256) softcap_kernel(float* x, size_t n, float cap) {
   pdl_launch_dependents();
   pdl_wait();
   const size_t step = (size_t)gridDim.x * blockDim.x;
@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(256) softcap_kernel(float* __restrict__ x, siz
 // ---------------------------------------------------------------------------
 template <typename TI, typename TT, typename TO>
 __global__ void __launch_bounds__(256)
-plain_act_kernel(const TI* __restrict__ x, int parts, size_t part_stride, TO* __restrict__ out, int T, int N, int act, const TokenTable token) {
+plain_act_kernel(const TI* x, int parts, size_t part_stride, TO* __restrict__ out, int T, int N, int act, const TokenTable token) {
   pdl_launch_dependents();
   pdl_wait();
   const size_t total = (size_t)T * N;

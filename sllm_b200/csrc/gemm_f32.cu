@@ -66,7 +66,7 @@ __host__ __device__ constexpr int sk_stage_floats(int MT) { return SK_ROWS * SK_
 
 template <int MT, bool VEC>
 __global__ void __launch_bounds__(SK_WARPS * 32)
-gemm_f32_skinny_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
+gemm_f32_skinny_kernel(const float* A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
                        int M, int N, int K, int S, int seg) {
   extern __shared__ __align__(16) float sm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -168,7 +168,7 @@ __host__ __device__ constexpr int tl_threads(int BM) { return BM == 32 ? 128 : 2
 // FOLD: a CTA takes all the segments of its tile, one after the other; else the segments are the CTAs of a cluster (or there is one).
 template <int BM, int BN, bool VEC, bool FOLD>
 __global__ void __launch_bounds__(tl_threads(BM), BM == 128 ? 1 : 2)
-gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
+gemm_f32_tile_kernel(const float* A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
                      int M, int N, int K, int S, int seg) {
   constexpr int THREADS = tl_threads(BM), TM = BM == 128 ? 8 : 4, TN = BN / 16;
   constexpr int WM = TM * 4, WN = TN * 8;            // a warp's share: lanes 4 x 8, the rows of a lane 4 (of W: 8) apart

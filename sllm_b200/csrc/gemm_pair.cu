@@ -105,7 +105,7 @@ struct TpGroups {
 template <int EPI, int BN>
 __global__ void __launch_bounds__(192, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
-                 const float* __restrict__ bias, void* __restrict__ out, int M, int N, int K, int* __restrict__ status,
+                 const float* __restrict__ bias, void* __restrict__ out, int M, int N, int K, int* status,
                  const TgExtra extra, const int ksplits, const int kb_per_split, const TpGroups groups) {
   extern __shared__ unsigned char tp_smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tp_smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -323,7 +323,7 @@ template <int EPI, int R2>
 __global__ void __launch_bounds__(TP_THREADS_WIDE, 1)
 gemm_pair_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                       const __grid_constant__ CUtensorMap map_out, int tma_out,
-                      const float* __restrict__ bias, void* __restrict__ out, int M, int N, int K, int* __restrict__ status,
+                      const float* __restrict__ bias, void* __restrict__ out, int M, int N, int K, int* status,
                       const TgExtra extra) {
   extern __shared__ unsigned char tp_smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tp_smem_raw) + 1023) & ~(uintptr_t)1023);

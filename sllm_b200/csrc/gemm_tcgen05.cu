@@ -42,7 +42,7 @@ constexpr int TG_TMEM_COLS = 512;                        // two accumulators of 
 template <int EPI>
 __global__ void __launch_bounds__(192, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
-                    const float* __restrict__ bias, void* __restrict__ out, int M, int N, int K, int* __restrict__ status) {
+                    const float* __restrict__ bias, void* __restrict__ out, int M, int N, int K, int* status) {
   extern __shared__ unsigned char tg_smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tg_smem_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + TG_STAGES * TG_STAGE_BYTES);

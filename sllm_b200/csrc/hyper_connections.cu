@@ -27,10 +27,10 @@ __device__ __forceinline__ float4 load4_of(const __nv_bfloat16* p) {
 
 template <typename T>
 __global__ void __launch_bounds__(HC_THREADS)
-embed_streams_kernel(const T* __restrict__ table, const int* __restrict__ ids, float* __restrict__ out, int H, int V, float scale, int copies,
+embed_streams_kernel(const T* __restrict__ table, const int* ids, float* __restrict__ out, int H, int V, float scale, int copies,
                      const T* __restrict__ pair_table, unsigned long long buckets, unsigned long long mul_prev, unsigned long long mul_cur,
-                     const int* __restrict__ positions, const int* __restrict__ seq_of_token, const int* __restrict__ q_start,
-                     const int* __restrict__ state_slots, float* __restrict__ before, int vec) {
+                     const int* positions, const int* seq_of_token, const int* q_start,
+                     const int* state_slots, float* before, int vec) {
   __shared__ int prev_s;
   pdl_launch_dependents();
   pdl_wait();
@@ -100,9 +100,9 @@ __device__ __forceinline__ void hc_out(__nv_bfloat16* p, const float (&v)[4]) {
 // VEC channels a thread at a time.
 template <int NS, int VEC, typename TO>
 __global__ void __launch_bounds__(HC_THREADS, NS > 0 && NS <= 4 ? 3 : 1)
-streams_step_kernel(float* __restrict__ streams, const float* __restrict__ term, int parts, size_t part_stride, const float* __restrict__ mix,
+streams_step_kernel(float* streams, const float* term, int parts, size_t part_stride, const float* __restrict__ mix,
                     const float* __restrict__ share, const float* __restrict__ into, const float* __restrict__ gain, float eps,
-                    const int* __restrict__ rows, TO* __restrict__ h, int T, int ns, int W) {
+                    const int* rows, TO* __restrict__ h, int T, int ns, int W) {
   constexpr int CAP = NS > 0 ? NS : HC_MAX_STREAMS;
   extern __shared__ __align__(16) float hc_u[];              // [W] the weighted sum
   __shared__ float red[33];

@@ -17,7 +17,7 @@ namespace sllm {
 
 // dst[i] = x[i] / rms(x) * gain[i] by the whole CTA
 template <typename TO>
-__device__ __forceinline__ void norm_row(const float* __restrict__ x, int n, const float* __restrict__ gain, float eps, TO* __restrict__ dst, float* red) {
+__device__ __forceinline__ void norm_row(const float* x, int n, const float* __restrict__ gain, float eps, TO* __restrict__ dst, float* red) {
   float ss = 0.f;
   for (int i = threadIdx.x; i < n; i += blockDim.x) ss = fmaf(x[i], x[i], ss);
   ss = block_sum(ss, red);
@@ -29,9 +29,9 @@ __device__ __forceinline__ void norm_row(const float* __restrict__ x, int n, con
 // `rot` channels rotated by position (rotate-half layout), written behind the latent; rows of the cache are D wide,
 // zeros beyond rank + tail.
 template <typename TC>
-__global__ void latent_write_kernel(const float* __restrict__ proj, int ld, int off, int rank, const float* __restrict__ gain,
-                                    float eps, const int* __restrict__ slot_mapping, TC* __restrict__ cache, int D, int tail,
-                                    int rot, const int* __restrict__ positions, const float* __restrict__ table, int max_pos,
+__global__ void latent_write_kernel(const float* proj, int ld, int off, int rank, const float* __restrict__ gain,
+                                    float eps, const int* slot_mapping, TC* __restrict__ cache, int D, int tail,
+                                    int rot, const int* positions, const float* __restrict__ table, int max_pos,
                                     int q_off, int q_n, const float* __restrict__ q_gain, TC* __restrict__ q_out) {
   __shared__ float red[33];
   pdl_launch_dependents();
@@ -69,8 +69,8 @@ constexpr int HL_BM = 64, HL_BN = 64, HL_BK = 16;
 
 template <typename TX, typename TW, typename TO>
 __global__ void __launch_bounds__(256)
-head_linear_kernel(const TX* __restrict__ x, int ldx, int xoff, const TW* __restrict__ w, TO* __restrict__ out,
-                   const float* __restrict__ gate, int ldg, int goff, int T, int H, int din, int dout, int xstride, int ldo,
+head_linear_kernel(const TX* x, int ldx, int xoff, const TW* __restrict__ w, TO* __restrict__ out,
+                   const float* gate, int ldg, int goff, int T, int H, int din, int dout, int xstride, int ldo,
                    int ostride, int gate_elem) {
   __shared__ float Xs[HL_BK][HL_BM + 4];
   __shared__ float Ws[HL_BK][HL_BN + 4];
@@ -135,8 +135,8 @@ constexpr int HM_BM = 64, HM_BN = 64, HM_BK = 32, HM_LD = HM_BK + 8;
 
 template <typename TX>
 __global__ void __launch_bounds__(128)
-head_linear_mma_kernel(const TX* __restrict__ x, int ldx, int xoff, const __nv_bfloat16* __restrict__ w,
-                       __nv_bfloat16* __restrict__ out, const float* __restrict__ gate, int ldg, int goff, int T, int H,
+head_linear_mma_kernel(const TX* x, int ldx, int xoff, const __nv_bfloat16* __restrict__ w,
+                       __nv_bfloat16* __restrict__ out, const float* gate, int ldg, int goff, int T, int H,
                        int din, int dout, int vec, int xstride, int ldo, int ostride, int gate_elem) {
   __shared__ __align__(16) __nv_bfloat16 Xs[HM_BM][HM_LD];
   __shared__ __align__(16) __nv_bfloat16 Ws[HM_BN][HM_LD];
@@ -223,8 +223,8 @@ head_linear_mma_kernel(const TX* __restrict__ x, int ldx, int xoff, const __nv_b
 constexpr int HF_KB = 4;          // k blocks of 32 a warp has in flight
 template <typename TX, int NT>
 __global__ void __launch_bounds__(64)
-head_linear_few_kernel(const TX* __restrict__ x, int ldx, int xoff, const __nv_bfloat16* __restrict__ w,
-                       __nv_bfloat16* __restrict__ out, const float* __restrict__ gate, int ldg, int goff, int T, int din, int dout,
+head_linear_few_kernel(const TX* x, int ldx, int xoff, const __nv_bfloat16* __restrict__ w,
+                       __nv_bfloat16* __restrict__ out, const float* gate, int ldg, int goff, int T, int din, int dout,
                        int xstride, int ldo, int ostride, int gate_elem) {
   const int h = blockIdx.y, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
   const int n0 = (blockIdx.x * 2 + (threadIdx.x >> 5)) * 16;
@@ -288,7 +288,7 @@ head_linear_few_kernel(const TX* __restrict__ x, int ldx, int xoff, const __nv_b
 
 // out[t, i] = x[t, off + i] / rms * gain[i]: a CTA per token (the latent queries go through)
 template <typename TO>
-__global__ void norm_cols_kernel(const float* __restrict__ x, int ld, int off, int n, const float* __restrict__ gain, float eps, TO* __restrict__ out) {
+__global__ void norm_cols_kernel(const float* x, int ld, int off, int n, const float* __restrict__ gain, float eps, TO* __restrict__ out) {
   __shared__ float red[33];
   pdl_launch_dependents();
   pdl_wait();

@@ -102,7 +102,7 @@ __device__ __forceinline__ void ls_finish(const float (&acc)[NT][4], int n0, int
 // (LsScale; unsplit launches only).
 template <int NT, int EPI, typename OUT, bool SCALED>
 __global__ void __launch_bounds__(256)
-linear_stream_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ W,
+linear_stream_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ W,
                      const float* __restrict__ bias, OUT* __restrict__ out, float* __restrict__ partial,
                      int M, int N, int K, int chunks_per_split, const LsScale scale) {
   extern __shared__ __align__(16) unsigned char ls_smem[];
@@ -513,7 +513,7 @@ static float* g_noalloc_ptr[NOALLOC_MAX_DEVICES];      // device address of the 
 static std::mutex g_noalloc_mutex;
 
 // out[i] = sum over splits of partial[s][i]
-__global__ void sum_partials_kernel(const float* __restrict__ partial, int splits, size_t n, float* __restrict__ out) {
+__global__ void sum_partials_kernel(const float* partial, int splits, size_t n, float* __restrict__ out) {
   pdl_wait();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;

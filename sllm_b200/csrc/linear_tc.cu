@@ -53,7 +53,7 @@ template <int BN, int EPI>
 __global__ void __launch_bounds__(192, 1)
 linear_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                  const float* __restrict__ bias, void* __restrict__ out, int M, int N, int K, int splits, int kb_per_split,
-                 int* __restrict__ status) {
+                 int* status) {
   using C = LtCfg<BN>;
   extern __shared__ unsigned char lt_smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(lt_smem_raw) + 1023) & ~(uintptr_t)1023);

@@ -112,8 +112,8 @@ struct WsNorm {
 #define WS_ROWS 3
 template <int NT, int EPI, typename OUT, bool SCALED, int FORM>
 __global__ void __launch_bounds__(WS_WARPS * 32, 2)
-linear_ws_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ W,
-                 const float* __restrict__ bias, OUT* __restrict__ out, float* __restrict__ residual,
+linear_ws_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ W,
+                 const float* __restrict__ bias, OUT* __restrict__ out, float* residual,
                  int M, int N, int K, const WsRope rope, const WsNorm norm, const int act, const TokenTable token, const int slices_) {
   constexpr int WS_DEPTH = ws_depth(NT);
   constexpr bool SLICED = FORM == WS_SLICED, ROWS = FORM == WS_ROWS;

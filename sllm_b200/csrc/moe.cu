@@ -27,7 +27,7 @@ __device__ __forceinline__ void warp_argmax(float& v, int& i) {
 }
 
 __global__ void __launch_bounds__(ROUTE_WARPS * 32)
-moe_route_kernel(const float* __restrict__ logits, const float* __restrict__ correction, int T, int E, int groups, int keep,
+moe_route_kernel(const float* logits, const float* __restrict__ correction, int T, int E, int groups, int keep,
                  int top, float scale, float* __restrict__ dense, int* __restrict__ idx, float* __restrict__ wts) {
   extern __shared__ float sm[];
   pdl_launch_dependents();
@@ -95,7 +95,7 @@ moe_route_kernel(const float* __restrict__ logits, const float* __restrict__ cor
 
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(256)
-moe_act_kernel(const TI* __restrict__ up, const float* __restrict__ dense, TO* __restrict__ out, int N, int E, int ff) {
+moe_act_kernel(const TI* up, const float* dense, TO* __restrict__ out, int N, int E, int ff) {
   pdl_launch_dependents();
   pdl_wait();
   const int t = blockIdx.x;
@@ -115,7 +115,7 @@ moe_act_kernel(const TI* __restrict__ up, const float* __restrict__ dense, TO* _
 // experts' columns to be multiples of 8, so that a thread's columns share one expert.  The columns of an expert that a
 // token does not use are not read.
 __global__ void __launch_bounds__(256)
-moe_act_vec_kernel(const __nv_bfloat16* __restrict__ up, const float* __restrict__ dense, __nv_bfloat16* __restrict__ out, int N,
+moe_act_vec_kernel(const __nv_bfloat16* up, const float* dense, __nv_bfloat16* __restrict__ out, int N,
                    int E, int ff) {
   pdl_launch_dependents();
   pdl_wait();

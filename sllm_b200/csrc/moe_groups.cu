@@ -17,7 +17,7 @@ constexpr int MG_TILE = 256, MG_MAX_EXPERTS = 256, MG_THREADS = 1024;
 
 // one block; the order of an expert's rows is whatever the counters give (no result depends on it)
 __global__ void __launch_bounds__(MG_THREADS)
-moe_assign_kernel(const int* __restrict__ idx, int n, int top, int E, int tiles, int* __restrict__ place, int* __restrict__ tile_expert, int* __restrict__ row_token) {
+moe_assign_kernel(const int* idx, int n, int top, int E, int tiles, int* __restrict__ place, int* __restrict__ tile_expert, int* __restrict__ row_token) {
   __shared__ int count[MG_MAX_EXPERTS], start[MG_MAX_EXPERTS + 1];
   const int tid = threadIdx.x;
   pdl_wait();
@@ -58,7 +58,7 @@ moe_assign_kernel(const int* __restrict__ idx, int n, int top, int E, int tiles,
 
 // a warp per row, 16 bytes a lane
 __global__ void __launch_bounds__(256)
-moe_gather_kernel(const uint4* __restrict__ x, const int* __restrict__ row_token, uint4* __restrict__ out, int rows, int pieces) {
+moe_gather_kernel(const uint4* x, const int* row_token, uint4* __restrict__ out, int rows, int pieces) {
   pdl_wait();
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= rows) return;
@@ -70,8 +70,8 @@ moe_gather_kernel(const uint4* __restrict__ x, const int* __restrict__ row_token
 
 // a block per token, four columns a thread
 __global__ void __launch_bounds__(256)
-moe_combine_kernel(const float* __restrict__ y, const int* __restrict__ place, const float* __restrict__ wts, int top, const float* __restrict__ shared,
-                   const float* __restrict__ shared_w, int ld_w, float* __restrict__ out, int add, int W) {
+moe_combine_kernel(const float* y, const int* place, const float* wts, int top, const float* shared,
+                   const float* shared_w, int ld_w, float* out, int add, int W) {
   pdl_wait();
   const int t = blockIdx.x;
   const float sw = shared_w != nullptr ? shared_w[(size_t)t * ld_w] : 1.0f;

@@ -16,7 +16,7 @@ namespace sllm {
 // stream[t, 2i] += sin(p * f_i), stream[t, 2i+1] += cos(p * f_i), p = positions[t], f = inv_freq[i].
 // The angle is a float32 product of the float32 position and the float32 frequency; sinf and cosf are
 // the accurate forms (their argument reduction is exact for angles of this size).
-__global__ void add_sinusoid_kernel(float* __restrict__ stream, const int* __restrict__ positions,
+__global__ void add_sinusoid_kernel(float* stream, const int* positions,
                                     const float* __restrict__ inv_freq, int W) {
   pdl_launch_dependents();
   pdl_wait();
@@ -54,8 +54,8 @@ __device__ __forceinline__ void pb_store4(__nv_bfloat16* p, float4 v) {
 // strides are multiples of 4 and every pointer is 16-byte aligned; four elements a thread, the partial sums
 // read with independent loads.
 template <bool VEC>
-__global__ void add_group_ssq_kernel(float* __restrict__ stream, const float* __restrict__ d0, int parts0, size_t stride0,
-                                     const float* __restrict__ d1, int parts1, size_t stride1,
+__global__ void add_group_ssq_kernel(float* stream, const float* d0, int parts0, size_t stride0,
+                                     const float* d1, int parts1, size_t stride1,
                                      float* __restrict__ rinv, int W, int groups, float eps) {
   pdl_launch_dependents();
   pdl_wait();
@@ -108,7 +108,7 @@ __global__ void add_group_ssq_kernel(float* __restrict__ stream, const float* __
 // 1 / sqrt(mean(x[group]^2) + eps) of every group of a row, into dst[groups] (shared memory): warps take groups in
 // turn; a group's sum is taken in an order that depends on its size only.
 template <bool VEC>
-__device__ __forceinline__ void group_roots(const float* __restrict__ row, float* dst, int groups, int gs, float eps) {
+__device__ __forceinline__ void group_roots(const float* row, float* dst, int groups, int gs, float eps) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int g = warp; g < groups; g += nw) {
     const float* x = row + (size_t)g * gs;
@@ -135,10 +135,10 @@ __device__ __forceinline__ void group_roots(const float* __restrict__ row, float
 // before or the portion's last), so that a stream with nothing pending needs no kernel before this one.
 // VEC: W and W / groups are multiples of 4 and every pointer is 16-byte aligned.
 template <typename TO, bool VEC>
-__global__ void group_norm_shift_kernel(const float* __restrict__ stream, const float* __restrict__ rinv,
+__global__ void group_norm_shift_kernel(const float* stream, const float* rinv,
                                         const float* __restrict__ gain, const float* __restrict__ mix,
-                                        float* __restrict__ state, const int* __restrict__ seq_of_token,
-                                        const int* __restrict__ q_start, const int* __restrict__ state_slots,
+                                        float* state, const int* seq_of_token,
+                                        const int* q_start, const int* state_slots,
                                         TO* __restrict__ out_h, TO* __restrict__ out_hs, int W, int groups, float eps) {
   extern __shared__ float s_ri[];          // [2][groups]: this row's roots, and the other row's
   pdl_launch_dependents();
@@ -218,7 +218,7 @@ __device__ __forceinline__ float act_gelu_tanh(float z) {
 // (interleave == I: all gates, then all ups).  VEC: I and interleave are multiples of 4 and the pointers 16-byte
 // aligned; four results a thread.
 template <typename TI, typename TO, int ACT, bool VEC>
-__global__ void act_mul_kernel(const TI* __restrict__ gu, TO* __restrict__ out, int I, int interleave) {
+__global__ void act_mul_kernel(const TI* gu, TO* __restrict__ out, int I, int interleave) {
   pdl_launch_dependents();
   pdl_wait();
   const size_t t = blockIdx.x;             // (rows on the grid's x: no limit of 65,535)
@@ -243,7 +243,7 @@ __global__ void act_mul_kernel(const TI* __restrict__ gu, TO* __restrict__ out, 
 
 // out[t, j] = tanh(x[t, col0 + j]), j < n; x float32 with row stride ld.
 template <typename TO>
-__global__ void tanh_cols_kernel(const float* __restrict__ x, int ld, int col0, int n, TO* __restrict__ out, int T) {
+__global__ void tanh_cols_kernel(const float* x, int ld, int col0, int n, TO* __restrict__ out, int T) {
   pdl_launch_dependents();
   pdl_wait();
   const size_t total = (size_t)T * n;
@@ -256,7 +256,7 @@ __global__ void tanh_cols_kernel(const float* __restrict__ x, int ld, int col0, 
 
 // stream[t, c] += rows[t, c] + vec[c] (rows may be absent): what a range of layers that runs again takes in before a pass.
 __global__ void __launch_bounds__(256)
-add_rows_kernel(float* __restrict__ stream, const float* __restrict__ rows, const float* __restrict__ vec, size_t n, int W) {
+add_rows_kernel(float* stream, const float* rows, const float* __restrict__ vec, size_t n, int W) {
   pdl_launch_dependents();
   pdl_wait();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -271,7 +271,7 @@ add_rows_kernel(float* __restrict__ stream, const float* __restrict__ rows, cons
 // A CTA per row; the row's sum of squares is taken once, in an order that depends on the width alone.
 template <typename TO>
 __global__ void __launch_bounds__(256)
-norm_pair_kernel(const float* __restrict__ stream, const float* __restrict__ gain_a, const float* __restrict__ gain_b, float eps,
+norm_pair_kernel(const float* stream, const float* __restrict__ gain_a, const float* __restrict__ gain_b, float eps,
                  TO* __restrict__ out_a, TO* __restrict__ out_b, int W) {
   __shared__ float red[33];
   pdl_launch_dependents();

@@ -58,7 +58,7 @@ __device__ __forceinline__ void rc_turn4(float* lo, float* hi, float4 x, float4 
 // four tokens a lane (two tensors: two tokens) in flight together.
 template <int DK, int NX, int LD0, int LD1, int THREADS>
 __device__ __forceinline__ void load_rotated(const RetentionParams& p, float* d0, float* d1, int off0, int off1, float mul0, float mul1,
-                                             const float* __restrict__ weight, int h, int t0, int pos0, int n) {
+                                             const float* weight, int h, int t0, int pos0, int n) {
   const int half = p.rot >> 1, dk = p.dk, l8 = threadIdx.x & 7;
   constexpr int TPP = THREADS / 8, AT = NX == 1 ? 4 : 2;                   // tokens a pass, passes whose loads are in flight
   static_assert(RC % (TPP * AT) == 0 || RC % TPP == 0, "whole passes");

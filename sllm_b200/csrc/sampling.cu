@@ -52,7 +52,7 @@ __device__ __forceinline__ MaxIdx better(MaxIdx a, MaxIdx b) {
 }
 
 // the first maximum of row[from, to), known to all threads; index 0x7fffffff: nothing there is above minus infinity
-__device__ MaxIdx part_argmax(const float* __restrict__ row, int from, int to, bool vec, MaxIdx* sh) {
+__device__ MaxIdx part_argmax(const float* row, int from, int to, bool vec, MaxIdx* sh) {
   MaxIdx best{-INFINITY, 0x7fffffff};
   if (vec) {                                         // whole 16-byte pieces
     // four values a load, four loads in flight; a thread's indices still ascend
@@ -102,7 +102,7 @@ struct RowPart {
 };
 
 // the row's first maximum (index 0 where nothing is above minus infinity), known to the first block; all blocks of the cluster call it
-__device__ MaxIdx row_argmax(const float* __restrict__ row, const RowPart& part, MaxIdx* sh, MaxIdx* parts /* [8] shared */) {
+__device__ MaxIdx row_argmax(const float* row, const RowPart& part, MaxIdx* sh, MaxIdx* parts /* [8] shared */) {
   MaxIdx r = part_argmax(row, part.from, part.to, part.vec, sh);
   if (part.blocks > 1) {
     cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
@@ -160,7 +160,7 @@ struct Select {
 
 // f(logit, index) over every `stride`th logit of the row from `first` on, eight loads in flight a thread
 template <class F>
-__device__ __forceinline__ void for_strided(const float* __restrict__ row, int first, int stride, int V, F f) {
+__device__ __forceinline__ void for_strided(const float* row, int first, int stride, int V, F f) {
   for (int i0 = first; i0 < V; i0 += stride * 8) {
     float l[8];
 #pragma unroll
@@ -176,10 +176,10 @@ __device__ __forceinline__ void for_strided(const float* __restrict__ row, int f
   }
 }
 template <class F>
-__device__ __forceinline__ void for_row(const float* __restrict__ row, int V, F f) { for_strided(row, threadIdx.x, SAMPLE_THREADS, V, f); }
+__device__ __forceinline__ void for_row(const float* row, int V, F f) { for_strided(row, threadIdx.x, SAMPLE_THREADS, V, f); }
 // the same over [base, base + len) cut at `end`, by one warp
 template <class F>
-__device__ __forceinline__ void for_part(const float* __restrict__ row, int base, int len, int end, F f) {
+__device__ __forceinline__ void for_part(const float* row, int base, int len, int end, F f) {
   const int lane = threadIdx.x & 31;
   for (int o = 0; o < len; o += 32 * 8) {
     float l[8];
@@ -278,7 +278,7 @@ constexpr int SEL_CANDIDATES = 4096;        // the chosen linear bin's keys are 
 // by_mass false: the key of the k-th largest eligible logit.  by_mass true: the first key, going
 // down, at which the cumulative mass reaches `target` (`target_is_fraction`: of the eligible total).
 // Eligible: key > floor_key where has_floor.  The result is in *st (shared), the same for all threads.
-__device__ void select_key(const float* __restrict__ row, int V, float mx, float inv_t, bool by_mass, int k,
+__device__ void select_key(const float* row, int V, float mx, float inv_t, bool by_mass, int k,
                            double target, bool target_is_fraction, bool has_floor, uint32_t floor_key,
                            int* hist_c, float* hist_m, int* bin_c, double* bin_m, uint32_t* cand, int* n_cand, Select* st) {
   const int warp = threadIdx.x >> 5;
@@ -393,7 +393,7 @@ struct FastShared {
 // indices in `dyn_smem`), the largest fifth one is recorded in fs->max_let_go (31 bits), *mx_out is
 // the row's maximum (first index among equals); *sum_out is the sum over the whole row of
 // expf((logit - max) / T), from a second pass.
-__device__ void collect_candidates(const float* __restrict__ row, int V, float inv_t, unsigned char* dyn_smem, MaxIdx* sh_mi,
+__device__ void collect_candidates(const float* row, int V, float inv_t, unsigned char* dyn_smem, MaxIdx* sh_mi,
                                    double* red, FastShared* fs, MaxIdx* mx_out, double* sum_out) {
   uint32_t* cand_key = reinterpret_cast<uint32_t*>(dyn_smem);
   int* cand_idx = reinterpret_cast<int*>(cand_key + FAST_CANDIDATES);
@@ -581,7 +581,7 @@ static_assert(TOPK_LIST * 8 <= SAMPLE_SMEM, "the list lives in the histograms' s
 
 // true: out[row] is written (by the first block).  false: the general path must take the row.  All blocks of the cluster call it; in the others
 // the result means nothing.
-__device__ bool sample_top_k_fast(const float* __restrict__ row, int V, const RowPart& part, float inv_t, int k, float pfrac, double u,
+__device__ bool sample_top_k_fast(const float* row, int V, const RowPart& part, float inv_t, int k, float pfrac, double u,
                                   unsigned char* dyn_smem, uint32_t* group_max /* [256] shared */, uint32_t* bound_s, int* count,
                                   FastShared* fs, int* out) {
   cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
@@ -670,7 +670,7 @@ __device__ bool sample_top_k_fast(const float* __restrict__ row, int V, const Ro
 
 constexpr int FAST_P_KEPT = SAMPLE_THREADS;
 
-__device__ bool sample_top_p_fast(const float* __restrict__ row, int V, float inv_t, float pfrac, double u,
+__device__ bool sample_top_p_fast(const float* row, int V, float inv_t, float pfrac, double u,
                                   unsigned char* dyn_smem, int* bin_c, double* bin_m, Select* sel, MaxIdx* sh_mi,
                                   FastShared* fs, MaxIdx* mx_out, int* out) {
   uint32_t* cand_key = reinterpret_cast<uint32_t*>(dyn_smem);
@@ -721,8 +721,8 @@ __device__ bool sample_top_p_fast(const float* __restrict__ row, int V, float in
 }
 
 __global__ void __launch_bounds__(SAMPLE_THREADS)
-sample_rows_kernel(const float* __restrict__ logits, int V, const float* __restrict__ temperature,
-                   const double* __restrict__ uniform, const int* __restrict__ top_k, const float* __restrict__ top_p,
+sample_rows_kernel(const float* logits, int V, const float* temperature,
+                   const double* uniform, const int* top_k, const float* top_p,
                    int* __restrict__ out, int blocks_log2) {
   extern __shared__ __align__(16) unsigned char sample_smem[];
   __shared__ MaxIdx sh_mi[32], parts_mi[8];
@@ -960,8 +960,8 @@ sample_rows_kernel(const float* __restrict__ logits, int V, const float* __restr
 
 // Repetition penalty in place (runtime/sampler.py:12-33): for each (row, id) pair, a positive logit is
 // divided by the row's penalty and a negative one multiplied.  The pairs name each (row, id) once.
-__global__ void repetition_penalty_kernel(float* __restrict__ logits, int V, const int* __restrict__ pair_row,
-                                          const int* __restrict__ pair_id, const float* __restrict__ pair_penalty, int n) {
+__global__ void repetition_penalty_kernel(float* logits, int V, const int* pair_row,
+                                          const int* pair_id, const float* pair_penalty, int n) {
   pdl_launch_dependents();
   pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -978,8 +978,8 @@ __global__ void repetition_penalty_kernel(float* __restrict__ logits, int V, con
 // decoded tokens alike) before the step runs; penalty_seen_kernel changes the wanted logits rows of
 // requests whose penalty is neither 0 nor 1.  Both read the step's description on the device, so they
 // can be part of a captured decode step.
-__global__ void mark_seen_kernel(unsigned char* __restrict__ seen, int V, const int* __restrict__ token_ids,
-                                 const int* __restrict__ seq_of_token, const int* __restrict__ state_slots, int T, int slots) {
+__global__ void mark_seen_kernel(unsigned char* seen, int V, const int* token_ids,
+                                 const int* seq_of_token, const int* state_slots, int T, int slots) {
   pdl_launch_dependents();
   pdl_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -988,9 +988,9 @@ __global__ void mark_seen_kernel(unsigned char* __restrict__ seen, int V, const 
   if (id >= 0 && id < V && slot >= 0 && slot < slots) seen[(size_t)slot * V + id] = 1;
 }
 
-__global__ void penalty_seen_kernel(float* __restrict__ logits, int V, const unsigned char* __restrict__ seen,
-                                    const int* __restrict__ logit_rows, const int* __restrict__ seq_of_token,
-                                    const int* __restrict__ state_slots, const float* __restrict__ penalty, int slots) {
+__global__ void penalty_seen_kernel(float* logits, int V, const unsigned char* seen,
+                                    const int* logit_rows, const int* seq_of_token,
+                                    const int* state_slots, const float* penalty, int slots) {
   pdl_launch_dependents();
   pdl_wait();
   const int row = blockIdx.y;

@@ -31,7 +31,7 @@ namespace sllm {
 __device__ __forceinline__ float sw_sigmoid(float z) { return 1.0f / (1.0f + expf(-z)); }
 
 // stream += term / rms(term) * post_gain (no term: nothing added); returns this thread's share of sum(stream^2)
-__device__ __forceinline__ float post_add(float* __restrict__ x, const float* __restrict__ term, size_t base, int parts,
+__device__ __forceinline__ float post_add(float* x, const float* term, size_t base, int parts,
                                           size_t part_stride, const float* __restrict__ post_gain, float post_eps, int W, float* red) {
   float ss = 0.f;
   if (term != nullptr) {
@@ -59,7 +59,7 @@ __device__ __forceinline__ float post_add(float* __restrict__ x, const float* __
 // The same with the row in registers (W <= 256 * PER): the stream's and the term's loads leave together, nothing is read
 // twice, and the sums run in the order of `post_add`, so both forms give the same bits.
 template <int PER>
-__device__ __forceinline__ float post_add_regs(float* __restrict__ x, const float* __restrict__ term, size_t base, int parts,
+__device__ __forceinline__ float post_add_regs(float* x, const float* term, size_t base, int parts,
                                                size_t part_stride, const float* __restrict__ post_gain, float post_eps, int W,
                                                float* red, float (&y)[PER]) {
   float v[PER];
@@ -104,7 +104,7 @@ __device__ __forceinline__ float post_add_regs(float* __restrict__ x, const floa
 // PER = 0: rows of any width, read from memory in every pass
 template <typename TO, int PER>
 __global__ void __launch_bounds__(256)
-post_add_norm_kernel(float* __restrict__ stream, const float* __restrict__ term, int parts, size_t part_stride,
+post_add_norm_kernel(float* stream, const float* term, int parts, size_t part_stride,
                      const float* __restrict__ post_gain, float post_eps, const float* __restrict__ pre_gain, float pre_eps,
                      TO* __restrict__ h, int W) {
   __shared__ float red[33];
@@ -312,7 +312,7 @@ static int pan_threads(int W) { return (W / 4 + 32 * PAN_V - 1) / (32 * PAN_V) *
 
 // h + conv(h) of one channel from its state row (oldest input first), which moves on by one
 template <typename TO>
-__device__ __forceinline__ void conv_one(float now, const float* __restrict__ w, float* __restrict__ s, int keep, TO* __restrict__ dst) {
+__device__ __forceinline__ void conv_one(float now, const float* __restrict__ w, float* s, int keep, TO* __restrict__ dst) {
   float acc = 0.f;
   for (int j = 0; j < keep; ++j) {
     const float v = s[j];
@@ -330,10 +330,10 @@ __device__ __forceinline__ void conv_one(float now, const float* __restrict__ w,
 // store, so the loads of its channels do not wait for one another.
 template <typename TO, int PER, int TAPS>
 __global__ void __launch_bounds__(256)
-post_add_norm_conv_kernel(float* __restrict__ stream, const float* __restrict__ term, int parts, size_t part_stride,
+post_add_norm_conv_kernel(float* stream, const float* term, int parts, size_t part_stride,
                           const float* __restrict__ post_gain, float post_eps, const float* __restrict__ pre_gain, float pre_eps,
-                          const float* __restrict__ conv_w, int taps, float* __restrict__ conv_state,
-                          const int* __restrict__ seq_of_token, const int* __restrict__ state_slots, TO* __restrict__ out, int W) {
+                          const float* __restrict__ conv_w, int taps, float* conv_state,
+                          const int* seq_of_token, const int* state_slots, TO* __restrict__ out, int W) {
   __shared__ float red[33];
   pdl_launch_dependents();
   pdl_wait();
@@ -399,8 +399,8 @@ constexpr int MG_WARPS = 16;
 // the runs, 32-byte rows).  A run's effect on what it meets is (keep, reach): S_out = keep * S_in + reach.
 template <typename TO, int CH>
 __global__ void __launch_bounds__(32 * MG_WARPS)
-mingru_scan_kernel(const float* __restrict__ proj, int ld, int off_z, int off_x, int off_g, float* __restrict__ state,
-                   const int* __restrict__ q_start, const int* __restrict__ state_slots, TO* __restrict__ out, int C) {
+mingru_scan_kernel(const float* proj, int ld, int off_z, int off_x, int off_g, float* state,
+                   const int* q_start, const int* state_slots, TO* __restrict__ out, int C) {
   constexpr int RUNS = MG_WARPS * (32 / CH);
   __shared__ float keep_s[RUNS][CH], reach_s[RUNS][CH];
   pdl_wait();
@@ -445,7 +445,7 @@ mingru_scan_kernel(const float* __restrict__ proj, int ld, int off_z, int off_x,
 
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(256)
-gated_clamp_act_kernel(const TI* __restrict__ gu, const float* __restrict__ dense, TO* __restrict__ out, int N, int E, int ff,
+gated_clamp_act_kernel(const TI* gu, const float* dense, TO* __restrict__ out, int N, int E, int ff,
                        int tail, int il, float limit, float alpha, int act) {
   pdl_launch_dependents();
   pdl_wait();
@@ -469,7 +469,7 @@ gated_clamp_act_kernel(const TI* __restrict__ gu, const float* __restrict__ dens
 
 // bfloat16 in and out, blocks of 8 (or a multiple): eight columns a thread, one 16-byte load each of gate and up
 __global__ void __launch_bounds__(256)
-gated_clamp_act_vec_kernel(const __nv_bfloat16* __restrict__ gu, const float* __restrict__ dense, __nv_bfloat16* __restrict__ out,
+gated_clamp_act_vec_kernel(const __nv_bfloat16* gu, const float* dense, __nv_bfloat16* __restrict__ out,
                            int N, int E, int ff, int tail, int il, float limit, float alpha, int act) {
   pdl_launch_dependents();
   pdl_wait();
@@ -503,7 +503,7 @@ constexpr int RS_WARPS = 4;
 
 // a warp per token
 __global__ void __launch_bounds__(RS_WARPS * 32)
-moe_route_top_softmax_kernel(const float* __restrict__ logits, int ld, int T, int E, int gated, int top, float scale, float* __restrict__ dense,
+moe_route_top_softmax_kernel(const float* logits, int ld, int T, int E, int gated, int top, float scale, float* __restrict__ dense,
                              int* __restrict__ idx, float* __restrict__ wts) {
   extern __shared__ float sm[];
   pdl_launch_dependents();
@@ -557,7 +557,7 @@ moe_route_top_softmax_kernel(const float* __restrict__ logits, int ld, int T, in
 // a thread per (token, head, pair or plain column)
 template <typename TO>
 __global__ void __launch_bounds__(256)
-rope_cols_kernel(const float* __restrict__ x, int ldx, int xoff, int xstride, int n, int rot, const int* __restrict__ positions,
+rope_cols_kernel(const float* x, int ldx, int xoff, int xstride, int n, int rot, const int* positions,
                  const float* __restrict__ table, int max_pos, TO* __restrict__ out, int ldo, int ooff, int ostride, int T, int H) {
   pdl_launch_dependents();
   pdl_wait();

@@ -24,11 +24,11 @@ __device__ __forceinline__ float sbs_silu(float z) { return z / (1.0f + expf(-z)
 
 template <typename TC>
 __global__ void __launch_bounds__(128)
-qk_norm_rope_kv_write_kernel(const float* __restrict__ qkv, int ld, const float* __restrict__ q_gain,
+qk_norm_rope_kv_write_kernel(const float* qkv, int ld, const float* __restrict__ q_gain,
                              const float* __restrict__ k_gain, const float* __restrict__ q_mul, float eps,
-                             const int* __restrict__ positions,
+                             const int* positions,
                              const float* __restrict__ table, int rot, int max_pos, int nq, int nkv, int dim, int vdim, int D,
-                             const int* __restrict__ slot_mapping, int page_size, int num_pages, TC* __restrict__ k_cache,
+                             const int* slot_mapping, int page_size, int num_pages, TC* __restrict__ k_cache,
                              TC* __restrict__ v_cache, TC* __restrict__ q_out, int T) {
   pdl_launch_dependents();
   pdl_wait();
@@ -107,9 +107,9 @@ template <int VEC, typename T> __device__ __forceinline__ void wn_store(T* p, co
 // and the product's rows are multiples of 4.
 template <typename TC, int VEC>
 __global__ void __launch_bounds__(256)
-whole_norm_kv_write_kernel(const float* __restrict__ qkv, int parts, size_t part_stride, int ld, const float* __restrict__ bias,
-                           const float* __restrict__ q_gain, const float* __restrict__ k_gain, float eps, const int* __restrict__ positions,
-                           float q_coef, int q_every, int nq, int nkv, int dim, int vdim, int D, const int* __restrict__ slot_mapping,
+whole_norm_kv_write_kernel(const float* qkv, int parts, size_t part_stride, int ld, const float* __restrict__ bias,
+                           const float* __restrict__ q_gain, const float* __restrict__ k_gain, float eps, const int* positions,
+                           float q_coef, int q_every, int nq, int nkv, int dim, int vdim, int D, const int* slot_mapping,
                            int page_size, int num_pages, TC* __restrict__ k_cache, TC* __restrict__ v_cache, TC* __restrict__ q_out) {
   extern __shared__ __align__(16) float wn_x[];                      // [(nq + nkv) * dim]
   __shared__ float red[33];
@@ -180,9 +180,9 @@ whole_norm_kv_write_kernel(const float* __restrict__ qkv, int parts, size_t part
 // convolution (a convolution in front of a sublayer that keeps the sublayer's input as it was beside it).
 template <int MODE, typename TO>
 __global__ void __launch_bounds__(256)
-short_conv_kernel(const float* __restrict__ x, int ld, int off, const float* __restrict__ w, const float* __restrict__ bias, int taps,
-                  const float* __restrict__ state, const int* __restrict__ seq_of_token, const int* __restrict__ q_start,
-                  const int* __restrict__ state_slots, TO* __restrict__ out, int C, int own_state) {
+short_conv_kernel(const float* x, int ld, int off, const float* __restrict__ w, const float* __restrict__ bias, int taps,
+                  const float* state, const int* seq_of_token, const int* q_start,
+                  const int* state_slots, TO* __restrict__ out, int C, int own_state) {
   pdl_launch_dependents();
   pdl_wait();
   const int t = blockIdx.x, c = blockIdx.y * blockDim.x + threadIdx.x;
@@ -209,8 +209,8 @@ short_conv_kernel(const float* __restrict__ x, int ld, int off, const float* __r
 // weights and of the state.  The sums run in the scalar kernel's order, so both give the same bits.
 template <int MODE, int TAPS, typename TO>
 __global__ void __launch_bounds__(128)
-short_conv_vec4_kernel(const float* __restrict__ x, int ld, int off, const float* __restrict__ w, const float* __restrict__ bias, float* __restrict__ state,
-                       const int* __restrict__ seq_of_token, const int* __restrict__ q_start, const int* __restrict__ state_slots,
+short_conv_vec4_kernel(const float* x, int ld, int off, const float* __restrict__ w, const float* __restrict__ bias, float* state,
+                       const int* seq_of_token, const int* q_start, const int* state_slots,
                        TO* __restrict__ out, int C, int own_state) {
   constexpr int KEEP = TAPS - 1;
   pdl_launch_dependents();
@@ -288,8 +288,8 @@ short_conv_vec4_kernel(const float* __restrict__ x, int ld, int off, const float
 // kernels above: the same bits.  grid (ceil(T / RUN), ceil(C / 512)).
 template <int MODE, int TAPS, typename TO, int RUN>
 __global__ void __launch_bounds__(128)
-short_conv_run_kernel(const float* __restrict__ x, int ld, int off, const float* __restrict__ w, const float* __restrict__ bias, const float* __restrict__ state,
-                      const int* __restrict__ seq_of_token, const int* __restrict__ q_start, const int* __restrict__ state_slots,
+short_conv_run_kernel(const float* x, int ld, int off, const float* __restrict__ w, const float* __restrict__ bias, const float* state,
+                      const int* seq_of_token, const int* q_start, const int* state_slots,
                       TO* __restrict__ out, int C, int T) {
   constexpr int KEEP = TAPS - 1;
   pdl_launch_dependents();
@@ -365,8 +365,8 @@ short_conv_run_kernel(const float* __restrict__ x, int ld, int off, const float*
 
 // grid (S, ceil(C / 256)): a thread per (request, channel) rewrites its state row in ascending order
 __global__ void __launch_bounds__(256)
-short_conv_state_kernel(const float* __restrict__ x, int ld, int off, int taps, float* __restrict__ state,
-                        const int* __restrict__ q_start, const int* __restrict__ state_slots, int C) {
+short_conv_state_kernel(const float* x, int ld, int off, int taps, float* state,
+                        const int* q_start, const int* state_slots, int C) {
   pdl_launch_dependents();
   pdl_wait();
   const int seq = blockIdx.x, c = blockIdx.y * blockDim.x + threadIdx.x;
@@ -381,8 +381,8 @@ short_conv_state_kernel(const float* __restrict__ x, int ld, int off, int taps, 
 
 // a CTA per token
 __global__ void __launch_bounds__(256)
-norm_mean_add_kernel(float* __restrict__ stream, const float* __restrict__ a, const float* __restrict__ ga,
-                     const float* __restrict__ b, const float* __restrict__ gb, float eps, int W) {
+norm_mean_add_kernel(float* stream, const float* a, const float* __restrict__ ga,
+                     const float* b, const float* __restrict__ gb, float eps, int W) {
   __shared__ float red[33];
   pdl_launch_dependents();
   pdl_wait();

@@ -414,7 +414,7 @@ static int launch_ssd(const SsdParams& p, int chunks, int runs, cudaStream_t str
 // VEC channels a thread at a time; the gated row waits in shared memory for its root mean square
 template <typename TO, int VEC>
 __global__ void __launch_bounds__(512)
-gated_group_norm_kernel(const float* __restrict__ y, const float* __restrict__ gate, int ldg, int off_g, const float* __restrict__ gain, float eps,
+gated_group_norm_kernel(const float* y, const float* gate, int ldg, int off_g, const float* __restrict__ gain, float eps,
                         int groups, TO* __restrict__ out, int n) {
   extern __shared__ __align__(16) float gg_v[];          // [n / groups]
   __shared__ float red[33];

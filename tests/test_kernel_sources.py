@@ -1,0 +1,36 @@
+"""What every kernel source has to keep, read from the sources: no GPU and no compiler needed, and none could show it (a load that the compiler moves in front of a wait gives
+the right number on most days)."""
+
+import glob
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "sllm_b200", "csrc")
+SOURCES = sorted(os.path.basename(f) for f in glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh")))
+
+# What no kernel of a step writes: matrices, gains, biases, tables, and constants of a layer.
+CONSTANTS = set("W w table pair_table bias gain gain_a gain_b q_gain k_gain post_gain pre_gain ga gb conv_w inv_freq correction sink rel q_mul mix share into vec".split())
+# What a kernel only writes.
+RESULTS = set("out out_h out_hs out_a out_b q_out h dst C idx wts dense place tile_expert row_token k_cache v_cache pk_cache pv_cache cache partial rinv".split())
+# Blocks in shared memory (chunked.cuh, delta_chunks.cu), and zero_rows' table, which its owner writes once.
+ELSEWHERE = {("chunked.cuh", n) for n in ("A", "B", "dst")} | {("delta_chunks.cu", n) for n in ("m", "v", "lt", "col", "A0", "A1", "B")} | {("elementwise.cu", "long long rows")}
+
+
+def code_of(name):
+    text = open(os.path.join(CSRC, name)).read()
+    return re.sub(r"//[^\n]*", "", re.sub(r"/\*.*?\*/", "", text, flags=re.S))
+
+
+@pytest.mark.parametrize("name", SOURCES)
+def test_what_an_earlier_kernel_writes_is_loaded_behind_the_wait(name):
+    """A kernel is set up while the one before it runs, and waits for it in `pdl_wait()`.  ``const __restrict__`` says that nobody writes there while the kernel runs, so the compiler may
+    move the load in front of the wait: a pointer to what the step itself produces has no such qualifier."""
+    wrong = []
+    for const, kind, pointer in re.findall(r"(const\s+)?((?:long\s+)?[\w:]+)\s*\*\s*__restrict__\s+(\w+)", code_of(name)):
+        if (name, pointer) in ELSEWHERE or (name, f"{kind} {pointer}") in ELSEWHERE:
+            continue
+        if pointer not in (CONSTANTS if const else RESULTS):
+            wrong.append(pointer)
+    assert not wrong, f"{name}: __restrict__ on {wrong}"
