@@ -123,6 +123,24 @@ void set_error(const char* msg);   // remembers the text for sllm_last_error()
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// What an earlier kernel of the step wrote, loaded where the code says so: behind the wait, and with the loads before and after it in flight (a plain load may be moved down to its first
+// use).  `_l2`: past L1, and in order with the kernel's own stores.
+__device__ __forceinline__ float load_now(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float load_now_l2(const float* p) {
+  float v;
+  asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 load_now_l2(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+  return v;
+}
+
 bool pdl_enabled();
 int num_sms();           // streaming multiprocessors of the current device (asked once per device)
 

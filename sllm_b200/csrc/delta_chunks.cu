@@ -180,8 +180,8 @@ __global__ void __launch_bounds__(DC_THREADS, 2) gated_delta_prep_kernel(const D
         const int t = 8 * warp + r + u, i = lane + 32 * m;
         const bool ok = t < n && i < p.dk;
         const float* src = p.proj + (size_t)(t0 + t) * p.ld + kh * p.dk + i;
-        k[u][m] = ok ? __ldg(src + p.off_k) : 0.f;
-        q[u][m] = ok ? __ldg(src + p.off_q) : 0.f;
+        k[u][m] = ok ? load_now(src + p.off_k) : 0.f;
+        q[u][m] = ok ? load_now(src + p.off_q) : 0.f;
       }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(DC_THREADS, 2) gated_delta_prep_kernel(const D
   if (tid < DV) {
     const float* v = p.proj + (size_t)t0 * p.ld + p.off_v + h * p.dv + tid;
 #pragma unroll 16
-    for (int t = 0; t < RC; ++t) qs[t * LV + tid] = t < n && tid < p.dv ? beta[t] * __ldg(v + (size_t)t * p.ld) : 0.f;
+    for (int t = 0; t < RC; ++t) qs[t * LV + tid] = t < n && tid < p.dv ? beta[t] * load_now(v + (size_t)t * p.ld) : 0.f;
   } else if (tid < DV + DK) {
     float f = 1.f;
     for (int run = 0; run < 4; ++run) {
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(DC_THREADS, 2) general_delta_prep_kernel(const
 #pragma unroll
       for (int m = 0; m < 2; ++m) {
         const int t = 8 * warp + u, i = lane + 32 * m;
-        k[u][m] = t < n && i < p.dk ? __ldg(p.proj + (size_t)(t0 + t) * p.ld + p.off_k + h * p.dk + i) : 0.f;
+        k[u][m] = t < n && i < p.dk ? load_now(p.proj + (size_t)(t0 + t) * p.ld + p.off_k + h * p.dk + i) : 0.f;
       }
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
@@ -336,10 +336,10 @@ __global__ void __launch_bounds__(DC_THREADS, 2) general_delta_prep_kernel(const
     for (int u = 0; u < 16; ++u) {
       const int t = 16 * run + u;
       const bool ok = in && t < n;
-      d[u] = ok ? __ldg(p.decay + (size_t)(t0 + t) * p.H * p.dk + h * p.dk + i) : 0.f;
-      r[u] = ok ? __ldg(row + (size_t)t * p.ld + p.off_q) : 0.f;
-      k[u] = ok ? __ldg(row + (size_t)t * p.ld + p.off_k) : 0.f;
-      a[u] = ok ? __ldg(row + (size_t)t * p.ld + p.off_a) : 0.f;
+      d[u] = ok ? load_now(p.decay + (size_t)(t0 + t) * p.H * p.dk + h * p.dk + i) : 0.f;
+      r[u] = ok ? load_now(row + (size_t)t * p.ld + p.off_q) : 0.f;
+      k[u] = ok ? load_now(row + (size_t)t * p.ld + p.off_k) : 0.f;
+      a[u] = ok ? load_now(row + (size_t)t * p.ld + p.off_a) : 0.f;
     }
     float f = 1.f;
 #pragma unroll
@@ -492,11 +492,11 @@ __global__ void __launch_bounds__(DC_THREADS) delta_scan_kernel(const DeltaChunk
     const size_t at = (size_t)(first + c) * p.H + h;
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      k[r] = __ldcg(p.keep + at * DK + k0 + r);
+      k[r] = load_now_l2(p.keep + at * DK + k0 + r);
 #pragma unroll
-      for (int q = 0; q < CN; ++q) n[r][q] = MODE == DC_GENERAL ? __ldcg(p.s + (at * DK + k0 + r) * DV + c0 + cl + q) : 0.f;
+      for (int q = 0; q < CN; ++q) n[r][q] = MODE == DC_GENERAL ? load_now_l2(p.s + (at * DK + k0 + r) * DV + c0 + cl + q) : 0.f;
     }
-    x = __ldcg(reinterpret_cast<const float4*>(p.xv + (at * RC + tid / 4) * DV + c0 + tid % 4 * 4));
+    x = load_now_l2(reinterpret_cast<const float4*>(p.xv + (at * RC + tid / 4) * DV + c0 + tid % 4 * 4));
   };
   fetch(0);
   if (AHEAD) bring(0, keep, add, xv);

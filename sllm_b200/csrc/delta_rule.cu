@@ -128,17 +128,17 @@ __global__ void __launch_bounds__(DR_THREADS) delta_rule_kernel(const DeltaParam
           const int i = lane + 32 * m;
           const bool in = tok && i < dk, turned = in && i < p.rot;
           const int j = i < half ? i + half : i - half, a_i = i < half ? i : i - half;
-          k[q][m] = in ? __ldg(row + p.off_k + h * dk + i) : 0.f;
-          r[q][m] = in ? __ldg(row + p.off_r + h * dk + i) : 0.f;
-          kp[q][m] = turned ? __ldg(row + p.off_k + h * dk + j) : 0.f;
-          rp[q][m] = turned ? __ldg(row + p.off_r + h * dk + j) : 0.f;
+          k[q][m] = in ? load_now(row + p.off_k + h * dk + i) : 0.f;
+          r[q][m] = in ? load_now(row + p.off_r + h * dk + i) : 0.f;
+          kp[q][m] = turned ? load_now(row + p.off_k + h * dk + j) : 0.f;
+          rp[q][m] = turned ? load_now(row + p.off_r + h * dk + j) : 0.f;
           cs[q][m] = turned ? __ldg(tab + a_i) : 1.f;
           sn[q][m] = turned ? (i < half ? -__ldg(tab + half + a_i) : __ldg(tab + half + a_i)) : 0.f;
         }
 #pragma unroll
         for (int m = 0; m < VPL; ++m) {
           const int j = c0 + lane + 32 * m;
-          v[q][m] = (tok && lane + 32 * m < COLS && j < dv) ? __ldg(row + p.off_v + h * dv + j) : 0.f;
+          v[q][m] = (tok && lane + 32 * m < COLS && j < dv) ? load_now(row + p.off_v + h * dv + j) : 0.f;
         }
       }
 #pragma unroll
@@ -168,18 +168,18 @@ __global__ void __launch_bounds__(DR_THREADS) delta_rule_kernel(const DeltaParam
         const bool tok = tt < nt;
         const int t = t0 + (tok ? tt : 0);
         const float* row = p.proj + (size_t)t * p.ld;
-        z[q] = __ldg(p.gates + (size_t)t * p.ldg + p.off_dt + h);
+        z[q] = load_now(p.gates + (size_t)t * p.ldg + p.off_dt + h);
 #pragma unroll
         for (int m = 0; m < PER_LANE; ++m) {
           const int i = lane + 32 * m;
           const bool in = tok && i < dk;
-          k[q][m] = in ? __ldg(row + p.off_k + kh * dk + i) : 0.f;
-          r[q][m] = in ? __ldg(row + p.off_r + kh * dk + i) : 0.f;
+          k[q][m] = in ? load_now(row + p.off_k + kh * dk + i) : 0.f;
+          r[q][m] = in ? load_now(row + p.off_r + kh * dk + i) : 0.f;
         }
 #pragma unroll
         for (int m = 0; m < VPL; ++m) {
           const int j = c0 + lane + 32 * m;
-          v[q][m] = (tok && lane + 32 * m < COLS && j < dv) ? __ldg(row + p.off_v + h * dv + j) : 0.f;
+          v[q][m] = (tok && lane + 32 * m < COLS && j < dv) ? load_now(row + p.off_v + h * dv + j) : 0.f;
         }
       }
       const float rate = -expf(__ldg(p.a_log + h)), bias = __ldg(p.dt_bias + h);
@@ -215,16 +215,16 @@ __global__ void __launch_bounds__(DR_THREADS) delta_rule_kernel(const DeltaParam
       for (int m = 0; m < PER_LANE; ++m) {
         const int i = lane + 32 * m;
         const bool in = tok && i < dk;
-        k[q][m] = in ? __ldg(row + p.off_k + kh * dk + i) : 0.f;
-        a[q][m] = (in && p.mode == 0) ? __ldg(row + p.off_a + h * dk + i) + __ldg(p.a_bias + h * dk + i) : 0.f;
+        k[q][m] = in ? load_now(row + p.off_k + kh * dk + i) : 0.f;
+        a[q][m] = (in && p.mode == 0) ? load_now(row + p.off_a + h * dk + i) + __ldg(p.a_bias + h * dk + i) : 0.f;
         if (p.mode == 4) a[q][m] = in ? __ldg(p.a_bias + h * dk + i) : 0.f;        // the gate's bias; k holds its logit
-        d[q][m] = (in && (p.mode == 0 || p.mode == 2)) ? __ldg(dec + i) : 0.f;
-        r[q][m] = in ? __ldg(row + p.off_r + kh * dk + i) : 0.f;
+        d[q][m] = (in && (p.mode == 0 || p.mode == 2)) ? load_now(dec + i) : 0.f;
+        r[q][m] = in ? load_now(row + p.off_r + kh * dk + i) : 0.f;
       }
 #pragma unroll
       for (int m = 0; m < VPL; ++m) {
         const int j = c0 + lane + 32 * m;
-        v[q][m] = (tok && lane + 32 * m < COLS && j < dv) ? __ldg(row + p.off_v + h * dv + j) : 0.f;
+        v[q][m] = (tok && lane + 32 * m < COLS && j < dv) ? load_now(row + p.off_v + h * dv + j) : 0.f;
       }
     }
 #pragma unroll
@@ -258,8 +258,8 @@ __global__ void __launch_bounds__(DR_THREADS) delta_rule_kernel(const DeltaParam
         sr = warp_sum(sr);
         const float rinv = p.r_scale / sqrtf(sr + 1e-6f);
         const float* gr = p.gates + (size_t)(t0 + tt) * p.ldg;
-        const float beta = sigmoidf_(__ldg(gr + p.off_b + h));
-        const float x = __ldg(gr + p.off_dt + h) + __ldg(p.dt_bias + h);
+        const float beta = sigmoidf_(load_now(gr + p.off_b + h));
+        const float x = load_now(gr + p.off_dt + h) + __ldg(p.dt_bias + h);
         const float g = expf(-expf(__ldg(p.a_log + h)) * (fmaxf(x, 0.f) + log1pf(expf(-fabsf(x)))));
         vmul = beta;
 #pragma unroll

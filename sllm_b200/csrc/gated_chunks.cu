@@ -101,8 +101,8 @@ __global__ void __launch_bounds__(2 * DK) gated_state_kernel(const GatedChunkPar
     for (int q = 0; q < 8; ++q) {
       const int t = half * (RC / 2) + b + q;
       const bool ok = in && t < n;
-      x[q] = ok ? __ldg(kp + (size_t)t * p.ld) : 0.f;
-      z[q] = MODE == GC_GATED && ok ? __ldg(zp + (size_t)t * p.H * p.dk) : 0.f;
+      x[q] = ok ? load_now(kp + (size_t)t * p.ld) : 0.f;
+      z[q] = MODE == GC_GATED && ok ? load_now(zp + (size_t)t * p.H * p.dk) : 0.f;
     }
 #pragma unroll
     for (int q = 7; q >= 0; --q) {
@@ -247,9 +247,9 @@ __global__ void __launch_bounds__(RC_OUT_THREADS) gated_out_kernel(const GatedCh
           const int t = 16 * warp + b + r, i = lane + 32 * m;
           const bool ok = t < n && i < p.dk;
           const float* src = p.proj + (size_t)(t0 + t) * p.ld + h * p.dk + i;
-          q[r][m] = ok ? __ldg(src + p.off_q) : 0.f;
-          x[r][m] = ok ? __ldg(src + p.off_k) : 0.f;
-          z[r][m] = MODE == GC_GATED && ok ? __ldg(p.z + (size_t)(t0 + t) * p.H * p.dk + h * p.dk + i) : 0.f;
+          q[r][m] = ok ? load_now(src + p.off_q) : 0.f;
+          x[r][m] = ok ? load_now(src + p.off_k) : 0.f;
+          z[r][m] = MODE == GC_GATED && ok ? load_now(p.z + (size_t)(t0 + t) * p.H * p.dk + h * p.dk + i) : 0.f;
         }
 #pragma unroll
       for (int r = 0; r < 4; ++r)

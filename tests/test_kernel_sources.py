@@ -34,3 +34,11 @@ def test_what_an_earlier_kernel_writes_is_loaded_behind_the_wait(name):
         if pointer not in (CONSTANTS if const else RESULTS):
             wrong.append(pointer)
     assert not wrong, f"{name}: __restrict__ on {wrong}"
+
+
+@pytest.mark.parametrize("name", SOURCES)
+def test_read_only_loads_are_of_constants(name):
+    """`__ldg` reads what nobody writes while the kernel runs, and the kernel runs while the one before it still writes (`__ldcg` is no more ordered behind the wait): both are for constants."""
+    arguments = [code_of(name)[m.end():].lstrip() for m in re.finditer(r"__ldc?g\(", code_of(name))]
+    constants = ("p.a_log", "p.skip", "p.a_bias", "p.dt_bias", "p.rel", "rel_h[", "bias", "tab ", "reinterpret_cast<const float4*>(bias", "reinterpret_cast<const float4*>(w ")
+    assert not [a[:60] for a in arguments if not a.startswith(constants)]
