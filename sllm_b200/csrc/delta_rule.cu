@@ -514,15 +514,33 @@ __global__ void delta_out_kernel(const float* o, const float* __restrict__ gain,
     if (q_start[seq + 1] - q_start[seq] > max_len) return;
   }
   const float* x = o + (size_t)row * dv;
+  const float* g = proj + (size_t)t * ld + off_g + h * dv;
+  auto finish = [&](int j, float v, float z, float inv) {
+    const float gate = gate_act == 2 ? 1.0f : (gate_act == 1 ? z * sigmoidf_(z) : sigmoidf_(z));
+    out[(size_t)t * out_ld + out_off + h * dv + j] = from_f32<TO>(v * inv * (gain != nullptr ? gain[h * dv + j] : 1.0f) * gate);
+  };
   float ss = 0.f;
+  constexpr int KEEP = 4;               // heads of up to 128 channels: the row and its gates are loaded before the sum
+  if (dv <= 32 * KEEP) {
+    float v[KEEP], z[KEEP];
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) {
+      v[k] = lane + 32 * k < dv ? x[lane + 32 * k] : 0.f;
+      z[k] = lane + 32 * k < dv && gate_act != 2 ? g[lane + 32 * k] : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) ss = fmaf(v[k], v[k], ss);
+    ss = warp_sum(ss);
+    const float inv = 1.0f / sqrtf(ss / (float)dv + eps);
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k)
+      if (lane + 32 * k < dv) finish(lane + 32 * k, v[k], z[k], inv);
+    return;
+  }
   for (int j = lane; j < dv; j += 32) ss = fmaf(x[j], x[j], ss);
   ss = warp_sum(ss);
   const float inv = 1.0f / sqrtf(ss / (float)dv + eps);
-  const float* g = proj + (size_t)t * ld + off_g + h * dv;
-  for (int j = lane; j < dv; j += 32) {
-    const float gate = gate_act == 2 ? 1.0f : (gate_act == 1 ? g[j] * sigmoidf_(g[j]) : sigmoidf_(g[j]));
-    out[(size_t)t * out_ld + out_off + h * dv + j] = from_f32<TO>(x[j] * inv * (gain != nullptr ? gain[h * dv + j] : 1.0f) * gate);
-  }
+  for (int j = lane; j < dv; j += 32) finish(j, x[j], gate_act != 2 ? g[j] : 0.f, inv);
 }
 
 // the same with a CTA per (t, h): a "head" of many hundred channels (one norm over all of a row's heads together)

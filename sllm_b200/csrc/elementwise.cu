@@ -193,12 +193,17 @@ __global__ void add_rmsnorm_rows_kernel(float* residual, const TD* delta,
     v[k] = i < H ? load4(residual + base + i) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   if (delta != nullptr) {
+    float4 d[VPT];                       // (all loads before the first store, which they are not free to pass)
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+      const int i = (threadIdx.x + k * blockDim.x) * 4;
+      d[k] = i < H ? load4(delta + base + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
 #pragma unroll
     for (int k = 0; k < VPT; ++k) {
       const int i = (threadIdx.x + k * blockDim.x) * 4;
       if (i < H) {
-        const float4 d = load4(delta + base + i);
-        v[k].x += d.x; v[k].y += d.y; v[k].z += d.z; v[k].w += d.w;
+        v[k].x += d[k].x; v[k].y += d[k].y; v[k].z += d[k].z; v[k].w += d[k].w;
         store4(residual + base + i, v[k]);
       }
     }

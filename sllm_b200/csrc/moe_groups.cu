@@ -13,7 +13,7 @@
 
 namespace sllm {
 
-constexpr int MG_TILE = 256, MG_MAX_EXPERTS = 256, MG_THREADS = 1024;
+constexpr int MG_TILE = 256, MG_MAX_EXPERTS = 256, MG_THREADS = 1024, MG_AHEAD = 4 /* choices whose loads are in flight */;
 
 // one block; the order of an expert's rows is whatever the counters give (no result depends on it)
 __global__ void __launch_bounds__(MG_THREADS)
@@ -24,14 +24,20 @@ moe_assign_kernel(const int* idx, int n, int top, int E, int tiles, int* __restr
   for (int e = tid; e < E; e += MG_THREADS) count[e] = 0;
   for (int r = tid; r < tiles * MG_TILE; r += MG_THREADS) row_token[r] = -1;
   __syncthreads();
-  for (int i0 = 0; i0 < n; i0 += MG_THREADS) {       // (whole warps: the lanes of one expert count together)
-    const int i = i0 + tid, e = i < n ? idx[i] : -1;
-    const unsigned peers = __match_any_sync(0xffffffffu, e);
-    const int leader = __ffs(peers) - 1, lane = tid & 31;
-    int base = 0;
-    if (e >= 0 && lane == leader) base = atomicAdd(&count[e], __popc(peers));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (i < n) place[i] = base + __popc(peers & ((1u << lane) - 1));
+  for (int i0 = 0; i0 < n; i0 += MG_AHEAD * MG_THREADS) {       // (whole warps: the lanes of one expert count together)
+    int chosen[MG_AHEAD];
+#pragma unroll
+    for (int u = 0; u < MG_AHEAD; ++u) chosen[u] = i0 + u * MG_THREADS + tid < n ? idx[i0 + u * MG_THREADS + tid] : -1;
+#pragma unroll
+    for (int u = 0; u < MG_AHEAD; ++u) {
+      const int i = i0 + u * MG_THREADS + tid, e = chosen[u];
+      const unsigned peers = __match_any_sync(0xffffffffu, e);
+      const int leader = __ffs(peers) - 1, lane = tid & 31;
+      int base = 0;
+      if (e >= 0 && lane == leader) base = atomicAdd(&count[e], __popc(peers));
+      base = __shfl_sync(0xffffffffu, base, leader);
+      if (i < n) place[i] = base + __popc(peers & ((1u << lane) - 1));
+    }
   }
   __syncthreads();
   if (tid == 0) {
@@ -49,10 +55,21 @@ moe_assign_kernel(const int* idx, int n, int top, int E, int tiles, int* __restr
       for (e = 0; t >= start[e + 1]; ++e) {}
     tile_expert[t] = e;
   }
-  for (int i = tid; i < n; i += MG_THREADS) {        // (a thread's own entries)
-    const int r = start[idx[i]] * MG_TILE + place[i];
-    place[i] = r;
-    row_token[r] = i / top;
+  for (int i0 = tid; i0 < n; i0 += MG_AHEAD * MG_THREADS) {        // (a thread's own entries)
+    int e[MG_AHEAD], at[MG_AHEAD];
+#pragma unroll
+    for (int u = 0; u < MG_AHEAD; ++u) {
+      const int i = i0 + u * MG_THREADS;
+      e[u] = i < n ? idx[i] : 0;
+      at[u] = i < n ? place[i] : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < MG_AHEAD; ++u) {
+      const int i = i0 + u * MG_THREADS, r = start[e[u]] * MG_TILE + at[u];
+      if (i >= n) break;
+      place[i] = r;
+      row_token[r] = i / top;
+    }
   }
 }
 
@@ -64,8 +81,15 @@ moe_gather_kernel(const uint4* x, const int* row_token, uint4* __restrict__ out,
   if (row >= rows) return;
   const int t = row_token[row];
   if (t < 0) return;
-#pragma unroll 4
-  for (int c = lane; c < pieces; c += 32) out[(size_t)row * pieces + c] = x[(size_t)t * pieces + c];
+  for (int c0 = lane; c0 < pieces; c0 += 256) {
+    uint4 v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (c0 + 32 * k < pieces) v[k] = x[(size_t)t * pieces + c0 + 32 * k];
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (c0 + 32 * k < pieces) out[(size_t)row * pieces + c0 + 32 * k] = v[k];
+  }
 }
 
 // a block per token, four columns a thread
