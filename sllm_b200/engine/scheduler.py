@@ -161,24 +161,26 @@ class Scheduler:
                 budget -= n
         # admission (pump): skip what does not fit, keep its place
         skipped, admitted = [], []
-        while self.waiting and len(self.running) < self.max_num_seqs and budget > 0:
-            r = self.waiting.popleft()
-            n = min(r.pending, self.chunk_size, budget)
-            if self.policy == "on_demand" and self.cache.groups:
-                # start with the pages there are; the rest of the prompt follows as they come free
-                n = min(n, self.cache.token_room())
-            total = len(r.prompt) + r.params.max_new if self.policy == "reserve" else r.num_computed + n
-            if n <= 0 or not self.cache.can_reserve(r.req_id, total):
-                skipped.append(r)
-                continue
-            admitted.append(self.cache.add_request(r.req_id, zero=False))
-            self.cache.reserve(r.req_id, total)
-            r.status = "running"
-            self.running.append(r)
-            plan.append(Planned(r, r.num_computed, n, r.num_computed + n == r.num_tokens))
-            planned_ids.add(r.req_id)
-            budget -= n
-        self.cache.zero_rows(admitted)
+        try:
+            while self.waiting and len(self.running) < self.max_num_seqs and budget > 0:
+                r = self.waiting.popleft()
+                n = min(r.pending, self.chunk_size, budget)
+                if self.policy == "on_demand" and self.cache.groups:
+                    # start with the pages there are; the rest of the prompt follows as they come free
+                    n = min(n, self.cache.token_room())
+                total = len(r.prompt) + r.params.max_new if self.policy == "reserve" else r.num_computed + n
+                if n <= 0 or not self.cache.can_reserve(r.req_id, total):
+                    skipped.append(r)
+                    continue
+                admitted.append(self.cache.add_request(r.req_id, zero=False))
+                self.cache.reserve(r.req_id, total)
+                r.status = "running"
+                self.running.append(r)
+                plan.append(Planned(r, r.num_computed, n, r.num_computed + n == r.num_tokens))
+                planned_ids.add(r.req_id)
+                budget -= n
+        finally:
+            self.cache.zero_rows(admitted)          # (also of those admitted before one that is refused: they are running)
         self.waiting.extendleft(reversed(skipped))
         self._trim_to_row_tiles(plan)
         return plan

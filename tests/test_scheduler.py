@@ -183,3 +183,18 @@ def test_the_last_portion_of_a_prompt_that_is_trimmed_samples_a_step_later():
     s.add("a", [0] * 35, SamplingParams(max_new=1))      # 35 = 2 tiles + 3
     log = run(s)
     assert [e[0][1:] for e in log] == [(0, 32, False), (32, 3, True)]
+
+
+def test_rows_of_the_admitted_are_zeroed_though_a_later_request_is_refused():
+    """A request whose id is live already (a program that also steps the engine itself) is refused; the one admitted before it runs on, from rows of zeros."""
+    import torch
+    s, cache = make()
+    table = torch.ones(cache.max_requests + 1, 3)
+    cache.register_slot_table("seen", table)
+    cache.add_request("b", zero=False)
+    s.add("a", [1, 2, 3], SamplingParams(max_new=2))
+    s.add("b", [1, 2, 3], SamplingParams(max_new=2))
+    with pytest.raises(ValueError):
+        s.schedule()
+    assert [r.req_id for r in s.running] == ["a"]
+    assert not table[cache.requests["a"].slot].any() and table[cache.requests["b"].slot].all()
