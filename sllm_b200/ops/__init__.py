@@ -1828,7 +1828,20 @@ def linear_scaled_supports(x: torch.Tensor, w: torch.Tensor) -> bool:
             and pair_supports(M, w.shape[0], K))
 
 
+LINEAR_NARROW_MAX_ROWS = TCGEN05_MIN_ROWS
 LINEAR_NARROW_MAX_COLS = 15    # a router's logits: fewer columns than a tile of any other kernel (figures in linear_stream.cu)
+
+
+def _narrow_takes(x, w, bias, out_dtype) -> bool:
+    """Whether `linear` has its own kernel for a product of so few columns.  What that kernel does not read as it lies (another type, operands that do not fit one another, a bias that is
+    broadcast) stays with the library's product, which takes it or refuses it."""
+    if w.dim() != 2:
+        return False
+    (M, K), N = x.shape, w.shape[0]
+    return (1 <= M <= LINEAR_NARROW_MAX_ROWS and 1 <= N <= LINEAR_NARROW_MAX_COLS and K >= 8 and K % 8 == 0 and w.shape[1] == K
+            and x.dtype == torch.bfloat16 and out_dtype in (torch.float32, torch.bfloat16) and w.device == x.device
+            and (bias is None or (bias.dtype == torch.float32 and tuple(bias.shape) == (N,) and bias.device == x.device))
+            and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
 def _stream_splits(N: int, K: int) -> int:
@@ -1877,8 +1890,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias, out_dtype: torch.dtype, allow
         if allow_partials and out_dtype == torch.float32 and pair_splits(M, N, K) > 1:
             return gemm_pair(x, w, bias, out_dtype, splits=pair_splits(M, N, K))
         return gemm_pair(x, w, bias, out_dtype)
-    if 1 <= M <= TCGEN05_MIN_ROWS and 1 <= N <= LINEAR_NARROW_MAX_COLS and K >= 8 and K % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 \
-            and out_dtype in (torch.float32, torch.bfloat16) and (bias is None or bias.dtype == torch.float32):
+    if _narrow_takes(x, w, bias, out_dtype):
         out = torch.empty((M, N), dtype=out_dtype, device=x.device)
         call("sllm_linear_narrow", _p(x), _p(w), _p(bias), _p(out), _dtc(out_dtype), M, N, K, _stream())
         return out

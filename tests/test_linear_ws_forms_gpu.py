@@ -186,3 +186,26 @@ def test_few_columns(M, N, K):
     plain = y - b
     assert bool(((ops.linear(x, w, None, torch.bfloat16) - plain).abs() <= bound + 2.0 ** -8 * plain.abs()).all())
     assert ops.launches["library"] == before
+
+
+def test_few_columns_of_what_the_kernel_does_not_read():
+    """Few columns of another type or off a 16-byte border, a bias that is broadcast or of another type: the library's product takes them, as it takes any; operands that do not fit one another and
+    a bias of another length are refused."""
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    g = torch.Generator(device=dev).manual_seed(3)
+    for dtype in (torch.float16, torch.float64):
+        x, w = torch.randn(5, 64, device=dev, generator=g, dtype=torch.float32).to(dtype), torch.randn(9, 64, device=dev, generator=g, dtype=torch.float32).to(dtype)
+        want = x.double() @ w.double().T
+        assert bool(((ops.linear(x, w, None, dtype) - want).abs() <= torch.finfo(dtype).eps * want.abs() + 65 * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)).all())
+    x, w = torch.randn(5, 64, device=dev, generator=g).bfloat16(), torch.randn(9, 64, device=dev, generator=g).bfloat16()
+    b = torch.randn(9, device=dev, generator=g)
+    y, bound = x.double() @ w.double().T, 66 * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T) + 2.0 ** -22
+    shifted = torch.empty(5 * 64 + 1, device=dev, dtype=torch.bfloat16)[1:].view(5, 64).copy_(x)
+    for xs, bias in ((shifted, b), (x, b[:1]), (x, b.bfloat16()), (x, b.double())):
+        before = ops.launches["library"]
+        assert bool(((ops.linear(xs, w, bias, torch.float32) - (y + bias.double())).abs() <= bound + 2.0 ** -22 * (y.abs() + bias.abs())).all())
+        assert ops.launches["library"] == before + 1
+    for xs, ws, bias in ((x, w[:, :56].contiguous(), None), (x[:, :56].contiguous(), w, None), (x, w, b[:8].contiguous()), (x, w.reshape(9, 8, 8), None)):
+        with pytest.raises((RuntimeError, ops.KernelError)):
+            ops.linear(xs, ws, bias, torch.float32)
