@@ -434,13 +434,16 @@ SLLM_EXPORT int sllm_linear_stream_silu_scaled(const void* x, const void* W, voi
 }
 
 // ---------------------------------------------------------------------------------------------
-// Products of fewer than 16 columns (a router's logits): out[M, N] = x[M, K] W[N, K]^T (+ bias).  A CTA a token, a warp a column in turn, 16 bytes a load; the first
-// rows of W (K up to LN_AHEAD * 256) lie in registers before the wait on the step's earlier kernels.  Bound by latency: one round trip for the token's row, a sum over the
-// warp.  (16 tokens, 8 columns, K = 2,048: 3.1 us in a graph of such products; 48 tokens, 9 columns 4.2 against 18.3 for the library's product, which took these before.)
+// Products of fewer than 16 columns (a router's logits): out[M, N] = x[M, K] W[N, K]^T (+ bias).  A warp a (token, column), 16 bytes a load, the first LN_AHEAD * 256 of a column's
+// weights in registers before the wait on the step's earlier kernels.  Bound by latency: one round trip for every LN_AHEAD * 256 columns of K (weights and activations together behind
+// the first), a sum over the warp; and for few tokens by what one SM draws from L2, so a CTA there has few columns
+// (ln_columns).  (In a graph of such products, us, with eight columns a CTA in two rounds and a loop behind K = 4,096 / so / the library's: 16 tokens, 8 columns, K = 2,048 3.1 / 1.7 / 4.6;
+// 48 tokens, 9 columns, K = 2,048 4.3 / 2.0 / 17.9; one token, 9 columns, K = 4,096 6.1 / 1.8 / 3.8, 15 columns, K = 11,008 16.0 / 3.9 / 4.1; 128 tokens, 15 columns, K = 8,192 15.7 / 6.6 /
+// 18.8, 10 columns 13.5 / 4.5 / 7.4.)
 // ---------------------------------------------------------------------------------------------
 namespace sllm {
 
-constexpr int LN_MAX_N = 15, LN_WARPS = 8, LN_AHEAD = 16;
+constexpr int LN_MAX_N = 15, LN_COLS = 4 /* of a CTA, at most */, LN_AHEAD = 16;
 
 __device__ __forceinline__ float ln_dot(const uint4& a, const uint4& b, float sum) {
   const __nv_bfloat162 *p = reinterpret_cast<const __nv_bfloat162*>(&a), *q = reinterpret_cast<const __nv_bfloat162*>(&b);
@@ -454,33 +457,37 @@ __device__ __forceinline__ float ln_dot(const uint4& a, const uint4& b, float su
 }
 
 template <typename OUT>
-__global__ void __launch_bounds__(LN_WARPS * 32)
+__global__ void __launch_bounds__(LN_COLS * 32)
 linear_narrow_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ W, const float* __restrict__ bias, OUT* __restrict__ out, int N, int K) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, n = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
   pdl_launch_dependents();
-  uint4 w[LN_AHEAD];
-  auto load_w = [&](int n) {
+  uint4 w[LN_AHEAD], v[LN_AHEAD];
+  auto load = [&](uint4 (&a)[LN_AHEAD], const __nv_bfloat16* row, int k0) {
 #pragma unroll
     for (int i = 0; i < LN_AHEAD; ++i) {
-      const int k = (lane + 32 * i) * 8;
-      w[i] = n < N && k < K ? *reinterpret_cast<const uint4*>(W + (size_t)n * K + k) : make_uint4(0u, 0u, 0u, 0u);
+      const int k = k0 + (lane + 32 * i) * 8;
+      a[i] = n < N && k < K ? *reinterpret_cast<const uint4*>(row + k) : make_uint4(0u, 0u, 0u, 0u);
     }
   };
-  load_w(warp);
+  load(w, W + (size_t)n * K, 0);
   pdl_wait();
-  const __nv_bfloat16* row = x + (size_t)blockIdx.x * K;
-  for (int n = warp; n < N; n += LN_WARPS) {
-    float sum = 0.f;
+  float sum = 0.f;
+  for (int k0 = 0; k0 < K; k0 += LN_AHEAD * 256) {
+    if (k0 > 0) load(w, W + (size_t)n * K, k0);
+    load(v, x + (size_t)blockIdx.x * K, k0);
 #pragma unroll
-    for (int i = 0; i < LN_AHEAD; ++i) {
-      const int k = (lane + 32 * i) * 8;
-      if (k < K) sum = ln_dot(*reinterpret_cast<const uint4*>(row + k), w[i], sum);
-    }
-    for (int k = (lane + 32 * LN_AHEAD) * 8; k < K; k += 256) sum = ln_dot(*reinterpret_cast<const uint4*>(row + k), *reinterpret_cast<const uint4*>(W + (size_t)n * K + k), sum);
-    if (n + LN_WARPS < N) load_w(n + LN_WARPS);
-    sum = warp_sum(sum);
-    if (lane == 0) out[(size_t)blockIdx.x * N + n] = from_f32<OUT>(sum + (bias ? bias[n] : 0.f));
+    for (int i = 0; i < LN_AHEAD; ++i)
+      if (k0 + (lane + 32 * i) * 8 < K) sum = ln_dot(v[i], w[i], sum);
   }
+  sum = warp_sum(sum);
+  if (lane == 0 && n < N) out[(size_t)blockIdx.x * N + n] = from_f32<OUT>(sum + (bias ? bias[n] : 0.f));
+}
+
+// Columns of a CTA: as few as make two CTAs an SM, at most (each reads the token's row again).
+static int ln_columns(int M, int N) {
+  int cols = 1;
+  while (cols < LN_COLS && (long long)M * ((N + cols - 1) / cols) > 2 * num_sms()) ++cols;
+  return cols < N ? cols : N;
 }
 
 }  // namespace sllm
@@ -488,10 +495,12 @@ linear_narrow_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ W
 SLLM_EXPORT int sllm_linear_narrow(const void* x, const void* W, const float* bias, void* out, int out_dtype, int M, int N, int K, cudaStream_t stream) {
   SLLM_REQUIRE(M >= 1 && N >= 1 && N <= LN_MAX_N && K >= 8 && K % 8 == 0, "linear_narrow: sizes M=%d N=%d K=%d (needs N<=15, K%%8==0)", M, N, K);
   SLLM_REQUIRE(((uintptr_t)x & 15) == 0 && ((uintptr_t)W & 15) == 0, "linear_narrow: operands must be 16-byte aligned");
+  const int cols = ln_columns(M, N);
+  const dim3 grid(M, (N + cols - 1) / cols);
   if (out_dtype == SLLM_BF16)
-    launch_kernel(linear_narrow_kernel<__nv_bfloat16>, M, LN_WARPS * 32, 0, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)W, bias, (__nv_bfloat16*)out, N, K);
+    launch_kernel(linear_narrow_kernel<__nv_bfloat16>, grid, cols * 32, 0, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)W, bias, (__nv_bfloat16*)out, N, K);
   else
-    launch_kernel(linear_narrow_kernel<float>, M, LN_WARPS * 32, 0, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)W, bias, (float*)out, N, K);
+    launch_kernel(linear_narrow_kernel<float>, grid, cols * 32, 0, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)W, bias, (float*)out, N, K);
   return launch_status("linear_narrow");
 }
 
