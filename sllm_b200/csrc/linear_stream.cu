@@ -325,14 +325,33 @@ linear_resident_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__
   ls_finish<NT, EPI, OUT>(acc, n0, g, t4, bias, out, M, N);
 }
 
-// Where the activations fit; with four token tiles the products of a warp (mma.sync, some 30 cycles each) are what takes the time, so there only where the form above is
-// worse off still: a norm owed, whose partial sums it adds token after token behind the stream, or too few rows for its CTAs.  (17 tokens, us, this / the form above: 9,728 x 896
-// with the activation 10.4 / 9.6, with a norm owed 11.0 / 13.4; 4,096 x 1,024 7.2 / 10.3, 6,144 x 1,536 10.3 / 15.3, 8,192 x 1,024 9.8 / 10.6, 32 tokens 11.0 / 10.6.)
-constexpr int LR_MANY_TOKENS_ROWS = 7168;
-static bool ls_resident(int M, int N, int K, int splits, bool scaled) {
-  const int nt = M <= 8 ? 1 : (M <= 16 ? 2 : 4);
-  return splits == 1 && M <= 32 && K * 16 * nt <= LR_X_MAX && (nt < 4 || scaled || N <= LR_MANY_TOKENS_ROWS);
+// Where the activations fit and this form is the faster one (the bits are the same).  With four token tiles the products of a warp (mma.sync, some 30 cycles each) are what takes the
+// time, so there only where the form above is worse off still: a norm owed, whose partial sums it adds token after token behind the stream, or too few rows for its CTAs.  Else by
+// how well the CTAs fill the SMs, three an SM (registers) or what the activations leave room for, against the form above with two of 128 rows: as long as all are on the SMs at
+// once the shorter CTAs win, in later waves only where they fill them better.  A CTA has 64 KB of loads in flight, which lie in L1: where the activations of an SM's CTAs leave less than
+// 92 KB of it, two CTAs an SM at most; less than 60 KB, one on every other SM.  (Us, the form above / this one.  8 tokens: 1,024 x 2,048 16.4 / 7.1, 9,728 x 1,536 13.3 / 9.1, 18,944
+// x 1,536 1.25 times as fast, 28,416 rows 1.08, 30,720 (1.1 waves) 0.94, 32,000 18.7 / 20.0, 36,864 0.88, 40,960 (1.4 waves against 1.1 of the other) 1.26, 65,536 1.0, 151,936 x 1,536
+// 81.9 / 73.9; K = 256 1,024 rows 1.98 / 1.76, 9,728 2.62 / 2.63, 32,000 4.4 / 5.2.  K = 4,096 9,728 rows 34.4 / 26.9, 24,576 0.98, 32,000 48.3 / 65.1; K = 6,400 4,096 rows 51.2 /
+// 39.2, 8,192 52.6 / 55.5, 9,472 53.1 / 64.9; K = 4,864 9,472 rows 40.7 / 23.4, K = 4,608 38.9 / 50.9.
+// 16 tokens: 9,728 x 2,048 18.1 / 15.2, 32,000 x 2,048 25.7 / 35.6, 9,728 x 3,200 27.7 / 41.2.  17 tokens: 9,728 x 896 with the activation 9.6 / 10.4, with a norm owed 13.4 / 11.0;
+// 4,096 x 1,024 10.3 / 7.2, 6,144 x 1,536 15.3 / 10.3, 8,192 x 1,024 10.6 / 9.8, 32 tokens 10.6 / 11.0.)
+constexpr int LR_MANY_TOKENS_ROWS = 7168, LR_CTAS = 3;
+static bool ls_resident(int M, int N, int K, int splits, bool gated, bool scaled) {
+  const int nt = M <= 8 ? 1 : (M <= 16 ? 2 : 4), bytes = K * 16 * nt;
+  if (splits != 1 || M > 32 || bytes > LR_X_MAX || (nt == 4 && !scaled && N > LR_MANY_TOKENS_ROWS)) return false;
+  if ((K <= 256 && scaled) || (K < 512 && nt == 4 && gated && !scaled)) return false;       // (two or three chunks: what comes before the stream is all of it)
+  const int sms = num_sms(), ctas = (N + LR_WARPS * 16 - 1) / (LR_WARPS * 16);
+  const int a_cta = bytes + 1152, fit = 227 * 1024 / a_cta, per_sm = fit < LR_CTAS ? fit : LR_CTAS;
+  if (per_sm * a_cta > 196 * 1024) return ctas <= sms / 2;
+  if (ctas <= sms) return true;
+  if (K <= 256 || (K < 512 && nt == 1 && scaled)) return false;
+  if (K < 512 || (nt < 4 && per_sm * a_cta > 164 * 1024) || (nt == 1 && scaled && K < 1536) || (nt == 2 && K < 896)) return ctas <= 2 * sms;
+  const long long places = (long long)per_sm * sms, above = (N + LS_ROWS - 1) / LS_ROWS, above_places = 2LL * sms;
+  const long long waves = (ctas + places - 1) / places, above_waves = (above + above_places - 1) / above_places;
+  return ctas * above_waves * above_places > above * waves * places;
 }
+// 1: the form with resident activations, 0: the other (epilogue as in sllm_linear_stream; scaled: sllm_linear_stream_silu_scaled)
+SLLM_EXPORT int sllm_linear_stream_resident(int M, int N, int K, int epilogue, int scaled) { return ls_resident(M, N, K, 1, epilogue != 0, scaled != 0) ? 1 : 0; }
 
 template <int NT, int EPI, typename OUT, bool SCALED>
 static int launch_resident(const __nv_bfloat16* x, const __nv_bfloat16* W, const float* bias, void* out, int M, int N, int K, cudaStream_t stream, const LsScale& scale) {
@@ -352,7 +371,7 @@ template <int NT, int EPI, typename OUT, bool SCALED = false>
 static int launch_ls(const __nv_bfloat16* x, const __nv_bfloat16* W, const float* bias, void* out, float* partial,
                      int M, int N, int K, int splits, cudaStream_t stream, const LsScale& scale = LsScale{}) {
   if constexpr (NT <= 4) {
-    if (ls_resident(M, N, K, splits, SCALED)) return launch_resident<NT, EPI, OUT, SCALED>(x, W, bias, out, M, N, K, stream, scale);
+    if (ls_resident(M, N, K, splits, EPI != EPI_STORE, SCALED)) return launch_resident<NT, EPI, OUT, SCALED>(x, W, bias, out, M, N, K, stream, scale);
   }
   constexpr size_t smem = sizeof(__nv_bfloat16) * 2 * 8 * NT * LS_XSTRIDE + (SCALED ? sizeof(float) * 8 * NT * LS_SSQ_MAX : 0);
   static bool configured = false;

@@ -121,6 +121,7 @@ def _declare(L):
         "sllm_linear_ws_rope": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int,
                                 c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p,
                                 c_void_p, c_int, c_float, c_int, c_void_p],
+        "sllm_linear_stream_resident": [c_int, c_int, c_int, c_int, c_int],
         "sllm_linear_narrow": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
         "sllm_linear_stream_supports": [c_int, c_int, c_int],
         "sllm_linear_stream_splits": [c_int, c_int],

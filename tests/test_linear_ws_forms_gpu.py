@@ -209,3 +209,20 @@ def test_few_columns_of_what_the_kernel_does_not_read():
     for xs, ws, bias in ((x, w[:, :56].contiguous(), None), (x[:, :56].contiguous(), w, None), (x, w, b[:8].contiguous()), (x, w.reshape(9, 8, 8), None)):
         with pytest.raises((RuntimeError, ops.KernelError)):
             ops.linear(xs, ws, bias, torch.float32)
+
+
+def test_which_streams_keep_their_activations():
+    """The line between the two streaming kernels (whose sums have the same order and so the same bits), on both sides of each of its borders, for 148 SMs."""
+    import sllm_b200.ops as ops
+    cuda_or_skip()
+    if ops.num_sms() != 148:
+        pytest.skip("the sizes are those of 148 SMs")
+    form = ops.lib().sllm_linear_stream_resident
+    store, silu = 0, 1
+    for M, N, K, epilogue, scaled, want in [
+            (1, 9472, 256, store, 0, 1), (1, 9488, 256, store, 0, 0), (8, 1024, 256, silu, 1, 0), (32, 1024, 256, silu, 0, 0), (32, 1024, 384, silu, 0, 0), (32, 1024, 512, silu, 0, 1),
+            (32, 7168, 896, store, 0, 1), (32, 7184, 896, store, 0, 0), (32, 7184, 896, silu, 1, 1), (8, 18944, 384, store, 0, 1), (8, 18960, 384, store, 0, 0),
+            (8, 28416, 1536, store, 0, 1), (8, 32000, 1536, store, 0, 0), (8, 40960, 1536, store, 0, 1), (8, 151936, 1536, store, 0, 1), (8, 28416, 896, silu, 1, 0), (8, 18944, 896, silu, 1, 1),
+            (16, 18944, 2048, store, 0, 1), (16, 18960, 2048, store, 0, 0), (16, 32000, 2048, store, 0, 0), (16, 4736, 3200, store, 0, 1), (16, 4752, 3200, store, 0, 0), (16, 64, 3328, store, 0, 0),
+            (8, 4736, 6400, store, 0, 1), (8, 4752, 6400, store, 0, 0), (8, 9472, 4864, store, 0, 1), (8, 4752, 4608, store, 0, 0), (8, 64, 6528, store, 0, 0), (33, 64, 128, store, 0, 0)]:
+        assert form(M, N, K, epilogue, scaled) == want, (M, N, K, epilogue, scaled)
