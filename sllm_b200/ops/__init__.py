@@ -1573,11 +1573,14 @@ LINEAR_TC_UNSPLIT = 12 << 20
 
 
 @functools.lru_cache(maxsize=4096)
-def _tc_unsplit_pays(M: int, N: int, K: int) -> bool:
-    """Whether a product of 17 to 32 tokens that cannot leave partial sums (or applies gate|up's activation) is better off here than with the streaming kernel although its matrix is
-    under `LINEAR_TC_LARGE`: there mma.sync's rate bounds four token tiles.  (32 tokens, us, streaming / this one: store 9,728 x 896 9.4 / 9.0, 12,288 x 1,536 16.3 / 12.7, 10,240 x 2,048
-    21.0 / 15.0; gate|up 17,920 x 1,536 20.2 / 16.0, with a norm owed 19.9 and here a norm kernel of 1.4 before it; 11,264 x 2,048 24.5 / 17.6 and 26.5.)"""
-    return STREAM_MAX_ROWS >= M >= LINEAR_TC_LARGE_FROM_ROWS and N * K >= LINEAR_TC_UNSPLIT and linear_tc_takes(M, N, K)
+def _tc_unsplit_pays(M: int, N: int, K: int, gated: bool = False) -> bool:
+    """Whether a product of 17 to 32 tokens that cannot leave partial sums (or, ``gated``, applies gate|up's activation) is better off here than with the streaming kernel although its matrix is
+    under `LINEAR_TC_LARGE`: there mma.sync's rate bounds four token tiles.  Only up to one 128-row tile an SM, and from a K on that is worth a tile's start: (32 tokens, us, streaming /
+    this one: store 14,336 x 896 10.8 / 10.0, 18,944 x 1,024 14.7 / 12.0, 10,240 x 2,048 21.0 / 15.0, 1,024 x 12,288 116.8 / 62.6, but 16,384 x 768 9.2 / 9.7, and with a second wave
+    19,072 x 1,024 15.6 / 16.7, 32,000 x 512 9.5 / 11.7, 98,304 x 128 10.8 / 14.1; gate|up 12,288 x 1,024 13.4 / 13.0, 17,920 x 1,536 20.2 / 16.4, 2,048 x 6,144 58.4 / 36.0, but
+    14,336 x 896 11.7 / 12.4, 20,480 x 1,536 22.1 / 24.1.)"""
+    return (STREAM_MAX_ROWS >= M >= LINEAR_TC_LARGE_FROM_ROWS and N * K >= LINEAR_TC_UNSPLIT and K >= (1024 if gated else 896) and -(-N // 128) <= num_sms()
+            and linear_tc_takes(M, N, K))
 
 
 @functools.lru_cache(maxsize=4096)
@@ -1984,10 +1987,8 @@ def linear_silu_mul(x: torch.Tensor, w_gate_up: torch.Tensor, interleave: int, o
         N = w_gate_up.shape[0]
         if ws_gated_supports(M, N, K):
             return linear_ws_gated(x, w_gate_up, None, "silu")
-        if stream_supports(M, N, K) and not (N % 16 == 0 and _tc_unsplit_pays(M, N, K)):
-            return linear_stream(x, w_gate_up, None, out_dtype, silu=True)
-        if N % 16 == 0 and _tc_unsplit_pays(M, N, K):
-            return linear_tc(x, w_gate_up, None, out_dtype, silu=True)
+        if stream_supports(M, N, K):
+            return (linear_tc if N % 16 == 0 and _tc_unsplit_pays(M, N, K, True) else linear_stream)(x, w_gate_up, None, out_dtype, silu=True)
         if PAIR_SILU_FROM_ROWS <= M <= TCGEN05_MIN_ROWS and N % 16 == 0 and _PAIR_GEMM != "off" and pair_supports(M, N, K):
             # 64..128 tokens: still bound by reading W once, and the pair kernel's narrow tiles (two accumulators, the
             # epilogue under the next tile) stream it faster than `linear_tc`, whose accumulator is 128 columns wide there

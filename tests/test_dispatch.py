@@ -44,6 +44,18 @@ def test_the_cut_of_a_context_fills_whole_waves(ops_with_sms):
         assert ops.choose_splits(120, 1, 512, 2) == 2 and ops.choose_splits(32, 1, 512, 2) == 4
 
 
+def test_products_of_17_to_32_tokens(ops_with_sms, monkeypatch):
+    """Up to one tile an SM, from 12 Mi elements and from a K on; with a norm owed on the input the rotary epilogue takes short reductions."""
+    ops, sms = ops_with_sms
+    monkeypatch.setattr(ops, "linear_tc_takes", lambda M, N, K: True)
+    pays = ops._tc_unsplit_pays
+    assert [pays(M, 12288, 1024) for M in (16, 17, 32, 33)] == [False, sms >= 96, sms >= 96, False]
+    wide = 128 * sms
+    for N, K, plain, gated in [(6144, 2048, True, True), (6144, 2032, False, False), (wide, 1536, True, True), (wide + 1, 1536, False, False), (wide, 896, wide * 896 >= 12 << 20, False), (wide, 768, False, False)]:
+        assert (pays(24, N, K), pays(24, N, K, True)) == (plain, gated), (N, K)
+    assert ops._ws_rope32_ok(16 * 2 * sms, 1024) and not ops._ws_rope32_ok(16 * 2 * sms + 1, 1024) and not ops._ws_rope32_ok(1152, 1056)
+
+
 def test_tile_shapes_of_a_prompt_portions_products(ops_with_sms):
     ops, sms = ops_with_sms
     pairs = sms // 2
