@@ -1878,7 +1878,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias, out_dtype: torch.dtype, allow
         return linear_ws(x, w, bias, out_dtype)
     if stream_supports(M, N, K):
         splits = _stream_splits(N, K) if (allow_partials and out_dtype == torch.float32) else 1
-        if splits == 1 and _tc_unsplit_pays(M, N, K):
+        if splits == 1 and out_dtype in (torch.float32, torch.bfloat16) and _tc_unsplit_pays(M, N, K):
             return linear_tc(x, w, bias, out_dtype)
         return linear_stream(x, w, bias, out_dtype, splits=splits)
     if allow_partials and out_dtype == torch.float32 and M <= LINEAR_TC_SPLIT_MAX_ROWS and K >= LINEAR_TC_SPLIT_MIN_K \

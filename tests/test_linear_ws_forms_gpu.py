@@ -226,3 +226,39 @@ def test_which_streams_keep_their_activations():
             (16, 18944, 2048, store, 0, 1), (16, 18960, 2048, store, 0, 0), (16, 32000, 2048, store, 0, 0), (16, 4736, 3200, store, 0, 1), (16, 4752, 3200, store, 0, 0), (16, 64, 3328, store, 0, 0),
             (8, 4736, 6400, store, 0, 1), (8, 4752, 6400, store, 0, 0), (8, 9472, 4864, store, 0, 1), (8, 4752, 4608, store, 0, 0), (8, 64, 6528, store, 0, 0), (33, 64, 128, store, 0, 0)]:
         assert form(M, N, K, epilogue, scaled) == want, (M, N, K, epilogue, scaled)
+
+
+def _silu_of(z, off):
+    """silu(gate) * up of rows interleaved by eight, in float64, and how far it is off where gate and up are off by ``off``."""
+    M, N = z.shape
+    gate, up = z.reshape(M, N // 16, 2, 8).unbind(2)
+    gate_off, up_off = off.reshape(M, N // 16, 2, 8).unbind(2)
+    want = torch.nn.functional.silu(gate) * up
+    lim = 2.0 ** -8 * want.abs() + 1.2 * (gate_off * up.abs() + up_off * gate.abs()) + 1e-5 * gate.abs() * up.abs() + 1e-30
+    return want.reshape(M, N // 2), lim.reshape(M, N // 2)
+
+
+@pytest.mark.parametrize("M", [16, 17, 32, 33])
+@pytest.mark.parametrize("N,K", [(12272, 1024), (12288, 1024), (6144, 2048), (14080, 896), (18944, 1024), (19072, 1024)])
+def test_medium_matrices_of_17_to_32_tokens(M, N, K, monkeypatch):
+    """Both sides of the lines between the streaming kernel and the one on tensor memory (2^23.6 elements, 1,024 columns with the activation, one tile an SM): which one runs, with and without the
+    activation, and what neither leaves is refused."""
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    g, x, w, b, y, bound = _product(dev, M, N, K)
+    ran = []
+    for name in ("linear_tc", "linear_stream", "linear_ws"):
+        monkeypatch.setattr(ops, name, lambda *a, _f=getattr(ops, name), _n=name, **k: (ran.append(_n), _f(*a, **k))[1])
+    on_tensor_memory = 17 <= M <= 32 and N * K >= 12 << 20 and -(-N // 128) <= ops.num_sms()
+    assert bool(((ops.linear(x, w, b, torch.float32) - y).abs() <= bound).all())
+    if 17 <= M <= 32:
+        assert ran == ["linear_tc" if on_tensor_memory else "linear_stream"]
+    if M <= 32:
+        with pytest.raises(ops.KernelError):                  # (no kernel for few tokens leaves float16)
+            ops.linear(x, w, b, torch.float16)
+    ran.clear()
+    plain, off = x.double() @ w.double().T, (K + 1) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+    want, lim = _silu_of(plain, off)
+    assert bool(((ops.linear_silu_mul(x, w, 8, torch.bfloat16) - want).abs() <= lim).all())
+    if 17 <= M <= 32:
+        assert ran == ["linear_tc" if on_tensor_memory and K >= 1024 else "linear_stream"]
