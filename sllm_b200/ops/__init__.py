@@ -1962,7 +1962,18 @@ def silu_scaled_supports(x, w_gate_up, interleave: int, out_dtype) -> bool:
     N = w_gate_up.shape[0]
     if not (x.is_cuda and x.dtype == torch.bfloat16 and out_dtype == torch.bfloat16 and interleave == 8 and N % 16 == 0):
         return False
-    return (M <= 32 and stream_supports(M, N, K) and not _tc_unsplit_pays(M, N, K)) or (M > TCGEN05_MIN_ROWS and _PAIR_GEMM != "off" and pair_supports(M, N, K))
+    return (M <= 32 and stream_supports(M, N, K)) or (M > TCGEN05_MIN_ROWS and _PAIR_GEMM != "off" and pair_supports(M, N, K))
+
+
+SILU_SCALED_BELOW, SILU_SCALED_MAX_K = 1 << 24, 1536
+
+
+def silu_scaled_pays(x, w_gate_up, interleave: int, out_dtype) -> bool:
+    """Whether `linear_silu_mul` had better get its input with the norm still owed: where it takes it, but for 17 to 32 tokens and matrices for which the product without one is so much the faster on
+    tensor memory (`_tc_unsplit_pays`) that a norm kernel before it pays.  (32 tokens, us, with the norm owed / the norm's kernel and the product: 12,288 x 1,024 12.9 / 14.1, 8,192 x 1,536 14.6 / 15.7,
+    12,288 x 1,280 13.0 / 15.1, 16,384 x 1,024 14.8 / 15.0; 9,728 x 1,408 15.7 / 15.2, 18,944 x 1,024 16.0 / 15.7, 16,384 x 1,536 18.6 / 17.1, 11,264 x 2,048 30.4 / 18.8, 4,096 x 4,096 47.6 / 27.5.)"""
+    (M, K), N = x.shape, w_gate_up.shape[0]
+    return silu_scaled_supports(x, w_gate_up, interleave, out_dtype) and not (_tc_unsplit_pays(M, N, K, True) and (N * K > SILU_SCALED_BELOW or K > SILU_SCALED_MAX_K))
 
 
 def linear_silu_mul(x: torch.Tensor, w_gate_up: torch.Tensor, interleave: int, out_dtype: torch.dtype,

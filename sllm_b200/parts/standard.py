@@ -269,7 +269,7 @@ class SwiGLU(FeedForward):
 
     def forward(self, x, step, residual=None, next_norm=None):
         if isinstance(x, OwedNorm):
-            if ops.silu_scaled_supports(x.x, self.gate_up.weight, self.interleave, self.dtype):
+            if ops.silu_scaled_pays(x.x, self.gate_up.weight, self.interleave, self.dtype):
                 act = ops.linear_silu_mul(x.x, self.gate_up.weight, self.interleave, self.dtype, scale=x.scale)
                 return self.down.into(act, residual, next_norm)
             x = x.plain()

@@ -262,3 +262,10 @@ def test_medium_matrices_of_17_to_32_tokens(M, N, K, monkeypatch):
     assert bool(((ops.linear_silu_mul(x, w, 8, torch.bfloat16) - want).abs() <= lim).all())
     if 17 <= M <= 32:
         assert ran == ["linear_tc" if on_tensor_memory and K >= 1024 else "linear_stream"]
+    if M <= 32:                                              # an input whose norm is owed is taken on either side
+        ssq = torch.rand(M, 56, device=dev, generator=g) * 4 * K / 56
+        scale = (ssq.double().sum(1, keepdim=True) / K + 1e-5).rsqrt()
+        want, lim = _silu_of(plain * scale, off * scale + 2.0 ** -20 * (plain * scale).abs())
+        assert ops.silu_scaled_supports(x, w, 8, torch.bfloat16)
+        assert bool(((ops.linear_silu_mul(x, w, 8, torch.bfloat16, scale=ops.RowScale(ssq, 56, 1e-5, K)) - want).abs() <= lim).all())
+        assert ops.silu_scaled_pays(x, w, 8, torch.bfloat16) == (not (on_tensor_memory and (N, K) in ((6144, 2048), (18944, 1024))))
