@@ -112,6 +112,7 @@ def _declare(L):
         "sllm_linear_ws": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
                            c_void_p, c_int, c_float, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
         "sllm_linear_ws_parts": [c_int, c_int],
+        "sllm_add_rmsnorm_form": [c_int, c_int, c_int, c_int],
         "sllm_zero_rows": [c_void_p, c_int, ctypes.c_longlong, c_void_p, c_int, c_void_p],
         "sllm_linear_ws_slices": [c_int, c_int],
         "sllm_linear_ws_side_by_side": [c_int, c_int, c_int],

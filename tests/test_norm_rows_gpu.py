@@ -24,7 +24,7 @@ def _close(got, want, scale, W):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("T", [1, 3, 300])
-@pytest.mark.parametrize("W", [4, 100, 128, 2048, 4096, 4100, 8192, 8196, 1001])
+@pytest.mark.parametrize("W", [4, 100, 128, 2048, 4096, 4100, 8192, 8196, 16388, 1001])
 def test_rows_in_registers(W, T, dtype):
     import sllm_b200.ops as ops
     dev = cuda_or_skip()
@@ -52,6 +52,16 @@ def test_rows_in_registers(W, T, dtype):
         assert bool(((stream.double() - (x + add)).abs() <= (W + 16) * 2.0 ** -24 * (x.abs() + add.abs() + 1)).all())
         want = norm(stream.double()) * b
         assert _close(h, want, want.abs(), W)
+
+
+def test_wide_rows_keep_their_16_byte_loads():
+    """The form a norm takes (0: a channel a load; 1, 2: one or two vectors of four a thread, in registers; 3: vectors of four, read twice; 4: many rows), on both sides of every border."""
+    cuda_or_skip()
+    from sllm_b200.ops._lib import lib
+    form = lib().sllm_add_rmsnorm_form
+    for H, few, many in ((4, 1, 4), (4096, 1, 4), (4100, 2, 4), (8192, 2, 4), (8196, 3, 4), (16384, 3, 4), (16388, 3, 3), (32768, 3, 3)):
+        assert [form(1, H, 0, 1), form(63, H, 1, 1), form(64, H, 1, 1), form(64, H, 2, 1), form(64, H, 1, 0)] == [few, few, many, few, 0]
+        assert form(1, H + 1, 0, 1) == form(64, H + 2, 0, 1) == 0
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
