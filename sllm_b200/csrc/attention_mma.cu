@@ -472,14 +472,10 @@ static int launch_attention(const AttnParams& p, int tiles, cudaStream_t stream)
   constexpr int BM = DECODE ? 16 : 128;
   constexpr size_t smem = sizeof(__nv_bfloat16) * (size_t)(BM + 2 * AttStages<DECODE>::value * ATT_BN) * (HD + 8) +
                           sizeof(int) * AttBtCache<DECODE>::value;
-  static bool configured = false;                 // per template instance
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attention_mma_kernel<HD, DECODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) {
-      set_error("attention_mma: cannot raise the shared memory limit");
-      return SLLM_ERR_LAUNCH;
-    }
-    configured = true;
+  static SharedLimit limit;                       // per template instance
+  if (!limit.raise(attention_mma_kernel<HD, DECODE>, smem)) {
+    set_error("attention_mma: cannot raise the shared memory limit");
+    return SLLM_ERR_LAUNCH;
   }
   dim3 grid((unsigned)tiles * p.nkv, 1, p.num_splits);
   launch_kernel(attention_mma_kernel<HD, DECODE>, grid, AttThreads<DECODE>::value, smem, stream, p);

@@ -673,13 +673,10 @@ template <int HD, int RT, bool CAP, bool REL>
 static int launch_tc(const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& rk, const CUtensorMap& rv,
                      const AttnTcParams& p, int tiles, cudaStream_t stream) {
   constexpr int smem = TcLayout<HD, RT>::SMEM;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(attention_tc_kernel<HD, RT, CAP, REL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
-      set_error("attention_tc: cannot raise the shared memory limit");
-      return SLLM_ERR_LAUNCH;
-    }
-    configured = true;
+  static SharedLimit limit;
+  if (!limit.raise(attention_tc_kernel<HD, RT, CAP, REL>, smem)) {
+    set_error("attention_tc: cannot raise the shared memory limit");
+    return SLLM_ERR_LAUNCH;
   }
   dim3 grid((unsigned)tiles * p.nkv, 1, p.num_splits);
   launch_kernel(attention_tc_kernel<HD, RT, CAP, REL>, grid, TcLayout<HD, RT>::THREADS, (size_t)smem, stream, mk, mv, rk, rv, p);

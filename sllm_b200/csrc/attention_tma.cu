@@ -615,13 +615,10 @@ template <int HD, bool CAP, bool REL>
 static int launch_ta(const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& rk, const CUtensorMap& rv,
                      const AttnTmaParams& p, int tiles, cudaStream_t stream) {
   constexpr size_t smem = ta_smem(HD);
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(attention_tma_decode_kernel<HD, CAP, REL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-      set_error("attention_tma: cannot raise the shared memory limit");
-      return SLLM_ERR_LAUNCH;
-    }
-    configured = true;
+  static SharedLimit limit;
+  if (!limit.raise(attention_tma_decode_kernel<HD, CAP, REL>, smem)) {
+    set_error("attention_tma: cannot raise the shared memory limit");
+    return SLLM_ERR_LAUNCH;
   }
   dim3 grid((unsigned)tiles * p.nkv, 1, p.num_splits);
   if (p.cluster) {

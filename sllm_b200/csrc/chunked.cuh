@@ -100,14 +100,10 @@ __device__ __forceinline__ void rc_store4(__nv_bfloat16* o, const float (&v)[4])
 }
 
 template <typename K>
-static int rc_smem(K kernel, size_t bytes, size_t& allowed) {
-  if (bytes > allowed) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
-      cudaGetLastError();
-      set_error("chunks: a kernel's shared memory could not be raised");
-      return SLLM_ERR_LAUNCH;
-    }
-    allowed = bytes;
+static int rc_smem(K kernel, size_t bytes, SharedLimit& limit) {
+  if (bytes > 48 * 1024 && !limit.raise(kernel, bytes)) {
+    set_error("chunks: a kernel's shared memory could not be raised");
+    return SLLM_ERR_LAUNCH;
   }
   return SLLM_OK;
 }

@@ -9,6 +9,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <mutex>
+
 #define SLLM_OK 0
 #define SLLM_ERR_ARG 1        // a size, pointer or dtype the kernel refuses
 #define SLLM_ERR_LAUNCH 2     // the launch itself failed (see cudaGetLastError text)
@@ -159,6 +161,26 @@ inline void launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_
   cfg.numAttrs = pdl_enabled() ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);   // errors are read by launch_status()
 }
+
+// The shared memory that a kernel has been told it may use, a device each: the setting belongs to a device's copy of the kernel, and a process may hold models on
+// several and launch from several threads.  One of these stands beside every launch that needs more than what any kernel gets.
+struct SharedLimit {
+  std::mutex mutex;
+  size_t allowed[64] = {};
+  template <typename Kernel>
+  bool raise(Kernel kernel, size_t bytes) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return false;
+    std::lock_guard<std::mutex> lock(mutex);
+    if (dev < 64 && bytes <= allowed[dev]) return true;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    if (dev < 64) allowed[dev] = bytes;
+    return true;
+  }
+};
 
 inline int launch_status(const char* what) {
   cudaError_t e = cudaGetLastError();

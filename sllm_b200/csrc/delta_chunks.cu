@@ -671,15 +671,15 @@ __global__ void __launch_bounds__(RC_OUT_THREADS) delta_chunk_out_kernel(const D
 
 template <int DK, int DV, int MODE>
 static int launch_delta_chunks(const DeltaChunkParams& p, int chunks, int runs, cudaStream_t stream) {
-  static size_t allowed_prep = 48 * 1024, allowed_scan = 48 * 1024, allowed_out = 48 * 1024;      // (per instantiation)
+  static SharedLimit prep_limit, scan_limit, out_limit;      // (per instantiation)
   const size_t smem_prep = MODE == DC_GATED ? GatedPrepSmem<DK, DV>::BYTES : GENERAL_PREP_BYTES;
   constexpr size_t smem_scan = DeltaScanSmem<DK>::BYTES, smem_out = DeltaOutSmem<DK, DV>::BYTES;
   void (*prep)(const DeltaChunkParams);
   if constexpr (MODE == DC_GATED) prep = gated_delta_prep_kernel<DK, DV>;
   else prep = general_delta_prep_kernel;
-  int rc = rc_smem(prep, smem_prep, allowed_prep);
-  if (rc == SLLM_OK) rc = rc_smem(delta_scan_kernel<DK, MODE>, smem_scan, allowed_scan);
-  if (rc == SLLM_OK) rc = rc_smem(delta_chunk_out_kernel<DK, DV, MODE>, smem_out, allowed_out);
+  int rc = rc_smem(prep, smem_prep, prep_limit);
+  if (rc == SLLM_OK) rc = rc_smem(delta_scan_kernel<DK, MODE>, smem_scan, scan_limit);
+  if (rc == SLLM_OK) rc = rc_smem(delta_chunk_out_kernel<DK, DV, MODE>, smem_out, out_limit);
   if (rc != SLLM_OK) return rc;
   const dim3 grid((unsigned)chunks, (unsigned)p.H);
   launch_kernel(prep, grid, DC_THREADS, smem_prep, stream, p);

@@ -585,14 +585,10 @@ static int launch_delta_rule(DeltaParams p, int S, cudaStream_t stream) {
   if (p.max_q > 0 && chunk > p.max_q) chunk = p.max_q;      // single decoded tokens: little shared memory, more CTAs an SM
   p.chunk = chunk;
   const size_t smem = 2 * per_token * chunk;
-  static size_t allowed = 48 * 1024;          // (per instantiation: what the kernel has been told it may use)
-  if (smem > allowed) {
-    if (cudaFuncSetAttribute(delta_rule_kernel<RPT, CB, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-      cudaGetLastError();
-      set_error("delta_rule: the kernel's shared memory could not be raised");
-      return SLLM_ERR_LAUNCH;
-    }
-    allowed = smem;
+  static SharedLimit limit;                   // (per instantiation)
+  if (smem > 48 * 1024 && !limit.raise(delta_rule_kernel<RPT, CB, KIND>, smem)) {
+    set_error("delta_rule: the kernel's shared memory could not be raised");
+    return SLLM_ERR_LAUNCH;
   }
   const dim3 grid((unsigned)S, (unsigned)p.H, (unsigned)((p.dv + DR_COLS - 1) / DR_COLS));
   launch_kernel(delta_rule_kernel<RPT, CB, KIND>, grid, DR_THREADS, smem, stream, p);

@@ -415,10 +415,10 @@ __global__ void __launch_bounds__(RC_OUT_THREADS) gated_out_kernel(const GatedCh
 
 template <int DK, int DV, int MODE>
 static int launch_gated(const GatedChunkParams& p, int chunks, int runs, cudaStream_t stream) {
-  static size_t allowed_state = 48 * 1024, allowed_out = 48 * 1024;      // (per instantiation)
+  static SharedLimit state_limit, out_limit;      // (per instantiation)
   constexpr size_t smem_state = (size_t)(RC * DK + RC * DV + DK) * 4, smem_out = GatedOutSmem<DK, DV>::BYTES;
-  int rc = rc_smem(gated_state_kernel<DK, DV, MODE>, smem_state, allowed_state);
-  if (rc == SLLM_OK) rc = rc_smem(gated_out_kernel<DK, DV, MODE>, smem_out, allowed_out);
+  int rc = rc_smem(gated_state_kernel<DK, DV, MODE>, smem_state, state_limit);
+  if (rc == SLLM_OK) rc = rc_smem(gated_out_kernel<DK, DV, MODE>, smem_out, out_limit);
   if (rc != SLLM_OK) return rc;
   const dim3 grid((unsigned)chunks, (unsigned)p.H);
   launch_kernel(gated_state_kernel<DK, DV, MODE>, grid, 2 * DK, smem_state, stream, p);

@@ -553,13 +553,10 @@ static void pair_launch_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&at
 template <int EPI, int R2>
 static int launch_tp_wide(const CUtensorMap& ma, const CUtensorMap& mw, const float* bias, void* out, int M, int N, int K,
                           int* status, cudaStream_t stream, const TgExtra& extra) {
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(gemm_pair_wide_kernel<EPI, R2>, cudaFuncAttributeMaxDynamicSharedMemorySize, TP_SMEM_WIDE) != cudaSuccess) {
-      set_error("gemm_pair: cannot raise the shared memory limit");
-      return SLLM_ERR_LAUNCH;
-    }
-    configured = true;
+  static SharedLimit limit;
+  if (!limit.raise(gemm_pair_wide_kernel<EPI, R2>, TP_SMEM_WIDE)) {
+    set_error("gemm_pair: cannot raise the shared memory limit");
+    return SLLM_ERR_LAUNCH;
   }
   // the result leaves through TMA stores where its rows are whole 16-byte pieces; else lane by lane
   const int out_cols = tg_gated(EPI) ? N / 2 : N, elem = TgBox<EPI>::ELEM;
@@ -583,13 +580,10 @@ static int launch_tp(const CUtensorMap& ma, const CUtensorMap& mw, const float* 
                      int* status, cudaStream_t stream, const TgExtra& extra, int ksplits, int kb_per_split, const TpGroups& groups = TpGroups{}) {
   auto kernel = gemm_pair_kernel<EPI, BN>;
   constexpr int TP_SMEM = TpCfg<BN>::SMEM, TP_BN = BN;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TP_SMEM) != cudaSuccess) {
-      set_error("gemm_pair: cannot raise the shared memory limit");
-      return SLLM_ERR_LAUNCH;
-    }
-    configured = true;
+  static SharedLimit limit;
+  if (!limit.raise(kernel, TP_SMEM)) {
+    set_error("gemm_pair: cannot raise the shared memory limit");
+    return SLLM_ERR_LAUNCH;
   }
   const int pairs_max = sllm::num_sms() / 2;
   const long long tiles = (long long)((M + 2 * TP_BM - 1) / (2 * TP_BM)) * ((N + TP_BN - 1) / TP_BN) * ksplits;

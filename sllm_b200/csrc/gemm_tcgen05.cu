@@ -175,13 +175,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 template <int EPI>
 static int launch_tg(const CUtensorMap& ma, const CUtensorMap& mw, const float* bias, void* out, int M, int N, int K,
                      int* status, cudaStream_t stream) {
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(gemm_tcgen05_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, TG_SMEM) != cudaSuccess) {
-      set_error("gemm_tcgen05: cannot raise the shared memory limit");
-      return SLLM_ERR_LAUNCH;
-    }
-    configured = true;
+  static SharedLimit limit;
+  if (!limit.raise(gemm_tcgen05_kernel<EPI>, TG_SMEM)) {
+    set_error("gemm_tcgen05: cannot raise the shared memory limit");
+    return SLLM_ERR_LAUNCH;
   }
   const int num_sms = sllm::num_sms();
   const long long tiles = (long long)((M + TG_BM - 1) / TG_BM) * ((N + TG_BN - 1) / TG_BN);

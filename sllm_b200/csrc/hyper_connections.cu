@@ -186,14 +186,10 @@ template <int NS, int VEC, typename TO>
 static int launch_streams_step(float* streams, const float* term, int parts, size_t part_stride, const float* mix, const float* share, const float* into,
                                const float* gain, float eps, const int* rows, TO* h, int R, int T, int ns, int W, cudaStream_t stream) {
   const size_t smem = gain != nullptr ? (size_t)W * sizeof(float) : 0;
-  static size_t allowed = 48 * 1024;              // (per instantiation)
-  if (smem > allowed) {
-    if (cudaFuncSetAttribute(streams_step_kernel<NS, VEC, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-      cudaGetLastError();
-      set_error("streams_step: rows so wide do not fit the shared memory");
-      return SLLM_ERR_LAUNCH;
-    }
-    allowed = smem;
+  static SharedLimit limit;                       // (per instantiation)
+  if (smem > 48 * 1024 && !limit.raise(streams_step_kernel<NS, VEC, TO>, smem)) {
+    set_error("streams_step: rows so wide do not fit the shared memory");
+    return SLLM_ERR_LAUNCH;
   }
   launch_kernel(streams_step_kernel<NS, VEC, TO>, (unsigned)R, HC_THREADS, smem, stream, streams, term, parts, part_stride, mix, share, into, gain, eps,
                 rows, h, T, ns, W);

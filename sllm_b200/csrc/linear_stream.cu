@@ -355,13 +355,10 @@ SLLM_EXPORT int sllm_linear_stream_resident(int M, int N, int K, int epilogue, i
 
 template <int NT, int EPI, typename OUT, bool SCALED>
 static int launch_resident(const __nv_bfloat16* x, const __nv_bfloat16* W, const float* bias, void* out, int M, int N, int K, cudaStream_t stream, const LsScale& scale) {
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(linear_resident_kernel<NT, EPI, OUT, SCALED>, cudaFuncAttributeMaxDynamicSharedMemorySize, LR_X_MAX) != cudaSuccess) {
-      set_error("linear_stream: cannot raise the shared memory limit");
-      return SLLM_ERR_LAUNCH;
-    }
-    configured = true;
+  static SharedLimit limit;
+  if (!limit.raise(linear_resident_kernel<NT, EPI, OUT, SCALED>, LR_X_MAX)) {
+    set_error("linear_stream: cannot raise the shared memory limit");
+    return SLLM_ERR_LAUNCH;
   }
   launch_kernel(linear_resident_kernel<NT, EPI, OUT, SCALED>, (N + LR_WARPS * 16 - 1) / (LR_WARPS * 16), LR_WARPS * 32, (size_t)K * 16 * NT, stream, x, W, bias, (OUT*)out, M, N, K, scale);
   return launch_status("linear_stream");
@@ -374,13 +371,10 @@ static int launch_ls(const __nv_bfloat16* x, const __nv_bfloat16* W, const float
     if (ls_resident(M, N, K, splits, EPI != EPI_STORE, SCALED)) return launch_resident<NT, EPI, OUT, SCALED>(x, W, bias, out, M, N, K, stream, scale);
   }
   constexpr size_t smem = sizeof(__nv_bfloat16) * 2 * 8 * NT * LS_XSTRIDE + (SCALED ? sizeof(float) * 8 * NT * LS_SSQ_MAX : 0);
-  static bool configured = false;
-  if (!configured && smem + 1024 > 48 * 1024) {      // (the kernel has a little static shared memory too)
-    if (cudaFuncSetAttribute(linear_stream_kernel<NT, EPI, OUT, SCALED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-      set_error("linear_stream: cannot raise the shared memory limit");
-      return SLLM_ERR_LAUNCH;
-    }
-    configured = true;
+  static SharedLimit limit;
+  if (smem + 1024 > 48 * 1024 && !limit.raise(linear_stream_kernel<NT, EPI, OUT, SCALED>, smem)) {      // (the kernel has a little static shared memory too)
+    set_error("linear_stream: cannot raise the shared memory limit");
+    return SLLM_ERR_LAUNCH;
   }
   const int total_chunks = K / LS_KC;
   const int per = (total_chunks + splits - 1) / splits;

@@ -245,13 +245,10 @@ static int lt_num_sms() { return sllm::num_sms(); }
 template <int BN, int EPI>
 static int launch_lt(const CUtensorMap& mw, const CUtensorMap& mx, const float* bias, void* out, int M, int N, int K,
                      int splits, int kb_per_split, int* status, cudaStream_t stream) {
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(linear_tc_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, LtCfg<BN>::SMEM) != cudaSuccess) {
-      set_error("linear_tc: cannot raise the shared memory limit");
-      return SLLM_ERR_LAUNCH;
-    }
-    configured = true;
+  static SharedLimit limit;
+  if (!limit.raise(linear_tc_kernel<BN, EPI>, LtCfg<BN>::SMEM)) {
+    set_error("linear_tc: cannot raise the shared memory limit");
+    return SLLM_ERR_LAUNCH;
   }
   const int units = ((N + LT_ROWS - 1) / LT_ROWS) * splits, sms = lt_num_sms();
   dim3 grid((unsigned)(units < sms ? units : sms));              // persistent: one CTA per SM walks the units

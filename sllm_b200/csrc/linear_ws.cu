@@ -28,6 +28,8 @@
 #include <cooperative_groups.h>
 #include <stdio.h>
 
+#include <atomic>
+
 #include "common.cuh"
 
 namespace sllm {
@@ -479,7 +481,7 @@ static bool ws_side_by_side(int M, int N, int K) {
   return ctas <= places || ctas * 100 >= (ctas + places - 1) / places * places * 84;
 }
 
-// The kernel, told once what shared memory it wants beside L1: what two CTAs need, at least WS_CARVEOUT per cent.  The loads in flight lie in L1, and an SM keeps the split that the kernel
+// The kernel, told once a device what shared memory it wants beside L1: what two CTAs need, at least WS_CARVEOUT per cent.  The loads in flight lie in L1, and an SM keeps the split that the kernel
 // before had as long as the next one's shared memory fits: behind the decode attention, which takes all of it, this kernel ran with 28 KB of L1 (at 7B sizes gate|up 65 us in place of 45,
 // down 67 in place of 25, as soon as no small kernel stood between them).  (8 requests at 7B sizes, 8 of 240 keys at a width of 2,048, 16 of 300, one of 700 at 4,096, ms: no preference 195, 20.0, 29.4, 17.2;
 // 0 per cent beyond what fits 131.6, 19.8, 29.4, 16.8; 30 131.6, 19.4, 28.6, 16.6; 60 138.9, 21.4, 28.9, 18.4.)
@@ -487,14 +489,12 @@ constexpr int WS_CARVEOUT = 30, WS_SM_SHARED = 228 * 1024;
 template <int NT, int EPI, typename OUT, bool SCALED, int FORM>
 static auto ws_kernel() {
   auto kernel = linear_ws_kernel<NT, EPI, OUT, SCALED, FORM>;
-  static bool told = false;
-  if (!told) {
-    cudaFuncAttributes at;
-    if (cudaFuncGetAttributes(&at, kernel) == cudaSuccess) {
-      const int fit = (int)(2 * (at.sharedSizeBytes + 1024) * 100 / WS_SM_SHARED) + 1;
-      cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, fit > WS_CARVEOUT ? fit : WS_CARVEOUT);      // (a preference; nothing depends on it but time)
-    }
-    told = true;
+  static std::atomic<unsigned long long> told{0};                       // a bit a device
+  int dev = 0;
+  cudaFuncAttributes at;
+  if (cudaGetDevice(&dev) == cudaSuccess && dev < 64 && !(told.fetch_or(1ull << dev) >> dev & 1) && cudaFuncGetAttributes(&at, kernel) == cudaSuccess) {
+    const int fit = (int)(2 * (at.sharedSizeBytes + 1024) * 100 / WS_SM_SHARED) + 1;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, fit > WS_CARVEOUT ? fit : WS_CARVEOUT);      // (a preference; nothing depends on it but time)
   }
   return kernel;
 }

@@ -356,10 +356,10 @@ __global__ void __launch_bounds__(RC_OUT_THREADS) chunk_out_kernel(const Retenti
 
 template <int DK, int DV, typename TO>
 static int launch_chunked(const RetentionParams& p, int chunks, int runs, TO* out, int out_ld, cudaStream_t stream) {
-  static size_t allowed_state = 48 * 1024, allowed_out = 48 * 1024;      // (per instantiation)
+  static SharedLimit state_limit, out_limit;      // (per instantiation)
   constexpr size_t smem_state = (size_t)(RC * DK + RC * DV + RC) * 4, smem_out = ChunkOutSmem<DK, DV>::BYTES;
-  int rc = rc_smem(chunk_state_kernel<DK, DV>, smem_state, allowed_state);
-  if (rc == SLLM_OK) rc = rc_smem(chunk_out_kernel<DK, DV, TO>, smem_out, allowed_out);
+  int rc = rc_smem(chunk_state_kernel<DK, DV>, smem_state, state_limit);
+  if (rc == SLLM_OK) rc = rc_smem(chunk_out_kernel<DK, DV, TO>, smem_out, out_limit);
   if (rc != SLLM_OK) return rc;
   const dim3 grid((unsigned)chunks, (unsigned)p.H);
   launch_kernel(chunk_state_kernel<DK, DV>, grid, 2 * DK, smem_state, stream, p);

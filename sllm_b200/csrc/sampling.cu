@@ -1027,9 +1027,8 @@ static void sample_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[2
 
 // Raises the kernel's limit of shared memory; what fits the GPU is asked with it raised, whichever call of a process comes first.
 static bool sample_smem_raised() {
-  static bool raised = false;
-  if (!raised) raised = cudaFuncSetAttribute(sample_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_SMEM) == cudaSuccess;
-  return raised;
+  static SharedLimit limit;
+  return limit.raise(sample_rows_kernel, SAMPLE_SMEM);
 }
 
 // Blocks a row (log2): as many as leave every row's cluster on the GPU at once.  A block fills an SM (1,024 threads of 64 registers) and a cluster lies in one

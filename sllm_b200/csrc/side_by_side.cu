@@ -445,14 +445,10 @@ SLLM_EXPORT int sllm_whole_norm_kv_write(const float* qkv, int parts, size_t par
                    (((uintptr_t)qkv | (uintptr_t)bias | (uintptr_t)q_gain | (uintptr_t)k_gain | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)q_out) & 15) == 0;
 #define LAUNCH(TC, VEC)                                                                                                                    \
   do {                                                                                                                                     \
-    static size_t allowed = 48 * 1024;                                                                                                     \
-    if (smem > allowed) {                                                                                                                  \
-      if (cudaFuncSetAttribute(whole_norm_kv_write_kernel<TC, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) { \
-        cudaGetLastError();                                                                                                                \
-        set_error("whole_norm: the kernel's shared memory could not be raised");                                                           \
-        return SLLM_ERR_LAUNCH;                                                                                                            \
-      }                                                                                                                                    \
-      allowed = smem;                                                                                                                      \
+    static SharedLimit limit;                                                                                                              \
+    if (smem > 48 * 1024 && !limit.raise(whole_norm_kv_write_kernel<TC, VEC>, smem)) {                                                     \
+      set_error("whole_norm: the kernel's shared memory could not be raised");                                                             \
+      return SLLM_ERR_LAUNCH;                                                                                                              \
     }                                                                                                                                      \
     launch_kernel(whole_norm_kv_write_kernel<TC, VEC>, (unsigned)T, 256, smem, stream, qkv, parts, part_stride, ld, bias, q_gain, k_gain, eps, \
                   positions, q_coef, q_every, nq, nkv, dim, vdim, D, slot_mapping, page_size, num_pages, (TC*)k_cache, (TC*)v_cache, (TC*)q_out); \

@@ -393,11 +393,11 @@ __global__ void __launch_bounds__(ST_THREADS) ssd_token_kernel(const SsdTokenPar
 
 template <int DK, int DV>
 static int launch_ssd(const SsdParams& p, int chunks, int runs, cudaStream_t stream) {
-  static size_t allowed_state = 48 * 1024, allowed_out = 48 * 1024;      // (per instantiation)
+  static SharedLimit state_limit, out_limit;      // (per instantiation)
   constexpr size_t for_state = (size_t)(RC * DK + RC * DV + 2 * RC + 4) * 4, for_scores = (size_t)2 * RC * (DK + 4) * 4;
   constexpr size_t smem_state = for_state > for_scores ? for_state : for_scores, smem_out = SsdOutSmem<DK, DV>::BYTES;
-  int rc = rc_smem(ssd_state_kernel<DK, DV>, smem_state, allowed_state);
-  if (rc == SLLM_OK) rc = rc_smem(ssd_out_kernel<DK, DV>, smem_out, allowed_out);
+  int rc = rc_smem(ssd_state_kernel<DK, DV>, smem_state, state_limit);
+  if (rc == SLLM_OK) rc = rc_smem(ssd_out_kernel<DK, DV>, smem_out, out_limit);
   if (rc != SLLM_OK) return rc;
   const dim3 grid((unsigned)chunks, (unsigned)p.H);
   launch_kernel(ssd_state_kernel<DK, DV>, dim3((unsigned)chunks, (unsigned)(p.H + p.groups)), 2 * DK, smem_state, stream, p);
@@ -524,8 +524,8 @@ SLLM_EXPORT int sllm_gated_group_norm(const float* y, const float* gate, int ldg
   const int per = vec ? size / 4 : size, threads = per >= 512 ? 512 : (per + 31) / 32 * 32;
 #define GG(TO_, VEC_)                                                                                                                        \
   do {                                                                                                                                       \
-    static size_t allowed = 48 * 1024;                                                                                                       \
-    if (int rc = rc_smem(gated_group_norm_kernel<TO_, VEC_>, smem, allowed)) return rc;                                                      \
+    static SharedLimit limit;                                                                                                                \
+    if (int rc = rc_smem(gated_group_norm_kernel<TO_, VEC_>, smem, limit)) return rc;                                                        \
     launch_kernel(gated_group_norm_kernel<TO_, VEC_>, blocks, threads, smem, stream, y, gate, ldg, off_g, gain, eps, groups, (TO_*)out, n);   \
     return launch_status("gated_group_norm");                                                                                                \
   } while (0)

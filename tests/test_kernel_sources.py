@@ -42,3 +42,12 @@ def test_read_only_loads_are_of_constants(name):
     arguments = [code_of(name)[m.end():].lstrip() for m in re.finditer(r"__ldc?g\(", code_of(name))]
     constants = ("p.a_log", "p.skip", "p.a_bias", "p.dt_bias", "p.rel", "rel_h[", "bias", "tab ", "reinterpret_cast<const float4*>(bias", "reinterpret_cast<const float4*>(w ")
     assert not [a[:60] for a in arguments if not a.startswith(constants)]
+
+
+@pytest.mark.parametrize("name", SOURCES)
+def test_settings_of_a_kernel_are_made_on_every_device(name):
+    """A kernel's limit of shared memory and its split of L1 lie with a device's copy of it: no flag or size of the whole process says that they have been set (`SharedLimit`; a bit a device)."""
+    code = code_of(name)
+    assert not re.findall(r"\bstatic (?:bool|int|size_t) \w+ =[^=(]*;", code)
+    if name not in ("common.cuh", "linear_ws.cu", "gemm_f32.cu"):           # (gemm_f32.cu sets it at every launch)
+        assert "cudaFuncSetAttribute" not in code
