@@ -53,6 +53,12 @@ struct WsRope {
   int max_pos, nq, nkv, hd, page_size, num_pages;
 };
 
+__device__ __forceinline__ int ws_position(const int* p) {        // which another kernel may be writing: from L2, and nothing stays in L1
+  int pos;
+  asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(pos) : "l"(p));
+  return pos;
+}
+
 __device__ __forceinline__ uint4 ws_ldg_stream(const void* p) {
   uint4 v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n"
@@ -131,6 +137,7 @@ linear_ws_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ W,
   constexpr bool AHEAD = (EPI == WS_EPI_RESID && !SCALED && (FORM == WS_ONE || FORM == WS_SLICED)) || EPI == WS_EPI_ROPE;
   constexpr bool BIAS_AHEAD = !(SCALED && NT == 2);
   constexpr int AHEAD_N = EPI == WS_EPI_ROPE ? 64 * NT : (16 * 8 * NT + WS_WARPS * 32 - 1) / (WS_WARPS * 32) * WS_WARPS * 32;
+  __shared__ int token_s[EPI == WS_EPI_ROPE ? 3 : 1][EPI == WS_EPI_ROPE ? 8 * NT : 1];      // rotary: the position its angles were copied for, its position, its slot
   __shared__ float ahead[AHEAD ? (EPI == WS_EPI_ROPE ? (BIAS_AHEAD ? 4 : 2) : 3) : 1][AHEAD ? AHEAD_N : 1];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t4 = lane & 3;
@@ -216,27 +223,26 @@ linear_ws_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ W,
   constexpr int GROUP = WS_DEPTH * KW;        // k blocks the CTA covers per group
   const int k_mine = k_first + warp % KW;
   int kb = k_mine;
-  int ahead_pos = 0, ahead_slot = -1;
-  if constexpr (EPI == WS_EPI_ROPE) {         // (the step's description was there before the step's first kernel)
-    const int tok = tid / 8;
-    if (tid < AHEAD_N && tok < M) {
-      if (rope.table != nullptr) ahead_pos = rope.positions[tok];
-      if (rope.slot_mapping != nullptr) ahead_slot = rope.slot_mapping[tok];
-    }
+  // Rotary: a token's position is taken twice.  Before the wait it may still be on its way from an earlier kernel, so it only says which angles to copy; behind the wait it is the token's, and the
+  // epilogue looks the angles up again where the two differ.  (Behind the wait alone the product waits for two misses one behind the other: 1,152 x 896, one token 2.45 -> 3.06 us.  In shared
+  // memory, because registers are weights in flight: 4,608 x 3,584 7.5 -> 8.5 us with two more.)
+  const int ahead_tok = tid / 8, ahead_i = tid % 8;
+  const bool ahead_mine = EPI == WS_EPI_ROPE && tid < AHEAD_N && ahead_tok < M;
+  int ahead_pos = 0;
+  if constexpr (EPI == WS_EPI_ROPE) {         // (one load a token: its eight threads copy the same angles)
+    if (ahead_mine && ahead_i == 0 && rope.table != nullptr) ahead_pos = token_s[0][ahead_tok] = min(max(ws_position(rope.positions + ahead_tok), 0), rope.max_pos - 1);
+    ahead_pos = __shfl_sync(0xffffffffu, ahead_pos, lane & 24);
   }
   load_w(wa0, wb0, kb);
   if constexpr (EPI == WS_EPI_ROPE) {
-    const int tok = tid / 8, i = tid % 8, half = rope.hd / 2, j = n0 % rope.hd + i;
-    if (tid < AHEAD_N && tok < M) {
-      const float* cs = rope.table + (size_t)min(max(ahead_pos, 0), rope.max_pos - 1) * rope.hd;        // cos[half] then sin[half]
-      if (rope.table != nullptr) {
-        ws_copy4(&ahead[0][tid], cs + j);
-        ws_copy4(&ahead[1][tid], cs + half + j);
-      }
-      if (BIAS_AHEAD && bias) {
-        ws_copy4(&ahead[BIAS_AHEAD ? 2 : 0][tid], bias + n0 + i);
-        ws_copy4(&ahead[BIAS_AHEAD ? 3 : 0][tid], bias + n0 + half + i);
-      }
+    if (ahead_mine && rope.table != nullptr) {
+      const float* cs = rope.table + (size_t)ahead_pos * rope.hd + n0 % rope.hd + ahead_i;        // cos[half] then sin[half]
+      ws_copy4(&ahead[0][tid], cs);
+      ws_copy4(&ahead[1][tid], cs + rope.hd / 2);
+    }
+    if (ahead_mine && BIAS_AHEAD && bias) {
+      ws_copy4(&ahead[BIAS_AHEAD ? 2 : 0][tid], bias + n0 + ahead_i);
+      ws_copy4(&ahead[BIAS_AHEAD ? 3 : 0][tid], bias + n0 + rope.hd / 2 + ahead_i);
     }
   }
   auto resid_at = [&](auto&& use) {           // the thread's outputs of the CTA's only group
@@ -253,6 +259,10 @@ linear_ws_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ W,
   }
   if constexpr (SLICED) cooperative_groups::this_cluster().sync();      // nobody writes to a CTA that has not begun
   pdl_wait();
+  if constexpr (EPI == WS_EPI_ROPE) {
+    if (ahead_mine && ahead_i == 0 && rope.table != nullptr) ws_copy4(&token_s[1][ahead_tok], rope.positions + ahead_tok);
+    if (ahead_mine && ahead_i == 0 && rope.slot_mapping != nullptr) ws_copy4(&token_s[2][ahead_tok], rope.slot_mapping + ahead_tok);
+  }
   load_x(x0, kb);
   if constexpr (EPI == WS_EPI_RESID && AHEAD) resid_at([&](int idx, int tok, int n) { ws_copy4(&ahead[2][idx], residual + (size_t)tok * N + n); });
   if constexpr (AHEAD) asm volatile("cp.async.commit_group;\n" ::);
@@ -330,8 +340,8 @@ linear_ws_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ W,
     if constexpr (EPI == WS_EPI_ROPE) {
       const int half = rope.hd / 2;
       const int head = m0 / rope.hd, j0 = m0 % rope.hd;            // j0 = 8c: the pair's lower dimension starts here
-      const int i = tid % 8, tok = tid / 8;                          // consecutive threads -> consecutive dimensions of one token; at most one output a thread
-      if (tid < AHEAD_N && tok < M) {
+      const int i = ahead_i, tok = ahead_tok;                        // consecutive threads -> consecutive dimensions of one token; at most one output a thread
+      if (ahead_mine) {
         float lo = 0.f, hi = 0.f;
 #pragma unroll
         for (int w = 0; w < WS_WARPS; ++w) { lo += red[w][i][tok]; hi += red[w][i + 8][tok]; }
@@ -347,14 +357,20 @@ linear_ws_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ W,
         if (head < rope.nq) {
           dst = rope.q_out + ((size_t)tok * rope.nq + head) * rope.hd;
         } else {
-          if (ahead_slot < 0 || ahead_slot / rope.page_size >= rope.num_pages) return;     // not written (padding row, borrowed cache)
+          const int slot = rope.slot_mapping != nullptr ? token_s[2][tok] : -1;
+          if (slot < 0 || slot / rope.page_size >= rope.num_pages) return;     // not written (padding row, borrowed cache)
           const bool is_k = head < rope.nq + rope.nkv;
           const int kvh = is_k ? head - rope.nq : head - rope.nq - rope.nkv;
           dst = (is_k ? rope.k_cache : rope.v_cache) +
-                (((size_t)(ahead_slot / rope.page_size) * rope.nkv + kvh) * rope.page_size + ahead_slot % rope.page_size) * rope.hd;
+                (((size_t)(slot / rope.page_size) * rope.nkv + kvh) * rope.page_size + slot % rope.page_size) * rope.hd;
         }
         if (rope.table != nullptr && head < rope.nq + rope.nkv) {
-          const float c = ahead[0][tid], sn = ahead[1][tid];
+          float c = ahead[0][tid], sn = ahead[1][tid];
+          const int pos = min(max(token_s[1][tok], 0), rope.max_pos - 1);
+          if (pos != token_s[0][tok]) {
+            c = rope.table[(size_t)pos * rope.hd + j0 + i];
+            sn = rope.table[(size_t)pos * rope.hd + half + j0 + i];
+          }
           const float a = lo * c - hi * sn, b = hi * c + lo * sn;
           lo = a;
           hi = b;
@@ -641,6 +657,7 @@ SLLM_EXPORT int sllm_linear_ws_rope_supports(int M, int N, int K, int nq, int nk
 // The fused q|k|v product of an attention layer with its bias, rotary encoding and cache write:
 // x [M, K] and W [(nq + 2 nkv) * hd, K] bfloat16; table null or rot == 0: no rotation, else rot == hd and
 // table [max_pos][2][hd/2] float32; slot_mapping null: keys and values are not written.  ssq_in: as for sllm_linear_ws.
+// W and bias are read before the wait on the stream's earlier kernels, positions and slot_mapping behind it.
 SLLM_EXPORT int sllm_linear_ws_rope(const void* x, const void* W, const float* bias, int M, int N, int K, const int* positions,
                                     const float* table, int rot, int max_pos, int nq, int nkv, int hd, const int* slot_mapping,
                                     int page_size, int num_pages, void* k_cache, void* v_cache, void* q_out,

@@ -5,6 +5,14 @@ library model code behind these functions.  Matrix products of the bfloat16
 path with many rows go to cuBLAS (as the reference's engine does,
 kernels/cuda/kernels.cu:752-767); everything else, and every product of the
 float32 path, runs in this package's own kernels.
+
+A kernel is set up while the ones before it in the stream still run, and waits for them before it
+reads what they wrote.  Two kinds of operands are read before that wait and have to be in place by
+then: what belongs to a model (matrices, gains, biases, tables of angles and of weights), in every
+function, and the step's description (tiles, lengths, block tables) in the attention functions.  A
+program that computes one of these on the device puts a copy, an event or a synchronisation between
+that and the first call here; the engine's are loaded, or copied from the host, before a step begins.
+Everything else, token ids, positions and slots among it, may come from the kernel just before.
 """
 
 from __future__ import annotations
@@ -1855,10 +1863,14 @@ def _stream_splits(N: int, K: int) -> int:
 def linear(x: torch.Tensor, w: torch.Tensor, bias, out_dtype: torch.dtype, allow_partials: bool = False,
            scale: "RowScale | None" = None) -> torch.Tensor:
     """``x @ w.T (+ bias)``; ``w`` is ``[N, K]``.  float32 operands: this package's
-    float32 kernel.  bfloat16 operands, float32 accumulation, result in ``out_dtype``: up
-    to 64 rows the weight-streaming kernel (which, if ``allow_partials``, may return a
-    float32 stack of partial sums ``[parts, M, N]`` for the consumer to add); beyond that
-    the library product."""
+    float32 kernel.  bfloat16 operands, float32 accumulation, result in ``out_dtype``: up to 32
+    rows a weight-streaming kernel (`linear_ws`, `linear_stream`; `linear_tc` for medium and large
+    matrices, from some number of rows on up to 128), beyond 128 rows the CTA-pair product
+    (`gemm_pair`), fewer than 16 columns of up to 128 rows a kernel of their own
+    (`_narrow_takes`), and the library's product for what is left (33 to 128 rows of small matrices,
+    few columns of more than 128 rows, sizes or types that no kernel here takes).  With
+    ``allow_partials`` the result may be a float32 stack of partial sums ``[parts, M, N]`` for the
+    consumer to add.  ``w`` and ``bias`` are read before the wait for earlier kernels (see above)."""
     if x.dtype != w.dtype:
         raise KernelError(f"linear: x is {x.dtype}, w is {w.dtype}")
     if scale is not None:                       # a norm still owed on x (see `linear_scaled_supports`)
@@ -2037,7 +2049,8 @@ def linear_rope_kv_write(x, w, bias, positions, table, rotary_dim, nq, nkv, hd, 
     product's epilogue: bias, rotary encoding of the query and key heads by the tokens' positions,
     the new keys and values written to ``slot_mapping`` of the paged caches (not written when it is
     None).  Returns the rotated queries ``[T, nq*hd]`` bfloat16.  Few tokens only (`qkv_rope_supports`).
-    ``scale``: a norm still owed on ``x`` (`RowScale`)."""
+    ``scale``: a norm still owed on ``x`` (`RowScale`).  ``w`` and ``bias`` are read before the wait for earlier
+    kernels, ``positions`` and ``slot_mapping`` behind it."""
     _chk(x, w, bias, positions, table, slot_mapping, k_cache, v_cache)
     M, K = x.shape
     N = w.shape[0]

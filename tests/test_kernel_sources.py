@@ -51,3 +51,13 @@ def test_settings_of_a_kernel_are_made_on_every_device(name):
     assert not re.findall(r"\bstatic (?:bool|int|size_t) \w+ =[^=(]*;", code)
     if name not in ("common.cuh", "linear_ws.cu", "gemm_f32.cu"):           # (gemm_f32.cu sets it at every launch)
         assert "cudaFuncSetAttribute" not in code
+
+
+def test_the_rotary_epilogue_reads_positions_and_slots_behind_the_wait():
+    """A slot read before the kernels that came earlier have finished would send keys and values to another request's page, without an error, a position turn them by another's angle."""
+    code = code_of("linear_ws.cu")
+    code = code[code.index("linear_ws_kernel("):]
+    wait = code.index("pdl_wait();")
+    early, late = code[:wait], code[wait:]
+    assert "rope.slot_mapping" not in early and early.count("rope.positions") == 1 and "token_s[0][ahead_tok] = min(max(ws_position(rope.positions" in early
+    assert "ws_copy4(&token_s[1][ahead_tok], rope.positions" in late and "ws_copy4(&token_s[2][ahead_tok], rope.slot_mapping" in late and "if (pos != token_s[0][tok])" in late

@@ -269,3 +269,43 @@ def test_medium_matrices_of_17_to_32_tokens(M, N, K, monkeypatch):
         assert ops.silu_scaled_supports(x, w, 8, torch.bfloat16)
         assert bool(((ops.linear_silu_mul(x, w, 8, torch.bfloat16, scale=ops.RowScale(ssq, 56, 1e-5, K)) - want).abs() <= lim).all())
         assert ops.silu_scaled_pays(x, w, 8, torch.bfloat16) == (not (on_tensor_memory and (N, K) in ((6144, 2048), (18944, 1024))))
+
+
+def test_rotary_epilogue_behind_the_kernel_that_makes_positions_and_slots():
+    """Positions and slots that the kernel just before writes are the ones that count, call after call: the same queries, keys and values as from buffers that were there long before."""
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    g = torch.Generator(device=dev).manual_seed(5)
+    M, K, nq, nkv, hd, ps, pages = 8, 256, 4, 2, 64, 16, 40
+    x, w = torch.randn(M, K, device=dev, generator=g).bfloat16(), torch.randn((nq + 2 * nkv) * hd, K, device=dev, generator=g).bfloat16()
+    b, table = torch.randn((nq + 2 * nkv) * hd, device=dev, generator=g), torch.randn(4096, 2, hd // 2, device=dev, generator=g)
+    many = [(torch.randint(0, 4096, (M,), device=dev, generator=g, dtype=torch.int32), torch.randperm(pages * ps, device=dev, generator=g)[:M].int()) for _ in range(40)]
+
+    def caches():
+        return [torch.zeros(pages, nkv, ps, hd, device=dev, dtype=torch.bfloat16) for _ in range(2)]
+    call = lambda pos, slots, kv: ops.linear_rope_kv_write(x, w, b, pos, table, hd, nq, nkv, hd, slots, *kv)  # noqa: E731
+    kept, made = caches(), caches()
+    torch.cuda.synchronize()
+    want = [call(pos, slots, kept) for pos, slots in many]
+    pos, slots = torch.zeros(M, device=dev, dtype=torch.int32), torch.zeros(M, device=dev, dtype=torch.int32)
+    got = []
+    for p, s in many:
+        torch.add(p, 0, out=pos)
+        torch.add(s, 0, out=slots)
+        got.append(call(pos, slots, made))
+    assert all(torch.equal(a, c) for a, c in zip(got, want)) and all(torch.equal(a, c) for a, c in zip(made, kept))
+
+
+def test_rotary_epilogue_of_17_to_32_tokens_with_a_norm_owed():
+    """Only where the norm is owed, up to 1,024 columns and rows for two CTAs an SM; the product itself is tested with the kernels."""
+    import sllm_b200.ops as ops
+    dev = cuda_or_skip()
+    cache, table = torch.empty(4, 2, 16, 64, device=dev, dtype=torch.bfloat16), torch.empty(8, 2, 32, device=dev)
+
+    def takes(M, nq, nkv, K, owed):
+        x, w = torch.empty(M, K, device=dev, dtype=torch.bfloat16), torch.empty((nq + 2 * nkv) * 64, K, device=dev, dtype=torch.bfloat16)
+        return ops.qkv_rope_supports(x, w, table, 64, nq, nkv, 64, cache, owed=owed)
+    for M, nq, nkv, K, plain, owed in [(16, 14, 2, 896, True, True), (17, 14, 2, 896, False, True), (32, 14, 2, 1024, False, True), (17, 14, 2, 1056, False, False), (33, 14, 2, 896, False, False)]:
+        assert (takes(M, nq, nkv, K, False), takes(M, nq, nkv, K, True)) == (plain, owed), (M, nq, nkv, K)
+    if ops.num_sms() == 148:
+        assert takes(32, 14, 30, 1024, True) and not takes(32, 14, 31, 1024, True)
