@@ -44,6 +44,25 @@ def test_the_cut_of_a_context_fills_whole_waves(ops_with_sms):
         assert ops.choose_splits(120, 1, 512, 2) == 2 and ops.choose_splits(32, 1, 512, 2) == 4
 
 
+def test_the_cut_of_a_context_whose_ranges_a_cluster_merges(ops_with_sms, monkeypatch):
+    """Ranges may be single key tiles where the cluster that merges them fits the GPU, and are what they were where it does not."""
+    ops, sms = ops_with_sms
+    places = {64: 3 * sms, 128: 2 * sms}
+    monkeypatch.setattr(ops, "_tma_ctas_per_sm", lambda hd: places[hd] // sms)
+    monkeypatch.setattr(ops, "tma_clustered", lambda tiles, nkv, s, hd: 2 <= s <= 8 and tiles * nkv * s * 100 <= places[hd] * (100 if s == 2 else 85))
+    for requests in (1, 2, 4, 8, 16, 24, 48, 64, 128):
+        for nkv in (1, 2, 4, 8):
+            for ctx in (1, 64, 127, 128, 240, 256, 512, 1024, 4096, 12001, 32768):
+                for hd in (64, 128):
+                    s, old = ops.choose_tma_splits(requests, nkv, ctx, hd), ops.choose_splits(requests, nkv, ctx, ops._tma_ctas_per_sm(hd))
+                    assert s == old or ops.tma_clustered(requests, nkv, s, hd) or s == 1, (requests, nkv, ctx, hd)
+                    assert -(-ctx // (-(-(-(-ctx // s)) // 64) * 64)) == s, (requests, nkv, ctx, hd)          # no range without keys
+    if sms == 148:
+        for requests, nkv, ctx, hd, want in [(8, 4, 127, 128, 1), (8, 4, 256, 128, 4), (8, 1, 256, 128, 4), (4, 2, 256, 64, 4), (16, 2, 512, 128, 4), (8, 4, 540, 128, 5), (8, 4, 1024, 128, 6), (8, 4, 4096, 128, 8),
+                                             (32, 2, 1024, 64, 4), (148, 1, 512, 128, 2), (149, 1, 512, 128, 1), (1, 4, 12001, 128, 63), (1, 4, 32768, 128, 74), (64, 4, 4096, 128, 1)]:
+            assert ops.choose_tma_splits(requests, nkv, ctx, hd) == want, (requests, nkv, ctx, hd)
+
+
 def test_products_of_17_to_32_tokens(ops_with_sms, monkeypatch):
     """Up to one tile an SM, from 12 Mi elements and from a K on; with a norm owed on the input the rotary epilogue takes short reductions."""
     ops, sms = ops_with_sms

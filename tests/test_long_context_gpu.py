@@ -198,3 +198,16 @@ def test_ranges_merged_by_a_cluster(splits, lens, hd):
             f = gate[b, 3:].double().sigmoid()[:, None] if gt is not None else 1.0
             want, size = torch.einsum("hn,hnd->hd", w, v) * f, torch.einsum("hn,hnd->hd", w, v.abs()) * f
             assert bool(((got[b].reshape(nq, hd) - want).abs() <= 3 * 2.0 ** -8 * size + 1e-6).all()), (b, n)
+
+
+def test_which_ranges_a_cluster_merges():
+    """Two CTAs an SM with heads of 128, three with heads of 64; pairs of ranges up to every place, more up to 85 % of the places (148 SMs)."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import sllm_b200.ops as ops
+    if ops.num_sms() != 148:
+        pytest.skip("the sizes are those of 148 SMs")
+    for tiles, nkv, splits, hd, want in [(8, 4, 1, 128, False), (8, 4, 7, 128, True), (8, 4, 8, 128, False), (1, 1, 8, 128, True), (1, 1, 9, 128, False), (148, 1, 2, 128, True), (149, 1, 2, 128, False),
+                                         (62, 1, 4, 128, True), (63, 1, 4, 128, False), (31, 1, 8, 128, True), (16, 2, 8, 128, False), (222, 1, 2, 64, True), (223, 1, 2, 64, False), (47, 2, 4, 64, True),
+                                         (95, 1, 4, 64, False)]:
+        assert ops.tma_clustered(tiles, nkv, splits, hd) == want, (tiles, nkv, splits, hd)
